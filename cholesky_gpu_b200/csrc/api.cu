@@ -292,25 +292,20 @@ DecisionParams make_dp(const mpchol_opts& o) {
   return dp;
 }
 
-// The lower triangle of an n x n column-major matrix, block column by block
-// column (rows from the block's diagonal down): one 2-D copy per block
-// column, about half of the matrix's bytes.  The factorization and the
-// operator products read nothing above the diagonal.
-// Block columns [j0, j1) only: copy_lower_cols.
-cudaError_t copy_lower_cols(float* dst, int ldd, const float* src, int lds, int n, int b, int j0,
-                            int j1, cudaMemcpyKind kind, cudaStream_t s) {
+// Block columns [j0, j1) of the lower triangle of a host matrix (rows from
+// the block's diagonal down) to the device: one 2-D copy per block column,
+// about half of the matrix's bytes.  The factorization and the operator
+// products read nothing above the diagonal.
+cudaError_t upload_lower_cols(float* dst, int ldd, const float* src, int lds, int n, int b, int j0,
+                              int j1, cudaStream_t s) {
   for (int c = j0 * b; c < n && c < j1 * b; c += b) {
     const int w = std::min(b, n - c);
     cudaError_t e = cudaMemcpy2DAsync(dst + (size_t)c * ldd + c, sizeof(float) * ldd,
                                       src + (size_t)c * lds + c, sizeof(float) * lds,
-                                      sizeof(float) * (n - c), w, kind, s);
+                                      sizeof(float) * (n - c), w, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
-}
-cudaError_t copy_lower_blocks(float* dst, int ldd, const float* src, int lds, int n, int b,
-                              cudaMemcpyKind kind, cudaStream_t s) {
-  return copy_lower_cols(dst, ldd, src, lds, n, b, 0, ceil_div(n, b), kind, s);
 }
 
 bool valid_copy_plan(const CopyPlan& p, int nb);
@@ -713,10 +708,9 @@ mpchol_status enqueue_factor(mpchol_factor_t* f, cudaStream_t stream, const Copy
   MPCHOL_CUDA_TRY(cudaEventRecord(f->ev_start, stream));
   MPCHOL_CUDA_TRY(cudaStreamWaitEvent(f->cp, f->ev_start, 0));
   for (int g = 0; g < plan->ng; ++g) {
-    MPCHOL_CUDA_TRY(copy_lower_cols(f->op, f->ld, hA, lda, n, b, plan->c0[g], plan->c1[g],
-                                    cudaMemcpyHostToDevice, f->cp));
-    MPCHOL_CUDA_TRY(copy_lower_cols(f->A, f->ld, f->op, f->ld, n, b, plan->c0[g], plan->c1[g],
-                                    cudaMemcpyDeviceToDevice, f->cp));
+    MPCHOL_CUDA_TRY(upload_lower_cols(f->op, f->ld, hA, lda, n, b, plan->c0[g], plan->c1[g], f->cp));
+    PHASE(MPCHOL_PH_SETUP, 1, f->cp,
+          launch_copy_lower(f->op, f->ld, f->A, f->ld, n, b, plan->c0[g] * b, plan->c1[g] * b, f->cp));
     MPCHOL_CUDA_TRY(cudaEventRecord(f->ev_grp[g], f->cp));
   }
   // the switching statistics of step 0 read the whole diagonal
@@ -1299,7 +1293,7 @@ mpchol_status mpchol_factor_compute(mpchol_factor_t* f, const float* dA, int lda
                                     mpchol_stream_t stream) {
   if (f == nullptr || dA == nullptr || lda < f->n) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  MPCHOL_CUDA_TRY(copy_lower_blocks(f->A, f->ld, dA, lda, f->n, f->b, cudaMemcpyDeviceToDevice, s));
+  PHASE(MPCHOL_PH_SETUP, 1, s, launch_copy_lower(dA, lda, f->A, f->ld, f->n, f->b, 0, f->n, s));
   return launch_factor(f, s);
 }
 
@@ -1360,9 +1354,9 @@ mpchol_status mpchol_solve_host(mpchol_factor_t* f, const float* hA, int lda, co
   }
   const CopyPlan& plan = f->plan;
   if (plan.ng <= 1) {
-    MPCHOL_CUDA_TRY(copy_lower_blocks(f->op, f->ld, hA, lda, n, b, cudaMemcpyHostToDevice, s));
+    MPCHOL_CUDA_TRY(upload_lower_cols(f->op, f->ld, hA, lda, n, b, 0, f->nsteps, s));
     MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->hb, hB, sizeof(double) * n * nrhs, cudaMemcpyHostToDevice, s));
-    MPCHOL_CUDA_TRY(copy_lower_blocks(f->A, f->ld, f->op, f->ld, n, b, cudaMemcpyDeviceToDevice, s));
+    PHASE(MPCHOL_PH_SETUP, 1, s, launch_copy_lower(f->op, f->ld, f->A, f->ld, n, b, 0, n, s));
     mpchol_status st = launch_factor(f, s);
     if (st != MPCHOL_OK) return st;
   } else {
@@ -1668,7 +1662,7 @@ int mpchol_precond_cg(double* dA, double* dX, double* dB, int n, int r, double n
   mpchol_status st = mpchol_factor_create(&o, n, &f);
   if (st != MPCHOL_OK) return -(100 + st);
   // FP64 -> FP32 directly into the factor's storage (src/mixed_cholesky.cu:122)
-  if (launch_f64_to_f32(dA, n, f->A, f->ld, n, s) != cudaSuccess) {
+  if (launch_copy_lower(dA, n, f->A, f->ld, n, f->b, 0, n, s) != cudaSuccess) {
     free_factor(f);
     return -(100 + MPCHOL_ERR_CUDA);
   }

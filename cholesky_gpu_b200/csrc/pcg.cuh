@@ -57,8 +57,12 @@ cudaError_t launch_pcg_loop_cond(cudaGraphConditionalHandle handle, int* ctl, co
 // misc device utilities (util.cu)
 cudaError_t launch_extract_diag(const float* A, int lda, int n, float* d, float* dtilde,
                                 cudaStream_t stream);
-cudaError_t launch_f64_to_f32(const double* src, int lds, float* dst, int ldd, int n,
-                              cudaStream_t stream);
+// Columns [c0, c1) of the lower block columns (rows from the column's block
+// diagonal down, block b) of src (FP32, or FP64 rounded to FP32) into dst, in
+// one launch.
+template <typename TS>
+cudaError_t launch_copy_lower(const TS* src, int lds, float* dst, int ldd, int n, int b, int c0,
+                              int c1, cudaStream_t stream);
 // Equilibration: ex[i] = exponent of row i from A's diagonal; then the lower
 // triangle of columns [c0, c1) is scaled to D A D
 // (unscale_rows = false) or the factor's rows scaled back by 2^ex[i] (true).

@@ -1,0 +1,27 @@
+"""Edges of the device paths that a size, an alignment or a format selects."""
+import numpy as np
+import pytest
+import torch
+
+import cholesky_gpu_b200 as mp
+from cholesky_gpu_b200 import matgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,pad,offset", [
+    (37, 0, 0), (130, 2, 0), (257, 3, 1), (256, 4, 4), (515, 5, 2), (1000, 0, 0), (999, 1, 3),
+])
+def test_operator_copy_is_exact_for_every_alignment(n, pad, offset):
+    """The copy of A's lower block columns (16-byte path, or scalar for columns
+    that start elsewhere) gives the same factor bit for bit wherever A lies."""
+    A = matgen.spd_matrix(n, 1e2, n).cuda()
+    ref = mp.factor(A, block_size=128, precision="fp32").lower()
+    lda = n + pad
+    store = torch.full((n * lda + offset,), float("nan"), device="cuda")
+    view = store[offset:].as_strided((n, n), (1, lda))      # column-major, leading dimension lda
+    view.copy_(A)
+    got = mp.factor(view, block_size=128, precision="fp32").lower()
+    assert torch.equal(got, ref)
+    L = np.linalg.cholesky(A.double().cpu().numpy())
+    assert np.linalg.norm(got.cpu().numpy() - L) / np.linalg.norm(L) < 1e-5
