@@ -121,6 +121,7 @@ SIGNATURES = {
     "mpchol_factor_compute": (_i, [_vp, _vp, _i, _vp]),
     "mpchol_factor": (_i, [ctypes.POINTER(Opts), _i, _vp, _i, ctypes.POINTER(_vp), _vp]),
     "mpchol_factor_destroy": (_i, [_vp]),
+    "mpchol_release_cached": (None, []),
     "mpchol_factor_info_get": (_i, [_vp, ctypes.POINTER(FactorInfo), _vp, _vp, _vp]),
     "mpchol_factor_lower": (_i, [_vp, ctypes.POINTER(_vp), ctypes.POINTER(_i), ctypes.POINTER(_i)]),
     "mpchol_factor_diags": (_i, [_vp, ctypes.POINTER(_vp), ctypes.POINTER(_vp)]),

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -131,13 +132,146 @@ struct FactorGraph {
 // iteration) and what it was captured for; nk: kernels per iteration.
 struct PcgGraph {
   cudaGraphExec_t exec = nullptr;
+  int calls = 0;              // calls in a row with the key below
   bool failed = false;        // the runtime refused the graph: iterations are launched directly
   const void* A = nullptr;
   int lda = 0, nr = 0, elem = 0;
   double tol2 = 0.0;
   long long nk[MPCHOL_NPHASES] = {};
 };
+
+// What a factor object needs from the driver: its device memory (one
+// allocation), pinned read-back buffers, streams and events.  On a B200 a
+// cudaMalloc above 2 MB costs 0.35 ms, a cudaFree 0.31 ms and a stream 0.06 to
+// 0.5 ms, ten times that on a busy host, and the drop-in entry points make
+// and free a factor object on every call.  So the resources of a freed object
+// are kept for the next one of about its size: at most kCacheCount sets of
+// kCacheBytes in all, idle ones only (the device is synchronized when a set
+// is put away, as a cudaFree would), given back by mpchol_release_cached, when
+// an allocation of the library fails, or when newer ones take their room.
+// Create + destroy at n = 3072: 3.6 ms with one allocation per buffer, 0.70
+// with one for all.
+struct Resources {
+  int device = -1;
+  char* arena = nullptr;
+  size_t bytes = 0;
+  int* h_done = nullptr;      // pinned
+  double* h_scal = nullptr;   // pinned
+  // look-ahead: the bulk of each step's trailing update runs on aux while the
+  // next diagonal block is factored on the caller's stream; capture_stream is
+  // used only to capture graphs
+  cudaStream_t aux = nullptr, capture_stream = nullptr;
+  cudaEvent_t ev_next = nullptr;    // the next block's columns are updated
+  cudaEvent_t ev_rest = nullptr;    // the rest of the step's update is done
+  cudaEvent_t ev_catch = nullptr;   // a step's catch-ups are done
+};
+constexpr size_t kCacheBytes = (size_t)512 << 20;
+constexpr size_t kCacheCount = 4;
+std::mutex g_cache_mu;
+std::vector<Resources> g_cache;   // oldest first
+
+void free_resources(Resources& r) {
+  if (r.arena) cudaFree(r.arena);
+  if (r.h_done) cudaFreeHost(r.h_done);
+  if (r.h_scal) cudaFreeHost(r.h_scal);
+  if (r.aux) cudaStreamDestroy(r.aux);
+  if (r.capture_stream) cudaStreamDestroy(r.capture_stream);
+  for (cudaEvent_t e : {r.ev_next, r.ev_rest, r.ev_catch})
+    if (e) cudaEventDestroy(e);
+  r = Resources{};
+}
+
+void release_cached() {
+  std::vector<Resources> all;
+  {
+    std::lock_guard<std::mutex> lk(g_cache_mu);
+    all.swap(g_cache);
+  }
+  for (Resources& r : all) free_resources(r);
+}
+
+// A set with at least `bytes` of device memory on the current device: the
+// smallest cached one that is not more than twice that, or a new one.
+bool acquire_resources(int device, size_t bytes, Resources* out) {
+  // binds the device's context to this thread, which an allocation would do
+  // and the tensor-map encoder needs
+  if (cudaSetDevice(device) != cudaSuccess) return false;
+  {
+    std::lock_guard<std::mutex> lk(g_cache_mu);
+    size_t best = g_cache.size();
+    for (size_t i = 0; i < g_cache.size(); ++i)
+      if (g_cache[i].device == device && g_cache[i].bytes >= bytes && g_cache[i].bytes / 2 <= bytes &&
+          (best == g_cache.size() || g_cache[i].bytes < g_cache[best].bytes))
+        best = i;
+    if (best < g_cache.size()) {
+      *out = g_cache[best];
+      g_cache.erase(g_cache.begin() + best);
+      return true;
+    }
+  }
+  Resources r;
+  r.device = device;
+  r.bytes = bytes;
+  bool ok = lib_malloc(reinterpret_cast<void**>(&r.arena), bytes) == cudaSuccess;
+  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&r.h_done), 2 * sizeof(int)) == cudaSuccess &&
+       cudaMallocHost(reinterpret_cast<void**>(&r.h_scal), sizeof(double) * 64) == cudaSuccess &&
+       cudaStreamCreateWithFlags(&r.aux, cudaStreamNonBlocking) == cudaSuccess &&
+       cudaStreamCreateWithFlags(&r.capture_stream, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t* e : {&r.ev_next, &r.ev_rest, &r.ev_catch})
+    ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    free_resources(r);
+    return false;
+  }
+  *out = r;
+  return true;
+}
+
+// Puts a set away (or frees it when it is larger than the cache may hold).
+void put_away_resources(Resources& r) {
+  if (r.arena == nullptr || r.bytes > kCacheBytes) {
+    free_resources(r);
+    return;
+  }
+  int cur = 0;
+  const bool there = cudaGetDevice(&cur) == cudaSuccess;
+  if (there && cur != r.device) cudaSetDevice(r.device);
+  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+  if (there && cur != r.device) cudaSetDevice(cur);
+  if (!idle) {
+    free_resources(r);
+    return;
+  }
+  std::vector<Resources> out;
+  {
+    std::lock_guard<std::mutex> lk(g_cache_mu);
+    g_cache.push_back(r);
+    size_t total = 0;
+    for (const Resources& c : g_cache) total += c.bytes;
+    while (g_cache.size() > kCacheCount || total > kCacheBytes) {
+      total -= g_cache.front().bytes;
+      out.push_back(g_cache.front());
+      g_cache.erase(g_cache.begin());
+    }
+  }
+  for (Resources& o : out) free_resources(o);
+  r = Resources{};
+}
+
 }  // namespace
+
+// A device allocation that gives the cached resources back before it fails.
+cudaError_t mpchol::lib_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  *p = nullptr;
+  release_cached();
+  e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
 
 // Run `expr` (which launches `nk` library kernels) as phase `ph`.
 #define PHASE(ph, nk, stream, expr)                 \
@@ -150,6 +284,7 @@ struct mpchol_factor {
   mpchol_opts opts;
   int n = 0, ld = 0, b = 0, nsteps = 0;
   int device = 0;
+  Resources res;              // device memory that holds the buffers down to loop_ctl, streams, ...
   float* A = nullptr;         // n columns x ld rows, factor in the lower triangle
   float* d = nullptr;         // original diagonal
   float* dtilde = nullptr;    // Schur-complement diagonal tracker
@@ -179,28 +314,19 @@ struct mpchol_factor {
   double* partials = nullptr; // 4 * VG * 8
   double* scal = nullptr;     // rho[2][8], alpha[8], bnorm2[8], misc
   int* done = nullptr;        // [0] converged flag, [1] iteration counter
-  int* h_done = nullptr;      // pinned
-  double* h_scal = nullptr;   // pinned
   PcgGraph graph;             // captured PCG loop (see run_pcg)
   FactorGraph fgraph;         // captured factorization (see launch_factor)
   int* loop_ctl = nullptr;    // its iteration count and budget
-  cudaStream_t capture_stream = nullptr;   // private stream used only to capture graphs
-  // look-ahead: the bulk of each step's trailing update runs on aux while
-  // the next diagonal block is factored on the caller's stream
   // host-buffer solves: the operator's lower triangle and the rhs / solution
   float* op = nullptr;        // n columns x ld, lower triangle
   double* hb = nullptr;       // n x 8
   double* hx = nullptr;       // n x 8
-  cudaStream_t aux = nullptr;
-  cudaEvent_t ev_next = nullptr;   // the next block's columns are updated
-  cudaEvent_t ev_rest = nullptr;   // the rest of the step's update is done
   // host-buffer solves with the copy of A overlapped (see CopyPlan): the
   // copy stream, one event per arrived group, the pinned diagonal of A, and
   // the quantized panels of the steps that late groups catch up with
   cudaStream_t cp = nullptr;
   cudaEvent_t ev_grp[kMaxGroups] = {};
   cudaEvent_t ev_start = nullptr;  // prior work on the caller's stream is done
-  cudaEvent_t ev_catch = nullptr;  // a step's catch-ups are done
   cudaEvent_t ev_diag = nullptr;   // the pinned diagonal has been copied
   float* h_diag = nullptr;
   uint8_t* hq8 = nullptr;
@@ -250,32 +376,23 @@ mpchol_status validate_opts(const mpchol_opts* o, int n) {
 
 template <typename T>
 cudaError_t dmalloc(T** p, size_t count) {
-  return cudaMalloc(reinterpret_cast<void**>(p), count * sizeof(T) + 256);
+  return lib_malloc(reinterpret_cast<void**>(p), count * sizeof(T) + 256);
 }
 
 void free_factor(mpchol_factor_t* f) {
   if (f == nullptr) return;
-  void* ptrs[] = {f->A, f->d, f->dtilde, f->rowsq, f->sh, f->winv, f->scratch64, f->q8,
-                  f->q16, f->rexp, f->mxexp, f->steps, f->status, f->pstatus, f->colacc,
-                  f->eqexp, f->wsup, f->trsv_ctr,
-                  f->vec, f->partials, f->scal, f->done, f->loop_ctl, f->op, f->hb, f->hx,
-                  f->hq8, f->hq16, f->hrexp, f->hmx};
+  void* ptrs[] = {f->op, f->hb, f->hx, f->hq8, f->hq16, f->hrexp, f->hmx};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (f->graph.exec) cudaGraphExecDestroy(f->graph.exec);
   if (f->fgraph.exec) cudaGraphExecDestroy(f->fgraph.exec);
-  if (f->capture_stream) cudaStreamDestroy(f->capture_stream);
-  if (f->aux) cudaStreamDestroy(f->aux);
-  if (f->ev_next) cudaEventDestroy(f->ev_next);
-  if (f->ev_rest) cudaEventDestroy(f->ev_rest);
   if (f->cp) cudaStreamDestroy(f->cp);
   for (cudaEvent_t e : f->ev_grp)
     if (e) cudaEventDestroy(e);
-  for (cudaEvent_t e : {f->ev_start, f->ev_catch, f->ev_diag})
+  for (cudaEvent_t e : {f->ev_start, f->ev_diag})
     if (e) cudaEventDestroy(e);
   if (f->h_diag) cudaFreeHost(f->h_diag);
-  if (f->h_done) cudaFreeHost(f->h_done);
-  if (f->h_scal) cudaFreeHost(f->h_scal);
+  put_away_resources(f->res);
   delete f;
 }
 
@@ -454,18 +571,6 @@ bool valid_copy_plan(const CopyPlan& p, int nb) {
   return true;
 }
 
-// The second stream of the look-ahead and its events (created once, outside
-// any stream capture).
-mpchol_status ensure_factor_streams(mpchol_factor_t* f) {
-  if (f->aux != nullptr) return MPCHOL_OK;
-  MPCHOL_CUDA_TRY(cudaStreamCreateWithFlags(&f->aux, cudaStreamNonBlocking));
-  MPCHOL_CUDA_TRY(cudaEventCreateWithFlags(&f->ev_next, cudaEventDisableTiming));
-  MPCHOL_CUDA_TRY(cudaEventCreateWithFlags(&f->ev_rest, cudaEventDisableTiming));
-  MPCHOL_CUDA_TRY(cudaEventCreateWithFlags(&f->ev_catch, cudaEventDisableTiming));
-  MPCHOL_CUDA_TRY(cudaDeviceGetAttribute(&f->nsm, cudaDevAttrMultiProcessorCount, f->device));
-  return MPCHOL_OK;
-}
-
 // One factorization of f->A in place, on `stream`, right-looking with a
 // look-ahead of one block.  Step k: the panel solve (with the step decision
 // and the panel quantization), then the trailing update of the tiles of
@@ -490,8 +595,6 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
   const int n = f->n, ld = f->ld, b = f->b;
   PotrfParams pp{o.diag_pert, o.pert, o.pivot_floor};
   const DecisionParams dp = make_dp(o);
-  mpchol_status es = ensure_factor_streams(f);
-  if (es != MPCHOL_OK) return es;
   const bool streamed = plan != nullptr && plan->ng > 1;
   const int cap = f->nsm > 1 ? f->nsm - 1 : 1;   // SMs for the concurrent part of the update
   MPCHOL_CUDA_TRY(cudaMemsetAsync(f->status, 0, sizeof(DevStatus), stream));
@@ -632,7 +735,7 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
     const int m = n - s - bs;
     if (m <= 0) break;
     if (rest_pending) {
-      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->ev_rest, 0));
+      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->res.ev_rest, 0));
       rest_pending = false;
     }
     const int next_bs = std::min(b, m);
@@ -648,10 +751,10 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
     bool caught = false, head_waits = false;
     while (streamed && joined < plan->ng && plan->join[joined] == k) {
       const int g = joined;
-      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(f->aux, f->ev_grp[g], 0));
+      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(f->res.aux, f->ev_grp[g], 0));
       for (int p = 0; p < k; ++p) {
         TileSel band{SEL_BAND, 0, tcol(p, plan->c0[g]), tcol(p, plan->c1[g]), 0};
-        if ((rs = syrk(p, band, cap, f->aux)) != MPCHOL_OK) return rs;
+        if ((rs = syrk(p, band, cap, f->res.aux)) != MPCHOL_OK) return rs;
       }
       caught = true;
       head_waits = head_waits || k + 1 >= plan->c0[g];
@@ -659,8 +762,8 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
       ++joined;
     }
     if (caught) {
-      MPCHOL_CUDA_TRY(cudaEventRecord(f->ev_catch, f->aux));
-      if (head_waits) MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->ev_catch, 0));
+      MPCHOL_CUDA_TRY(cudaEventRecord(f->res.ev_catch, f->res.aux));
+      if (head_waits) MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->res.ev_catch, 0));
     }
     const int jc = ceil_div(next_bs, 128);   // 128-tile columns of block k+1
     if ((rs = syrk(k, TileSel{SEL_NEXT, jc}, 0, stream)) != MPCHOL_OK) return rs;
@@ -669,17 +772,17 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
     const int jend = tcol(k, joined_end);
     const TileSel rest = jend >= T ? TileSel{SEL_REST, jc} : TileSel{SEL_BAND, jc, 0, jend, jc};
     if (sel_tile_count(T, rest) > 0) {
-      MPCHOL_CUDA_TRY(cudaEventRecord(f->ev_next, stream));
-      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(f->aux, f->ev_next, 0));
-      if ((rs = syrk(k, rest, cap, f->aux)) != MPCHOL_OK) return rs;
-      MPCHOL_CUDA_TRY(cudaEventRecord(f->ev_rest, f->aux));
+      MPCHOL_CUDA_TRY(cudaEventRecord(f->res.ev_next, stream));
+      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(f->res.aux, f->res.ev_next, 0));
+      if ((rs = syrk(k, rest, cap, f->res.aux)) != MPCHOL_OK) return rs;
+      MPCHOL_CUDA_TRY(cudaEventRecord(f->res.ev_rest, f->res.aux));
       rest_pending = true;
     } else if (caught) {
-      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->ev_catch, 0));
+      MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->res.ev_catch, 0));
     }
     if ((rs = potrf(k + 1, rest_pending)) != MPCHOL_OK) return rs;
   }
-  if (rest_pending) MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->ev_rest, 0));
+  if (rest_pending) MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->res.ev_rest, 0));
   if (streamed) MPCHOL_CUDA_TRY(cudaStreamWaitEvent(stream, f->ev_grp[plan->ng - 1], 0));
   // equilibrated: L of A is D^-1 times the factor of D A D (rows times 2^e_i)
   if (o.equilibrate && !streamed)
@@ -750,17 +853,13 @@ mpchol_status launch_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyP
     return enqueue_factor(f, stream, plan, hA, lda, hA_dev);
   }
   if (g.exec == nullptr) {
-    mpchol_status es = ensure_factor_streams(f);
-    if (es != MPCHOL_OK) return es;
-    if (f->capture_stream == nullptr)
-      MPCHOL_CUDA_TRY(cudaStreamCreateWithFlags(&f->capture_stream, cudaStreamNonBlocking));
     long long before[MPCHOL_NPHASES];
     launch_counts(before);
-    bool ok = cudaStreamBeginCapture(f->capture_stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    bool ok = cudaStreamBeginCapture(f->res.capture_stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
-      const mpchol_status st = enqueue_factor(f, f->capture_stream, plan, hA, lda, hA_dev);
+      const mpchol_status st = enqueue_factor(f, f->res.capture_stream, plan, hA, lda, hA_dev);
       cudaGraph_t graph = nullptr;
-      const cudaError_t ce = cudaStreamEndCapture(f->capture_stream, &graph);
+      const cudaError_t ce = cudaStreamEndCapture(f->res.capture_stream, &graph);
       ok = st == MPCHOL_OK && ce == cudaSuccess && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
       if (graph) cudaGraphDestroy(graph);
     }
@@ -867,8 +966,7 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
   }
   const double tol2 = po.rel_tol * po.rel_tol;
   int it = 0;         // iterations executed on the device
-  int launched = 0;   // iterations counted against max_it (the direct path also counts
-                      // iterations enqueued past convergence, which return at once)
+  int launched = 0;   // iterations counted against max_it
   bool converged = false;
   const int max_restarts = 3;
   for (int restart = 0;; ++restart) {
@@ -878,17 +976,17 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_residual(bb, Ap, r, n, nr, part_rr, stream));
     PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_rr, misc, nr, stream));
     // convergence of the true residual
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_scal, misc, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_scal + 8, bnorm2, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal, misc, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal + 8, bnorm2, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
     // the factorization's status rides along with the first check: a failed
     // factor (NOT_SPD, TIMEOUT) is not iterated with
     if (restart == 0)
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_scal + 48, f->status, sizeof(DevStatus),
+      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal + 48, f->status, sizeof(DevStatus),
                                       cudaMemcpyDeviceToHost, stream));
     MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
     if (restart == 0) {
       DevStatus fst;
-      memcpy(&fst, f->h_scal + 48, sizeof(DevStatus));
+      memcpy(&fst, f->res.h_scal + 48, sizeof(DevStatus));
       if (fst.code != 0) {
         if (rep != nullptr) memset(rep, 0, sizeof(*rep));
         return (mpchol_status)fst.code;
@@ -896,7 +994,7 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     }
     converged = true;
     for (int k = 0; k < nrhs; ++k)
-      if (!(f->h_scal[k] <= tol2 * f->h_scal[8 + k])) converged = false;
+      if (!(f->res.h_scal[k] <= tol2 * f->res.h_scal[8 + k])) converged = false;
     if (converged || launched >= po.max_it || restart > max_restarts) break;
     mpchol_status s1 = apply_precond(f, r, tmp, z, nr, nullptr, stream);
     if (s1 != MPCHOL_OK) return s1;
@@ -921,19 +1019,26 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     // The iterations run in a device-side loop: one launch of a CUDA graph
     // whose WHILE node repeats one iteration until the recursive residual
     // meets the tolerance, an error is recorded or the budget is spent, with
-    // no host round trip in between.  Captured once per operator / rhs
-    // count / tolerance.
+    // no host round trip in between.  Captured per operator / rhs count /
+    // tolerance, on the third call in a row with the same ones: capture and
+    // instantiation cost about 300 us, which an object that solves once or
+    // twice (the drop-in driver, a gradient step) does not earn back.
     PcgGraph& g = f->graph;
-    bool use_graph = !profiling_on() && !g.failed;
-    if (use_graph && (g.exec == nullptr || g.A != (const void*)dA || g.lda != lda || g.nr != nr ||
-                      g.elem != (int)sizeof(TA) || g.tol2 != tol2)) {
-      if (g.exec) cudaGraphExecDestroy(g.exec);
-      g.exec = nullptr;
+    if (restart == 0) {
+      if (g.A != (const void*)dA || g.lda != lda || g.nr != nr || g.elem != (int)sizeof(TA) ||
+          g.tol2 != tol2) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+        g.calls = 0;
+        g.A = dA; g.lda = lda; g.nr = nr; g.elem = (int)sizeof(TA); g.tol2 = tol2;
+      }
+      if (g.calls < 3) ++g.calls;
+    }
+    bool use_graph = !profiling_on() && !g.failed && g.calls >= 3;
+    if (use_graph && g.exec == nullptr) {
       // capture on a private stream (the caller's may be the legacy default
       // stream, which cannot be captured); the graph is launched into the
       // caller's stream
-      if (f->capture_stream == nullptr)
-        MPCHOL_CUDA_TRY(cudaStreamCreateWithFlags(&f->capture_stream, cudaStreamNonBlocking));
       long long before[MPCHOL_NPHASES];
       launch_counts(before);
       cudaGraph_t graph = nullptr;
@@ -952,15 +1057,15 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
       }
       if (ok) {
         cudaGraph_t body = cp.conditional.phGraph_out[0];
-        ok = cudaStreamBeginCaptureToGraph(f->capture_stream, body, nullptr, nullptr, 0,
+        ok = cudaStreamBeginCaptureToGraph(f->res.capture_stream, body, nullptr, nullptr, 0,
                                            cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         if (ok) {
-          const mpchol_status s0 = iteration(0, f->capture_stream);
+          const mpchol_status s0 = iteration(0, f->res.capture_stream);
           const bool cond_ok =
               s0 == MPCHOL_OK && launch_pcg_loop_cond(handle, f->loop_ctl, f->done, f->pstatus,
-                                                      f->scal, nr, f->capture_stream) == cudaSuccess;
+                                                      f->scal, nr, f->res.capture_stream) == cudaSuccess;
           cudaGraph_t captured = nullptr;
-          const cudaError_t ce = cudaStreamEndCapture(f->capture_stream, &captured);
+          const cudaError_t ce = cudaStreamEndCapture(f->res.capture_stream, &captured);
           ok = cond_ok && ce == cudaSuccess && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
         }
       }
@@ -976,20 +1081,18 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
         g.exec = nullptr;
         g.failed = true;
         use_graph = false;
-      } else {
-        g.A = dA; g.lda = lda; g.nr = nr; g.elem = (int)sizeof(TA); g.tol2 = tol2;
       }
     }
     if (use_graph) {
       PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_pcg_loop_init(f->loop_ctl, po.max_it - launched, stream));
       MPCHOL_CUDA_TRY(cudaGraphLaunch(g.exec, stream));
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_done, f->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_done, f->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
       DevStatus st;
       MPCHOL_CUDA_TRY(cudaMemcpyAsync(&st, f->pstatus, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
       MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
       if (st.code == MPCHOL_ERR_TIMEOUT) return MPCHOL_ERR_TIMEOUT;
-      add_launch_counts(g.nk, f->h_done[1] - it);
-      it = f->h_done[1];                // iterations actually executed on the device
+      add_launch_counts(g.nk, f->res.h_done[1] - it);
+      it = f->res.h_done[1];                // iterations actually executed on the device
       launched = it;
       continue;                         // the true residual decides (residual replacement restart)
     }
@@ -1003,14 +1106,15 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
         cur ^= 1;
       }
       launched += chunk;
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_done, f->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_done, f->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
       DevStatus st;
       MPCHOL_CUDA_TRY(cudaMemcpyAsync(&st, f->pstatus, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
       MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
       if (st.code == MPCHOL_ERR_TIMEOUT) return MPCHOL_ERR_TIMEOUT;
-      it = f->h_done[1];                // iterations actually executed on the device
-      if (f->h_done[0]) stop = true;    // recursive residual met the tolerance
+      it = f->res.h_done[1];                // iterations actually executed on the device
+      if (f->res.h_done[0]) stop = true;    // recursive residual met the tolerance
       if (st.code == MPCHOL_PCG_BREAKDOWN) stop = true;
+      if (f->res.h_done[0]) launched = it;  // those enqueued past it returned at once
     }
     // the loop exits on max_it or when the recursive residual says done; the
     // next pass re-checks the true residual (residual replacement restart)
@@ -1031,16 +1135,16 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     }
     PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_dot(r, z, n, nr, part_rz, nullptr, stream));
     PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_rz, misc + 24, nr, stream));
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_scal, misc, sizeof(double) * 32, cudaMemcpyDeviceToHost, stream));
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->h_scal + 32, bnorm2, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal, misc, sizeof(double) * 32, cudaMemcpyDeviceToHost, stream));
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal + 32, bnorm2, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
     MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
     double relmax = 0.0, bemax = 0.0, prmax = 0.0;
-    const double frob = sqrt(f->h_scal[16]);
+    const double frob = sqrt(f->res.h_scal[16]);
     for (int k = 0; k < nrhs; ++k) {
-      const double rr = f->h_scal[k], xx = f->h_scal[8 + k], bb2 = f->h_scal[32 + k];
+      const double rr = f->res.h_scal[k], xx = f->res.h_scal[8 + k], bb2 = f->res.h_scal[32 + k];
       const double rel = bb2 > 0 ? sqrt(rr / bb2) : sqrt(rr);
       const double be = sqrt(rr) / (frob * sqrt(xx) + sqrt(bb2));
-      const double pr = bb2 > 0 ? sqrt(fabs(f->h_scal[24 + k]) / bb2) : 0.0;
+      const double pr = bb2 > 0 ? sqrt(fabs(f->res.h_scal[24 + k]) / bb2) : 0.0;
       relmax = std::max(relmax, rel);
       bemax = std::max(bemax, be);
       prmax = std::max(prmax, pr);
@@ -1230,37 +1334,49 @@ mpchol_status mpchol_factor_create(const mpchol_opts* opts, int n, mpchol_factor
   f->b = opts->block_size;
   f->nsteps = (n + f->b - 1) / f->b;
   cudaGetDevice(&f->device);
-  const size_t nv = (size_t)n * 8;
-  bool ok = dmalloc(&f->A, (size_t)f->ld * n) == cudaSuccess &&
-            dmalloc(&f->d, n) == cudaSuccess && dmalloc(&f->dtilde, n) == cudaSuccess &&
-            dmalloc(&f->rowsq, n) == cudaSuccess && dmalloc(&f->sh, n) == cudaSuccess &&
-            dmalloc(&f->winv, (size_t)8 * 32 * 32) == cudaSuccess &&
-            dmalloc(&f->scratch64, potrf_scratch64_elems(256)) == cudaSuccess &&
-            dmalloc(&f->q8, (size_t)3 * n * f->b) == cudaSuccess &&
-            dmalloc(&f->q16, (size_t)2 * n * f->b) == cudaSuccess &&
-            dmalloc(&f->rexp, (size_t)3 * n) == cudaSuccess &&
-            dmalloc(&f->mxexp, (size_t)n * (f->b / 32)) == cudaSuccess &&
-            dmalloc(&f->steps, f->nsteps + 1) == cudaSuccess &&
-            dmalloc(&f->status, 1) == cudaSuccess && dmalloc(&f->pstatus, 1) == cudaSuccess &&
-            dmalloc(&f->colacc, (size_t)f->nsteps * kColCopies * f->b) == cudaSuccess &&
-            dmalloc(&f->eqexp, n) == cudaSuccess &&
-            dmalloc(&f->wsup, solve_wsup_elems(n)) == cudaSuccess &&
-            dmalloc(&f->trsv_ctr, trsv_counter_ints(n)) == cudaSuccess &&
-            dmalloc(&f->vec, 8 * nv) == cudaSuccess &&
-            dmalloc(&f->partials, (size_t)5 * pcg_vgrid() * 8) == cudaSuccess &&
-            dmalloc(&f->scal, 64) == cudaSuccess && dmalloc(&f->done, 2) == cudaSuccess &&
-            dmalloc(&f->loop_ctl, 2) == cudaSuccess &&
-            cudaMallocHost(reinterpret_cast<void**>(&f->h_done), 2 * sizeof(int)) == cudaSuccess &&
-            cudaMallocHost(reinterpret_cast<void**>(&f->h_scal), sizeof(double) * 64) == cudaSuccess;
-  if (!ok) {
-    cudaGetLastError();
+  const size_t nv = (size_t)n * 8, nbq = (size_t)n * f->b;
+  // one device allocation holds every buffer (see Resources)
+  auto carve = [&](char* base) -> size_t {
+    size_t off = 0;
+    auto take = [&](auto*& p, size_t count) {
+      using T = std::remove_reference_t<decltype(*p)>;
+      p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+      off += (count * sizeof(T) + 256 + 255) / 256 * 256;   // 256 bytes of slack each
+    };
+    take(f->A, (size_t)f->ld * n);
+    take(f->d, n);
+    take(f->dtilde, n);
+    take(f->rowsq, n);
+    take(f->sh, n);
+    take(f->winv, (size_t)8 * 32 * 32);
+    take(f->scratch64, potrf_scratch64_elems(256));
+    take(f->q8, 3 * nbq);
+    take(f->q16, 2 * nbq);
+    take(f->rexp, (size_t)3 * n);
+    take(f->mxexp, (size_t)n * (f->b / 32));
+    take(f->steps, f->nsteps + 1);
+    take(f->status, 1);
+    take(f->pstatus, 1);
+    take(f->colacc, (size_t)f->nsteps * kColCopies * f->b);
+    take(f->eqexp, n);
+    take(f->wsup, solve_wsup_elems(n));
+    take(f->trsv_ctr, trsv_counter_ints(n));
+    take(f->vec, 8 * nv);
+    take(f->partials, (size_t)5 * pcg_vgrid() * 8);
+    take(f->scal, 64);
+    take(f->done, 2);
+    take(f->loop_ctl, 2);
+    return off;
+  };
+  if (!acquire_resources(f->device, carve(nullptr), &f->res)) {
     free_factor(f);
     return MPCHOL_ERR_ALLOC;
   }
+  carve(f->res.arena);
+  cudaDeviceGetAttribute(&f->nsm, cudaDevAttrMultiProcessorCount, f->device);
   if (opts->left) {
     // the quantized panels of every step (the left-looking schedule applies
     // each panel to the later block columns one at a time)
-    const size_t nbq = (size_t)n * f->b;
     const int hist = f->nsteps;
     if (dmalloc(&f->hq8, (size_t)hist * 3 * nbq) != cudaSuccess ||
         dmalloc(&f->hq16, (size_t)hist * 2 * nbq) != cudaSuccess ||
@@ -1456,6 +1572,8 @@ mpchol_status mpchol_factor(const mpchol_opts* opts, int n, const float* dA, int
   }
   return s;
 }
+
+void mpchol_release_cached(void) { release_cached(); }
 
 mpchol_status mpchol_factor_destroy(mpchol_factor_t* f) {
   if (f == nullptr) return MPCHOL_ERR_BAD_ARG;

@@ -52,7 +52,7 @@ __global__ void batch_load_kernel(const BatchSys* __restrict__ sys, const float*
 
 template <typename T>
 cudaError_t dalloc(T** p, size_t count) {
-  return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
+  return lib_malloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
 }
 
 }  // namespace

@@ -190,4 +190,7 @@ __host__ __device__ inline int ceil_div(long long a, long long b) { return (int)
 
 namespace mpchol {
 void record_cuda_error(cudaError_t e, const char* what, const char* file, int line);
+// cudaMalloc that gives the library's cached resources back and tries again
+// before it reports that memory ran out.
+cudaError_t lib_malloc(void** p, size_t bytes);
 }

@@ -192,6 +192,11 @@ MPCHOL_API mpchol_status mpchol_factor_compute(mpchol_factor_t* f, const float* 
 MPCHOL_API mpchol_status mpchol_factor(const mpchol_opts* opts, int n, const float* dA, int lda,
                             mpchol_factor_t** out, mpchol_stream_t stream);
 MPCHOL_API mpchol_status mpchol_factor_destroy(mpchol_factor_t* f);
+/* The device memory, streams and events of destroyed factor objects are kept
+ * for the next object of about the same size (at most 4 sets, 512 MiB in all,
+ * per process); this gives them back to the driver.  An allocation of the
+ * library that fails does the same before it reports MPCHOL_ERR_ALLOC. */
+MPCHOL_API void mpchol_release_cached(void);
 /* Synchronizes `stream`; fills info; hStepPrec (nullable, length nsteps)
  * receives each step's trailing-update precision, hStepFp64 (nullable) the
  * FP64-diagonal flags. */

@@ -25,3 +25,36 @@ def test_operator_copy_is_exact_for_every_alignment(n, pad, offset):
     assert torch.equal(got, ref)
     L = np.linalg.cholesky(A.double().cpu().numpy())
     assert np.linalg.norm(got.cpu().numpy() - L) / np.linalg.norm(L) < 1e-5
+
+
+def test_resources_of_a_freed_factor_serve_the_next_one():
+    """Objects made and freed in turn (with other sizes between, in threads on
+    streams of their own, after the cache was given back) factor as a lone one."""
+    import threading
+    from cholesky_gpu_b200 import _lib
+    sizes = (200, 900, 513, 900)
+    mats = {n: matgen.spd_matrix(n, 1e2, n).cuda() for n in set(sizes)}
+    opts = dict(block_size=128, precision="fp16x2")
+    _lib.load().mpchol_release_cached()
+    ref = {n: mp.factor(A, **opts).lower() for n, A in mats.items()}
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(order):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for n in order:
+                    f = mp.factor(mats[n], **opts)
+                    if not torch.equal(f.lower(), ref[n]):
+                        bad.append(n)
+                    del f
+        except Exception as e:      # a thread's exception does not fail the test by itself
+            bad.append(e)
+    threads = [threading.Thread(target=work, args=(o,)) for o in (sizes, sizes[::-1], sizes * 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    _lib.load().mpchol_release_cached()
+    work(sizes)
+    assert not bad
