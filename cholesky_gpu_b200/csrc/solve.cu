@@ -652,129 +652,124 @@ symv_kernel(const TA* __restrict__ A, int lda, int n, const double* __restrict__
 // ---- setup: super-block inverses by recursive doubling ---------------------
 // For a lower-triangular [A 0; B C], inv = [A^-1 0; X C^-1] with
 // X = -C^-1 (B A^-1).  The inverses W_S of the RS-row diagonal super-blocks
-// are built bottom-up: the 128-row diagonal blocks in FP64 inside one CTA each
-// (32-row tiles, then the 32 -> 64 -> 128 doublings), then the 128 -> 1024
-// doublings as 128 x 128 FP32 GEMM tiles over all super-blocks at once.
+// are built bottom-up: the 128-row diagonal blocks in FP64 (32-row tiles on
+// the FP64 tensor cores), then the 128 -> 1024 doublings as 64 x 64 FP32 GEMM
+// tiles over all super-blocks at once.
 // Storage: W_S is RS x RS column-major at wsup + S*RS*RS.  Its lower 128-tiles
 // hold the inverse (diagonal tiles with a zero upper part); the strictly
 // upper 128-tiles are scratch for the doubling products T = B A^-1 and are
 // never read by the solves.
 
-constexpr int BLD = RB + 1;     // padded column stride of the shared tiles
+// FP64 32 x 32 tiles in shared memory: column-major, 36 doubles per column,
+// so both DMMA fragment patterns (four consecutive rows of four columns 36
+// apart) read 16 different 8-byte banks per half-warp.
+constexpr int DT = 32;
+constexpr int DLD = 36;
+constexpr int DTSZ = DT * DLD;
+constexpr int BT = RB / DT;                       // tiles per 128-block side
+__host__ __device__ constexpr int dtri(int i, int j) { return i * (i + 1) / 2 + j; }
+// the block's ten lower tiles, the column's solved tiles below its diagonal
+// one, one product
+constexpr int BI_TILES = BT * (BT + 1) / 2 + (BT - 1) + 1;
+constexpr size_t kBlockInvSmem = (size_t)BI_TILES * DTSZ * sizeof(double);
 
-// One 128-row diagonal block per CTA (256 threads), FP64 in shared memory;
-// the FP32 result goes to its diagonal tile of W_S.  Rows and columns past n
-// are identity.
+// The 32 x 32 product A B added to the warp's two 8 x 8 blocks: rows 8 mb..,
+// columns 8 nb.. and 8 (nb + 1)..
+__device__ __forceinline__ void dtile_mma(const double* A, const double* B, int mb, int nb, int g,
+                                          int t, double (&acc)[2][2]) {
+#pragma unroll
+  for (int k0 = 0; k0 < DT; k0 += 4) {
+    const double a = A[(k0 + t) * DLD + 8 * mb + g];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) dmma_m8n8k4(acc[u], a, B[(8 * (nb + u) + g) * DLD + k0 + t]);
+  }
+}
+
+// Columns 32 q .. 32 q + 31 of the inverse of one 128-row diagonal block
+// (bid.x = 4 block + q), 256 threads, FP64; the FP32 result goes to its
+// diagonal tile of W_S.  Rows and columns past n are identity.  The columns
+// of an inverse are independent, so four CTAs share a block and each runs
+// only the tile rows from q down:
+//   W_q = L_qq^-1,  W_i = -L_ii^-1 (L_iq W_q + .. + L_i,i-1 W_i-1)
+// with the diagonal tiles inverted side by side, one warp each.  Latency
+// bound (the 32 dependent steps of a tile inverse, then up to three pairs of
+// products): 13 us for up to 37 blocks, 45 us for the 128 blocks of n = 16384
+// (one CTA per block with 8-byte shared loads per FMA: 80 and 84 us).
 __device__ __forceinline__ void
 block_inverse_body(const float* __restrict__ L, int ldl, int n, float* __restrict__ wsup, uint3 bid) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  double* W = reinterpret_cast<double*>(sm_raw);            // [RB][BLD], column-major
-  float* Ls = reinterpret_cast<float*>(W + RB * BLD);        // [RB][BLD], column-major
-  const int g = bid.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int i0 = g * RB;
+  double* Lt = reinterpret_cast<double*>(sm_raw);           // tile (i, j) at dtri(i, j) * DTSZ
+  double* Wt = Lt + BT * (BT + 1) / 2 * DTSZ;               // W_i, i > q, at (i - 1) * DTSZ
+  double* Pt = Wt + (BT - 1) * DTSZ;                        // the product
+  const int g0 = bid.x / BT, q = bid.x % BT;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = g0 * RB;
   const int nb = min(RB, n - i0);
-  // 16 loads in flight per thread before their shared-memory stores
-  constexpr int LB = 16;
-  for (int e0 = tid; e0 < RB * RB; e0 += LB * NTH) {
-    float v[LB];
+  // the lower tiles of tile columns q.., four loads in flight per thread
+  for (int j = q; j < BT; ++j)
+    for (int i = j; i < BT; ++i) {
+      float v[DT * DT / NTH];
 #pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int e = e0 + u * NTH;
-      const int col = e / RB, row = e % RB;
-      if (row < nb && col < nb) v[u] = (row >= col) ? L[(size_t)(i0 + col) * ldl + i0 + row] : 0.0f;
-      else v[u] = (row == col) ? 1.0f : 0.0f;
-    }
+      for (int u = 0; u < DT * DT / NTH; ++u) {
+        const int e = tid + u * NTH, c = DT * j + e / DT, r = DT * i + e % DT;
+        v[u] = (r < nb && c < nb) ? (r >= c ? L[(size_t)(i0 + c) * ldl + i0 + r] : 0.0f)
+                                  : (r == c ? 1.0f : 0.0f);
+      }
 #pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int e = e0 + u * NTH;
-      const int col = e / RB, row = e % RB;
-      Ls[col * BLD + row] = v[u];
-      W[col * BLD + row] = 0.0;
+      for (int u = 0; u < DT * DT / NTH; ++u) {
+        const int e = tid + u * NTH;
+        Lt[dtri(i, j) * DTSZ + (e / DT) * DLD + e % DT] = (double)v[u];
+      }
     }
+  __syncthreads();
+  // diagonal tiles, in place: lane j of warp w solves L_tt w = e_j (t = q + w;
+  // right-looking, the column held in registers)
+  if (q + warp < BT) {
+    double* T = Lt + dtri(q + warp, q + warp) * DTSZ;
+    const double rinv = 1.0 / T[lane * DLD + lane];
+    double w[DT];
+#pragma unroll
+    for (int i = 0; i < DT; ++i) w[i] = (i == lane) ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < DT; ++k) {
+      w[k] *= __shfl_sync(0xffffffffu, rinv, k);
+#pragma unroll
+      for (int i = k + 1; i < DT; ++i) w[i] = fma(-T[k * DLD + i], w[k], w[i]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < DT; ++i) T[lane * DLD + i] = w[i];
   }
   __syncthreads();
-  // 32-row diagonal tiles: warp t, lane j solves L_tt w = e_j (right-looking,
-  // the column held in registers)
-  if (warp < RB / 32) {
-    const int t0 = warp * 32;
-    double w[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) w[i] = (i == lane) ? 1.0 : 0.0;
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      w[k] = w[k] / (double)Ls[(t0 + k) * BLD + t0 + k];
-#pragma unroll
-      for (int i = k + 1; i < 32; ++i) w[i] -= (double)Ls[(t0 + k) * BLD + t0 + i] * w[k];
-    }
-#pragma unroll
-    for (int i = 0; i < 32; ++i) W[(t0 + lane) * BLD + t0 + i] = w[i];
+  const int S = i0 / RS, tb = (i0 % RS) / RB;
+  float* out = wsup + (size_t)S * RS * RS + (size_t)(tb * RB + DT * q) * RS + tb * RB;
+  // rows above the tile column are zero, then its diagonal tile
+  for (int e = tid; e < DT * DT * (q + 1); e += NTH) {
+    const int c = e % DT, r = e / DT;              // r < 32 (q + 1)
+    out[(size_t)c * RS + r] = r < DT * q ? 0.0f : (float)Lt[dtri(q, q) * DTSZ + c * DLD + r - DT * q];
   }
-  __syncthreads();
-  // doublings h = 32 (two pairs) and h = 64 (one pair) inside the block;
-  // output e of a level: row r = e % h, column c = (e / h) % h of pair e / h^2
-  // Every output of a doubling runs over the whole k range of its pair: the
-  // inverses stored in W are zero above their diagonals, so the extra terms
-  // add zeros, and a thread's outputs advance together (independent
-  // accumulators instead of one dependent chain after another).
-  for (int h = 32; h < RB; h *= 2) {
-    const int per = (RB / (2 * h)) * h * h / NTH;    // outputs per thread: 8 or 16
-    int pa[16], pb[16];                               // per output: operand bases
-    double acc[16];
-    // T = B A^-1 -> the pair's upper-right block (scratch):
-    // T[r][c] = sum_k L[a0+h+r][a0+k] * Ainv[k][c]
+  const int g = lane >> 2, t = lane & 3, mb = warp >> 1, nb8 = 2 * (warp & 1);
+  for (int i = q + 1; i < BT; ++i) {
+    double acc[2][2] = {};
+    dtile_mma(Lt + dtri(i, q) * DTSZ, Lt + dtri(q, q) * DTSZ, mb, nb8, g, t, acc);
+    for (int j = q + 1; j < i; ++j)
+      dtile_mma(Lt + dtri(i, j) * DTSZ, Wt + (j - 1) * DTSZ, mb, nb8, g, t, acc);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int e = tid + NTH * q;
-      const int r = e % h, c = (e / h) % h, a0 = (e / (h * h)) * 2 * h;
-      pa[q] = a0 * BLD + a0 + h + r;                  // Ls[(a0 + k) * BLD + a0 + h + r]
-      pb[q] = (a0 + c) * BLD + a0;                    // W[(a0 + c) * BLD + a0 + k]
-      acc[q] = 0.0;
-    }
-    for (int k = 0; k < h; ++k) {
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int q = 0; q < 16; ++q)
-        if (q < per) acc[q] += (double)Ls[pa[q] + k * BLD] * W[pb[q] + k];
-    }
+      for (int e = 0; e < 2; ++e) Pt[(8 * (nb8 + u) + 2 * t + e) * DLD + 8 * mb + g] = -acc[u][e];
     __syncthreads();
+    double x[2][2] = {};
+    dtile_mma(Lt + dtri(i, i) * DTSZ, Pt, mb, nb8, g, t, x);
 #pragma unroll
-    for (int q = 0; q < 16; ++q)
-      if (q < per) {
-        const int e = tid + NTH * q;
-        const int r = e % h, c = (e / h) % h, a0 = (e / (h * h)) * 2 * h;
-        W[(a0 + h + c) * BLD + a0 + r] = acc[q];
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * (nb8 + u) + 2 * t + e, r = 8 * mb + g;
+        Wt[(i - 1) * DTSZ + c * DLD + r] = x[u][e];
+        out[(size_t)c * RS + DT * i + r] = (float)x[u][e];
       }
     __syncthreads();
-    // X = -C^-1 T -> the pair's lower-left block; the scratch is cleared:
-    // X[r][c] = -sum_k Cinv[r][k] * T[k][c]
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int e = tid + NTH * q;
-      const int r = e % h, c = (e / h) % h, a0 = (e / (h * h)) * 2 * h;
-      pa[q] = (a0 + h) * BLD + a0 + h + r;            // W[(a0 + h + k) * BLD + a0 + h + r]
-      pb[q] = (a0 + h + c) * BLD + a0;                // W[(a0 + h + c) * BLD + a0 + k]
-      acc[q] = 0.0;
-    }
-    for (int k = 0; k < h; ++k) {
-#pragma unroll
-      for (int q = 0; q < 16; ++q)
-        if (q < per) acc[q] += W[pa[q] + k * BLD] * W[pb[q] + k];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-      if (q < per) {
-        const int e = tid + NTH * q;
-        const int r = e % h, c = (e / h) % h, a0 = (e / (h * h)) * 2 * h;
-        W[(a0 + c) * BLD + a0 + h + r] = -acc[q];
-        W[(a0 + h + c) * BLD + a0 + r] = 0.0;
-      }
-    __syncthreads();
-  }
-  const int S = i0 / RS, t = (i0 % RS) / RB;
-  float* out = wsup + (size_t)S * RS * RS + (size_t)(t * RB) * RS + t * RB;
-  for (int e = tid; e < RB * RB; e += NTH) {
-    const int col = e / RB, row = e % RB;
-    out[(size_t)col * RS + row] = (float)W[col * BLD + row];
   }
 }
 
@@ -783,104 +778,143 @@ block_inverse_kernel(const float* __restrict__ L, int ldl, int n, float* __restr
   block_inverse_body(L, ldl, n, wsup, blockIdx);
 }
 
-// C(128x128) = A(128 x K) * B(K x 128), A and B column-major, FP32 FMA.
-// 256 threads, 8 x 8 outputs each (rows tx*4+{0..3}, 64+tx*4+{0..3}).  K
-// advances in chunks of GK (a multiple of GK): the next chunk is loaded into
-// registers (coalesced: 128 consecutive rows of A, GK consecutive k of each B
-// column) while the current one is multiplied from shared memory.
-constexpr int GK = 32;
-constexpr int GPT = GK * RB / NTH;   // elements of A (and of B) per thread per chunk
-constexpr int BLDK = GK + 1;         // padded column stride of the staged B chunk
+// C(64 x 64) = A(64 x K) B(K x 64), all column-major, FP32 FMA, by 256 threads
+// as four groups of 64: group q takes k = 8 q .. 8 q + 7 of every 32-deep
+// chunk with 8 x 8 outputs per thread, and the groups' sums are added at the
+// end in a fixed order.  A 64 x 64 tile per CTA spreads a super-block's
+// largest doubling over 64 SMs (128 x 128 tiles: 16) and the split of K keeps
+// the 8 x 8 register blocks that shared memory's return path needs (four
+// 16-byte reads per 64 FMAs and k).  The next chunk travels in registers.
+// The six launches of n = 1024 take 107 us (128 x 128 tiles: 266), those of n =
+// 16384 312 us (385).
+// Rows of A past a_rows are zero.  Thread (tx, ty): rows 4 tx.. and 32 + 4
+// tx.., columns ty + 8 j.
+constexpr int GT = 64;
+constexpr int GKC = 32;
+constexpr int GLDB = GKC + 4;                        // floats per staged column of B
+constexpr int G_AS = GKC * GT, G_BS = GT * GLDB;
+constexpr int G_SMEM = 2 * (G_AS + G_BS);            // two chunks; the reduction reuses them
+static_assert(G_SMEM >= 2 * GT * GT, "two groups' sums fit");
 
-__device__ __forceinline__ int acc_col_of(int ty, int b) { return b < 4 ? ty * 4 + b : 64 + ty * 4 + (b - 4); }
-
-__device__ __forceinline__ void gemm128_load(const float* A, int lda, int a_rows_valid,
-                                             const float* B, int ldb, int k0, float (&ra)[GPT],
-                                             float (&rb)[GPT]) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void gemm64_load(const float* A, int lda, int a_rows, const float* B,
+                                            int ldb, int k0, float4 (&ra)[2], float4 (&rb)[2]) {
 #pragma unroll
-  for (int q = 0; q < GPT; ++q) {
-    const int e = tid + NTH * q;
-    const int r = e % RB, kk = e / RB;          // A: rows fastest
-    ra[q] = (r < a_rows_valid) ? A[(size_t)(k0 + kk) * lda + r] : 0.0f;
-    const int k = e % GK, c = e / GK;           // B: k fastest within a column
-    rb[q] = B[(size_t)c * ldb + k0 + k];
+  for (int u = 0; u < 2; ++u) {
+    const int e = threadIdx.x + NTH * u;
+    const int r = 4 * (e % (GT / 4));
+    const float* p = A + (size_t)(k0 + e / (GT / 4)) * lda + r;
+    if (r + 3 < a_rows) {
+      ra[u] = *reinterpret_cast<const float4*>(p);
+    } else {
+      ra[u].x = r < a_rows ? p[0] : 0.0f;
+      ra[u].y = r + 1 < a_rows ? p[1] : 0.0f;
+      ra[u].z = r + 2 < a_rows ? p[2] : 0.0f;
+      ra[u].w = 0.0f;
+    }
+    rb[u] = *reinterpret_cast<const float4*>(B + (size_t)(e / (GKC / 4)) * ldb + k0 + 4 * (e % (GKC / 4)));
   }
 }
 
-__device__ void gemm128(const float* A, int lda, int a_rows_valid, const float* B, int ldb, int K,
-                        float (&acc)[8][8], float* As, float* Bs) {
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  float ra[GPT], rb[GPT];
-  gemm128_load(A, lda, a_rows_valid, B, ldb, 0, ra, rb);
-  for (int k0 = 0; k0 < K; k0 += GK) {
+__device__ __forceinline__ void gemm64(const float* A, int lda, int a_rows, const float* B, int ldb,
+                                       int K, float (&acc)[8][8], float* sm) {
+  const int tid = threadIdx.x, grp = tid / 64, tx = tid % 8, ty = (tid % 64) / 8;
+  float4 ra[2], rb[2];
+  gemm64_load(A, lda, a_rows, B, ldb, 0, ra, rb);
+  for (int k0 = 0, buf = 0; k0 < K; k0 += GKC, buf ^= 1) {
+    float* As = sm + buf * (G_AS + G_BS);            // [k][row]
+    float* Bs = As + G_AS;                           // [column][k]
 #pragma unroll
-    for (int q = 0; q < GPT; ++q) {
-      const int e = tid + NTH * q;
-      As[(e / RB) * RB + e % RB] = ra[q];
-      Bs[(e / GK) * BLDK + e % GK] = rb[q];      // B column-major in shared memory too
+    for (int u = 0; u < 2; ++u) {
+      const int e = tid + NTH * u;
+      *reinterpret_cast<float4*>(As + 4 * e) = ra[u];
+      *reinterpret_cast<float4*>(Bs + (e / (GKC / 4)) * GLDB + 4 * (e % (GKC / 4))) = rb[u];
+    }
+    __syncthreads();   // this buffer's last reader passed the previous barrier
+    if (k0 + GKC < K) gemm64_load(A, lda, a_rows, B, ldb, k0 + GKC, ra, rb);
+#pragma unroll 1
+    for (int kq = 0; kq < 8; kq += 4) {
+      const int k = 8 * grp + kq;
+      float4 b[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        b[j] = *reinterpret_cast<const float4*>(Bs + (ty + 8 * j) * GLDB + k);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 a0 = *reinterpret_cast<const float4*>(As + (k + e) * GT + 4 * tx);
+        const float4 a1 = *reinterpret_cast<const float4*>(As + (k + e) * GT + 32 + 4 * tx);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float bv = e == 0 ? b[j].x : (e == 1 ? b[j].y : (e == 2 ? b[j].z : b[j].w));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(av[i], bv, acc[i][j]);
+        }
+      }
+    }
+  }
+  // groups 2 and 3 onto 0 and 1, then 1 onto 0
+#pragma unroll
+  for (int half = 2; half >= 1; half >>= 1) {
+    __syncthreads();
+    if (grp >= half && grp < 2 * half) {
+      float* d = sm + (grp - half) * GT * GT + (tid % 64);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d[(j * 8 + i) * 64] = acc[i][j];
     }
     __syncthreads();
-    if (k0 + GK < K) gemm128_load(A, lda, a_rows_valid, B, ldb, k0 + GK, ra, rb);
-#pragma unroll 4
-    for (int kk = 0; kk < GK; ++kk) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[kk * RB + tx * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[kk * RB + 64 + tx * 4]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      float bv[8];
+    if (grp < half) {
+      const float* d = sm + grp * GT * GT + (tid % 64);
 #pragma unroll
-      for (int b = 0; b < 8; ++b) bv[b] = Bs[acc_col_of(ty, b) * BLDK + kk];
+      for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
+        for (int i = 0; i < 8; ++i) acc[i][j] += d[(j * 8 + i) * 64];
     }
-    __syncthreads();
   }
 }
 
-__device__ __forceinline__ int acc_row(int a) { return a < 4 ? (threadIdx.x % 16) * 4 + a : 64 + (threadIdx.x % 16) * 4 + (a - 4); }
-__device__ __forceinline__ int acc_col(int b) { return b < 4 ? (threadIdx.x / 16) * 4 + b : 64 + (threadIdx.x / 16) * 4 + (b - 4); }
-
-// One doubling level of half-size h (a multiple of RB) for pair blockIdx.y of
-// super-block blockIdx.z; blockIdx.x enumerates the (h/RB)^2 output tiles.
+// One doubling level of half-size h (a multiple of RB) for pair bid.y of
+// super-block bid.z; bid.x enumerates the (h/GT)^2 output tiles.
 //   PHASE 0:  T(ti,tj) = sum_{kt >= tj} L(h + ti, kt) A^-1(kt, tj)  -> upper-right scratch
 //   PHASE 1:  X(ti,tj) = -sum_{kt <= ti} C^-1(ti, kt) T(kt, tj)     -> lower-left block
-// (128-tile indices relative to the pair's origin a0 = 2 h * pair).  Tiles
+// (64-tile indices relative to the pair's origin a0 = 2 h * pair).  Tiles
 // whose rows start at or past n are skipped: the solves never read them.
 template <int PHASE>
 __device__ __forceinline__ void
 superinv_gemm_body(const float* __restrict__ L, int ldl, int n, float* __restrict__ wsup, int h, uint3 bid) {
-  __shared__ __align__(16) float As[GK * RB];
-  __shared__ __align__(16) float Bs[RB * BLDK];
-  const int tpr = h / RB;
+  __shared__ __align__(16) float sm[G_SMEM];
+  const int tpr = h / GT;
   const int ti = bid.x / tpr, tj = bid.x % tpr;
   const int S = bid.z, s0 = S * RS, a0 = bid.y * 2 * h;
-  const int grow = s0 + a0 + h + ti * RB;          // first global row of the output tile
+  const int grow = s0 + a0 + h + ti * GT;          // first global row of the output tile
   if (grow >= n) return;
   float* W = wsup + (size_t)S * RS * RS;
   float acc[8][8] = {};
+  float* out;
   if (PHASE == 0) {
-    gemm128(L + (size_t)(s0 + a0 + tj * RB) * ldl + grow, ldl, min(RB, n - grow),
-            W + (size_t)(a0 + tj * RB) * RS + a0 + tj * RB, RS, h - tj * RB, acc, As, Bs);
-    float* T = W + (size_t)(a0 + h + tj * RB) * RS + a0 + ti * RB;
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int b = 0; b < 8; ++b) T[(size_t)acc_col(b) * RS + acc_row(a)] = acc[a][b];
+    gemm64(L + (size_t)(s0 + a0 + tj * GT) * ldl + grow, ldl, min(GT, n - grow),
+           W + (size_t)(a0 + tj * GT) * RS + a0 + tj * GT, RS, h - tj * GT, acc, sm);
+    out = W + (size_t)(a0 + h + tj * GT) * RS + a0 + ti * GT;
   } else {
-    gemm128(W + (size_t)(a0 + h) * RS + a0 + h + ti * RB, RS, RB,
-            W + (size_t)(a0 + h + tj * RB) * RS + a0, RS, (ti + 1) * RB, acc, As, Bs);
-    float* X = W + (size_t)(a0 + tj * RB) * RS + a0 + h + ti * RB;
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int b = 0; b < 8; ++b) X[(size_t)acc_col(b) * RS + acc_row(a)] = -acc[a][b];
+    gemm64(W + (size_t)(a0 + h) * RS + a0 + h + ti * GT, RS, GT,
+           W + (size_t)(a0 + h + tj * GT) * RS + a0, RS, (ti + 1) * GT, acc, sm);
+    out = W + (size_t)(a0 + tj * GT) * RS + a0 + h + ti * GT;
   }
+  if (threadIdx.x >= 64) return;                   // group 0 holds the sums
+  const float sg = PHASE == 0 ? 1.0f : -1.0f;
+  const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh)
+      *reinterpret_cast<float4*>(out + (size_t)(ty + 8 * j) * RS + 32 * hh + 4 * tx) =
+          make_float4(sg * acc[4 * hh][j], sg * acc[4 * hh + 1][j], sg * acc[4 * hh + 2][j],
+                      sg * acc[4 * hh + 3][j]);
 }
 
 template <int PHASE>
-__global__ void __launch_bounds__(NTH)
+__global__ void __launch_bounds__(NTH, 2)
 superinv_gemm_kernel(const float* __restrict__ L, int ldl, int n, float* __restrict__ wsup, int h) {
   superinv_gemm_body<PHASE>(L, ldl, n, wsup, h, blockIdx);
 }
@@ -1353,12 +1387,12 @@ __global__ void vec_slot_batched_kernel(const BatchSys* __restrict__ sys, int sr
 __global__ void __launch_bounds__(NTH)
 block_inverse_batched_kernel(const BatchSys* __restrict__ sys) {
   const BatchSys& S = sys[blockIdx.y];
-  if ((int)blockIdx.x * RB >= S.n) return;
+  if ((int)(blockIdx.x / BT) * RB >= S.n) return;
   block_inverse_body(S.A, S.ld, S.n, S.wsup, make_uint3(blockIdx.x, 0, 0));
 }
 
 template <int PHASE>
-__global__ void __launch_bounds__(NTH)
+__global__ void __launch_bounds__(NTH, 2)
 superinv_gemm_batched_kernel(const BatchSys* __restrict__ sys, int h, int max_super) {
   const BatchSys& S = sys[blockIdx.z / max_super];
   const int sup = blockIdx.z % max_super;
@@ -1458,8 +1492,7 @@ cudaError_t solve_init_attributes() {
 
 cudaError_t solve_set_attributes() {
   cudaError_t e;
-  const size_t inv = (size_t)RB * BLD * (sizeof(double) + sizeof(float));
-  if ((e = set_dyn(block_inverse_kernel, inv)) != cudaSuccess) return e;
+  if ((e = set_dyn(block_inverse_kernel, kBlockInvSmem)) != cudaSuccess) return e;
 #define SET_NR(NRC)                                                                         \
   if ((e = set_dyn(symv_kernel<float, NRC>, red_bytes(NRC))) != cudaSuccess) return e;      \
   if ((e = set_dyn(symv_kernel<double, NRC>, red_bytes(NRC))) != cudaSuccess) return e;
@@ -1471,7 +1504,7 @@ cudaError_t solve_set_attributes() {
   if ((e = set_dyn(symv_staged_kernel<NRC>, symv_staged_smem<NRC>())) != cudaSuccess) return e;
   SET_NRP(1) SET_NRP(2) SET_NRP(4) SET_NRP(8)
 #undef SET_NRP
-  if ((e = set_dyn(block_inverse_batched_kernel, inv)) != cudaSuccess) return e;
+  if ((e = set_dyn(block_inverse_batched_kernel, kBlockInvSmem)) != cudaSuccess) return e;
 #define SET_NRB(NRC)                                                                              \
   if ((e = set_dyn(symv_staged_batched_kernel<NRC>, symv_batched_smem<NRC>())) != cudaSuccess) return e; \
   if ((e = set_dyn(trmv_super_batched_kernel<NRC, false>, red_bytes(NRC))) != cudaSuccess) return e; \
@@ -1522,12 +1555,16 @@ cudaError_t launch_symv_skip(const TA* A, int lda, int n, const double* x, doubl
 template cudaError_t launch_symv_skip<float>(const float*, int, int, const double*, double*, int, const int*, cudaStream_t, double*, int);
 template cudaError_t launch_symv_skip<double>(const double*, int, int, const double*, double*, int, const int*, cudaStream_t, double*, int);
 
+// Pairs of the doubling level h whose second half has rows below n, in a
+// super-block of the first min(n, RS) rows; 0: the level is not launched.
+int doubling_pairs(int n, int h) { return ceil_div(std::max(0, std::min(n, RS) - h), 2 * h); }
+
 cudaError_t launch_solve_setup(const float* L, int ldl, int n, float* wsup, cudaStream_t stream) {
-  const size_t inv = (size_t)RB * BLD * (sizeof(double) + sizeof(float));
-  block_inverse_kernel<<<ceil_div(n, RB), NTH, inv, stream>>>(L, ldl, n, wsup);
+  block_inverse_kernel<<<BT * ceil_div(n, RB), NTH, kBlockInvSmem, stream>>>(L, ldl, n, wsup);
   const int nbs = ceil_div(n, RS);
   for (int h = RB; h < RS; h *= 2) {
-    const dim3 grid((h / RB) * (h / RB), RS / (2 * h), nbs);
+    if (doubling_pairs(n, h) == 0) break;
+    const dim3 grid((h / GT) * (h / GT), doubling_pairs(n, h), nbs);
     superinv_gemm_kernel<0><<<grid, NTH, 0, stream>>>(L, ldl, n, wsup, h);
     superinv_gemm_kernel<1><<<grid, NTH, 0, stream>>>(L, ldl, n, wsup, h);
   }
@@ -1535,9 +1572,8 @@ cudaError_t launch_solve_setup(const float* L, int ldl, int n, float* wsup, cuda
 }
 
 int solve_setup_launches(int n) {
-  (void)n;
   int k = 1;
-  for (int h = RB; h < RS; h *= 2) k += 2;
+  for (int h = RB; h < RS && doubling_pairs(n, h) > 0; h *= 2) k += 2;
   return k;
 }
 
@@ -1559,11 +1595,11 @@ cudaError_t launch_symv_batched(const BatchSys* sys, int nsys, int ntiles, int x
 
 cudaError_t launch_solve_setup_batched(const BatchSys* sys, int nsys, int max_n,
                                        cudaStream_t stream) {
-  const size_t inv = (size_t)RB * BLD * (sizeof(double) + sizeof(float));
-  block_inverse_batched_kernel<<<dim3(ceil_div(max_n, RB), nsys), NTH, inv, stream>>>(sys);
+  block_inverse_batched_kernel<<<dim3(BT * ceil_div(max_n, RB), nsys), NTH, kBlockInvSmem, stream>>>(sys);
   const int max_super = ceil_div(max_n, RS);
   for (int h = RB; h < RS; h *= 2) {
-    const dim3 grid((h / RB) * (h / RB), RS / (2 * h), nsys * max_super);
+    if (doubling_pairs(max_n, h) == 0) break;
+    const dim3 grid((h / GT) * (h / GT), doubling_pairs(max_n, h), nsys * max_super);
     superinv_gemm_batched_kernel<0><<<grid, NTH, 0, stream>>>(sys, h, max_super);
     superinv_gemm_batched_kernel<1><<<grid, NTH, 0, stream>>>(sys, h, max_super);
   }

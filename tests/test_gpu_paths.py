@@ -58,3 +58,17 @@ def test_resources_of_a_freed_factor_serve_the_next_one():
     _lib.load().mpchol_release_cached()
     work(sizes)
     assert not bad
+
+
+@pytest.mark.parametrize("n", [31, 33, 96, 128, 129, 191, 385, 640, 1023, 1025, 1500])
+def test_preconditioner_apply_at_block_and_super_block_edges(n):
+    """z = M^-1 r through the block and super-block inverses against the FP64
+    solve with the factor itself.  The inverses are exact to FP32 rounding:
+    kappa(L) = 10, so 1e-5 leaves two digits."""
+    A = matgen.spd_matrix(n, 1e2, n).cuda()
+    f = mp.factor(A, block_size=128, precision="fp32")
+    L = f.lower().double()
+    R = matgen.rhs(n, 3, 5).cuda()
+    Z = f.apply_precond(R)
+    ref = torch.cholesky_solve(R, L)
+    assert ((Z - ref).norm() / ref.norm()).item() < 1e-5
