@@ -72,3 +72,45 @@ def test_preconditioner_apply_at_block_and_super_block_edges(n):
     Z = f.apply_precond(R)
     ref = torch.cholesky_solve(R, L)
     assert ((Z - ref).norm() / ref.norm()).item() < 1e-5
+
+
+@pytest.mark.parametrize("n,d,lower", [
+    (1, 3, False), (63, 16, True), (65, 17, False), (2047, 15, True), (2305, 33, True),
+])
+def test_rbf_build_at_tile_edges(n, d, lower):
+    """Both tile heights of the builder, ragged in rows and features: 1e-13 of
+    the FP64 kernel (64 differences of FP32 values squared in FP64: d * 2^-53
+    relative in the exponent, which is below 30 here), zeros above a lower build."""
+    from cholesky_gpu_b200.autograd import rbf_build
+    from oracle import oracle as O
+    X = matgen.gaussian_points(n, d, n)
+    K64, K32 = rbf_build(torch.from_numpy(X).cuda(), 2.0, 0.25, lower_only=lower)
+    want, _ = O.rbf_kernel_f64(X, 2.0, 0.25)
+    if lower:
+        want = np.tril(want)
+    got = K64.cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
+    assert np.array_equal(K32.cpu().numpy(), got.astype(np.float32))
+
+
+@pytest.mark.parametrize("n,d", [(1, 1), (17, 128), (130, 9), (3199, 3), (3201, 8), (6401, 7), (6465, 120)])
+def test_rbf_grad_contraction_at_row_tile_edges(n, d):
+    """The 16-, 32- and 64-row variants against dense FP64: sums of n terms,
+    relative error of a norm below 1e-13."""
+    from cholesky_gpu_b200.autograd import rbf_grad_contract
+    g = torch.Generator(device="cuda").manual_seed(n)
+    X = torch.randn((n, d), generator=g, device="cuda")
+    a, b = (torch.randn(n, generator=g, device="cuda", dtype=torch.float64) for _ in range(2))
+    ell = float(d) ** 0.5
+    P, s = rbf_grad_contract(X, ell, a, b)
+    Xd = X.double()
+    r2 = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    for k in range(d):
+        r2 += (Xd[:, k].unsqueeze(1) - Xd[:, k].unsqueeze(0)) ** 2
+    K = torch.exp(-r2 / (2 * ell * ell))
+    Z = torch.cat([a.unsqueeze(1), b.unsqueeze(1), a.unsqueeze(1) * Xd, b.unsqueeze(1) * Xd], 1)
+    want = K @ Z
+    assert ((P - want).norm() / want.norm()).item() < 1e-13
+    ws = (a @ ((K * r2) @ b)).item()
+    scale = (a.abs() @ ((K * r2) @ b.abs())).item()
+    assert abs(s.item() - ws) <= 1e-13 * max(scale, 1e-300)
