@@ -61,17 +61,13 @@ size_t potrf_smem_bytes(int bs);
 size_t potrf_scratch64_elems(int bs);
 // Also writes the inverses of the 32x32 diagonal tiles of the factored block
 // to winv (ceil(bs/32) tiles, column-major 32x32 each) for the panel solve.
-// tmap32: TMA map over A (FP32, n x n, column stride lda) with 32 x 32 boxes.
 // With diagonal perturbation, the block's rows first receive the previous
 // step's rounding shift, sh += u(prev->prec) * rowsq (prev null: none).
-// compact: the small-code variant, for a POTRF that runs beside a long
-// trailing update (the fully unrolled one is faster on its own but slows
-// down several times when its instructions are refetched through a busy L2).
-cudaError_t launch_potrf(const CUtensorMap& tmap32, float* A, int lda, int n, int s, int bs,
+cudaError_t launch_potrf(float* A, int lda, int s, int bs,
                          const float* d, float* sh, const PotrfParams& p,
                          const int* fp64_flag, double* scratch64, float* winv, DevStatus* st,
                          bool may_fp64, cudaStream_t stream, const StepState* prev = nullptr,
-                         const float* rowsq = nullptr, bool compact = false);
+                         const float* rowsq = nullptr);
 
 // ---- panel TRSM + fused diagonal tracker, decision and quantization ------
 // Where the panel solve writes the quantized panel: one K-major code panel
@@ -99,8 +95,8 @@ __host__ __device__ inline int rexp_slot(int fmt) { return fmt == E4M3 ? 0 : (fm
 // (step->prec).  Before its rows' sums of squares are overwritten, each CTA
 // adds the previous step's rounding shift u(prev->prec) * rowsq to qa.sh for
 // its rows (prev null: first step); the rows of the next diagonal block get
-// theirs in its POTRF.  tmapX: TMA map over A with 32 x bs boxes; tmap32 as
-// for launch_potrf.
+// theirs in its POTRF.  tmapX: TMA map over A with 32 x bs boxes; tmap32: with
+// 32 x 32 boxes.
 // colacc (coherence rule, nullable otherwise): kColCopies x bs FP64
 // accumulators, zeroed before the launch, that receive the panel's column
 // sums (slab i adds into copy i % kColCopies).

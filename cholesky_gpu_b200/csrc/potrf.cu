@@ -6,11 +6,9 @@
 // up to 256 x 256 as a blocked right-looking Cholesky on dense 32 x 32 tiles in
 // shared memory (column-major, lane i of a warp always owns row i, so every
 // shared access is either contiguous across lanes or a broadcast):
-//   * the lower tiles are staged by TMA (one thread issues the 2-D copies,
-//     an mbarrier counts the bytes) and written back by TMA stores;
-//   * one warp factors each diagonal tile with the tile's rows held in
-//     registers, one tile ahead of the trailing update of the other warps;
-//   * warps solve the tiles below and update the trailing tiles;
+//   * a warp owns a row of tiles: it solves them from left to right, each
+//     close behind the factor of its diagonal tile, then factors its own;
+//   * other warps update the tiles ahead of their turn;
 //   * the inverses of the diagonal tiles are formed for the panel solve.
 // Blocks flagged near-indefinite by the switching criterion are factored in
 // FP64 by a second kernel on a global (L2-resident) scratch.
@@ -287,21 +285,19 @@ __device__ void invert_tile(const T* l, const T* inv, float* out, int lane) {
   }
 }
 
-template <typename T, bool TMA, int CB>
-__device__ void potrf_block(const CUtensorMap* tmap, T* tiles, float* A, int lda, int n, int s,
-                            int bs, const float* d, float* sh, const PotrfParams& p,
-                            float* winv, DevStatus* st, const StepState* prev = nullptr,
-                            const float* rowsq = nullptr) {
+// ---- FP64 blocks -------------------------------------------------------------
+template <typename T, int CB>
+__device__ void potrf_block(T* tiles, float* A, int lda, int s, int bs, const float* d, float* sh,
+                            const PotrfParams& p, float* winv, DevStatus* st,
+                            const StepState* prev, const float* rowsq) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int NT = (bs + TS - 1) / TS;
-  const int ntiles = NT * (NT + 1) / 2;
   __shared__ T s_shift[256];
   __shared__ T s_pmin[256];
   __shared__ T s_inv[256];
   __shared__ __align__(16) T s_col[2 * TS];
-  __shared__ int s_fail, s_pert, s_ok;
-  __shared__ __align__(8) uint64_t bar;
-  if (tid == 0) { s_fail = -1; s_pert = 0; s_ok = 1; }
+  __shared__ int s_fail, s_pert;
+  if (tid == 0) { s_fail = -1; s_pert = 0; }
   const int prev_prec = (prev != nullptr && p.diag_pert && sh) ? prev->prec : FP32;
   for (int i = tid; i < NT * TS; i += blockDim.x) {
     T shv = T(0), pm = T(0);
@@ -319,59 +315,30 @@ __device__ void potrf_block(const CUtensorMap* tmap, T* tiles, float* A, int lda
     s_shift[i] = shv;
     s_pmin[i] = pm;
   }
-  if (TMA) {
-    // stage the lower tiles with TMA (the lanes of warp 0 issue the copies);
-    // rows/columns past n arrive as zeros
-    if (warp == 0) {
-      if (lane == 0) {
-        tc::mbar_init(&bar, 1);
-        tc::fence_mbar_init();
-        tc::mbar_expect_tx(&bar, (uint32_t)(ntiles * TSZ * sizeof(float)));
-      }
-      __syncwarp();
-      for (int t = lane; t < ntiles; t += 32) {
-        int I = 0;
-        while ((I + 1) * (I + 2) / 2 <= t) ++I;
-        const int J = t - I * (I + 1) / 2;
-        tc::tma_load_2d(tiles + t * TSZ, tmap, &bar, s + I * TS, s + J * TS);
-      }
-      if (lane == 0 && !tc::mbar_wait(&bar, 0)) {
-        s_ok = 0;
-        set_status(st, MPCHOL_ERR_TIMEOUT, s);
-        tc::mbar_wait(&bar, 0);
-      }
-    }
-    __syncthreads();
-    if (!s_ok) return;
-    // identity padding past the block (only the last block can be partial)
-    for (int i = bs + tid; i < NT * TS; i += blockDim.x)
-      tiles[tidx(i / TS, i / TS) * TSZ + (i % TS) * TS + (i % TS)] = T(1);
-  } else {
-    // FP64 path: batched loads from the FP32 matrix
-    const int total = NT * NT * TSZ;
-    for (int base = 0; base < total; base += 8 * blockDim.x) {
-      float v[8];
-      int dst[8];
+  // FP64 path: batched loads from the FP32 matrix
+  const int total = NT * NT * TSZ;
+  for (int base = 0; base < total; base += 8 * blockDim.x) {
+    float v[8];
+    int dst[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = base + q * blockDim.x + tid;
-        dst[q] = -1;
-        v[q] = 0.0f;
-        if (e < total) {
-          const int T2 = e / TSZ, rc = e % TSZ;
-          const int I = T2 % NT, J = T2 / NT, c = rc / TS, r = rc % TS;
-          if (I >= J) {
-            const int gr = I * TS + r, gc = J * TS + c;
-            dst[q] = tidx(I, J) * TSZ + c * TS + r;
-            if (gr < bs && gc < bs) v[q] = A[(size_t)(s + gc) * lda + (s + gr)];
-            else v[q] = (gr == gc) ? 1.0f : 0.0f;
-          }
+    for (int q = 0; q < 8; ++q) {
+      const int e = base + q * blockDim.x + tid;
+      dst[q] = -1;
+      v[q] = 0.0f;
+      if (e < total) {
+        const int T2 = e / TSZ, rc = e % TSZ;
+        const int I = T2 % NT, J = T2 / NT, c = rc / TS, r = rc % TS;
+        if (I >= J) {
+          const int gr = I * TS + r, gc = J * TS + c;
+          dst[q] = tidx(I, J) * TSZ + c * TS + r;
+          if (gr < bs && gc < bs) v[q] = A[(size_t)(s + gc) * lda + (s + gr)];
+          else v[q] = (gr == gc) ? 1.0f : 0.0f;
         }
       }
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (dst[q] >= 0) tiles[dst[q]] = T(v[q]);
     }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (dst[q] >= 0) tiles[dst[q]] = T(v[q]);
   }
   __syncthreads();
   // Step J: (A) the tiles below diagonal tile J are solved, one per warp;
@@ -442,78 +409,526 @@ __device__ void potrf_block(const CUtensorMap* tmap, T* tiles, float* A, int lda
     if (tid == 0) set_status(st, MPCHOL_ERR_NOT_SPD, s + s_fail);
     return;
   }
-  // write back: TMA stores of the lower tiles (FP32 path), or a coalesced loop
-  // that rounds the FP64 tiles to FP32.  The strictly upper part of a
-  // diagonal tile is written back as it was staged; it is never read as data.
-  if (TMA) {
-    tc::fence_proxy_async_smem();
-    __syncthreads();
-    if (warp == 0) {   // the lanes of warp 0 issue the stores
-      for (int t = lane; t < ntiles; t += 32) {
-        int I = 0;
-        while ((I + 1) * (I + 2) / 2 <= t) ++I;
-        const int J = t - I * (I + 1) / 2;
-        tc::tma_store_2d(tmap, tiles + t * TSZ, s + I * TS, s + J * TS);
-      }
-      tc::bulk_commit();
-    }
-  } else {
-    for (int c = warp; c < bs; c += nwarps) {
-      const int J = c / TS, cc = c % TS;
-      for (int r = c + lane; r < bs; r += TS) {
-        const int I = r / TS, rr = r % TS;
-        A[(size_t)(s + c) * lda + (s + r)] = (float)tiles[tidx(I, J) * TSZ + cc * TS + rr];
-      }
+  // write back, rounded to FP32
+  for (int c = warp; c < bs; c += nwarps) {
+    const int J = c / TS, cc = c % TS;
+    for (int r = c + lane; r < bs; r += TS) {
+      const int I = r / TS, rr = r % TS;
+      A[(size_t)(s + c) * lda + (s + r)] = (float)tiles[tidx(I, J) * TSZ + cc * TS + rr];
     }
   }
   // inverses of the diagonal tiles, used by the panel solve
   for (int J = warp; J < NT; J += nwarps)
     invert_tile<T, CB>(tiles + tidx(J, J) * TSZ, s_inv + J * TS, winv + J * TS * TS, lane);
   if (tid == 0 && s_pert) atomicAdd(&st->perturbed, s_pert);
-  if (TMA && warp == 0) tc::bulk_wait_read();   // smem must outlive the stores' reads
-  (void)n;
 }
 
-// FP32 blocks: tiles in shared memory, staged by TMA.  Separate kernels for
-// the two precisions keep the FP64 register footprint out of the FP32 path.
-// CB = TS unrolls the tile loops fully (fastest on its own); CB = 4 keeps the
-// kernel's code about a quarter of that size, so it stays cache-resident and
-// fast while a trailing update saturates L2 beside it.
-template <int CB>
+// ---- FP32 blocks -------------------------------------------------------------
+// The chain of a block is its 256 pivots; the rest (28 tile solves and 84 tile
+// products) has to stay off it.  Warp I (0 .. 7) owns tile row I, lane = row:
+//   * for each tile column J < I it solves X(I, J), eight columns behind the
+//     factor of diagonal tile J (follow_tile), having applied column J - 1 to
+//     the tile itself;
+//   * while it solves X(I, I - 1) it applies the finished columns to its
+//     diagonal tile, kept in registers, so that its factor starts as soon as
+//     the solve ends;
+//   * it factors the diagonal tile (chain_tile), eight columns at a time: the
+//     8 x 8 diagonal block goes to every lane through shared memory, each lane
+//     factors it in registers (no shuffle on the pivot chain) and solves its
+//     own row with it, and the update of the columns beyond the next eight
+//     overlaps the next eight pivots;
+//   * then it inverts the tile for the panel solve.
+// The other warps apply columns 0 .. J - 2 to the tiles of column J >= 2 before
+// their row's warp gets there, in the order of those deadlines.  The warps meet
+// only on mbarriers (a column step of a factor, a solved tile, a tile brought
+// up to date), all of one use and waited for in an order without cycles.
+// Every element is one fma chain over the columns in order, whatever the
+// schedule.  The loops stay rolled (register arrays shift by eight columns):
+// instruction fetch, not arithmetic, bounded fully unrolled forms, whose code
+// was refetched in every phase.  One SM's FP32 rate is the floor: 116 K warp
+// fmas, about 41 K cycles at the 0.7 of peak that three-operand fmas reach.
+// 256 x 256: 47 us a launch alone and 53 - 68 us beside a trailing update; one
+// pivot per shared-memory round trip with block barriers between tile solves
+// and updates took 72 us, and 77 - 105 us beside the update.
+constexpr int NPW = 8;          // panel warps: warp w holds tile row w
+constexpr int SUB = 8;          // columns per step of the chain
+constexpr int NSUB = TS / SUB;
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpack2(uint64_t d, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+}
+// two fused multiply-adds in one issue slot, each rounded as fmaf
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// a[0..7] -= x l[0..7], nx2 = (-x, -x), l 16-byte aligned
+__device__ __forceinline__ void axpy8(float* a, uint64_t nx2, const float* l) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(l + 4 * q);
+    unpack2(fma2(nx2, v.x, pack2(a[4 * q], a[4 * q + 1])), a[4 * q], a[4 * q + 1]);
+    unpack2(fma2(nx2, v.y, pack2(a[4 * q + 2], a[4 * q + 3])), a[4 * q + 2], a[4 * q + 3]);
+  }
+}
+
+// What the pivot rule needs of one tile column's rows, and what it found.
+struct PivotRule {
+  const float* shift;     // 32 entries each
+  const float* pmin;
+  const float* thr;       // a finite pivot above thr is taken as it is
+  int nreal, diag_pert;
+};
+struct PivotLog {
+  int fail = -1, npert = 0;
+};
+
+// Eight columns with the pivot rule in full (a pivot at or below its floor, not
+// finite or denormal among them): D the 8 x 8 diagonal block by rows, x the
+// lane's row, i its row in the block.  Uniform over the warp but for x.
+__device__ __noinline__ void rare_block(const float* D, const PivotRule& pr, int c0, int i, float* x,
+                                        float* my_inv, int lane, PivotLog* log) {
+  float d[SUB * SUB];
+  for (int e = 0; e < SUB * SUB; ++e) d[e] = D[e];
+  for (int k = 0; k < SUB; ++k) {
+    const Pivot<float> p = eval_pivot<float>(d[k * SUB + k], c0 + k < pr.nreal, pr.shift[c0 + k],
+                                             pr.pmin[c0 + k], pr.diag_pert);
+    log->npert += p.pert ? 1 : 0;
+    if (p.bad && log->fail < 0) log->fail = c0 + k;
+    if (lane == k) *my_inv = p.r;
+    const float xk = i == k ? p.piv * p.r : x[k] * p.r;
+    x[k] = xk;
+    for (int e = k + 1; e < SUB; ++e) d[e * SUB + k] *= p.r;
+    for (int e = k + 1; e < SUB; ++e)
+      for (int c = k + 1; c <= e; ++c)
+        d[e * SUB + c] = fmaf(-d[e * SUB + k], d[c * SUB + k], d[e * SUB + c]);
+    for (int c = k + 1; c < SUB; ++c) x[c] = fmaf(-xk, d[c * SUB + k], x[c]);
+  }
+}
+
+// The factor of a diagonal tile whose rows the lanes hold in a (column j of the
+// lane's row in a[j]), into t (lower triangle); inv[k] = 1 / L(k,k); sub[s] is
+// arrived at once columns 8 s .. 8 s + 7 are in shared memory.  D: an 8 x 8
+// buffer.
+__device__ __forceinline__ void chain_tile(float (&a)[TS], float* t, float* inv, float* D, int lane,
+                                           const PivotRule& pr, uint64_t* sub, PivotLog& log) {
+  float xp[SUB] = {};                              // the previous eight columns of the row
+#pragma unroll 1
+  for (int s = 0; s < NSUB; ++s) {
+    const int c0 = SUB * s;
+    const int i = lane - c0;                       // row of the diagonal block
+    if (i >= 0 && i < SUB) {
+      *reinterpret_cast<float4*>(D + i * SUB) = make_float4(a[0], a[1], a[2], a[3]);
+      *reinterpret_cast<float4*>(D + i * SUB + 4) = make_float4(a[4], a[5], a[6], a[7]);
+    }
+    __syncwarp();
+    float d[SUB][SUB];
+#pragma unroll
+    for (int r = 0; r < SUB; ++r)
+#pragma unroll
+      for (int q = 0; q <= r / 4; ++q) {
+        const float4 v = *reinterpret_cast<const float4*>(D + r * SUB + 4 * q);
+        d[r][4 * q] = v.x; d[r][4 * q + 1] = v.y; d[r][4 * q + 2] = v.z; d[r][4 * q + 3] = v.w;
+      }
+    float sh[SUB], th[SUB];
+    load_n<SUB>(pr.shift + c0, sh);
+    load_n<SUB>(pr.thr + c0, th);
+    // the columns after the next eight, by the previous eight
+    if (s == 1 || s == 2) {
+      const float* tp = t + (c0 - SUB) * TS + c0 + SUB;
+#pragma unroll
+      for (int m = 0; m < SUB; ++m) axpy8(a + SUB, pack2(-xp[m], -xp[m]), tp + m * TS);
+      if (s == 1) {
+#pragma unroll
+        for (int m = 0; m < SUB; ++m) axpy8(a + 2 * SUB, pack2(-xp[m], -xp[m]), tp + m * TS + SUB);
+      }
+    }
+    float x[SUB], my_inv = 1.0f;
+    bool plain = true;
+#pragma unroll
+    for (int c = 0; c < SUB; ++c) x[c] = a[c];
+#pragma unroll
+    for (int k = 0; k < SUB; ++k) {
+      const float piv = d[k][k] + sh[k];
+      float r;   // rsqrtf's value for every normal argument, at less than half its latency
+      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
+      plain = plain && piv > th[k] && piv <= 3.402823466e38f;
+      my_inv = lane == k ? r : my_inv;
+      x[k] = i == k ? piv * r : x[k] * r;
+#pragma unroll
+      for (int e = k + 1; e < SUB; ++e) d[e][k] *= r;
+#pragma unroll
+      for (int e = k + 1; e < SUB; ++e)
+#pragma unroll
+        for (int c = k + 1; c <= e; ++c) d[e][c] = fmaf(-d[e][k], d[c][k], d[e][c]);
+#pragma unroll
+      for (int c = k + 1; c < SUB; ++c) x[c] = fmaf(-x[k], d[c][k], x[c]);
+    }
+    if (!plain) {
+      float xr[SUB], ir = 1.0f;
+#pragma unroll
+      for (int c = 0; c < SUB; ++c) xr[c] = a[c];
+      rare_block(D, pr, c0, i, xr, &ir, lane, &log);
+#pragma unroll
+      for (int c = 0; c < SUB; ++c) x[c] = xr[c];
+      my_inv = ir;
+    }
+#pragma unroll
+    for (int c = 0; c < SUB; ++c) {
+      if (c <= i) t[(c0 + c) * TS + lane] = x[c];
+      xp[c] = x[c];
+    }
+    if (lane < SUB) inv[c0 + lane] = my_inv;
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&sub[s]);
+    if (s + 1 < NSUB) {
+#pragma unroll
+      for (int m = 0; m < SUB; ++m)
+        axpy8(a + SUB, pack2(-x[m], -x[m]), t + (c0 + m) * TS + c0 + SUB);
+    }
+#pragma unroll
+    for (int j = 0; j < TS - SUB; ++j) a[j] = a[j + SUB];
+  }
+}
+
+// A 32 x 32 tile spread over the warp as 8 x 4 blocks per lane, rows in pairs
+// for packed fmas.  The blocks' numbers interleave the lane's bits so that four
+// neighbouring lanes read two different vectors of each operand: such a
+// 16-byte shared load takes 2.2 cycles of an SM, one with four different
+// vectors 4.0.  The values are kept negated, so that the accumulation adds.
+struct TileAcc {
+  uint64_t v[4][4];                                // [column][row pair]
+};
+__device__ __forceinline__ int blk_row(int lane) { return 8 * ((lane & 1) | ((lane >> 1) & 2)); }
+__device__ __forceinline__ int blk_col(int lane) { return 4 * (((lane >> 1) & 1) | ((lane >> 2) & 6)); }
+constexpr uint64_t kSigns = 0x8000000080000000ull;
+__device__ __forceinline__ void acc_load(TileAcc& c, const float* t, int lane) {
+  t += blk_col(lane) * TS + blk_row(lane);
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(t + u * TS + 4 * q);
+      c.v[u][2 * q] = w.x ^ kSigns;
+      c.v[u][2 * q + 1] = w.y ^ kSigns;
+    }
+}
+__device__ __forceinline__ void acc_store(const TileAcc& c, float* t, int lane) {
+  t += blk_col(lane) * TS + blk_row(lane);
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      ulonglong2 w;
+      w.x = c.v[u][2 * q] ^ kSigns;
+      w.y = c.v[u][2 * q + 1] ^ kSigns;
+      *reinterpret_cast<ulonglong2*>(t + u * TS + 4 * q) = w;
+    }
+}
+// c -= A B^T over columns [k0, k1) (a multiple of 8) of the tiles a and b
+__device__ __forceinline__ void acc_product(TileAcc& c, const float* a, const float* b, int lane, int k0,
+                                            int k1) {
+  a += blk_row(lane);
+  b += blk_col(lane);
+#pragma unroll 8
+  for (int k = k0; k < k1; ++k) {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(a + k * TS);
+    const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(a + k * TS + 4);
+    const uint64_t av[4] = {a0.x, a0.y, a1.x, a1.y};
+    float bv[4];
+    load_n<4>(b + k * TS, bv);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint64_t bb = pack2(bv[u], bv[u]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) c.v[u][i] = fma2(av[i], bb, c.v[u][i]);
+    }
+  }
+}
+
+// X L^T = A for the tile whose rows the lanes hold in a, below diagonal tile l,
+// eight columns behind its factor (sub as above), into x.  crit: dg, this
+// row's diagonal tile, receives -X X^T on the way.
+// Returns false if a bounded wait gave up.
+__device__ __forceinline__ bool follow_tile(float (&a)[TS], float* x, const float* l, const float* inv,
+                                            int lane, uint64_t* sub, bool crit, TileAcc& dg) {
+  bool ok = true;
+#pragma unroll 1
+  for (int s = 0; s < NSUB; ++s) {
+    const int c0 = SUB * s;
+    ok = tc::mbar_wait(&sub[s], 0) && ok;
+    const float* lb = l + c0 * TS + c0;            // L(c0 + c, c0 + m) at m * 32 + c
+    float iv[SUB];
+    load_n<SUB>(inv + c0, iv);
+#pragma unroll
+    for (int m = 0; m < SUB; ++m) {
+      float lm[SUB];
+      load_n<SUB>(lb + m * TS, lm);
+      a[m] *= iv[m];
+#pragma unroll
+      for (int c = m + 1; c < SUB; ++c) a[c] = fmaf(-a[m], lm[c], a[c]);
+    }
+#pragma unroll
+    for (int m = 0; m < SUB; ++m) x[(c0 + m) * TS + lane] = a[m];
+#pragma unroll
+    for (int g = 1; g < NSUB; ++g) {
+      if (s + g < NSUB) {
+#pragma unroll
+        for (int m = 0; m < SUB; ++m) axpy8(a + SUB * g, pack2(-a[m], -a[m]), lb + m * TS + SUB * g);
+      }
+    }
+    if (crit) {
+      __syncwarp();
+      acc_product(dg, x, x, lane, c0, c0 + SUB);
+    }
+#pragma unroll
+    for (int j = 0; j < TS - SUB; ++j) a[j] = a[j + SUB];
+  }
+  return ok;
+}
+
+// Tile t of the lower ones (at most NPW rows of them), numbered by rows.
+__device__ __forceinline__ void tile_of(int t, int& I, int& J) {
+  I = 0;
+#pragma unroll
+  for (int r = 1; r < NPW; ++r) I += t >= r * (r + 1) / 2 ? 1 : 0;
+  J = t - I * (I + 1) / 2;
+}
+// The block's lower tiles from global memory and back.  Whole tiles whose
+// columns start on 16-byte boundaries move as 16-byte vectors, eight lanes to
+// a column of 32 rows, nine loads in flight per thread (36 boxes by TMA take
+// one thread's issue about 80 cycles each); anything else element by element,
+// identity past the block.  The strictly upper part of a diagonal tile is
+// left alone in global memory.
+__device__ __forceinline__ void load_tiles(float* tiles, const float* A, int lda, int bs, int ntiles,
+                                           bool vec, int tid) {
+  if (vec) {
+    const int r4 = 4 * (tid & 7), c = (tid & 255) >> 3;
+    for (int t0 = tid >> 8; t0 < ntiles; t0 += 18) {
+      float4 v[9];
+#pragma unroll
+      for (int u = 0; u < 9; ++u)
+        if (t0 + 2 * u < ntiles) {
+          int I, J;
+          tile_of(t0 + 2 * u, I, J);
+          v[u] = *reinterpret_cast<const float4*>(A + (size_t)(J * TS + c) * lda + I * TS + r4);
+        }
+#pragma unroll
+      for (int u = 0; u < 9; ++u)
+        if (t0 + 2 * u < ntiles) *reinterpret_cast<float4*>(tiles + (t0 + 2 * u) * TSZ + c * TS + r4) = v[u];
+    }
+  } else {
+#pragma unroll 4
+    for (int e = tid; e < ntiles * TSZ; e += 512) {
+      int I, J;
+      tile_of(e / TSZ, I, J);
+      const int r = I * TS + e % TS, c = J * TS + e % TSZ / TS;
+      tiles[e] = r < bs && c < bs ? A[(size_t)c * lda + r] : (r == c ? 1.0f : 0.0f);
+    }
+  }
+}
+__device__ __forceinline__ void store_tiles(const float* tiles, float* A, int lda, int bs, int ntiles,
+                                            bool vec, int tid) {
+  if (vec) {
+    const int r4 = 4 * (tid & 7), c = (tid & 255) >> 3;
+#pragma unroll 2
+    for (int t = tid >> 8; t < ntiles; t += 2) {
+      int I, J;
+      tile_of(t, I, J);
+      const float4 v = *reinterpret_cast<const float4*>(tiles + t * TSZ + c * TS + r4);
+      float* g = A + (size_t)(J * TS + c) * lda + I * TS + r4;
+      if (I > J || r4 >= c) {
+        *reinterpret_cast<float4*>(g) = v;
+      } else if (r4 + 3 >= c) {                      // the vector the diagonal crosses
+        if (r4 + 1 >= c) g[1] = v.y;
+        if (r4 + 2 >= c) g[2] = v.z;
+        g[3] = v.w;
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int e = tid; e < ntiles * TSZ; e += 512) {
+      int I, J;
+      tile_of(e / TSZ, I, J);
+      const int r = I * TS + e % TS, c = J * TS + e % TSZ / TS;
+      if (r < bs && c < bs && r >= c) A[(size_t)c * lda + r] = tiles[e];
+    }
+  }
+}
+
+__device__ __forceinline__ void
+potrf_f32_block(float* tiles, float* A, int lda, int s, int bs, const float* d, float* sh,
+                const PotrfParams& p, const int* fp64_flag, float* winv, DevStatus* st,
+                const StepState* prev, const float* rowsq) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  const int NT = (bs + TS - 1) / TS;
+  const int ntiles = NT * (NT + 1) / 2;
+  __shared__ __align__(16) float s_shift[256];
+  __shared__ __align__(16) float s_pmin[256];
+  __shared__ __align__(16) float s_thr[256];
+  __shared__ __align__(16) float s_inv[256];
+  __shared__ __align__(16) float s_D[NPW][SUB * SUB];
+  __shared__ int s_fail, s_pert, s_ok;
+  // sub: column steps of the factors; done: solved tiles; fresh: tiles brought
+  // up to date by the helpers
+  __shared__ __align__(8) uint64_t sub[NPW * NSUB], done[NPW * (NPW + 1) / 2],
+      fresh[NPW * (NPW + 1) / 2];
+  float* const Ab = A + (size_t)s * lda + s;
+  const bool vec = (reinterpret_cast<uintptr_t>(Ab) & 15) == 0 && lda % 4 == 0 && bs % TS == 0;
+  if (tid >= 32 && tid < 32 + NPW * (NPW + 1) / 2) {
+    if (tid - 32 < NPW * NSUB) tc::mbar_init(&sub[tid - 32], 1);
+    tc::mbar_init(&done[tid - 32], 1);
+    tc::mbar_init(&fresh[tid - 32], 1);
+    tc::fence_mbar_init();
+  }
+  if (tid == 96) {
+    s_fail = NPW * TS;       // none
+    s_pert = 0;
+    s_ok = st->code == 0 && (fp64_flag == nullptr || *fp64_flag == 0);
+  }
+  const int prev_prec = (prev != nullptr && p.diag_pert && sh) ? prev->prec : FP32;
+  for (int i = tid; i < NT * TS; i += blockDim.x) {
+    // rows past the block are identity: their pivots are 1
+    float shv = 0.0f, pm = 0.0f, th = 1.175494351e-38f;
+    if (i < bs) {
+      if (p.diag_pert && sh) {
+        float shf = sh[s + i];
+        if (prev_prec != FP32)   // the previous step's shift for this row
+          shf = __fmaf_rn(unit_roundoff(prev_prec), rowsq[s + i], shf);
+        s_inv[i] = shf;          // stored once the block is known to be this kernel's
+        shv = p.pert * shf;
+      }
+      pm = p.pivot_floor * d[s + i];
+      // NaN bounds take every pivot to the full rule
+      if (p.diag_pert && !(pm < th)) th = pm >= th ? pm : 3.402823466e38f;
+    }
+    s_shift[i] = shv;
+    s_pmin[i] = pm;
+    s_thr[i] = th;
+  }
+  load_tiles(tiles, Ab, lda, bs, ntiles, vec, tid);
+  __syncthreads();
+  if (!s_ok) return;
+  if (p.diag_pert && sh && prev_prec != FP32)
+    for (int i = tid; i < bs; i += blockDim.x) sh[s + i] = s_inv[i];
+  __syncthreads();
+  bool ok = true;
+  if (warp < NT) {
+    const int I = warp;
+    float a[TS];
+    TileAcc acc;
+    float* const mine = tiles + tidx(I, I) * TSZ;
+#pragma unroll 1
+    for (int J = 0; J < I; ++J) {
+      float* x = tiles + tidx(I, J) * TSZ;
+      if (J >= 1) {
+        if (J >= 2) ok = tc::mbar_wait(&fresh[tidx(I, J)], 0) && ok;
+        ok = tc::mbar_wait(&done[tidx(J, J - 1)], 0) && ok;
+        acc_load(acc, x, lane);
+        acc_product(acc, tiles + tidx(I, J - 1) * TSZ, tiles + tidx(J, J - 1) * TSZ, lane, 0, TS);
+        acc_store(acc, x, lane);
+        __syncwarp();
+      }
+#pragma unroll
+      for (int j = 0; j < TS; ++j) a[j] = x[j * TS + lane];
+      const bool crit = J == I - 1;
+      if (crit) {
+        if (I >= 2) ok = tc::mbar_wait(&fresh[tidx(I, I)], 0) && ok;
+        acc_load(acc, mine, lane);
+      }
+      ok = follow_tile(a, x, tiles + tidx(J, J) * TSZ, s_inv + J * TS, lane, sub + J * NSUB, crit, acc) && ok;
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&done[tidx(I, J)]);
+    }
+    if (I > 0) acc_store(acc, mine, lane);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < TS; ++j) a[j] = mine[j * TS + lane];
+    PivotLog log;
+    const PivotRule pr{s_shift + I * TS, s_pmin + I * TS, s_thr + I * TS, min(TS, bs - I * TS), p.diag_pert};
+    chain_tile(a, mine, s_inv + I * TS, s_D[I], lane, pr, sub + I * NSUB, log);
+    if (lane == 0) {
+      if (log.fail >= 0) atomicMin(&s_fail, I * TS + log.fail);
+      if (log.npert) atomicAdd(&s_pert, log.npert);
+    }
+    // the inverse for the panel solve, where the SM has issue slots to spare;
+    // the first tiles' and the last one's wait for the end
+    if (I >= 2 && I < NT - 1)
+      invert_tile<float, SUB>(mine, s_inv + I * TS, winv + I * TS * TS, lane);
+  } else {
+    // tile (I, K), K >= 2, by columns 0 .. K - 2, in column order over all
+    // helpers: a task waits only for tiles that need tasks of earlier columns
+    const int nhelp = nwarps - NT;
+    int task = 0;
+    for (int K = 2; K < NT; ++K)
+      for (int I = K; I < NT; ++I, ++task) {
+        if (task % nhelp != warp - NT) continue;
+        TileAcc acc;
+        acc_load(acc, tiles + tidx(I, K) * TSZ, lane);
+#pragma unroll 1
+        for (int j = 0; j < K - 1; ++j) {
+          ok = tc::mbar_wait(&done[tidx(K, j)], 0) && ok;
+          ok = tc::mbar_wait(&done[tidx(I, j)], 0) && ok;
+          acc_product(acc, tiles + tidx(I, j) * TSZ, tiles + tidx(K, j) * TSZ, lane, 0, TS);
+        }
+        acc_store(acc, tiles + tidx(I, K) * TSZ, lane);
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&fresh[tidx(I, K)]);
+      }
+  }
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0) set_status(st, MPCHOL_ERR_TIMEOUT, s);
+    return;
+  }
+  if (s_fail < NT * TS) {
+    if (tid == 0) set_status(st, MPCHOL_ERR_NOT_SPD, s + s_fail);
+    return;
+  }
+  store_tiles(tiles, Ab, lda, bs, ntiles, vec, tid);
+  if (warp < 2 ? warp < NT : warp == NT - 1)
+    invert_tile<float, SUB>(tiles + tidx(warp, warp) * TSZ, s_inv + warp * TS, winv + warp * TS * TS, lane);
+  if (tid == 0 && s_pert) atomicAdd(&st->perturbed, s_pert);
+}
+
+// Separate kernels for the two precisions keep the FP64 register footprint out
+// of the FP32 path.
 __global__ void __launch_bounds__(512, 1)
-potrf_f32_kernel(const __grid_constant__ CUtensorMap tmap, float* A, int lda, int n, int s, int bs,
+potrf_f32_kernel(float* A, int lda, int s, int bs,
                  const float* d, float* sh, PotrfParams p, const int* fp64_flag, float* winv,
                  DevStatus* st, const StepState* prev, const float* rowsq) {
   tc::grid_dep_wait();      // the block's update and the step state are final
   tc::grid_dep_trigger();   // the next kernel may be scheduled (it waits too)
-  if (st->code != 0) return;
-  if (fp64_flag != nullptr && *fp64_flag != 0) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  potrf_block<float, true, CB>(&tmap, reinterpret_cast<float*>(smem_raw), A, lda, n, s, bs, d, sh, p,
-                           winv, st, prev, rowsq);
+  potrf_f32_block(reinterpret_cast<float*>(smem_raw), A, lda, s, bs, d, sh, p, fp64_flag, winv, st, prev,
+                  rowsq);
 }
 
-// Batched: CTA i factors the current diagonal block of system i (tiles in
-// shared memory, staged with plain coalesced loads: one tensor map per
-// system would not fit the launch).
+// Batched: CTA i factors the current diagonal block of system i.
 __global__ void __launch_bounds__(512, 1)
 potrf_batched_kernel(BatchSys* __restrict__ sys, int s, int b, PotrfParams p) {
   const BatchSys& S = sys[blockIdx.x];
   const int bs = min(b, S.n - s);
   if (bs <= 0 || S.st->code != 0) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  potrf_block<float, false, TS>(nullptr, reinterpret_cast<float*>(smem_raw), S.A, S.ld, S.n, s, bs,
-                            S.d, S.sh, p, S.winv, S.st);
+  potrf_f32_block(reinterpret_cast<float*>(smem_raw), S.A, S.ld, s, bs, S.d, S.sh, p, nullptr, S.winv,
+                  S.st, nullptr, nullptr);
 }
 
 // FP64 blocks (flagged near-indefinite): tiles in a global scratch.
 __global__ void __launch_bounds__(256, 1)
-potrf_f64_kernel(float* A, int lda, int n, int s, int bs, const float* d, float* sh,
+potrf_f64_kernel(float* A, int lda, int s, int bs, const float* d, float* sh,
                  PotrfParams p, const int* fp64_flag, double* scratch64, float* winv, DevStatus* st,
                  const StepState* prev, const float* rowsq) {
   if (st->code != 0) return;
   if (fp64_flag == nullptr || *fp64_flag == 0) return;
-  potrf_block<double, false, 8>(nullptr, scratch64, A, lda, n, s, bs, d, sh, p, winv, st, prev, rowsq);
+  potrf_block<double, 8>(scratch64, A, lda, s, bs, d, sh, p, winv, st, prev, rowsq);
 }
 
 }  // namespace
@@ -525,27 +940,22 @@ size_t potrf_scratch64_elems(int bs) {
 }
 size_t potrf_smem_bytes(int bs) { return potrf_scratch64_elems(bs) * sizeof(float); }
 
-cudaError_t launch_potrf(const CUtensorMap& tmap32, float* A, int lda, int n, int s, int bs,
+cudaError_t launch_potrf(float* A, int lda, int s, int bs,
                          const float* d, float* sh, const PotrfParams& p,
                          const int* fp64_flag, double* scratch64, float* winv, DevStatus* st,
                          bool may_fp64, cudaStream_t stream, const StepState* prev,
-                         const float* rowsq, bool compact) {
+                         const float* rowsq) {
   const size_t smem = potrf_smem_bytes(256);
-  cudaError_t e = cudaFuncSetAttribute(potrf_f32_kernel<4>,
+  cudaError_t e = cudaFuncSetAttribute(potrf_f32_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(potrf_f32_kernel<TS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
   if (e != cudaSuccess) return e;
   PdlLaunch L(dim3(1), dim3(512), smem, stream);
   const int* flag = may_fp64 ? fp64_flag : nullptr;
-  e = compact ? cudaLaunchKernelEx(&L.cfg, potrf_f32_kernel<4>, tmap32, A, lda, n, s, bs, d, sh, p,
-                                   flag, winv, st, prev, rowsq)
-              : cudaLaunchKernelEx(&L.cfg, potrf_f32_kernel<TS>, tmap32, A, lda, n, s, bs, d, sh, p,
-                                   flag, winv, st, prev, rowsq);
+  e = cudaLaunchKernelEx(&L.cfg, potrf_f32_kernel, A, lda, s, bs, d, sh, p, flag, winv, st,
+                         prev, rowsq);
   if (e != cudaSuccess) return e;
   if (may_fp64)
-    potrf_f64_kernel<<<1, 256, 0, stream>>>(A, lda, n, s, bs, d, sh, p, fp64_flag, scratch64, winv, st,
+    potrf_f64_kernel<<<1, 256, 0, stream>>>(A, lda, s, bs, d, sh, p, fp64_flag, scratch64, winv, st,
                                             prev, rowsq);
   return cudaGetLastError();
 }

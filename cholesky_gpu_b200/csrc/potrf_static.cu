@@ -22,7 +22,6 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "pcg.cuh"
-#include "tmap.cuh"
 
 using namespace mpchol;
 
@@ -65,7 +64,7 @@ extern "C" MPCHOL_API mpchol_status mpchol_potrf_static(float* dA, int lda, int 
   if (dA == nullptr || dInfo == nullptr) return MPCHOL_ERR_BAD_ARG;
   if (n < 1 || n > kMaxBlock || lda < n) return MPCHOL_ERR_BAD_ARG;
   if (!(pivot_floor >= 0.0f)) return MPCHOL_ERR_BAD_ARG;
-  // TMA needs the matrix base and its column stride on 16-byte boundaries
+  // documented requirement: the matrix base and its column stride on 16-byte boundaries
   if ((reinterpret_cast<uintptr_t>(dA) & 15) != 0 || (lda % 4) != 0) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   int dev = 0;
@@ -83,14 +82,10 @@ extern "C" MPCHOL_API mpchol_status mpchol_potrf_static(float* dA, int lda, int 
     return MPCHOL_ERR_CUDA;
   }
   StaticScratch* sc = slot.addr;
-  CUtensorMap tmap;
-  if (!encode_tmap_2d(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dA, n, n, lda, 32, 32,
-                      CU_TENSOR_MAP_SWIZZLE_NONE))
-    return MPCHOL_ERR_CUDA;
   MPCHOL_CUDA_TRY(cudaMemsetAsync(&sc->status, 0, sizeof(DevStatus), stream));
   MPCHOL_CUDA_TRY(launch_extract_diag(dA, lda, n, sc->diag, sc->diag_copy, stream));
   const PotrfParams pp{pivot_floor > 0.0f ? 1 : 0, 0.0f, pivot_floor};
-  MPCHOL_CUDA_TRY(launch_potrf(tmap, dA, lda, n, 0, n, sc->diag, nullptr, pp, nullptr, nullptr,
+  MPCHOL_CUDA_TRY(launch_potrf(dA, lda, 0, n, sc->diag, nullptr, pp, nullptr, nullptr,
                                sc->winv, &sc->status, false, stream));
   potrf_static_info_kernel<<<1, 1, 0, stream>>>(&sc->status, dInfo);
   MPCHOL_CUDA_TRY(cudaGetLastError());

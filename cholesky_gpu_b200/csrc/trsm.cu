@@ -65,9 +65,6 @@ size_t trsm_smem_floats(int tr, int bs) {
 __device__ __forceinline__ void pair_sync(int J) {   // the two warps of tile column J
   asm volatile("bar.sync %0, 64;" ::"r"(J + 1) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
-}
 
 // The slab solve.  The warp pair of tile column J (warps 2J, 2J + 1; w = 2J +
 // h) computes the TR x 32 tile X_J: thread t of the pair (t = 32 h + lane)
@@ -162,7 +159,7 @@ __device__ bool slab_solve(float* Xs, int bs, const float* Lt, const float* Wt, 
     for (int j = 0; j < 4; ++j)
       *reinterpret_cast<float4*>(xj + q * XH + (cl + j) * 32) =
           make_float4(acc[q][0][j], acc[q][1][j], acc[q][2][j], acc[q][3][j]);
-  mbar_arrive(&ready[J]);                              // release: X_J to the later tiles
+  tc::mbar_arrive(&ready[J]);                              // release: X_J to the later tiles
   return ok;
 }
 

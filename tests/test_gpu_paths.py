@@ -114,3 +114,38 @@ def test_rbf_grad_contraction_at_row_tile_edges(n, d):
     ws = (a @ ((K * r2) @ b)).item()
     scale = (a.abs() @ ((K * r2) @ b.abs())).item()
     assert abs(s.item() - ws) <= 1e-13 * max(scale, 1e-300)
+
+
+@pytest.mark.parametrize("n", [1, 8, 31, 32, 40, 63, 64, 95, 128, 160, 200, 224, 255, 256])
+def test_diagonal_factor_at_tile_edges(n):
+    """One diagonal block of every tile count, ragged and whole, against FP64
+    (kappa = 1e2: FP32 Cholesky is within n * 2^-24 * kappa^0.5 of it), with
+    pivots that need no repair."""
+    A = matgen.spd_matrix(n, 1e2, 3 * n) if n > 1 else torch.full((1, 1), 4.0)
+    f = mp.factor(A.cuda(), block_size=256, precision="fp32")
+    assert f.info().n_perturbed == 0
+    L = np.linalg.cholesky(A.double().numpy())
+    assert np.linalg.norm(f.lower().cpu().numpy() - L) / np.linalg.norm(L) < 1e-5
+
+
+@pytest.mark.parametrize("row,value", [(0, -1.0), (7, 0.0), (8, 1e-40), (37, -2.0), (100, float("nan")),
+                                       (255, float("inf"))])
+def test_diagonal_factor_takes_the_full_pivot_rule_for_rare_pivots(row, value):
+    """A pivot at or below its floor is repaired to max(|pivot|, floor) and
+    counted; one that is not finite fails at its row.  The matrix is diagonal,
+    so every pivot is known exactly."""
+    d = torch.linspace(1.0, 2.0, 256)
+    d[row] = value
+    f = mp.factor(torch.diag(d).cuda(), block_size=256, precision="fp32", pert=0.0)
+    info = f.info()
+    if not np.isfinite(value):
+        assert info.status != 0 and info.fail_row == row
+        return
+    assert info.status == 0 and info.n_perturbed == (0 if value > 0 else 1)
+    # 1 / sqrt times the repaired pivot; a zero pivot has a zero floor here, and
+    # 0 * (1 / sqrt(0)) is not a number
+    stored = d.double().numpy()
+    piv = np.where(np.arange(256) == row, np.maximum(np.abs(stored), 1e-7 * stored), stored)
+    want = np.where(piv > 0, np.sqrt(piv), np.nan)
+    got = torch.diagonal(f.lower()).cpu().numpy()
+    assert np.allclose(got, want, rtol=1e-6, atol=0.0, equal_nan=True)
