@@ -148,3 +148,28 @@ def test_diagonal_factor_takes_the_full_pivot_rule_for_rare_pivots(row, value):
     want = np.sqrt(np.where(np.arange(256) == row, np.maximum(np.abs(stored), 1e-7 * stored), stored))
     got = torch.diagonal(f.lower()).cpu().numpy()
     assert np.allclose(got, want, rtol=1e-6, atol=0.0)
+
+
+@pytest.mark.parametrize("m,k,pad", [(1, 32, 0), (33, 64, 3), (127, 40, 0), (128, 256, 1), (129, 96, 4),
+                                     (640, 256, 0), (1920, 17, 0), (2049, 32, 3), (2300, 256, 0)])
+def test_fp32_trailing_update_sizes(m, k, pad):
+    """Every kernel of the FP32 update (32-tiles, 128-tiles), ragged sizes and
+    unaligned panels, against FP64: sums of k products of N(0,1) values in
+    FP32, relative error of the update's norm below k * 2^-24."""
+    import ctypes  # noqa: F401
+    from cholesky_gpu_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    ld = m + pad
+    P = torch.randn((k, ld), generator=g, device="cuda")       # column-major m x k, stride ld
+    C = torch.randn((m, ld), generator=g, device="cuda")
+    before = C.clone()
+    _lib.check(_lib.load().mpchol_syrk_update(C.data_ptr(), ld, m, k, _lib.PREC_FP32, None, None,
+                                              P.data_ptr(), ld, torch.cuda.current_stream().cuda_stream))
+    Pd = P[:, :m].double().t()
+    want = Pd @ Pd.t()
+    got = (before - C)[:, :m].t().double()
+    low = torch.ones((m, m), dtype=torch.bool, device="cuda").tril()
+    assert ((got - want)[low].norm() / want[low].norm()).item() < max(k, 8) * 2.0 ** -24 + 2.0 ** -23
+    C2 = C.clone()
+    C2[:, :m].t()[low] = before[:, :m].t()[low]
+    assert torch.equal(C2, before)                              # nothing else is touched
