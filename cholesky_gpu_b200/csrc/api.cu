@@ -151,12 +151,16 @@ struct PcgGraph {
 // an allocation of the library fails, or when newer ones take their room.
 // Create + destroy at n = 3072: 3.6 ms with one allocation per buffer, 0.70
 // with one for all.
+// The scalar block of a factor object (doubles): misc at 0, ||b||^2 at 32, rho
+// at 40, the factor's and the solve's status at 56, done and loop control at 60.
+constexpr int kScalBnorm = 32, kScalRho = 40, kScalStatus = 56, kScalDone = 60, kScalDoubles = 64;
+static_assert(sizeof(DevStatus) == 16, "two status words take four doubles");
+
 struct Resources {
   int device = -1;
   char* arena = nullptr;
   size_t bytes = 0;
-  int* h_done = nullptr;      // pinned
-  double* h_scal = nullptr;   // pinned
+  double* h_scal = nullptr;   // pinned, kScalDoubles
   // look-ahead: the bulk of each step's trailing update runs on aux while the
   // next diagonal block is factored on the caller's stream; capture_stream is
   // used only to capture graphs
@@ -172,7 +176,6 @@ std::vector<Resources> g_cache;   // oldest first
 
 void free_resources(Resources& r) {
   if (r.arena) cudaFree(r.arena);
-  if (r.h_done) cudaFreeHost(r.h_done);
   if (r.h_scal) cudaFreeHost(r.h_scal);
   if (r.aux) cudaStreamDestroy(r.aux);
   if (r.capture_stream) cudaStreamDestroy(r.capture_stream);
@@ -213,8 +216,7 @@ bool acquire_resources(int device, size_t bytes, Resources* out) {
   r.device = device;
   r.bytes = bytes;
   bool ok = lib_malloc(reinterpret_cast<void**>(&r.arena), bytes) == cudaSuccess;
-  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&r.h_done), 2 * sizeof(int)) == cudaSuccess &&
-       cudaMallocHost(reinterpret_cast<void**>(&r.h_scal), sizeof(double) * 64) == cudaSuccess &&
+  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&r.h_scal), sizeof(double) * kScalDoubles) == cudaSuccess &&
        cudaStreamCreateWithFlags(&r.aux, cudaStreamNonBlocking) == cudaSuccess &&
        cudaStreamCreateWithFlags(&r.capture_stream, cudaStreamNonBlocking) == cudaSuccess;
   for (cudaEvent_t* e : {&r.ev_next, &r.ev_rest, &r.ev_catch})
@@ -311,8 +313,10 @@ struct mpchol_factor {
   bool solve_ready = false;
   // PCG workspace (sized for 8 rhs)
   double* vec = nullptr;      // x, r, z, p, Ap, b, tmp, work : 8 * n * 8
-  double* partials = nullptr; // 4 * VG * 8
-  double* scal = nullptr;     // rho[2][8], alpha[8], bnorm2[8], misc
+  double* partials = nullptr; // 6 * VG * 8
+  // one block that a solve reads back at once (kScalDoubles): misc[32],
+  // bnorm2[8], rho[2][8], both status words, done, the loop's control words
+  double* scal = nullptr;
   int* done = nullptr;        // [0] converged flag, [1] iteration counter
   PcgGraph graph;             // captured PCG loop (see run_pcg)
   FactorGraph fgraph;         // captured factorization (see launch_factor)
@@ -881,23 +885,16 @@ mpchol_status ensure_solve(mpchol_factor_t* f, cudaStream_t stream) {
   return MPCHOL_OK;
 }
 
-// kernels per triangular solve: the input preparation, the persistent solve
-int trsv_launch_count(int n) {
-  (void)n;
-  return 2;
-}
-
-// z = M^-1 r for NR-padded vectors (tmp, work: n x nr scratch)
-mpchol_status apply_precond(mpchol_factor_t* f, const double* r, double* tmp, double* z, int nr,
-                            const int* skip, cudaStream_t stream) {
-  double* work = f->vec + 7 * (size_t)f->n * 8;
-  const int nk = trsv_launch_count(f->n);
-  PHASE(MPCHOL_PH_TRSV, nk, stream,
-        launch_trsv_persistent(false, f->A, f->ld, f->n, f->wsup, r, tmp, work, nr, f->trsv_ctr,
-                               skip, f->pstatus, stream));
-  PHASE(MPCHOL_PH_TRSV, nk, stream,
-        launch_trsv_persistent(true, f->A, f->ld, f->n, f->wsup, tmp, z, work, nr, f->trsv_ctr,
-                               skip, f->pstatus, stream));
+// out = M^-1 w: the forward and the backward solve; w and mid are consumed (see
+// launch_trsv_persistent for what is zero on entry).
+mpchol_status apply_precond(mpchol_factor_t* f, double* w, double* mid, double* out, int nr, const int* skip,
+                            cudaStream_t stream) {
+  PHASE(MPCHOL_PH_TRSV, 1, stream,
+        launch_trsv_persistent(false, f->A, f->ld, f->n, f->wsup, w, mid, nr, f->trsv_ctr, skip, f->pstatus,
+                               stream));
+  PHASE(MPCHOL_PH_TRSV, 1, stream,
+        launch_trsv_persistent(true, f->A, f->ld, f->n, f->wsup, mid, out, nr,
+                               f->trsv_ctr + trsv_counter_ints(f->n), skip, f->pstatus, stream));
   return MPCHOL_OK;
 }
 
@@ -922,221 +919,205 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
   const int n = f->n;
   const int nr = pcg_padded_nrhs(nrhs);
   const size_t nv = (size_t)n * 8;
-  double* x = f->vec;
-  double* r = x + nv;
-  double* z = r + nv;
-  double* p = z + nv;
-  double* Ap = p + nv;
-  double* bb = Ap + nv;
-  double* tmp = bb + nv;
-  const int VG = pcg_vgrid();
-  double* part_pAp = f->partials;
-  double* part_rr = part_pAp + (size_t)VG * 8;
-  double* part_rz = part_rr + (size_t)VG * 8;
-  double* part_misc = part_rz + (size_t)VG * 8;
-  // shares of ||A||_F^2 (for the backward error), filled by the first
-  // operator product when it streams A through the staged kernel
-  double* part_fro = part_misc + (size_t)VG * 8;
-  const bool fro_fused = symv_staged_ok(dA, lda);
-  double* rho[2] = {f->scal, f->scal + 8};
-  double* alpha = f->scal + 16;
-  double* bnorm2 = f->scal + 24;
-  double* misc = f->scal + 32;   // [0..7] rr true, [8..15] xnorm2, [16] frob2
+  const size_t np = (size_t)pcg_vgrid() * 8;
+  PcgVectors v;
+  v.n = n;
+  v.nr = nr;
+  v.x = f->vec;
+  v.r = v.x + nv;
+  v.z = v.r + nv;
+  v.p = v.z + nv;
+  v.Ap = v.p + nv;
+  v.b = v.Ap + nv;
+  v.tmp = v.b + nv;
+  v.work = v.tmp + nv;
+  v.part_pAp = f->partials;
+  v.part_rr = v.part_pAp + np;
+  v.part_rz = v.part_rr + np;
+  v.part_xx = v.part_rz + np;
+  v.part_bb = v.part_xx + np;
+  // shares of ||A||_F^2 (for the backward error): from the first operator
+  // product when that streams A through the staged kernel
+  v.part_fro = v.part_bb + np;
+  v.misc = f->scal;
+  v.bnorm2 = f->scal + kScalBnorm;
+  v.rho = f->scal + kScalRho;
+  v.done = f->done;
+  v.ctl = f->loop_ctl;
+  v.ctr = f->trsv_ctr;
+  v.nctr = 2 * (int)trsv_counter_ints(n);
+  v.status = f->pstatus;
+  constexpr bool fro_fused = sizeof(TA) == 4;
   mpchol_status ss = ensure_solve(f, stream);
   if (ss != MPCHOL_OK) return ss;
-  MPCHOL_CUDA_TRY(cudaMemsetAsync(f->pstatus, 0, sizeof(DevStatus), stream));
-  MPCHOL_CUDA_TRY(cudaMemsetAsync(f->done, 0, 2 * sizeof(int), stream));
-  PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_pad_columns(dB, n, nrhs, bb, nr, stream));
-  PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_dot(bb, bb, n, nr, part_misc, nullptr, stream));
-  PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_misc, bnorm2, nr, stream));
-  // x0
+  PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_pcg_begin(v, dB, nrhs, po.x0_precond != 0, stream));
   if (po.x0_precond) {
-    mpchol_status s0 = apply_precond(f, bb, tmp, x, nr, nullptr, stream);
+    mpchol_status s0 = apply_precond(f, v.work, v.tmp, v.x, nr, nullptr, stream);
     if (s0 != MPCHOL_OK) return s0;
-  } else {
-    MPCHOL_CUDA_TRY(cudaMemsetAsync(x, 0, sizeof(double) * (size_t)n * nr, stream));
   }
   const double tol2 = po.rel_tol * po.rel_tol;
-  int it = 0;         // iterations executed on the device
-  int launched = 0;   // iterations counted against max_it
+  int it = 0;                 // iterations executed on the device
   bool converged = false;
   const int max_restarts = 3;
-  for (int restart = 0;; ++restart) {
-    // r = b - A x ; z = M^-1 r ; p = z ; rho = r^T z
-    PHASE(MPCHOL_PH_SYMV, 1, stream, launch_symv_skip<TA>(dA, lda, n, x, Ap, nr, nullptr, stream,
-                                                          fro_fused ? part_fro : nullptr, VG));
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_residual(bb, Ap, r, n, nr, part_rr, stream));
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_rr, misc, nr, stream));
-    // convergence of the true residual
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal, misc, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal + 8, bnorm2, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
-    // the factorization's status rides along with the first check: a failed
-    // factor (NOT_SPD, TIMEOUT) is not iterated with
-    if (restart == 0)
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal + 48, f->status, sizeof(DevStatus),
-                                      cudaMemcpyDeviceToHost, stream));
+  DevStatus st{};
+  // r = b - A x, its norms and x's, the device's own verdict on the tolerance,
+  // and the inputs of z = M^-1 r
+  auto true_residual = [&](bool first) -> mpchol_status {
+    double* fro = first && fro_fused ? v.part_fro : nullptr;
+    PHASE(MPCHOL_PH_SYMV, 1, stream,
+          launch_symv_skip<TA>(dA, lda, n, v.x, v.Ap, nr, nullptr, stream, fro, pcg_vgrid()));
+    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_residual(v, stream));
+    if (first && !fro_fused && rep != nullptr)
+      PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_frob_lower<TA>(dA, lda, n, v.part_fro, stream));
+    const bool have_fro = first && (fro_fused || rep != nullptr);
+    PHASE(MPCHOL_PH_PCG_VEC, 1, stream,
+          launch_residual_reduce(v, first, have_fro, tol2, f->status, stream));
+    return MPCHOL_OK;
+  };
+  // the scalar block, once the stream has got here
+  auto read_back = [&]() -> mpchol_status {
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal, f->scal, sizeof(double) * kScalDoubles,
+                                    cudaMemcpyDeviceToHost, stream));
     MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
-    if (restart == 0) {
-      DevStatus fst;
-      memcpy(&fst, f->res.h_scal + 48, sizeof(DevStatus));
-      if (fst.code != 0) {
-        if (rep != nullptr) memset(rep, 0, sizeof(*rep));
-        return (mpchol_status)fst.code;
+    memcpy(&st, f->res.h_scal + kScalStatus + 2, sizeof(DevStatus));
+    int dn[2];
+    memcpy(dn, f->res.h_scal + kScalDone, sizeof(dn));
+    it = dn[1];
+    return MPCHOL_OK;
+  };
+  // One PCG iteration.  Every kernel returns at once after *done is set.
+  auto iteration = [&](const cudaGraphConditionalHandle* loop, cudaStream_t s) -> mpchol_status {
+    PHASE(MPCHOL_PH_SYMV, 1, s, launch_symv_skip<TA>(dA, lda, n, v.p, v.Ap, nr, v.done, s));
+    PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_dot_pAp(v, s));
+    PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_update_xr(v, s));
+    mpchol_status s2 = apply_precond(f, v.work, v.tmp, v.z, nr, v.done, s);
+    if (s2 != MPCHOL_OK) return s2;
+    PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_dot_rz(v, s));
+    PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_update_p(v, tol2, loop, s));
+    return MPCHOL_OK;
+  };
+  if ((ss = true_residual(true)) != MPCHOL_OK) return ss;
+  // The iterations run in a device-side loop: one launch of a CUDA graph
+  // whose WHILE node repeats one iteration until the recursive residual meets
+  // the tolerance, an error is recorded or the budget is spent, with no host
+  // round trip in between.  Captured per operator / rhs count / tolerance, on
+  // the third call in a row with the same ones: capture and instantiation cost
+  // about 300 us, which an object that solves once or twice (the drop-in
+  // driver, a gradient step) does not earn back.
+  PcgGraph& g = f->graph;
+  if (g.A != (const void*)dA || g.lda != lda || g.nr != nr || g.elem != (int)sizeof(TA) || g.tol2 != tol2) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+    g.calls = 0;
+    g.A = dA; g.lda = lda; g.nr = nr; g.elem = (int)sizeof(TA); g.tol2 = tol2;
+  }
+  if (g.calls < 3) ++g.calls;
+  bool use_graph = !profiling_on() && !g.failed && g.calls >= 3 && po.max_it > 0;
+  if (use_graph && g.exec == nullptr) {
+    // capture on a private stream (the caller's may be the legacy default
+    // stream, which cannot be captured); the graph is launched into the
+    // caller's stream
+    long long before[MPCHOL_NPHASES];
+    launch_counts(before);
+    cudaGraph_t graph = nullptr;
+    cudaGraphConditionalHandle handle = 0;
+    cudaGraphNodeParams cp = {};
+    cudaGraphNode_t node = nullptr;
+    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
+              cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+    if (ok) {
+      cp.type = cudaGraphNodeTypeConditional;
+      cp.conditional.handle = handle;
+      cp.conditional.type = cudaGraphCondTypeWhile;
+      cp.conditional.size = 1;
+      ok = cudaGraphAddNode(&node, graph, nullptr, 0, &cp) == cudaSuccess;
+    }
+    if (ok) {
+      cudaGraph_t body = cp.conditional.phGraph_out[0];
+      ok = cudaStreamBeginCaptureToGraph(f->res.capture_stream, body, nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+      if (ok) {
+        const mpchol_status s0 = iteration(&handle, f->res.capture_stream);
+        cudaGraph_t captured = nullptr;
+        const cudaError_t ce = cudaStreamEndCapture(f->res.capture_stream, &captured);
+        ok = s0 == MPCHOL_OK && ce == cudaSuccess && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
       }
     }
-    converged = true;
-    for (int k = 0; k < nrhs; ++k)
-      if (!(f->res.h_scal[k] <= tol2 * f->res.h_scal[8 + k])) converged = false;
-    if (converged || launched >= po.max_it || restart > max_restarts) break;
-    mpchol_status s1 = apply_precond(f, r, tmp, z, nr, nullptr, stream);
-    if (s1 != MPCHOL_OK) return s1;
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_copy(z, p, n, nr, stream));
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_dot(r, z, n, nr, part_rz, nullptr, stream));
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_rz, rho[0], nr, stream));
-    MPCHOL_CUDA_TRY(cudaMemsetAsync(f->done, 0, sizeof(int), stream));
-    // One PCG iteration; rho[cur] is the current r^T z, rho[cur^1] receives
-    // the next one.  Every kernel returns at once after *done is set.
-    auto iteration = [&](int cur, cudaStream_t s) -> mpchol_status {
-      PHASE(MPCHOL_PH_SYMV, 2, s, launch_symv_skip<TA>(dA, lda, n, p, Ap, nr, f->done, s));
-      PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_dot(p, Ap, n, nr, part_pAp, f->done, s));
-      PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_update_xr(x, r, p, Ap, n, nr, part_pAp, rho[cur], alpha, part_rr,
-                                  f->done, f->pstatus, s));
-      mpchol_status s2 = apply_precond(f, r, tmp, z, nr, f->done, s);
-      if (s2 != MPCHOL_OK) return s2;
-      PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_dot(r, z, n, nr, part_rz, f->done, s));
-      PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_update_p(p, z, n, nr, part_rz, rho[cur], rho[cur ^ 1], part_rr,
-                                 bnorm2, tol2, f->done, f->done, f->done + 1, s));
-      return MPCHOL_OK;
-    };
-    // The iterations run in a device-side loop: one launch of a CUDA graph
-    // whose WHILE node repeats one iteration until the recursive residual
-    // meets the tolerance, an error is recorded or the budget is spent, with
-    // no host round trip in between.  Captured per operator / rhs count /
-    // tolerance, on the third call in a row with the same ones: capture and
-    // instantiation cost about 300 us, which an object that solves once or
-    // twice (the drop-in driver, a gradient step) does not earn back.
-    PcgGraph& g = f->graph;
-    if (restart == 0) {
-      if (g.A != (const void*)dA || g.lda != lda || g.nr != nr || g.elem != (int)sizeof(TA) ||
-          g.tol2 != tol2) {
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
-        g.calls = 0;
-        g.A = dA; g.lda = lda; g.nr = nr; g.elem = (int)sizeof(TA); g.tol2 = tol2;
-      }
-      if (g.calls < 3) ++g.calls;
+    if (graph) cudaGraphDestroy(graph);
+    long long after[MPCHOL_NPHASES];
+    launch_counts(after);
+    for (int i = 0; i < MPCHOL_NPHASES; ++i) g.nk[i] = after[i] - before[i];
+    add_launch_counts(g.nk, -1);   // nothing ran during capture
+    if (!ok) {
+      cudaGetLastError();            // the refusal is not an error of this call
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+      g.exec = nullptr;
+      g.failed = true;
+      use_graph = false;
     }
-    bool use_graph = !profiling_on() && !g.failed && g.calls >= 3;
-    if (use_graph && g.exec == nullptr) {
-      // capture on a private stream (the caller's may be the legacy default
-      // stream, which cannot be captured); the graph is launched into the
-      // caller's stream
-      long long before[MPCHOL_NPHASES];
-      launch_counts(before);
-      cudaGraph_t graph = nullptr;
-      cudaGraphConditionalHandle handle = 0;
-      cudaGraphNodeParams cp = {};
-      cudaGraphNode_t node = nullptr;
-      bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
-                cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault) ==
-                    cudaSuccess;
-      if (ok) {
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        ok = cudaGraphAddNode(&node, graph, nullptr, 0, &cp) == cudaSuccess;
-      }
-      if (ok) {
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        ok = cudaStreamBeginCaptureToGraph(f->res.capture_stream, body, nullptr, nullptr, 0,
-                                           cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-        if (ok) {
-          const mpchol_status s0 = iteration(0, f->res.capture_stream);
-          const bool cond_ok =
-              s0 == MPCHOL_OK && launch_pcg_loop_cond(handle, f->loop_ctl, f->done, f->pstatus,
-                                                      f->scal, nr, f->res.capture_stream) == cudaSuccess;
-          cudaGraph_t captured = nullptr;
-          const cudaError_t ce = cudaStreamEndCapture(f->res.capture_stream, &captured);
-          ok = cond_ok && ce == cudaSuccess && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
+  }
+  for (int restart = 0;; ++restart) {
+    if (po.max_it > 0 && restart <= max_restarts && it < po.max_it) {
+      // The iterations are enqueued without waiting for the residual's
+      // verdict: if it is met already (or the factor failed), done is set and
+      // they return at once.
+      mpchol_status s1 = apply_precond(f, v.work, v.tmp, v.z, nr, v.done, stream);
+      if (s1 != MPCHOL_OK) return s1;
+      PHASE(MPCHOL_PH_PCG_VEC, 2, stream, launch_pcg_start(v, po.max_it - it, stream));
+      if (use_graph) {
+        MPCHOL_CUDA_TRY(cudaGraphLaunch(g.exec, stream));
+      } else {
+        // chunks of check_every iterations, until the recursive residual meets
+        // the tolerance
+        const int it0 = it;
+        for (int launched = 0; it0 + launched < po.max_it;) {
+          const int chunk = std::min(po.check_every, po.max_it - it0 - launched);
+          for (int c = 0; c < chunk; ++c) {
+            mpchol_status s3 = iteration(nullptr, stream);
+            if (s3 != MPCHOL_OK) return s3;
+          }
+          launched += chunk;
+          mpchol_status rs = read_back();
+          if (rs != MPCHOL_OK) return rs;
+          int dn0;
+          memcpy(&dn0, f->res.h_scal + kScalDone, sizeof(int));
+          if (st.code == MPCHOL_ERR_TIMEOUT) return MPCHOL_ERR_TIMEOUT;
+          if (dn0 != 0 || st.code != 0) break;
         }
       }
-      if (graph) cudaGraphDestroy(graph);
-      long long after[MPCHOL_NPHASES];
-      launch_counts(after);
-      for (int i = 0; i < MPCHOL_NPHASES; ++i) g.nk[i] = after[i] - before[i];
-      add_launch_counts(g.nk, -1);   // nothing ran during capture
-      g.nk[MPCHOL_PH_PCG_VEC] += 1;  // the loop condition kernel
-      if (!ok) {
-        cudaGetLastError();            // the refusal is not an error of this call
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
-        g.failed = true;
-        use_graph = false;
-      }
-    }
-    if (use_graph) {
-      PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_pcg_loop_init(f->loop_ctl, po.max_it - launched, stream));
-      MPCHOL_CUDA_TRY(cudaGraphLaunch(g.exec, stream));
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_done, f->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-      DevStatus st;
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(&st, f->pstatus, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
-      MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
-      if (st.code == MPCHOL_ERR_TIMEOUT) return MPCHOL_ERR_TIMEOUT;
-      add_launch_counts(g.nk, f->res.h_done[1] - it);
-      it = f->res.h_done[1];                // iterations actually executed on the device
-      launched = it;
-      continue;                         // the true residual decides (residual replacement restart)
-    }
-    int cur = 0;
-    bool stop = false;
-    while (launched < po.max_it && !stop) {
-      const int chunk = std::min(po.check_every, po.max_it - launched);
-      for (int c = 0; c < chunk; ++c) {
-        mpchol_status s3 = iteration(cur, stream);
-        if (s3 != MPCHOL_OK) return s3;
-        cur ^= 1;
-      }
-      launched += chunk;
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_done, f->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
-      DevStatus st;
-      MPCHOL_CUDA_TRY(cudaMemcpyAsync(&st, f->pstatus, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
-      MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
-      if (st.code == MPCHOL_ERR_TIMEOUT) return MPCHOL_ERR_TIMEOUT;
-      it = f->res.h_done[1];                // iterations actually executed on the device
-      if (f->res.h_done[0]) stop = true;    // recursive residual met the tolerance
-      if (st.code == MPCHOL_PCG_BREAKDOWN) stop = true;
-      if (f->res.h_done[0]) launched = it;  // those enqueued past it returned at once
-    }
-    // the loop exits on max_it or when the recursive residual says done; the
-    // next pass re-checks the true residual (residual replacement restart)
-  }
-  // report
-  DevStatus st;
-  if (read_status(f->pstatus, stream, &st) != 0) return MPCHOL_ERR_CUDA;
-  MPCHOL_CUDA_TRY(cudaMemcpy2DAsync(dX, sizeof(double) * n, x, sizeof(double) * n,
-                                    sizeof(double) * n, nrhs, cudaMemcpyDeviceToDevice, stream));
-  if (rep != nullptr) {
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_dot(x, x, n, nr, part_misc, nullptr, stream));
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_misc, misc + 8, nr, stream));
-    if (fro_fused) {
-      PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_fro, misc + 16, 1, stream));
+      // the true residual decides (residual replacement restart)
+      const int it_before = it;
+      if ((ss = true_residual(false)) != MPCHOL_OK) return ss;
+      mpchol_status rs = read_back();
+      if (rs != MPCHOL_OK) return rs;
+      if (use_graph) add_launch_counts(g.nk, it - it_before);
     } else {
-      PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_frob_lower<TA>(dA, lda, n, part_misc, stream));
-      PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_misc, misc + 16, 1, stream));
+      mpchol_status rs = read_back();
+      if (rs != MPCHOL_OK) return rs;
     }
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_dot(r, z, n, nr, part_rz, nullptr, stream));
-    PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_reduce_partials(part_rz, misc + 24, nr, stream));
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal, misc, sizeof(double) * 32, cudaMemcpyDeviceToHost, stream));
-    MPCHOL_CUDA_TRY(cudaMemcpyAsync(f->res.h_scal + 32, bnorm2, sizeof(double) * 8, cudaMemcpyDeviceToHost, stream));
-    MPCHOL_CUDA_TRY(cudaStreamSynchronize(stream));
+    // a failed factor (NOT_SPD, TIMEOUT) is not iterated with
+    DevStatus fst;
+    memcpy(&fst, f->res.h_scal + kScalStatus, sizeof(DevStatus));
+    if (fst.code != 0) {
+      if (rep != nullptr) memset(rep, 0, sizeof(*rep));
+      return (mpchol_status)fst.code;
+    }
+    if (st.code == MPCHOL_ERR_TIMEOUT) return MPCHOL_ERR_TIMEOUT;
+    converged = true;
+    for (int k = 0; k < nrhs; ++k)
+      if (!(f->res.h_scal[k] <= tol2 * f->res.h_scal[kScalBnorm + k])) converged = false;
+    if (converged || it >= po.max_it || restart > max_restarts) break;
+  }
+  MPCHOL_CUDA_TRY(cudaMemcpyAsync(dX, v.x, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, stream));
+  if (rep != nullptr) {
     double relmax = 0.0, bemax = 0.0, prmax = 0.0;
-    const double frob = sqrt(f->res.h_scal[16]);
+    const double* h = f->res.h_scal;
+    const double frob = sqrt(h[16]);
     for (int k = 0; k < nrhs; ++k) {
-      const double rr = f->res.h_scal[k], xx = f->res.h_scal[8 + k], bb2 = f->res.h_scal[32 + k];
+      const double rr = h[k], xx = h[8 + k], bb2 = h[kScalBnorm + k];
       const double rel = bb2 > 0 ? sqrt(rr / bb2) : sqrt(rr);
       const double be = sqrt(rr) / (frob * sqrt(xx) + sqrt(bb2));
-      const double pr = bb2 > 0 ? sqrt(fabs(f->res.h_scal[24 + k]) / bb2) : 0.0;
+      const double pr = bb2 > 0 ? sqrt(fabs(h[24 + k]) / bb2) : 0.0;
       relmax = std::max(relmax, rel);
       bemax = std::max(bemax, be);
       prmax = std::max(prmax, pr);
@@ -1147,7 +1128,6 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     rep->backward_error = bemax;
     rep->precond_residual = prmax;
   }
-  if (st.code == MPCHOL_PCG_BREAKDOWN) return MPCHOL_PCG_BREAKDOWN;
   if (st.code != 0) return (mpchol_status)st.code;
   return converged ? MPCHOL_OK : MPCHOL_PCG_MAXIT;
 }
@@ -1347,17 +1327,19 @@ mpchol_status mpchol_factor_create(const mpchol_opts* opts, int n, mpchol_factor
     take(f->rexp, (size_t)3 * n);
     take(f->mxexp, (size_t)n * (f->b / 32));
     take(f->steps, f->nsteps + 1);
-    take(f->status, 1);
-    take(f->pstatus, 1);
     take(f->colacc, (size_t)f->nsteps * kColCopies * f->b);
     take(f->eqexp, n);
     take(f->wsup, solve_wsup_elems(n));
-    take(f->trsv_ctr, trsv_counter_ints(n));
+    take(f->trsv_ctr, 2 * trsv_counter_ints(n));
     take(f->vec, 8 * nv);
-    take(f->partials, (size_t)5 * pcg_vgrid() * 8);
-    take(f->scal, 64);
-    take(f->done, 2);
-    take(f->loop_ctl, 2);
+    take(f->partials, (size_t)6 * pcg_vgrid() * 8);
+    take(f->scal, kScalDoubles);
+    if (base) {
+      f->status = reinterpret_cast<DevStatus*>(f->scal + kScalStatus);
+      f->pstatus = f->status + 1;
+      f->done = reinterpret_cast<int*>(f->scal + kScalDone);
+      f->loop_ctl = f->done + 2;
+    }
     return off;
   };
   if (!acquire_resources(f->device, carve(nullptr), &f->res)) {
@@ -1731,12 +1713,14 @@ mpchol_status mpchol_apply_precond(mpchol_factor_t* f, const double* dR, double*
   if (ss != MPCHOL_OK) return ss;
   const int nr = pcg_padded_nrhs(nrhs);
   const size_t nv = (size_t)f->n * 8;
-  double* rp = f->vec + 5 * nv;     // bb slot
+  double* rp = f->vec + 5 * nv;     // b slot
   double* tmp = f->vec + 6 * nv;
+  double* work = f->vec + 7 * nv;
   double* zp = f->vec + 2 * nv;     // z slot
   MPCHOL_CUDA_TRY(cudaMemsetAsync(f->pstatus, 0, sizeof(DevStatus), s));
   PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_pad_columns(dR, f->n, nrhs, rp, nr, s));
-  ss = apply_precond(f, rp, tmp, zp, nr, nullptr, s);
+  PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_trsv_prep(rp, work, tmp, zp, f->n, nr, f->trsv_ctr, s));
+  ss = apply_precond(f, work, tmp, zp, nr, nullptr, s);
   if (ss != MPCHOL_OK) return ss;
   MPCHOL_CUDA_TRY(cudaMemcpy2DAsync(dZ, sizeof(double) * f->n, zp, sizeof(double) * f->n,
                                     sizeof(double) * f->n, nrhs, cudaMemcpyDeviceToDevice, s));
@@ -1750,8 +1734,9 @@ mpchol_status mpchol_symv(const float* dA, int lda, int n, const double* dX, dou
   if (dA == nullptr || dX == nullptr || dY == nullptr || n <= 0 || lda < n) return MPCHOL_ERR_BAD_ARG;
   if (nrhs != 1 && nrhs != 2 && nrhs != 4 && nrhs != 8) return MPCHOL_ERR_BAD_ARG;
   MPCHOL_CUDA_TRY(solve_init_attributes());
-  PHASE(MPCHOL_PH_SYMV, 1, reinterpret_cast<cudaStream_t>(stream), launch_symv_skip<float>(dA, lda, n, dX, dY, nrhs, nullptr,
-                                          reinterpret_cast<cudaStream_t>(stream)));
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  PHASE(MPCHOL_PH_SYMV, 1, s, launch_zero_vec(dY, (long long)n * nrhs, s));
+  PHASE(MPCHOL_PH_SYMV, 1, s, launch_symv_skip<float>(dA, lda, n, dX, dY, nrhs, nullptr, s));
   return MPCHOL_OK;
 }
 

@@ -63,30 +63,205 @@ __device__ __forceinline__ void sum_partials(const double* partials, double (&ou
   __syncthreads();
 }
 
+// ---- the kernels of one solve ------------------------------------------------
+// What a solve launches beside its operator products and triangular solves.
+// Each of these vector passes also prepares what the next kernels start from
+// (zeroed accumulation targets, the triangular solves' input and counters), so
+// that an iteration is seven launches; a boundary costs 1.5 us or more of an
+// iteration that takes 20 at n = 1024.
+
+// The inputs of one application z = M^-1 r: work = r, tmp and z zero, the two
+// triangular solves' counters zero.
+struct PrecPrep {
+  double* work;
+  double* tmp;
+  double* z;
+  int* ctr;
+  int nctr;
+};
+__device__ __forceinline__ void clear_counters(const PrecPrep& pp) {
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < pp.nctr; i += NTH) pp.ctr[i] = 0;
+}
+
+// b (padded to NR columns), its partial ||b||^2, and the start of the solve:
+// the first application's inputs (x0) or x = 0, Ap and z zero, the solve's
+// status and done flags clear.
 template <int NR>
 __global__ void __launch_bounds__(NTH)
-dot_kernel(const double* __restrict__ a, const double* __restrict__ b, int n, double* partials,
-           const int* skip) {
-  if (skip != nullptr && *skip) return;
+pcg_begin_kernel(const double* __restrict__ B, int nrhs, int n, double* __restrict__ bb, double* partials,
+                 PrecPrep pp, double* __restrict__ Ap, double* __restrict__ z, bool x0, DevStatus* st,
+                 int* done) {
   double v[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) v[k] = 0.0;
   for (int i = blockIdx.x * NTH + threadIdx.x; i < n; i += VG * NTH)
 #pragma unroll
-    for (int k = 0; k < NR; ++k) v[k] = fma(a[(size_t)k * n + i], b[(size_t)k * n + i], v[k]);
+    for (int k = 0; k < NR; ++k) {
+      const size_t o = (size_t)k * n + i;
+      const double t = k < nrhs ? B[o] : 0.0;
+      bb[o] = t;
+      v[k] = fma(t, t, v[k]);
+      if (x0) {
+        pp.work[o] = t;
+        pp.tmp[o] = 0.0;
+      }
+      pp.z[o] = 0.0;   // x
+      Ap[o] = 0.0;
+      z[o] = 0.0;
+    }
+  clear_counters(pp);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *st = DevStatus{0, 0, 0, 0};
+    done[0] = done[1] = 0;
+  }
   block_reduce_store<NR>(v, partials);
 }
 
-// alpha = rho / (p^T A p); x += alpha p; r -= alpha A p; partial ||r||^2.
-// A right-hand side whose pAp or rho is zero (already converged exactly) or
-// not finite takes alpha = 0; a negative pAp records PCG_BREAKDOWN.
+// r = b - A x (Ap on entry, zero on exit), the partials of ||r||^2, ||x||^2 and
+// r^T z (z: the last application's result), and the inputs of the next
+// application to r.
+template <int NR>
+__global__ void __launch_bounds__(NTH)
+residual_kernel(const double* __restrict__ b, double* __restrict__ Ap, double* __restrict__ r,
+                const double* __restrict__ x, int n, double* rr_partials, double* xx_partials,
+                double* rz_partials, PrecPrep pp) {
+  double v[NR], w[NR], u[NR];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) v[k] = w[k] = u[k] = 0.0;
+  for (int i = blockIdx.x * NTH + threadIdx.x; i < n; i += VG * NTH)
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const size_t o = (size_t)k * n + i;
+      const double rv = b[o] - Ap[o], xv = x[o];
+      Ap[o] = 0.0;
+      r[o] = rv;
+      v[k] = fma(rv, rv, v[k]);
+      w[k] = fma(xv, xv, w[k]);
+      u[k] = fma(rv, pp.z[o], u[k]);
+      pp.work[o] = rv;
+      pp.tmp[o] = 0.0;
+      pp.z[o] = 0.0;
+    }
+  clear_counters(pp);
+  block_reduce_store<NR>(v, rr_partials);
+  __syncthreads();
+  block_reduce_store<NR>(w, xx_partials);
+  __syncthreads();
+  block_reduce_store<NR>(u, rz_partials);
+}
+
+// Reduces the partials of a residual pass, one block each: ||r||^2 (and, in the
+// first pass, ||b||^2), ||x||^2, r^T z, ||A||_F^2 (null: elsewhere).  done is
+// set when every rhs meets the tolerance or the factor has failed, so that the
+// iterations enqueued behind it return at once; it is cleared otherwise.
+template <int NR>
+__global__ void __launch_bounds__(NTH)
+residual_reduce_kernel(const double* rr_partials, const double* bb_partials, const double* xx_partials,
+                       const double* rz_partials, const double* fro_partials, double* misc, double* bnorm2,
+                       double tol2, const DevStatus* factor_st, int* done) {
+  double s[NR];
+  if (blockIdx.x == 0) {
+    double bn[NR];
+    if (bb_partials != nullptr) {
+      sum_partials<NR>(bb_partials, bn);
+    } else {
+#pragma unroll
+      for (int k = 0; k < NR; ++k) bn[k] = bnorm2[k];
+    }
+    sum_partials<NR>(rr_partials, s);
+    if (threadIdx.x == 0) {
+      int all = 1;
+#pragma unroll
+      for (int k = 0; k < NR; ++k) {
+        misc[k] = s[k];
+        bnorm2[k] = bn[k];
+        if (!(s[k] <= tol2 * bn[k])) all = 0;
+      }
+      done[0] = (all || factor_st->code != 0) ? 1 : 0;
+    }
+  } else if (blockIdx.x == 3) {
+    if (fro_partials == nullptr) return;
+    double f[1];
+    sum_partials<1>(fro_partials, f);
+    if (threadIdx.x == 0) misc[16] = f[0];
+  } else {
+    sum_partials<NR>(blockIdx.x == 1 ? xx_partials : rz_partials, s);
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int k = 0; k < NR; ++k) misc[(blockIdx.x == 1 ? 8 : 24) + k] = s[k];
+  }
+}
+
+// p = z, partial r^T z: the first search direction.
+template <int NR>
+__global__ void __launch_bounds__(NTH)
+pcg_start_kernel(const double* __restrict__ r, const double* __restrict__ z, double* __restrict__ p, int n,
+                 double* partials, const int* skip) {
+  if (*skip) return;
+  double v[NR];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) v[k] = 0.0;
+  for (int i = blockIdx.x * NTH + threadIdx.x; i < n; i += VG * NTH)
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const size_t o = (size_t)k * n + i;
+      const double zv = z[o];
+      p[o] = zv;
+      v[k] = fma(r[o], zv, v[k]);
+    }
+  block_reduce_store<NR>(v, partials);
+}
+
+// rho_0 = r^T z from its partials; ctl: iterations begun by this loop, its budget.
+template <int NR>
+__global__ void __launch_bounds__(NTH)
+pcg_loop_begin_kernel(const double* partials, double* rho, int* ctl, int budget) {
+  double s[NR];
+  sum_partials<NR>(partials, s);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < NR; ++k) rho[k] = s[k];
+    ctl[0] = 0;
+    ctl[1] = budget;
+  }
+}
+
+// partial a^T b.  count (null: none): the iteration count, incremented once (no
+// block of this kernel reads it); zero (null: none): a vector cleared on the
+// way, the product's target for the next iteration.
+template <int NR>
+__global__ void __launch_bounds__(NTH)
+dot_kernel(const double* __restrict__ a, const double* __restrict__ b, int n, double* partials,
+           const int* skip, int* count, double* __restrict__ zero) {
+  if (skip != nullptr && *skip) return;
+  if (count != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *count += 1;
+  double v[NR];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) v[k] = 0.0;
+  for (int i = blockIdx.x * NTH + threadIdx.x; i < n; i += VG * NTH)
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const size_t o = (size_t)k * n + i;
+      v[k] = fma(a[o], b[o], v[k]);
+      if (zero != nullptr) zero[o] = 0.0;
+    }
+  block_reduce_store<NR>(v, partials);
+}
+
+// alpha = rho / (p^T A p); x += alpha p; r -= alpha A p; partial ||r||^2; the
+// inputs of the application to r.  A right-hand side whose pAp or rho is zero
+// (already converged exactly) or not finite takes alpha = 0; a negative pAp
+// records PCG_BREAKDOWN.  rho holds two sets of 8, used in turn: iteration c
+// (ctl[0], from 1) reads set (c - 1) % 2 and writes the other.
 template <int NR>
 __global__ void __launch_bounds__(NTH)
 update_xr_kernel(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
                  const double* __restrict__ Ap, int n, const double* pAp_partials,
-                 const double* rho, double* alpha_out, double* rr_partials, const int* skip,
-                 DevStatus* st) {
-  if (skip != nullptr && *skip) return;
+                 const double* rho_sets, const int* ctl, double* rr_partials, const int* skip,
+                 DevStatus* st, PrecPrep pp) {
+  if (*skip) return;
+  const double* rho = rho_sets + 8 * ((ctl[0] - 1) & 1);
   double pAp[NR], al[NR];
   sum_partials<NR>(pAp_partials, pAp);
 #pragma unroll
@@ -95,7 +270,6 @@ update_xr_kernel(double* __restrict__ x, double* __restrict__ r, const double* _
     al[k] = (pAp[k] != 0.0 && isfinite(a)) ? a : 0.0;
     if (!(pAp[k] >= 0.0) && threadIdx.x == 0 && blockIdx.x == 0) set_status(st, MPCHOL_PCG_BREAKDOWN, k);
   }
-  if (blockIdx.x == 0 && threadIdx.x < NR) alpha_out[threadIdx.x] = al[threadIdx.x];
   double v[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) v[k] = 0.0;
@@ -107,39 +281,53 @@ update_xr_kernel(double* __restrict__ x, double* __restrict__ r, const double* _
       const double rn = fma(-al[k], Ap[o], r[o]);
       r[o] = rn;
       v[k] = fma(rn, rn, v[k]);
+      pp.work[o] = rn;
+      pp.tmp[o] = 0.0;
+      pp.z[o] = 0.0;
     }
   }
+  clear_counters(pp);
   block_reduce_store<NR>(v, rr_partials);
 }
 
 // rho_new = r^T z (from partials); beta = rho_new / rho_old; p = z + beta p.
-// Writes rho_new to rho_out (a different buffer from rho_old) and, from the
-// ||r||^2 partials, sets *done when every rhs has ||r|| <= tol * ||b||.
-template <int NR>
+// From the ||r||^2 partials, sets *done when every rhs has ||r|| <= tol * ||b||
+// (a block that starts after that skips its part of p, which nothing reads
+// any more).  LOOP: also sets the condition of the device-side loop this
+// iteration is the body of: continue while the recursive residual is above
+// the tolerance, no error is recorded and the budget is not spent (the budget
+// alone ends it, whatever the other flags hold).
+template <int NR, bool LOOP>
 __global__ void __launch_bounds__(NTH)
-update_p_kernel(double* __restrict__ p, const double* __restrict__ z, int n,
-                const double* rz_partials, const double* rho_old, double* rho_out,
-                const double* rr_partials, const double* bnorm2, double tol2, int* done,
-                const int* skip, int* iters) {
-  if (skip != nullptr && *skip) return;
+update_p_kernel(double* __restrict__ p, const double* __restrict__ z, int n, const double* rz_partials,
+                double* rho_sets, const int* ctl, const double* rr_partials, const double* bnorm2,
+                double tol2, int* done, const DevStatus* st, cudaGraphConditionalHandle handle) {
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  if (*reinterpret_cast<volatile int*>(done)) {
+    if (LOOP && first) cudaGraphSetConditional(handle, 0u);
+    return;
+  }
+  const int cur = (ctl[0] - 1) & 1;
   double rz[NR], be[NR];
   sum_partials<NR>(rz_partials, rz);
 #pragma unroll
   for (int k = 0; k < NR; ++k) {
-    const double b = rz[k] / rho_old[k];
-    be[k] = (rho_old[k] != 0.0 && isfinite(b)) ? b : 0.0;
+    const double old = rho_sets[8 * cur + k];
+    const double b = rz[k] / old;
+    be[k] = (old != 0.0 && isfinite(b)) ? b : 0.0;
   }
   double rr[NR];
   sum_partials<NR>(rr_partials, rr);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (first) {
     int all = 1;
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
-      rho_out[k] = rz[k];
+      rho_sets[8 * (cur ^ 1) + k] = rz[k];
       if (!(rr[k] <= tol2 * bnorm2[k])) all = 0;
     }
-    *done = all;
-    *iters += 1;
+    done[0] = all;
+    done[1] += 1;
+    if (LOOP) cudaGraphSetConditional(handle, (ctl[0] < ctl[1] && !all && st->code == 0) ? 1u : 0u);
   }
   for (int i = blockIdx.x * NTH + threadIdx.x; i < n; i += VG * NTH)
 #pragma unroll
@@ -147,43 +335,6 @@ update_p_kernel(double* __restrict__ p, const double* __restrict__ z, int n,
       const size_t o = (size_t)k * n + i;
       p[o] = fma(be[k], p[o], z[o]);
     }
-}
-
-// out = sum of partials (fixed order) for the first NR slots; used to form
-// rho_0 = r_0^T z_0 and ||b||^2 on the device.
-template <int NR>
-__global__ void __launch_bounds__(NTH) reduce_partials_kernel(const double* partials, double* out) {
-  double s[NR];
-  sum_partials<NR>(partials, s);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < NR; ++k) out[k] = s[k];
-}
-
-// r = b - y (y = A x), partial ||r||^2
-template <int NR>
-__global__ void __launch_bounds__(NTH)
-residual_kernel(const double* __restrict__ b, const double* __restrict__ y, double* __restrict__ r,
-                int n, double* rr_partials) {
-  double v[NR];
-#pragma unroll
-  for (int k = 0; k < NR; ++k) v[k] = 0.0;
-  for (int i = blockIdx.x * NTH + threadIdx.x; i < n; i += VG * NTH)
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const size_t o = (size_t)k * n + i;
-      const double rv = b[o] - y[o];
-      r[o] = rv;
-      v[k] = fma(rv, rv, v[k]);
-    }
-  block_reduce_store<NR>(v, rr_partials);
-}
-
-template <int NR>
-__global__ void copy_kernel(const double* __restrict__ a, double* __restrict__ b, int n) {
-  for (long long i = blockIdx.x * (long long)NTH + threadIdx.x; i < (long long)n * NR;
-       i += (long long)VG * NTH)
-    b[i] = a[i];
 }
 
 // ---- batched PCG (one launch for every system of a batch) ------------------
@@ -426,42 +577,49 @@ frob_batched_kernel(const BatchSys* __restrict__ sys) {
 int pcg_padded_nrhs(int nrhs) { return nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : 8; }
 int pcg_vgrid() { return VG; }
 
-cudaError_t launch_dot(const double* a, const double* b, int n, int nrhs, double* partials,
-                       const int* skip, cudaStream_t stream) {
-  NR_DISPATCH(nrhs, (dot_kernel<NRC><<<VG, NTH, 0, stream>>>(a, b, n, partials, skip)));
+namespace {
+PrecPrep prep_of(const PcgVectors& v, double* target) {
+  return PrecPrep{v.work, v.tmp, target, v.ctr, v.nctr};
+}
+}  // namespace
+
+cudaError_t launch_pcg_begin(const PcgVectors& v, const double* B, int nrhs, bool x0, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (pcg_begin_kernel<NRC><<<VG, NTH, 0, stream>>>(B, nrhs, v.n, v.b, v.part_bb, prep_of(v, v.x), v.Ap, v.z, x0, v.status, v.done)));
   return cudaGetLastError();
 }
-
-cudaError_t launch_update_xr(double* x, double* r, const double* p, const double* Ap, int n,
-                             int nrhs, const double* pAp_partials, const double* rho,
-                             double* alpha_out, double* rr_partials, const int* skip,
-                             DevStatus* st, cudaStream_t stream) {
-  NR_DISPATCH(nrhs, (update_xr_kernel<NRC><<<VG, NTH, 0, stream>>>(x, r, p, Ap, n, pAp_partials, rho, alpha_out, rr_partials, skip, st)));
+cudaError_t launch_residual(const PcgVectors& v, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (residual_kernel<NRC><<<VG, NTH, 0, stream>>>(v.b, v.Ap, v.r, v.x, v.n, v.part_rr, v.part_xx, v.part_rz, prep_of(v, v.z))));
   return cudaGetLastError();
 }
-
-cudaError_t launch_update_p(double* p, const double* z, int n, int nrhs, const double* rz_partials,
-                            const double* rho_old, double* rho_out, const double* rr_partials,
-                            const double* bnorm2, double tol2, int* done, const int* skip,
-                            int* iters, cudaStream_t stream) {
-  NR_DISPATCH(nrhs, (update_p_kernel<NRC><<<VG, NTH, 0, stream>>>(p, z, n, rz_partials, rho_old, rho_out, rr_partials, bnorm2, tol2, done, skip, iters)));
+cudaError_t launch_residual_reduce(const PcgVectors& v, bool first, bool fro, double tol2,
+                                   const DevStatus* factor_st, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (residual_reduce_kernel<NRC><<<4, NTH, 0, stream>>>(v.part_rr, first ? v.part_bb : nullptr, v.part_xx, v.part_rz, fro ? v.part_fro : nullptr, v.misc, v.bnorm2, tol2, factor_st, v.done)));
   return cudaGetLastError();
 }
-
-cudaError_t launch_reduce_partials(const double* partials, double* out, int nrhs,
-                                   cudaStream_t stream) {
-  NR_DISPATCH(nrhs, (reduce_partials_kernel<NRC><<<1, NTH, 0, stream>>>(partials, out)));
+cudaError_t launch_pcg_start(const PcgVectors& v, int budget, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (pcg_start_kernel<NRC><<<VG, NTH, 0, stream>>>(v.r, v.z, v.p, v.n, v.part_rz, v.done)));
+  NR_DISPATCH(v.nr, (pcg_loop_begin_kernel<NRC><<<1, NTH, 0, stream>>>(v.part_rz, v.rho, v.ctl, budget)));
   return cudaGetLastError();
 }
-
-cudaError_t launch_residual(const double* b, const double* y, double* r, int n, int nrhs,
-                            double* rr_partials, cudaStream_t stream) {
-  NR_DISPATCH(nrhs, (residual_kernel<NRC><<<VG, NTH, 0, stream>>>(b, y, r, n, rr_partials)));
+cudaError_t launch_dot_pAp(const PcgVectors& v, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (dot_kernel<NRC><<<VG, NTH, 0, stream>>>(v.p, v.Ap, v.n, v.part_pAp, v.done, v.ctl, nullptr)));
   return cudaGetLastError();
 }
-
-cudaError_t launch_copy(const double* a, double* b, int n, int nrhs, cudaStream_t stream) {
-  NR_DISPATCH(nrhs, (copy_kernel<NRC><<<VG, NTH, 0, stream>>>(a, b, n)));
+cudaError_t launch_update_xr(const PcgVectors& v, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (update_xr_kernel<NRC><<<VG, NTH, 0, stream>>>(v.x, v.r, v.p, v.Ap, v.n, v.part_pAp, v.rho, v.ctl, v.part_rr, v.done, v.status, prep_of(v, v.z))));
+  return cudaGetLastError();
+}
+cudaError_t launch_dot_rz(const PcgVectors& v, cudaStream_t stream) {
+  NR_DISPATCH(v.nr, (dot_kernel<NRC><<<VG, NTH, 0, stream>>>(v.r, v.z, v.n, v.part_rz, v.done, nullptr, v.Ap)));
+  return cudaGetLastError();
+}
+cudaError_t launch_update_p(const PcgVectors& v, double tol2, const cudaGraphConditionalHandle* loop,
+                            cudaStream_t stream) {
+  if (loop != nullptr) {
+    NR_DISPATCH(v.nr, (update_p_kernel<NRC, true><<<VG, NTH, 0, stream>>>(v.p, v.z, v.n, v.part_rz, v.rho, v.ctl, v.part_rr, v.bnorm2, tol2, v.done, v.status, *loop)));
+  } else {
+    NR_DISPATCH(v.nr, (update_p_kernel<NRC, false><<<VG, NTH, 0, stream>>>(v.p, v.z, v.n, v.part_rz, v.rho, v.ctl, v.part_rr, v.bnorm2, tol2, v.done, v.status, cudaGraphConditionalHandle{})));
+  }
   return cudaGetLastError();
 }
 
@@ -513,36 +671,5 @@ cudaError_t launch_frob_batched(const BatchSys* sys, int nsys, cudaStream_t stre
   return cudaGetLastError();
 }
 
-
-namespace {
-// Loop control of the device-side PCG loop: ctl[0] counts the iterations run
-// by this launch of the loop, ctl[1] is how many it may run.
-__global__ void pcg_loop_init_kernel(int* ctl, int max_iters) {
-  ctl[0] = 0;
-  ctl[1] = max_iters;
-}
-// After each iteration: the new r^T z becomes the current one (rho[8..] ->
-// rho[0..]), and the loop runs again only if the recursive residual has not
-// met the tolerance, no error was recorded and the iteration budget is not
-// spent.  The budget alone ends the loop, whatever the other flags hold.
-__global__ void pcg_loop_cond_kernel(cudaGraphConditionalHandle handle, int* ctl, const int* done,
-                                     const DevStatus* st, double* rho, int nr) {
-  const int c = ctl[0] + 1;
-  ctl[0] = c;
-  for (int k = 0; k < nr; ++k) rho[k] = rho[8 + k];
-  const bool more = c < ctl[1] && done[0] == 0 && st->code == 0;
-  cudaGraphSetConditional(handle, more ? 1u : 0u);
-}
-}  // namespace
-
-cudaError_t launch_pcg_loop_init(int* ctl, int max_iters, cudaStream_t stream) {
-  pcg_loop_init_kernel<<<1, 1, 0, stream>>>(ctl, max_iters);
-  return cudaGetLastError();
-}
-cudaError_t launch_pcg_loop_cond(cudaGraphConditionalHandle handle, int* ctl, const int* done,
-                                 const DevStatus* st, double* rho, int nr, cudaStream_t stream) {
-  pcg_loop_cond_kernel<<<1, 1, 0, stream>>>(handle, ctl, done, st, rho, nr);
-  return cudaGetLastError();
-}
 
 }  // namespace mpchol

@@ -12,47 +12,59 @@ cudaError_t solve_init_attributes();
 int solve_super_rows();
 size_t solve_wsup_elems(int n);
 int solve_setup_launches(int n);
+// y += A x (the lower triangle of A, FP32 or FP64); y is zero on entry for a
+// product.  An FP32 A is streamed through the staged kernel, which then also
+// fills `fro` (shares of ||A||_F^2 for up to nfro CTAs, the rest zero).
+cudaError_t launch_zero_vec(double* y, long long count, cudaStream_t stream);
 template <typename TA>
 cudaError_t launch_symv_skip(const TA* A, int lda, int n, const double* x, double* y, int nrhs,
                              const int* skip, cudaStream_t stream, double* fro = nullptr,
                              int nfro = 0);
-// True when launch_symv_skip streams A through the staged kernel (FP32, 16-byte
-// aligned columns); only then does it fill `fro` (per-CTA shares of ||A||_F^2).
-template <typename TA>
-bool symv_staged_ok(const TA* A, int lda);
 // 128-block inverses into winv, then the super-block inverses into wsup.
 cudaError_t launch_solve_setup(const float* L, int ldl, int n, float* wsup, cudaStream_t stream);
-// out = L^-1 in (forward) or L^-T in (backward) through the super-block
-// inverses wsup: one launch that prepares work <- in, out <- 0 and clears the
-// counters, then one persistent cooperative launch; work is an n x nrhs
-// scratch, counters trsv_counter_ints(n) ints.
+// out = L^-1 w (forward) or L^-T w (backward) through the super-block inverses
+// wsup, one persistent cooperative launch: w is consumed, out (n x nrhs) and
+// the trsv_counter_ints(n) counters are zero on entry.  launch_trsv_prep: w <-
+// in, and for the forward-then-backward pair its targets mid and out and both
+// sets of counters zero.
 size_t trsv_counter_ints(int n);
+cudaError_t launch_trsv_prep(const double* in, double* w, double* mid, double* out, int n, int nrhs,
+                             int* counters, cudaStream_t stream);
 cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n,
-                                   const float* wsup, const double* in, double* out,
-                                   double* work, int nrhs, int* counters, const int* skip,
-                                   DevStatus* st, cudaStream_t stream);
-cudaError_t launch_dot(const double* a, const double* b, int n, int nrhs, double* partials,
-                       const int* skip, cudaStream_t stream);
-cudaError_t launch_update_xr(double* x, double* r, const double* p, const double* Ap, int n,
-                             int nrhs, const double* pAp_partials, const double* rho,
-                             double* alpha_out, double* rr_partials, const int* skip,
-                             DevStatus* st, cudaStream_t stream);
-cudaError_t launch_update_p(double* p, const double* z, int n, int nrhs, const double* rz_partials,
-                            const double* rho_old, double* rho_out, const double* rr_partials,
-                            const double* bnorm2, double tol2, int* done, const int* skip,
-                            int* iters, cudaStream_t stream);
-cudaError_t launch_reduce_partials(const double* partials, double* out, int nrhs,
-                                   cudaStream_t stream);
-cudaError_t launch_residual(const double* b, const double* y, double* r, int n, int nrhs,
-                            double* rr_partials, cudaStream_t stream);
-cudaError_t launch_copy(const double* a, double* b, int n, int nrhs, cudaStream_t stream);
-// Device-side PCG loop (a WHILE node of a CUDA graph): ctl[0] <- 0,
-// ctl[1] <- max_iters before the loop; after each iteration the condition
-// kernel copies rho[8..8+nr) to rho[0..nr) and sets the loop condition
-// (continue while ctl[0] < ctl[1], *done == 0 and no recorded error).
-cudaError_t launch_pcg_loop_init(int* ctl, int max_iters, cudaStream_t stream);
-cudaError_t launch_pcg_loop_cond(cudaGraphConditionalHandle handle, int* ctl, const int* done,
-                                 const DevStatus* st, double* rho, int nr, cudaStream_t stream);
+                                   const float* wsup, double* w, double* out, int nrhs, int* counters,
+                                   const int* skip, DevStatus* st, cudaStream_t stream);
+// What the kernels of one solve work on: n x nr vectors (column-major, ld n;
+// nr = 1, 2, 4 or 8), partial sums of pcg_vgrid() blocks, and the scalars
+// that never leave the device.
+struct PcgVectors {
+  int n, nr;
+  double *x, *r, *z, *p, *Ap, *b, *tmp, *work;
+  double *part_pAp, *part_rr, *part_rz, *part_xx, *part_bb, *part_fro;
+  double* rho;       // two sets of 8, used in turn by iteration
+  double* bnorm2;    // 8
+  double* misc;      // true ||r||^2 at 0, ||x||^2 at 8, ||A||_F^2 at 16, r^T z at 24
+  int* done;         // [0] converged or failed, [1] iterations of the solve
+  int* ctl;          // [0] iterations of the current loop, [1] its budget
+  int* ctr;          // the two triangular solves' counters
+  int nctr;
+  DevStatus* status;
+};
+// In the order of a solve.  begin: b from B, the start state, and (x0) the
+// inputs of the application that gives x.  residual: r = b - A x from Ap, and
+// the inputs of z = M^-1 r; residual_reduce: its norms and *done.  start: p = z,
+// rho, the loop's budget.  An iteration: Ap = A p, dot_pAp, update_xr (leaves
+// the inputs of z = M^-1 r), the application, dot_rz (clears Ap), update_p
+// (loop: sets the WHILE node's condition).
+cudaError_t launch_pcg_begin(const PcgVectors& v, const double* B, int nrhs, bool x0, cudaStream_t stream);
+cudaError_t launch_residual(const PcgVectors& v, cudaStream_t stream);
+cudaError_t launch_residual_reduce(const PcgVectors& v, bool first, bool fro, double tol2,
+                                   const DevStatus* factor_st, cudaStream_t stream);
+cudaError_t launch_pcg_start(const PcgVectors& v, int budget, cudaStream_t stream);
+cudaError_t launch_dot_pAp(const PcgVectors& v, cudaStream_t stream);
+cudaError_t launch_update_xr(const PcgVectors& v, cudaStream_t stream);
+cudaError_t launch_dot_rz(const PcgVectors& v, cudaStream_t stream);
+cudaError_t launch_update_p(const PcgVectors& v, double tol2, const cudaGraphConditionalHandle* loop,
+                            cudaStream_t stream);
 
 // misc device utilities (util.cu)
 cudaError_t launch_extract_diag(const float* A, int lda, int n, float* d, float* dtilde,

@@ -490,6 +490,19 @@ __device__ __forceinline__ void tile_mma_x8(const float* Ts, const double* x_c, 
   }
 }
 
+// A tile whose columns need not start on 16-byte boundaries, by 4-byte
+// copies into the plain (BL = false) or blocked (BL = true) layout.
+template <bool BL>
+__device__ __forceinline__ void stage_tile_4b(float* dst, const float* T, int ld, int rows_valid,
+                                              int cols_valid) {
+#pragma unroll 4
+  for (int e = threadIdx.x; e < TILE_ELEMS; e += NTH) {
+    const int c = e / RB, r = e % RB;
+    const bool ok = c < cols_valid && r < rows_valid;
+    cp_async4(dst + (BL ? bl_off(r, c) : c * RB + r), ok ? T + (size_t)c * ld + r : T, ok ? 4 : 0);
+  }
+}
+
 // Shared memory of the staged SYMV: STAGES x (tile + x_J + x_I) + column sums.
 // 8 rhs: one 84 KB stage per CTA and two CTAs per SM (each CTA's load
 // overlaps the other's tile pass; 16 warps hide the DMMA and shared-memory
@@ -513,7 +526,7 @@ constexpr size_t symv_staged_smem() {
 template <int NR>
 __global__ void __launch_bounds__(NTH, NR >= 8 ? 2 : 1)
 symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __restrict__ x,
-                   double* __restrict__ y, const int* skip, double* fro, int nfro) {
+                   double* __restrict__ y, const int* skip, double* fro, int nfro, int al16) {
   if (skip != nullptr && *skip) return;
   constexpr int STAGES = symv_stages<NR>();
   constexpr bool MMA = NR == 8;
@@ -530,12 +543,15 @@ symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __
     tri_of(t, I, J);
     const int i0 = I * RB, j0 = J * RB;
     const int ni = min(RB, n - i0), nj = min(RB, n - j0);
+    const float* T = A + (size_t)j0 * lda + i0;
     if (MMA) {
-      stage_tile_bl(tiles + stage * TE, A + (size_t)j0 * lda + i0, lda, ni, nj);
+      if (al16) stage_tile_bl(tiles + stage * TE, T, lda, ni, nj);
+      else stage_tile_4b<true>(tiles + stage * TE, T, lda, ni, nj);
       stage_vec_x8(x, n, j0, nj, vecs + (2 * stage) * VEC);
       stage_vec_x8(x, n, i0, ni, vecs + (2 * stage + 1) * VEC);
     } else {
-      stage_tile(tiles + stage * TE, A + (size_t)j0 * lda + i0, lda, ni, nj);
+      if (al16) stage_tile(tiles + stage * TE, T, lda, ni, nj);
+      else stage_tile_4b<false>(tiles + stage * TE, T, lda, ni, nj);
       stage_vec<NR>(x, n, j0, nj, vecs + (2 * stage) * VEC);
       stage_vec<NR>(x, n, i0, ni, vecs + (2 * stage + 1) * VEC);
     }
@@ -1233,19 +1249,6 @@ __device__ __forceinline__ double* bslot(const BatchSys& S, int slot, int nr) {
   return S.vec + (size_t)slot * S.n * nr;
 }
 
-// A tile whose columns need not start on 16-byte boundaries, by 4-byte
-// copies into the plain (BL = false) or blocked (BL = true) layout.
-template <bool BL>
-__device__ __forceinline__ void stage_tile_4b(float* dst, const float* T, int ld, int rows_valid,
-                                              int cols_valid) {
-#pragma unroll 4
-  for (int e = threadIdx.x; e < TILE_ELEMS; e += NTH) {
-    const int c = e / RB, r = e % RB;
-    const bool ok = c < cols_valid && r < rows_valid;
-    cp_async4(dst + (BL ? bl_off(r, c) : c * RB + r), ok ? T + (size_t)c * ld + r : T, ok ? 4 : 0);
-  }
-}
-
 // One unit of the batched operator product: tile (I, J) of one system's
 // lower triangle.  A == nullptr: the system has converged, nothing to do.
 struct SymvUnit {
@@ -1430,23 +1433,22 @@ panel_batched_kernel(const BatchSys* __restrict__ sys, int sup, int v_slot, int 
                         use_skip ? S.done : nullptr, make_uint3(blockIdx.x, blockIdx.y, 0));
 }
 
-// The persistent solve's inputs: work <- in, out <- 0 and its dependency
-// counters cleared, in one launch.
-__global__ void trsv_prep_kernel(const double* __restrict__ in, double* __restrict__ work,
-                                 double* __restrict__ out, long long count, int* counters,
-                                 int ncounters, const int* skip) {
-  if (skip != nullptr && *skip) return;
+// The inputs of a forward and a backward solve: w <- in, their targets zero and
+// their dependency counters cleared.
+__global__ void trsv_prep_kernel(const double* __restrict__ in, double* __restrict__ w,
+                                 double* __restrict__ mid, double* __restrict__ out, long long count,
+                                 int* counters, int ncounters) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (long long i = t0; i < count; i += stride) {
-    work[i] = in[i];
+    w[i] = in[i];
+    mid[i] = 0.0;
     out[i] = 0.0;
   }
   for (long long i = t0; i < ncounters; i += stride) counters[i] = 0;
 }
 
-__global__ void zero_vec_kernel(double* __restrict__ a, long long count, const int* skip) {
-  if (skip != nullptr && *skip) return;
+__global__ void zero_vec_kernel(double* __restrict__ a, long long count) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
        i += (long long)gridDim.x * blockDim.x)
     a[i] = 0.0;
@@ -1494,7 +1496,6 @@ cudaError_t solve_set_attributes() {
   cudaError_t e;
   if ((e = set_dyn(block_inverse_kernel, kBlockInvSmem)) != cudaSuccess) return e;
 #define SET_NR(NRC)                                                                         \
-  if ((e = set_dyn(symv_kernel<float, NRC>, red_bytes(NRC))) != cudaSuccess) return e;      \
   if ((e = set_dyn(symv_kernel<double, NRC>, red_bytes(NRC))) != cudaSuccess) return e;
   SET_NR(1) SET_NR(2) SET_NR(4) SET_NR(8)
 #undef SET_NR
@@ -1525,28 +1526,25 @@ int sm_count() {
   return c;
 }
 
-// FP32 operators whose columns start on 16-byte boundaries stream through
-// the staged persistent kernel; others (and FP64 operators) take one CTA per
-// tile with register loads.
-template <typename TA>
-bool symv_staged_ok(const TA* A, int lda) {
-  return sizeof(TA) == 4 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
+cudaError_t launch_zero_vec(double* y, long long count, cudaStream_t stream) {
+  zero_vec_kernel<<<148, 256, 0, stream>>>(y, count);
+  return cudaGetLastError();
 }
-template bool symv_staged_ok<float>(const float*, int);
-template bool symv_staged_ok<double>(const double*, int);
 
+// FP32 operators stream through the staged persistent kernel (4-byte copies
+// where columns do not start on 16-byte boundaries: n = 2999, 4 rhs, 28 us by
+// register loads of one tile per CTA against 22 us); FP64 operators take one
+// CTA per tile with register loads.
 template <typename TA>
 cudaError_t launch_symv_skip(const TA* A, int lda, int n, const double* x, double* y, int nrhs,
                              const int* skip, cudaStream_t stream, double* fro, int nfro) {
-  const long long cnt = (long long)n * nrhs;
-  zero_vec_kernel<<<148, 256, 0, stream>>>(y, cnt, skip);
   const int T = ceil_div(n, RB);
   const int ntiles = T * (T + 1) / 2;
-  if (symv_staged_ok(A, lda)) {
+  if constexpr (sizeof(TA) == 4) {
     int grid = std::min(ntiles, (nrhs >= 8 ? 2 : 1) * sm_count());
     if (fro != nullptr) grid = std::min(grid, nfro);   // one Frobenius partial per CTA
-    const float* Af = reinterpret_cast<const float*>(A);
-    NR_SWITCH(nrhs, (symv_staged_kernel<NRC><<<grid, NTH, symv_staged_smem<NRC>(), stream>>>(Af, lda, n, x, y, skip, fro, nfro)));
+    const int al16 = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
+    NR_SWITCH(nrhs, (symv_staged_kernel<NRC><<<grid, NTH, symv_staged_smem<NRC>(), stream>>>(A, lda, n, x, y, skip, fro, nfro, al16)));
   } else {
     NR_SWITCH(nrhs, (symv_kernel<TA, NRC><<<ntiles, NTH, red_bytes(NRC), stream>>>(A, lda, n, x, y, skip)));
   }
@@ -1632,17 +1630,18 @@ cudaError_t launch_trsv_batched(bool backward, const BatchSys* sys, int nsys, in
 
 size_t trsv_counter_ints(int n) { return 1 + 2 * (size_t)ceil_div(n, RB); }
 
-// The persistent solve: work <- in, out <- 0 and the counters
-// (trsv_counter_ints(n) ints) cleared in one launch, then one cooperative
-// launch over every resident CTA.
+cudaError_t launch_trsv_prep(const double* in, double* w, double* mid, double* out, int n, int nrhs,
+                             int* counters, cudaStream_t stream) {
+  trsv_prep_kernel<<<148, 256, 0, stream>>>(in, w, mid, out, (long long)n * nrhs, counters,
+                                            2 * (int)trsv_counter_ints(n));
+  return cudaGetLastError();
+}
+
+// One cooperative launch over every resident CTA.
 cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n,
-                                   const float* wsup, const double* in, double* out,
-                                   double* work, int nrhs, int* counters, const int* skip,
-                                   DevStatus* st, cudaStream_t stream) {
-  const long long cnt = (long long)n * nrhs;
+                                   const float* wsup, double* work, double* out, int nrhs, int* counters,
+                                   const int* skip, DevStatus* st, cudaStream_t stream) {
   cudaError_t e;
-  trsv_prep_kernel<<<148, 256, 0, stream>>>(in, work, out, cnt, counters, (int)trsv_counter_ints(n),
-                                            skip);
   static int grid_cache[64][2][4] = {};
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -95,7 +95,7 @@ __global__ void frob_lower_kernel(const TA* __restrict__ A, int lda, int n, doub
     }
   }
   s += 2.0 * ((s4[0] + s4[1]) + (s4[2] + s4[3]));
-  __shared__ double red[8];
+  __shared__ double red[32];
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -211,7 +211,7 @@ template cudaError_t launch_copy_lower<double>(const double*, int, float*, int, 
 
 template <typename TA>
 cudaError_t launch_frob_lower(const TA* A, int lda, int n, double* partials, cudaStream_t stream) {
-  frob_lower_kernel<TA><<<pcg_vgrid(), 256, 0, stream>>>(A, lda, n, partials);
+  frob_lower_kernel<TA><<<pcg_vgrid(), 1024, 0, stream>>>(A, lda, n, partials);
   return cudaGetLastError();
 }
 template cudaError_t launch_frob_lower<float>(const float*, int, int, double*, cudaStream_t);
