@@ -152,8 +152,10 @@ struct PcgGraph {
 // Create + destroy at n = 3072: 3.6 ms with one allocation per buffer, 0.70
 // with one for all.
 // The scalar block of a factor object (doubles): misc at 0, ||b||^2 at 32, rho
-// at 40, the factor's and the solve's status at 56, done and loop control at 60.
-constexpr int kScalBnorm = 32, kScalRho = 40, kScalStatus = 56, kScalDone = 60, kScalDoubles = 64;
+// at 40, the factor's and the solve's status at 56, done and loop control at 60,
+// the small solve's barrier at 62.
+constexpr int kScalBnorm = 32, kScalRho = 40, kScalStatus = 56, kScalDone = 60, kScalBarrier = 62,
+              kScalDoubles = 64;
 static_assert(sizeof(DevStatus) == 16, "two status words take four doubles");
 
 struct Resources {
@@ -950,8 +952,9 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
   constexpr bool fro_fused = sizeof(TA) == 4;
   mpchol_status ss = ensure_solve(f, stream);
   if (ss != MPCHOL_OK) return ss;
-  PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_pcg_begin(v, dB, nrhs, po.x0_precond != 0, stream));
-  if (po.x0_precond) {
+  const bool small = pcg_small_ok(n, nr, sizeof(TA), f->nsm);
+  if (!small) PHASE(MPCHOL_PH_PCG_VEC, 1, stream, launch_pcg_begin(v, dB, nrhs, po.x0_precond != 0, stream));
+  if (!small && po.x0_precond) {
     mpchol_status s0 = apply_precond(f, v.work, v.tmp, v.x, nr, nullptr, stream);
     if (s0 != MPCHOL_OK) return s0;
   }
@@ -996,7 +999,18 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     PHASE(MPCHOL_PH_PCG_VEC, 1, s, launch_update_p(v, tol2, loop, s));
     return MPCHOL_OK;
   };
-  if ((ss = true_residual(true)) != MPCHOL_OK) return ss;
+  if (small) {
+    // the solve's status, done and loop words and the barrier's, then all of it
+    MPCHOL_CUDA_TRY(cudaMemsetAsync(f->pstatus, 0, sizeof(double) * (kScalDoubles - kScalStatus - 2), stream));
+    PHASE(MPCHOL_PH_PCG_VEC, 1, stream,
+          launch_pcg_small<TA>(dA, lda, dB, nrhs, dX, f->wsup, v, tol2, po.max_it, max_restarts,
+                               po.x0_precond != 0, f->status,
+                               reinterpret_cast<unsigned*>(f->scal + kScalBarrier), stream));
+    mpchol_status rs = read_back();
+    if (rs != MPCHOL_OK) return rs;
+  } else if ((ss = true_residual(true)) != MPCHOL_OK) {
+    return ss;
+  }
   // The iterations run in a device-side loop: one launch of a CUDA graph
   // whose WHILE node repeats one iteration until the recursive residual meets
   // the tolerance, an error is recorded or the budget is spent, with no host
@@ -1012,7 +1026,7 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     g.A = dA; g.lda = lda; g.nr = nr; g.elem = (int)sizeof(TA); g.tol2 = tol2;
   }
   if (g.calls < 3) ++g.calls;
-  bool use_graph = !profiling_on() && !g.failed && g.calls >= 3 && po.max_it > 0;
+  bool use_graph = !small && !profiling_on() && !g.failed && g.calls >= 3 && po.max_it > 0;
   if (use_graph && g.exec == nullptr) {
     // capture on a private stream (the caller's may be the legacy default
     // stream, which cannot be captured); the graph is launched into the
@@ -1057,7 +1071,9 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     }
   }
   for (int restart = 0;; ++restart) {
-    if (po.max_it > 0 && restart <= max_restarts && it < po.max_it) {
+    if (small) {
+      // read back above
+    } else if (po.max_it > 0 && restart <= max_restarts && it < po.max_it) {
       // The iterations are enqueued without waiting for the residual's
       // verdict: if it is met already (or the factor failed), done is set and
       // they return at once.
@@ -1106,9 +1122,10 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
     converged = true;
     for (int k = 0; k < nrhs; ++k)
       if (!(f->res.h_scal[k] <= tol2 * f->res.h_scal[kScalBnorm + k])) converged = false;
-    if (converged || it >= po.max_it || restart > max_restarts) break;
+    if (small || converged || it >= po.max_it || restart > max_restarts) break;
   }
-  MPCHOL_CUDA_TRY(cudaMemcpyAsync(dX, v.x, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, stream));
+  if (!small)
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(dX, v.x, sizeof(double) * n * nrhs, cudaMemcpyDeviceToDevice, stream));
   if (rep != nullptr) {
     double relmax = 0.0, bemax = 0.0, prmax = 0.0;
     const double* h = f->res.h_scal;

@@ -66,6 +66,16 @@ cudaError_t launch_dot_rz(const PcgVectors& v, cudaStream_t stream);
 cudaError_t launch_update_p(const PcgVectors& v, double tol2, const cudaGraphConditionalHandle* loop,
                             cudaStream_t stream);
 
+// A whole solve in one cooperative launch (pcg_small.cu), for systems it fits:
+// nr padded right-hand sides, operator elements of elem bytes.  bar: a zeroed
+// word; v's status zero on entry.  Writes X (n x nrhs), the scalars of v, done
+// (converged, iterations).
+bool pcg_small_ok(int n, int nr, int elem, int nsm);
+template <typename TA>
+cudaError_t launch_pcg_small(const TA* A, int lda, const double* B, int nrhs, double* X, const float* W,
+                             const PcgVectors& v, double tol2, int max_it, int max_restarts, bool x0,
+                             const DevStatus* factor_st, unsigned* bar, cudaStream_t stream);
+
 // misc device utilities (util.cu)
 cudaError_t launch_extract_diag(const float* A, int lda, int n, float* d, float* dtilde,
                                 cudaStream_t stream);

@@ -173,3 +173,43 @@ def test_fp32_trailing_update_sizes(m, k, pad):
     C2 = C.clone()
     C2[:, :m].t()[low] = before[:, :m].t()[low]
     assert torch.equal(C2, before)                              # nothing else is touched
+
+
+@pytest.mark.parametrize("n,nrhs,f64", [(1, 1, False), (7, 3, False), (8, 1, True), (129, 8, False),
+                                        (511, 2, True), (513, 5, False), (1000, 1, False), (1017, 4, True),
+                                        (1024, 8, False), (1024, 1, True), (1024, 8, True), (1025, 2, False)])
+def test_small_solves_match_the_dense_solve(n, nrhs, f64):
+    """The one-launch solve at the edges of its range (and the sizes that fall
+    to the general path): iterations as for a general-path order, residual at
+    the tolerance, solution within kappa * tolerance of the FP64 dense solve."""
+    A = matgen.spd_matrix(n, 1e3, n).cuda() if n > 1 else torch.full((1, 1), 2.0, device="cuda")
+    B = matgen.rhs(n, nrhs, n + 1).cuda().reshape(n, -1)
+    f = mp.factor(A, block_size=128, precision="fp16")
+    Ad = A.double()
+    for x0 in (True, False):
+        X, rep = f.pcg(Ad if f64 else A, B, rel_tol=1e-11, x0_precond=x0)
+        assert rep.converged and rep.rel_residual <= 1e-11
+        true = ((B - Ad @ X).norm(dim=0) / B.norm(dim=0)).max().item()
+        assert true <= 2e-11
+        ref = torch.linalg.solve(Ad, B)
+        assert ((X - ref).norm() / ref.norm()).item() <= 1e-8
+        fro, xn = Ad.norm().item(), X.norm(dim=0)
+        be = ((B - Ad @ X).norm(dim=0) / (fro * xn + B.norm(dim=0))).max().item()
+        assert abs(rep.backward_error - be) <= 0.5 * be + 1e-15
+
+
+def test_small_solve_stops_at_its_iteration_budget_and_reports_failures():
+    n = 300
+    A = matgen.spd_matrix(n, 1e4, 3).cuda()
+    B = matgen.rhs(n, 2, 4).cuda()
+    f = mp.factor(A, block_size=128, precision="fp16")
+    for budget in (0, 1, 3):
+        X, rep = f.pcg(A, B, rel_tol=1e-14, max_it=budget)
+        assert rep.iterations == budget and not rep.converged
+    bad = -A
+    with pytest.raises(mp.MpcholError) as e:
+        mp.factor(bad, block_size=128, precision="fp16", diag_pert=0).pcg(A, B)
+    assert e.value.status == 2
+    with pytest.raises(mp.MpcholError) as e:      # an indefinite operator: p^T A p < 0
+        f.pcg(bad, B)
+    assert e.value.status == 6
