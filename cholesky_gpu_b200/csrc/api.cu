@@ -344,7 +344,7 @@ struct mpchol_factor {
   CopyPlan plan;
   int nsm = 0;
   CUtensorMap tmap32;         // TMA map over A, 32 x 32 boxes
-  CUtensorMap tmapX;          // TMA map over A, 32 x b boxes (panel slabs)
+  CUtensorMap tmapX, tmapX16; // TMA maps over A, 32 x b and 16 x b boxes (panel slabs)
 };
 
 namespace {
@@ -712,7 +712,7 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
       if (m <= 0) break;
       const QuantAll qa = qa_for(k);
       PHASE(MPCHOL_PH_TRSM, 1, stream,
-            launch_trsm_panel(f->tmapX, f->tmap32, f->A, ld, n, s, bs, f->winv, f->d, f->dtilde,
+            launch_trsm_panel(f->tmapX, f->tmapX16, f->tmap32, f->A, ld, n, s, bs, f->winv, f->d, f->dtilde,
                               f->rowsq, &f->steps[k], &f->steps[k + 1], std::min(b, m), dp, qa,
                               f->status, stream, k > 0 ? &f->steps[k - 1] : nullptr,
                               dp.coherence ? f->colacc + (size_t)k * kColCopies * b : nullptr));
@@ -740,7 +740,7 @@ mpchol_status run_factor(mpchol_factor_t* f, cudaStream_t stream, const CopyPlan
     // panel solve, step decision and panel quantization in one launch
     const QuantAll qa = qa_for(k);
     PHASE(MPCHOL_PH_TRSM, 1, stream,
-          launch_trsm_panel(f->tmapX, f->tmap32, f->A, ld, n, s, bs, f->winv, f->d, f->dtilde,
+          launch_trsm_panel(f->tmapX, f->tmapX16, f->tmap32, f->A, ld, n, s, bs, f->winv, f->d, f->dtilde,
                             f->rowsq, &f->steps[k], &f->steps[k + 1], next_bs, dp, qa, f->status,
                             stream, k > 0 ? &f->steps[k - 1] : nullptr,
                             dp.coherence ? f->colacc + (size_t)k * kColCopies * b : nullptr));
@@ -1388,6 +1388,8 @@ mpchol_status mpchol_factor_create(const mpchol_opts* opts, int n, mpchol_factor
   if (!encode_tmap_2d(&f->tmap32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, f->A, n, n, f->ld, 32, 32,
                       CU_TENSOR_MAP_SWIZZLE_NONE) ||
       !encode_tmap_2d(&f->tmapX, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, f->A, n, n, f->ld, 32,
+                      f->b, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+      !encode_tmap_2d(&f->tmapX16, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, f->A, n, n, f->ld, 16,
                       f->b, CU_TENSOR_MAP_SWIZZLE_NONE)) {
     free_factor(f);
     return MPCHOL_ERR_CUDA;

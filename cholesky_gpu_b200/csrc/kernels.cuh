@@ -88,20 +88,21 @@ struct QuantAll {
 __host__ __device__ inline int q8_slot(int fmt) { return fmt == E4M3 ? 0 : (fmt == E5M2 ? 1 : 2); }
 __host__ __device__ inline int rexp_slot(int fmt) { return fmt == E4M3 ? 0 : (fmt == E5M2 ? 1 : 2); }
 // Solves X * L11^T = A21 in place for rows [s+bs, n) of block column s, one
-// slab of 32 or 64 rows per CTA; subtracts each row's sum of squares from dtilde,
+// slab of 16, 32 or 64 rows per CTA; subtracts each row's sum of squares from dtilde,
 // stores it in rowsq, folds the switching statistics into step (and the FP64
 // flag of the next diagonal block into next), and writes the slab's codes in
 // every candidate format.  The last CTA to finish resolves the step precision
 // (step->prec).  Before its rows' sums of squares are overwritten, each CTA
 // adds the previous step's rounding shift u(prev->prec) * rowsq to qa.sh for
 // its rows (prev null: first step); the rows of the next diagonal block get
-// theirs in its POTRF.  tmapX: TMA map over A with 32 x bs boxes; tmap32: with
+// theirs in its POTRF.  tmapX, tmapX16: TMA maps over A with 32 x bs and 16 x bs boxes; tmap32: with
 // 32 x 32 boxes.
 // colacc (coherence rule, nullable otherwise): kColCopies x bs FP64
 // accumulators, zeroed before the launch, that receive the panel's column
 // sums (slab i adds into copy i % kColCopies).
 constexpr int kColCopies = 8;
-cudaError_t launch_trsm_panel(const CUtensorMap& tmapX, const CUtensorMap& tmap32, float* A,
+cudaError_t launch_trsm_panel(const CUtensorMap& tmapX, const CUtensorMap& tmapX16,
+                              const CUtensorMap& tmap32, float* A,
                               int lda, int n, int s, int bs, const float* winv, const float* d,
                               float* dtilde, float* rowsq, StepState* step, StepState* next,
                               int next_bs, const DecisionParams& dp, const QuantAll& qa,

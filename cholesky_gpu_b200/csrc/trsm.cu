@@ -6,8 +6,8 @@
 // (src/kernels_macros.cuh:191-211).
 //
 // X * L11^T = A21 for the m rows below the diagonal block.  Rows are
-// independent, so one CTA of 16 warps owns a slab of 32 or 64 rows (64 while
-// the panel has more 32-row slabs than the GPU has SMs).  TMA stages the slab
+// independent, so one CTA of 16 warps owns a slab of 16, 32 or 64 rows (the
+// smallest of which the panel has at most one per SM, else 64).  TMA stages the slab
 // and all of L11: the strictly-lower 32 x 32 tiles L_{J,M} as 2-D boxes and
 // the inverses of the diagonal tiles L_JJ, which the POTRF kernel wrote, as
 // 1-D bulk copies, one mbarrier per tile row.  The solve is a pipeline over
@@ -41,11 +41,36 @@ constexpr int MAXNT = 8;     // tiles per block column (b <= 256)
 
 __device__ __forceinline__ int tl(int I, int M) { return I * (I - 1) / 2 + M; }  // I > M
 
-// The slab in shared memory: 32-row halves, each column-major with its 32
-// rows contiguous (the layout of a 32 x bs TMA box), so lane l reading row l
-// (or l + 32) of one column touches 32 different banks.
+// The slab of TR rows in shared memory: parts of HR = min(TR, 32) rows, each
+// column-major with its rows contiguous (the layout of an HR x bs TMA box), so
+// lane l reading row l of one column of a 32- or 64-row slab touches 32
+// different banks.
+template <int TR>
+struct Slab {
+  static constexpr int HR = TR < 32 ? TR : 32;   // rows per part
+  static constexpr int RPL = TR / HR;            // parts
+  static constexpr int RT = HR / 8;              // rows of a part per thread of the solve
+};
+template <int TR>
 __device__ __forceinline__ int xoff(int r, int c, int bs) {
-  return (r >> 5) * bs * 32 + c * 32 + (r & 31);
+  constexpr int HR = Slab<TR>::HR;
+  return (r / HR) * bs * HR + c * HR + r % HR;
+}
+template <int N>
+__device__ __forceinline__ void load_rows(const float* p, float (&v)[N]) {
+  if constexpr (N == 4) {
+    const float4 w = *reinterpret_cast<const float4*>(p);
+    v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+  } else {
+    static_assert(N == 2, "two or four rows per thread");
+    const float2 w = *reinterpret_cast<const float2*>(p);
+    v[0] = w.x; v[1] = w.y;
+  }
+}
+template <int N>
+__device__ __forceinline__ void store_rows(float* p, const float (&v)[N]) {
+  if constexpr (N == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
 }
 
 // Code staging panel of the epilogue (32-bit words): FP16X2 hi + lo rows of
@@ -68,75 +93,70 @@ __device__ __forceinline__ void pair_sync(int J) {   // the two warps of tile co
 
 // The slab solve.  The warp pair of tile column J (warps 2J, 2J + 1; w = 2J +
 // h) computes the TR x 32 tile X_J: thread t of the pair (t = 32 h + lane)
-// holds a block of 4 RPL rows x 4 columns in registers, rows 4 rg .. 4 rg + 3
-// of each 32-row half (rg = t % 8) and columns 4 cg .. 4 cg + 3 (cg = t / 8),
-// so every k step of the tile products reads 16-byte vectors of X (one per
-// half) and of L (one), and a quarter-warp's eight X vectors are 128
-// contiguous bytes.  Lt: L11's tiles L_{I,M} (I > M) at tl(I, M) * TSZ; Wt:
-// the inverses W_JJ = L_JJ^-1, tile J at J * TSZ; both column-major (L(c, m)
-// at m * 32 + c, W(c, m) zero for m > c).  lrow[J] (null: already staged)
-// completes when tile row J has landed; ready[J] (64 arrivals) when X_J is
-// final:
+// holds RT rows of each part (rows RT rg ..) x 4 columns (4 cg ..) in
+// registers, so every k step of the tile products reads a vector of X per part
+// and one of L.  The lane's bits interleave into rg and cg so that four
+// neighbouring lanes read two different vectors of each (2.2 cycles of the
+// SM's shared memory per 16-byte load; 4.0 when they read four).  Lt: L11's
+// tiles L_{I,M} (I > M) at tl(I, M) * TSZ; Wt: the inverses W_JJ = L_JJ^-1,
+// tile J at J * TSZ; both column-major (L(c, m) at m * 32 + c, W(c, m) zero
+// for m > c).  lrow[J] (null: already staged) completes when tile row J has
+// landed; ready[J] (64 arrivals) when X_J is final:
 //   X_J = (A_J - sum_{K<J} X_K L_{J,K}^T) W_JJ^T.
 // Each output is one fma chain in a fixed order: the update over K, then m;
 // the diagonal multiply over m.  Returns false if a bounded wait gave up.
-template <int RPL>
+template <int TR>
 __device__ bool slab_solve(float* Xs, int bs, const float* Lt, const float* Wt, uint64_t* lrow,
                            uint64_t* ready, int tid) {
+  constexpr int HR = Slab<TR>::HR, RPL = Slab<TR>::RPL, RT = Slab<TR>::RT;
   const int NT = bs / 32;
   const int warp = tid >> 5, lane = tid & 31;
   const int J = warp >> 1, h = warp & 1;
   if (J >= NT) return true;
-  const int XH = bs * 32;                              // floats per 32-row half
-  const int t = 32 * h + lane;
-  const int rg = t & 7, cg = t >> 3;
-  const int r0 = 4 * rg;                               // rows r0.. of each half
+  const int XH = bs * HR;                              // floats per part
+  const int rg = (lane & 1) | ((lane >> 1) & 6), cg = ((lane >> 1) & 1) | ((lane >> 3) & 2) | (h << 2);
+  const int r0 = RT * rg;                              // rows r0.. of each part
   const int cl = 4 * cg;                               // columns cl.. of the tile
   bool ok = lrow == nullptr || tc::mbar_wait(&lrow[J], 0);
-  float acc[RPL][4][4];                                // [half][row][column]
+  float acc[RPL][4][RT];                               // [part][column][row]
 #pragma unroll
   for (int q = 0; q < RPL; ++q)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float4 v = *reinterpret_cast<const float4*>(Xs + q * XH + (32 * J + cl + j) * 32 + r0);
-      acc[q][0][j] = v.x; acc[q][1][j] = v.y; acc[q][2][j] = v.z; acc[q][3][j] = v.w;
-    }
+    for (int j = 0; j < 4; ++j) load_rows<RT>(Xs + q * XH + (32 * J + cl + j) * HR + r0, acc[q][j]);
 #pragma unroll 1
   for (int K = 0; K < J; ++K) {
     ok = tc::mbar_wait(&ready[K], 0) && ok;
     const float* L = Lt + (size_t)tl(J, K) * TSZ + cl;
-    const float* xk = Xs + 32 * K * 32 + r0;
+    const float* xk = Xs + 32 * K * HR + r0;
 #pragma unroll 8
     for (int m = 0; m < 32; ++m) {
       const float4 lv = *reinterpret_cast<const float4*>(L + m * 32);
       const float l[4] = {lv.x, lv.y, lv.z, lv.w};
 #pragma unroll
       for (int q = 0; q < RPL; ++q) {
-        const float4 xv = *reinterpret_cast<const float4*>(xk + q * XH + m * 32);
-        const float x[4] = {xv.x, xv.y, xv.z, xv.w};
+        float x[RT];
+        load_rows<RT>(xk + q * XH + m * HR, x);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[q][i][j] = fmaf(-x[i], l[j], acc[q][i][j]);
+          for (int i = 0; i < RT; ++i) acc[q][j][i] = fmaf(-x[i], l[j], acc[q][j][i]);
       }
     }
   }
   // the updated tile into the slab, then X_J = Y W_JJ^T
-  float* xj = Xs + 32 * J * 32 + r0;
+  float* xj = Xs + 32 * J * HR + r0;
 #pragma unroll
   for (int q = 0; q < RPL; ++q)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float4*>(xj + q * XH + (cl + j) * 32) =
-          make_float4(acc[q][0][j], acc[q][1][j], acc[q][2][j], acc[q][3][j]);
+    for (int j = 0; j < 4; ++j) store_rows<RT>(xj + q * XH + (cl + j) * HR, acc[q][j]);
   pair_sync(J);
   const float* W = Wt + (size_t)J * TSZ + cl;
 #pragma unroll
   for (int q = 0; q < RPL; ++q)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[q][i][j] = 0.0f;
+      for (int i = 0; i < RT; ++i) acc[q][j][i] = 0.0f;
   const int mend = 16 * h + 16;                        // W(c, m) = 0 for m > c (the warp's columns)
 #pragma unroll 8
   for (int m = 0; m < mend; ++m) {
@@ -144,22 +164,20 @@ __device__ bool slab_solve(float* Xs, int bs, const float* Lt, const float* Wt, 
     const float w[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
     for (int q = 0; q < RPL; ++q) {
-      const float4 yv = *reinterpret_cast<const float4*>(xj + q * XH + m * 32);
-      const float y[4] = {yv.x, yv.y, yv.z, yv.w};
+      float y[RT];
+      load_rows<RT>(xj + q * XH + m * HR, y);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[q][i][j] = fmaf(y[i], w[j], acc[q][i][j]);
+        for (int i = 0; i < RT; ++i) acc[q][j][i] = fmaf(y[i], w[j], acc[q][j][i]);
     }
   }
   pair_sync(J);                                        // every read of Y is done
 #pragma unroll
   for (int q = 0; q < RPL; ++q)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float4*>(xj + q * XH + (cl + j) * 32) =
-          make_float4(acc[q][0][j], acc[q][1][j], acc[q][2][j], acc[q][3][j]);
-  tc::mbar_arrive(&ready[J]);                              // release: X_J to the later tiles
+    for (int j = 0; j < 4; ++j) store_rows<RT>(xj + q * XH + (cl + j) * HR, acc[q][j]);
+  tc::mbar_arrive(&ready[J]);                          // release: X_J to the later tiles
   return ok;
 }
 
@@ -178,7 +196,7 @@ __device__ __forceinline__ void slab_row_partials(const float* Xs, int bs, float
   if (part < NT) {
 #pragma unroll 8
     for (int c = part * 32; c < part * 32 + 32; ++c) {
-      const float v = Xs[xoff(r, c, bs)];
+      const float v = Xs[xoff<TR>(r, c, bs)];
       sq = __fmaf_rn(v, v, sq);
       amax = fmaxf(amax, fabsf(v));
     }
@@ -222,7 +240,7 @@ __device__ __forceinline__ void stage_codes8(const float* Xs, int bs, int nrows,
   const int cb = part * 32;
   float v[32];
 #pragma unroll
-  for (int u = 0; u < 32; ++u) v[u] = Xs[xoff(r, cb + u, bs)];
+  for (int u = 0; u < 32; ++u) v[u] = Xs[xoff<TR>(r, cb + u, bs)];
   float inv;
   if constexpr (MX) {
     float mx[8];
@@ -270,7 +288,7 @@ __device__ void quantize_slab(const float* Xs, int bs, int nrows, int gi0, int m
     if (cw == 32) {
 #pragma unroll
       for (int c = c0; c < c0 + 32; c += 2) {
-        const float x0 = Xs[xoff(r, c, bs)] * inv, x1 = Xs[xoff(r, c + 1, bs)] * inv;
+        const float x0 = Xs[xoff<TR>(r, c, bs)] * inv, x1 = Xs[xoff<TR>(r, c + 1, bs)] * inv;
         const __half2 h = __floats2half2_rn(x0, x1);
         hi[r * sw + c / 2] = *reinterpret_cast<const uint32_t*>(&h);
         if (fmt == FP16X2) {   // x - hi is exact in FP32
@@ -281,13 +299,17 @@ __device__ void quantize_slab(const float* Xs, int bs, int nrows, int gi0, int m
     }
     if (live && part == 0) qa.rexp[2][gi] = (int8_t)e;
     __syncthreads();
+    // a warp per row (no index division)
     const int wpr = bs / 2;                    // words per row
+#pragma unroll 2
+    for (int rr = tid >> 5; rr < nrows; rr += NTHR / 32) {
+      uint32_t* dh = reinterpret_cast<uint32_t*>(qa.q16 + (size_t)(gi0 + rr) * qa.ldq);
+      uint32_t* dl = reinterpret_cast<uint32_t*>(qa.q16 + (size_t)(m + gi0 + rr) * qa.ldq);
 #pragma unroll 4
-    for (int q = tid; q < nrows * wpr; q += NTHR) {
-      const int rr = q / wpr, w = q % wpr;
-      reinterpret_cast<uint32_t*>(qa.q16 + (size_t)(gi0 + rr) * qa.ldq)[w] = hi[rr * sw + w];
-      if (fmt == FP16X2)
-        reinterpret_cast<uint32_t*>(qa.q16 + (size_t)(m + gi0 + rr) * qa.ldq)[w] = lo[rr * sw + w];
+      for (int w = tid & 31; w < wpr; w += 32) {
+        dh[w] = hi[rr * sw + w];
+        if (fmt == FP16X2) dl[w] = lo[rr * sw + w];
+      }
     }
   } else {
     switch (fmt) {
@@ -303,30 +325,31 @@ __device__ void quantize_slab(const float* Xs, int bs, int nrows, int gi0, int m
     const int sw = bs / 4 + 1;
     const int wpr = bs / 4;
 #pragma unroll 4
-    for (int q4 = tid; q4 < nrows * wpr; q4 += NTHR) {
-      const int rr = q4 / wpr, w = q4 % wpr;
-      reinterpret_cast<uint32_t*>(q + (size_t)(gi0 + rr) * qa.ldq)[w] = stage[rr * sw + w];
+    for (int rr = tid >> 5; rr < nrows; rr += NTHR / 32) {
+      uint32_t* d = reinterpret_cast<uint32_t*>(q + (size_t)(gi0 + rr) * qa.ldq);
+#pragma unroll 2
+      for (int w = tid & 31; w < wpr; w += 32) d[w] = stage[rr * sw + w];
     }
   }
   __syncthreads();                             // the staging panel is reused
 }
 
-// Panel solve with the quantization of the panel fused in; one slab of TR =
-// 32 * RPL rows per CTA (the launch may exceed the resident CTAs: no CTA
+// Panel solve with the quantization of the panel fused in; one slab of TR
+// rows per CTA (the launch may exceed the resident CTAs: no CTA
 // waits on another).  Each CTA stages its slab and L11 by TMA, solves the
 // slab, writes it back, folds its rows into the diagonal tracker and the
 // switching statistics, and writes the slab's codes in every candidate
 // format (the step's precision is not known yet; the trailing update reads
 // the panel of the one the step picks).  The CTA that finishes last (a
 // ticket counter) resolves the step precision.
-template <int RPL>
+template <int TR>
 __global__ void __launch_bounds__(NTHR, 1)
 trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_constant__ CUtensorMap tmap32,
                   float* __restrict__ A, int lda, int n, int s, int bs, const float* __restrict__ winv,
                   const float* __restrict__ d, float* __restrict__ dtilde, float* __restrict__ rowsq,
                   StepState* step, StepState* next, int next_bs, DecisionParams dp, DevStatus* st,
                   QuantAll qa, const StepState* prev, double* __restrict__ colacc) {
-  constexpr int TR = 32 * RPL;
+  constexpr int HR = Slab<TR>::HR, RPL = Slab<TR>::RPL;
   extern __shared__ __align__(128) float sm[];
   const int NT = bs / 32;
   float* Xs = sm;                                        // the slab (xoff layout)
@@ -369,8 +392,8 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
   __syncthreads();
   const bool issued = s_ok != 0;
   if (issued && tid == 0) {
-    tc::mbar_expect_tx(&barx, (uint32_t)(RPL * bs * 32 * sizeof(float)));
-    for (int q = 0; q < RPL; ++q) tc::tma_load_2d(Xs + q * bs * 32, &tmapX, &barx, row0 + 32 * q, s);
+    tc::mbar_expect_tx(&barx, (uint32_t)(TR * bs * sizeof(float)));
+    for (int q = 0; q < RPL; ++q) tc::tma_load_2d(Xs + q * bs * HR, &tmapX, &barx, row0 + HR * q, s);
     for (int J = 0; J < NT; ++J) {
       tc::mbar_expect_tx(&lrow[J], (uint32_t)((J + 1) * TSZ * sizeof(float)));
       for (int M = 0; M < J; ++M)
@@ -386,7 +409,7 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
   }
   __syncthreads();
   if (s_ok) {
-    if (!slab_solve<RPL>(Xs, bs, Lt, Wt, lrow, ready, tid)) {
+    if (!slab_solve<TR>(Xs, bs, Lt, Wt, lrow, ready, tid)) {
       s_ok = 0;
       set_status(st, MPCHOL_ERR_TIMEOUT, row0);
     }
@@ -405,7 +428,7 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
     __syncthreads();
     if (tid == 0) {
       for (int q = 0; q < RPL; ++q)
-        if (row0 + 32 * q < n) tc::tma_store_2d(&tmapX, Xs + q * bs * 32, row0 + 32 * q, s);
+        if (row0 + HR * q < n) tc::tma_store_2d(&tmapX, Xs + q * bs * HR, row0 + HR * q, s);
       tc::bulk_commit();
     }
     // ---- Schur diagonal tracker and switching statistics of the slab -----
@@ -445,7 +468,7 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
 #pragma unroll 8
       for (int q = 0; q < TR; ++q) {
         const int r = (q + tid) & (TR - 1);
-        cs += (r < nrows) ? Xs[xoff(r, tid, bs)] : 0.0f;
+        cs += (r < nrows) ? Xs[xoff<TR>(r, tid, bs)] : 0.0f;
       }
       atomicAdd(colacc + (size_t)(slab % kColCopies) * bs + tid, (double)cs);
       __threadfence();
@@ -559,7 +582,7 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
   }
   for (int e = tid; e < bs * TR; e += NTHR) {
     const int c = e / TR, r = e % TR;
-    Xs[xoff(r, c, bs)] = (r < nrows) ? A[(size_t)(s + c) * ld + row0 + r] : 0.0f;
+    Xs[xoff<TR>(r, c, bs)] = (r < nrows) ? A[(size_t)(s + c) * ld + row0 + r] : 0.0f;
   }
   for (int I = 1; I < NT; ++I)
     for (int M = 0; M < I; ++M)
@@ -569,7 +592,7 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
       }
   for (int e = tid; e < NT * TSZ; e += NTHR) Wt[e] = S.winv[e];
   __syncthreads();
-  if (!slab_solve<1>(Xs, bs, Lt, Wt, nullptr, ready, tid)) {
+  if (!slab_solve<TR>(Xs, bs, Lt, Wt, nullptr, ready, tid)) {
     s_ok = 0;
     set_status(S.st, MPCHOL_ERR_TIMEOUT, row0);
   }
@@ -577,7 +600,7 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
   if (!s_ok) return;
   for (int e = tid; e < bs * TR; e += NTHR) {
     const int c = e / TR, r = e % TR;
-    if (r < nrows) S.A[(size_t)(s + c) * ld + row0 + r] = Xs[xoff(r, c, bs)];
+    if (r < nrows) S.A[(size_t)(s + c) * ld + row0 + r] = Xs[xoff<TR>(r, c, bs)];
   }
   __shared__ float s_sq[NTHR / TR][TR];
   slab_row_partials<TR>(Xs, bs, s_sq, nullptr, tid);
@@ -603,21 +626,20 @@ int sm_count() {
   return nsm;
 }
 
-template <int RPL>
+template <int TR>
 cudaError_t launch_panel(const CUtensorMap& tmapX, const CUtensorMap& tmap32, float* A, int lda,
                          int n, int s, int bs, const float* winv, const float* d, float* dtilde,
                          float* rowsq, StepState* step, StepState* next, int next_bs,
                          const DecisionParams& dp, const QuantAll& qa, DevStatus* st,
                          cudaStream_t stream, const StepState* prev, double* colacc) {
-  constexpr int TR = 32 * RPL;
   const int m = n - s - bs;
   const size_t smem = trsm_smem_floats(TR, bs) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(trsm_panel_kernel<RPL>,
+  cudaError_t e = cudaFuncSetAttribute(trsm_panel_kernel<TR>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(trsm_smem_floats(TR, 256) * sizeof(float)));
   if (e != cudaSuccess) return e;
   PdlLaunch L(dim3(ceil_div(m, TR)), dim3(NTHR), smem, stream);
-  e = cudaLaunchKernelEx(&L.cfg, trsm_panel_kernel<RPL>, tmapX, tmap32, A, lda, n, s, bs, winv, d,
+  e = cudaLaunchKernelEx(&L.cfg, trsm_panel_kernel<TR>, tmapX, tmap32, A, lda, n, s, bs, winv, d,
                          dtilde, rowsq, step, next, next_bs, dp, st, qa, prev, colacc);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
@@ -625,7 +647,8 @@ cudaError_t launch_panel(const CUtensorMap& tmapX, const CUtensorMap& tmap32, fl
 
 }  // namespace
 
-cudaError_t launch_trsm_panel(const CUtensorMap& tmapX, const CUtensorMap& tmap32, float* A,
+cudaError_t launch_trsm_panel(const CUtensorMap& tmapX, const CUtensorMap& tmapX16,
+                              const CUtensorMap& tmap32, float* A,
                               int lda, int n, int s, int bs, const float* winv, const float* d,
                               float* dtilde, float* rowsq, StepState* step, StepState* next,
                               int next_bs, const DecisionParams& dp, const QuantAll& qa,
@@ -635,13 +658,18 @@ cudaError_t launch_trsm_panel(const CUtensorMap& tmapX, const CUtensorMap& tmap3
   if (m <= 0) return cudaSuccess;
   if (bs % 32 != 0 || bs > 32 * MAXNT) return cudaErrorInvalidValue;
   // 64-row slabs while the panel has more 32-row slabs than the GPU has SMs
-  // (throughput: L11 staged once per 64 rows); 32-row slabs otherwise
-  // (latency: the per-CTA chain is half as long)
-  if (ceil_div(m, 32) > sm_count())
-    return launch_panel<2>(tmapX, tmap32, A, lda, n, s, bs, winv, d, dtilde, rowsq, step, next,
-                           next_bs, dp, qa, st, stream, prev, colacc);
-  return launch_panel<1>(tmapX, tmap32, A, lda, n, s, bs, winv, d, dtilde, rowsq, step, next,
-                         next_bs, dp, qa, st, stream, prev, colacc);
+  // (throughput: L11 staged once per 64 rows); below that the smallest slabs
+  // that all run at once (latency: a CTA's work follows its rows).  B200, b =
+  // 256, panel solve: T64 us for a 64-row slab, T32 for 32 rows, T16 for 16.
+  const int nsm = sm_count();
+  if (ceil_div(m, 32) > nsm)
+    return launch_panel<64>(tmapX, tmap32, A, lda, n, s, bs, winv, d, dtilde, rowsq, step, next,
+                            next_bs, dp, qa, st, stream, prev, colacc);
+  if (ceil_div(m, 16) > nsm)
+    return launch_panel<32>(tmapX, tmap32, A, lda, n, s, bs, winv, d, dtilde, rowsq, step, next,
+                            next_bs, dp, qa, st, stream, prev, colacc);
+  return launch_panel<16>(tmapX16, tmap32, A, lda, n, s, bs, winv, d, dtilde, rowsq, step, next,
+                          next_bs, dp, qa, st, stream, prev, colacc);
 }
 
 cudaError_t launch_trsm_batched(BatchSys* sys, int nact, int s, int b, int max_m,
