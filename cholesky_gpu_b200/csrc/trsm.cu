@@ -18,13 +18,18 @@
 //   X_J = (A_J - sum_{K<J} X_K L_{J,K}^T) L_JJ^-T,
 // where the pair of tile J applies X_K as soon as the pair of tile K has
 // published it (an mbarrier per tile, bounded waits), so the only chain is
-// one tile update plus one diagonal multiply per tile column.  The epilogue
-// writes the slab back (TMA stores), folds each row's sum of squares into the
-// Schur-diagonal tracker dtilde, reduces the switching statistics (max
-// d/dtilde, min dtilde, the reference-literal choice, the panel's column sums)
-// and the near-indefinite flag of the next diagonal block, and writes the
-// slab's codes in every candidate format.  The last CTA to finish (a ticket
-// counter) resolves the step precision.
+// one tile update plus one diagonal multiply per tile column.  A finished pair
+// sums its tile's rows and columns and writes its MX codes while the chain goes
+// on.  The epilogue writes the slab back (TMA stores), folds each row's sum of
+// squares into the Schur-diagonal tracker dtilde, reduces the switching
+// statistics (max d/dtilde, min dtilde, the reference-literal choice) and the
+// near-indefinite flag of the next diagonal block, and writes the slab's codes
+// in the other candidate formats, straight from the slab.  The last CTA to take
+// a ticket (a counter) resolves the step precision.
+//
+// Against one thread that issued every copy (about 80 cycles each), sums after
+// the solve and codes staged in shared memory on their way out (n = 1024 / 8192
+// solve, b = 256, B200): 580 -> 561 and 4459 -> 4260 us end to end.
 #include <algorithm>
 
 #include "common.cuh"
@@ -73,18 +78,11 @@ __device__ __forceinline__ void store_rows(float* p, const float (&v)[N]) {
   else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
 }
 
-// Code staging panel of the epilogue (32-bit words): FP16X2 hi + lo rows of
-// bs / 2 + 1 words, or 8-bit code rows of bs / 4 + 1 words.
-size_t stage_words(int tr, int bs) {
-  return std::max((size_t)2 * tr * (bs / 2 + 1), (size_t)tr * (bs / 4 + 1));
-}
-// Shared memory of both panel kernels (floats): the slab, then L11's
-// strictly-lower tiles and the inverses of its diagonal tiles (the code
-// staging panel reuses that space once the solve is done).
+// Shared memory of both panel kernels (floats): the slab, L11's strictly-lower
+// tiles and the inverses of its diagonal tiles.
 size_t trsm_smem_floats(int tr, int bs) {
   const int NT = bs / 32;
-  const size_t lw = (size_t)(NT * (NT - 1) / 2 + NT) * TSZ;
-  return (size_t)bs * tr + std::max(lw, stage_words(tr, bs));
+  return (size_t)bs * tr + (size_t)(NT * (NT - 1) / 2 + NT) * TSZ;
 }
 
 __device__ __forceinline__ void pair_sync(int J) {   // the two warps of tile column J
@@ -103,11 +101,13 @@ __device__ __forceinline__ void pair_sync(int J) {   // the two warps of tile co
 // for m > c).  lrow[J] (null: already staged) completes when tile row J has
 // landed; ready[J] (64 arrivals) when X_J is final:
 //   X_J = (A_J - sum_{K<J} X_K L_{J,K}^T) W_JJ^T.
-// Each output is one fma chain in a fixed order: the update over K, then m;
-// the diagonal multiply over m.  Returns false if a bounded wait gave up.
-template <int TR>
+// post(J, t) runs in the pair's threads once both warps' parts of X_J are
+// written.  Each output is one fma chain in a fixed order: the update over K,
+// then m; the diagonal multiply over m.  Returns false if a bounded wait gave
+// up.
+template <int TR, typename Post>
 __device__ bool slab_solve(float* Xs, int bs, const float* Lt, const float* Wt, uint64_t* lrow,
-                           uint64_t* ready, int tid) {
+                           uint64_t* ready, int tid, Post post) {
   constexpr int HR = Slab<TR>::HR, RPL = Slab<TR>::RPL, RT = Slab<TR>::RT;
   const int NT = bs / 32;
   const int warp = tid >> 5, lane = tid & 31;
@@ -178,31 +178,29 @@ __device__ bool slab_solve(float* Xs, int bs, const float* Lt, const float* Wt, 
 #pragma unroll
     for (int j = 0; j < 4; ++j) store_rows<RT>(xj + q * XH + (cl + j) * HR, acc[q][j]);
   tc::mbar_arrive(&ready[J]);                          // release: X_J to the later tiles
+  pair_sync(J);
+  post(J, 32 * h + lane);
   return ok;
 }
 
-// Per-row sum of squares and max |x| of the solved slab: thread (r, part) =
-// (tid % TR, tid / TR) covers row r's 32 columns `part` (sums of squares as a
-// chain of FMAs in column order), leaving the partials in s_sq / s_amax
-// [part][r]; the row's sum is then the partials added in part order (row_sq).
-// One fixed order for the streaming and the batched kernel, so both give the
-// same bits.
+// Per-row sums of squares of the solved slab (batched kernel): thread (r, part)
+// = (tid % TR, tid / TR) covers row r's 32 columns `part` (a chain of FMAs in
+// column order), leaving the partials in s_sq[part][r]; the row's sum is then
+// the partials added in part order (row_sq).  The streaming kernel's pairs sum
+// in the same order, so both give the same bits.
 template <int TR>
-__device__ __forceinline__ void slab_row_partials(const float* Xs, int bs, float (*s_sq)[TR],
-                                                  float (*s_amax)[TR], int tid) {
+__device__ __forceinline__ void slab_row_partials(const float* Xs, int bs, float (*s_sq)[TR], int tid) {
   const int NT = bs / 32;
   const int r = tid % TR, part = tid / TR;
-  float sq = 0.0f, amax = 0.0f;
+  float sq = 0.0f;
   if (part < NT) {
 #pragma unroll 8
     for (int c = part * 32; c < part * 32 + 32; ++c) {
       const float v = Xs[xoff<TR>(r, c, bs)];
       sq = __fmaf_rn(v, v, sq);
-      amax = fmaxf(amax, fabsf(v));
     }
   }
   s_sq[part][r] = sq;
-  if (s_amax != nullptr) s_amax[part][r] = amax;
 }
 template <int TR>
 __device__ __forceinline__ float row_sq(float (*s_sq)[TR], int NT, int r) {
@@ -224,114 +222,80 @@ __device__ __forceinline__ uint32_t code8_x2(float a, float b) {
   }
 }
 
-// 8-bit codes of thread (r, part)'s 32-column block in format FMT into the
-// staging panel (row stride bs/4 + 1 words): the block's values are read once
-// into registers; an MX format takes the block's own E8M0 scale, the others
-// the row's power-of-two scale (from the row maximum rmax).
-template <int TR, int FMT>
-__device__ __forceinline__ void stage_codes8(const float* Xs, int bs, int nrows, int gi0, float rmax,
-                                             const QuantAll& qa, uint32_t* stage, int tid) {
-  constexpr bool MX = FMT == MXFP8 || FMT == MXFP6E2M3 || FMT == MXFP6E3M2 || FMT == MXFP4;
-  const int r = tid % TR, part = tid / TR;
-  const int gi = gi0 + r;
-  const bool live = r < nrows;
-  if (part >= bs / 32) return;
-  const int sw = bs / 4 + 1;
-  const int cb = part * 32;
-  float v[32];
+// N scaled values as N bytes at dst (N = 8, 16 or 32; dst aligned to the
+// smaller of N and 16).
+template <int FMT, int N>
+__device__ __forceinline__ void put_codes8(const float (&v)[N], float inv, uint8_t* dst) {
+  uint32_t w[N / 4];
 #pragma unroll
-  for (int u = 0; u < 32; ++u) v[u] = Xs[xoff<TR>(r, cb + u, bs)];
-  float inv;
-  if constexpr (MX) {
-    float mx[8];
+  for (int c = 0; c < N; c += 4)
+    w[c / 4] = code8_x2<FMT>(v[c] * inv, v[c + 1] * inv) | (code8_x2<FMT>(v[c + 2] * inv, v[c + 3] * inv) << 16);
+  if constexpr (N == 8) *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+  else
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      mx[u] = fmaxf(fmaxf(fabsf(v[u]), fabsf(v[u + 8])), fmaxf(fabsf(v[u + 16]), fabsf(v[u + 24])));
-    const float bmax = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])),
-                             fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
-    const int eb = mx_scale_exp(bmax, FMT);
-    inv = pow2f(-eb);
-    if (live) qa.mxexp[(size_t)gi * qa.ldmx + part] = (uint8_t)(eb + 127);
-  } else {
-    const int e = row_scale_exp(rmax, FMT);
-    inv = pow2f(-e);
-    if (live && part == 0) qa.rexp[rexp_slot(FMT)][gi] = (int8_t)e;
-  }
-#pragma unroll
-  for (int c = 0; c < 32; c += 4) {
-    const uint32_t w01 = code8_x2<FMT>(v[c] * inv, v[c + 1] * inv);
-    const uint32_t w23 = code8_x2<FMT>(v[c + 2] * inv, v[c + 3] * inv);
-    stage[r * sw + (cb + c) / 4] = w01 | (w23 << 16);
-  }
+    for (int q = 0; q < N / 16; ++q)
+      reinterpret_cast<uint4*>(dst)[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
 }
 
-// Codes of one solved slab in one format.  Thread (r, part) = (tid % TR,
-// tid / TR) converts row r's 32-column block `part` (for an MX format with
-// its own scale) into packed words of a shared staging panel (row stride
-// bs/4 + 1 words for 8-bit codes, bs/2 + 1 for 16-bit ones, so the
-// column-wise writes of 32 consecutive rows hit 32 banks); the CTA then
-// copies the staged rows out as coalesced 4-byte words.
+// One row's 32-column block (values v, largest magnitude amax) in an MX format:
+// its own E8M0 scale, then its codes.
+template <int FMT>
+__device__ __forceinline__ void put_mx_block(const float (&v)[32], float amax, const QuantAll& qa, int gi,
+                                             int block) {
+  const int eb = mx_scale_exp(amax, FMT);
+  qa.mxexp[(size_t)gi * qa.ldmx + block] = (uint8_t)(eb + 127);
+  put_codes8<FMT>(v, pow2f(-eb), qa.q8[q8_slot(FMT)] + (size_t)gi * qa.ldq + 32 * block);
+}
+
+// The codes of a solved slab that take the row's power-of-two scale (FP16 and
+// FP16X2, E4M3, E5M2), straight from the slab to global memory: thread (r,
+// part) = (tid % TR, tid / TR) converts TR / 2 columns of row r, 16 bytes or
+// more of codes in one piece.
 template <int TR>
-__device__ void quantize_slab(const float* Xs, int bs, int nrows, int gi0, int m, int fmt, float rmax,
-                              const QuantAll& qa, uint32_t* stage, int tid) {
-  const int r = tid % TR, part = tid / TR;
-  const int cw = part < bs / 32 ? 32 : 0;      // columns of this thread
-  const int c0 = part * 32;
+__device__ __forceinline__ void quantize_rows_of_slab(const float* Xs, int bs, int nrows, int gi0, int m,
+                                                      float (*s_rmax)[TR], const QuantAll& qa, int tid) {
+  constexpr int CW = TR / 2;
+  const int r = tid % TR, c0 = tid / TR * CW;
+  if (r >= nrows || c0 >= bs) return;
+  const bool f16 = (qa.cand >> FP16) & 1u, f16x2 = (qa.cand >> FP16X2) & 1u;
+  const bool e4 = (qa.cand >> E4M3) & 1u, e5 = (qa.cand >> E5M2) & 1u;
+  if (!(f16 || f16x2 || e4 || e5)) return;
   const int gi = gi0 + r;
-  const bool live = r < nrows;
-  if (fmt == FP16 || fmt == FP16X2) {
-    const int sw = bs / 2 + 1;
-    uint32_t* hi = stage;
-    uint32_t* lo = stage + TR * sw;
+  float rmax = 0.0f, v[CW];
+  for (int q = 0; q < bs / 32; ++q) rmax = fmaxf(rmax, s_rmax[q][r]);
+#pragma unroll
+  for (int u = 0; u < CW; ++u) v[u] = Xs[xoff<TR>(r, c0 + u, bs)];
+  if (f16 || f16x2) {
     const int e = row_scale_exp(rmax, FP16);
     const float inv = pow2f(-e);
-    if (cw == 32) {
+    if (c0 == 0) qa.rexp[2][gi] = (int8_t)e;
+    uint4* dh = reinterpret_cast<uint4*>(qa.q16 + (size_t)gi * qa.ldq + c0);
+    uint4* dl = reinterpret_cast<uint4*>(qa.q16 + (size_t)(m + gi) * qa.ldq + c0);
 #pragma unroll
-      for (int c = c0; c < c0 + 32; c += 2) {
-        const float x0 = Xs[xoff<TR>(r, c, bs)] * inv, x1 = Xs[xoff<TR>(r, c + 1, bs)] * inv;
+    for (int q = 0; q < CW / 8; ++q) {
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float x0 = v[8 * q + 2 * u] * inv, x1 = v[8 * q + 2 * u + 1] * inv;
         const __half2 h = __floats2half2_rn(x0, x1);
-        hi[r * sw + c / 2] = *reinterpret_cast<const uint32_t*>(&h);
-        if (fmt == FP16X2) {   // x - hi is exact in FP32
-          const float2 hf = __half22float2(h);
-          lo[r * sw + c / 2] = f32x2_to_f16x2(x0 - hf.x, x1 - hf.y);
-        }
+        hi[u] = *reinterpret_cast<const uint32_t*>(&h);
+        const float2 hf = __half22float2(h);   // x - hi is exact in FP32
+        lo[u] = f32x2_to_f16x2(x0 - hf.x, x1 - hf.y);
       }
-    }
-    if (live && part == 0) qa.rexp[2][gi] = (int8_t)e;
-    __syncthreads();
-    // a warp per row (no index division)
-    const int wpr = bs / 2;                    // words per row
-#pragma unroll 2
-    for (int rr = tid >> 5; rr < nrows; rr += NTHR / 32) {
-      uint32_t* dh = reinterpret_cast<uint32_t*>(qa.q16 + (size_t)(gi0 + rr) * qa.ldq);
-      uint32_t* dl = reinterpret_cast<uint32_t*>(qa.q16 + (size_t)(m + gi0 + rr) * qa.ldq);
-#pragma unroll 4
-      for (int w = tid & 31; w < wpr; w += 32) {
-        dh[w] = hi[rr * sw + w];
-        if (fmt == FP16X2) dl[w] = lo[rr * sw + w];
-      }
-    }
-  } else {
-    switch (fmt) {
-      case E4M3: stage_codes8<TR, E4M3>(Xs, bs, nrows, gi0, rmax, qa, stage, tid); break;
-      case E5M2: stage_codes8<TR, E5M2>(Xs, bs, nrows, gi0, rmax, qa, stage, tid); break;
-      case MXFP8: stage_codes8<TR, MXFP8>(Xs, bs, nrows, gi0, rmax, qa, stage, tid); break;
-      case MXFP6E2M3: stage_codes8<TR, MXFP6E2M3>(Xs, bs, nrows, gi0, rmax, qa, stage, tid); break;
-      case MXFP6E3M2: stage_codes8<TR, MXFP6E3M2>(Xs, bs, nrows, gi0, rmax, qa, stage, tid); break;
-      default: stage_codes8<TR, MXFP4>(Xs, bs, nrows, gi0, rmax, qa, stage, tid); break;
-    }
-    __syncthreads();
-    uint8_t* q = qa.q8[q8_slot(fmt)];
-    const int sw = bs / 4 + 1;
-    const int wpr = bs / 4;
-#pragma unroll 4
-    for (int rr = tid >> 5; rr < nrows; rr += NTHR / 32) {
-      uint32_t* d = reinterpret_cast<uint32_t*>(q + (size_t)(gi0 + rr) * qa.ldq);
-#pragma unroll 2
-      for (int w = tid & 31; w < wpr; w += 32) d[w] = stage[rr * sw + w];
+      dh[q] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      if (f16x2) dl[q] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
   }
-  __syncthreads();                             // the staging panel is reused
+  if (e4) {
+    const int e = row_scale_exp(rmax, E4M3);
+    if (c0 == 0) qa.rexp[rexp_slot(E4M3)][gi] = (int8_t)e;
+    put_codes8<E4M3>(v, pow2f(-e), qa.q8[q8_slot(E4M3)] + (size_t)gi * qa.ldq + c0);
+  }
+  if (e5) {
+    const int e = row_scale_exp(rmax, E5M2);
+    if (c0 == 0) qa.rexp[rexp_slot(E5M2)][gi] = (int8_t)e;
+    put_codes8<E5M2>(v, pow2f(-e), qa.q8[q8_slot(E5M2)] + (size_t)gi * qa.ldq + c0);
+  }
 }
 
 // Panel solve with the quantization of the panel fused in; one slab of TR
@@ -350,27 +314,50 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
                   StepState* step, StepState* next, int next_bs, DecisionParams dp, DevStatus* st,
                   QuantAll qa, const StepState* prev, double* __restrict__ colacc) {
   constexpr int HR = Slab<TR>::HR, RPL = Slab<TR>::RPL;
+  constexpr int SW = TR > 32 ? 2 : 1;                    // warps that hold the slab's rows
   extern __shared__ __align__(128) float sm[];
   const int NT = bs / 32;
   float* Xs = sm;                                        // the slab (xoff layout)
   float* Lt = Xs + (size_t)bs * TR;                      // L_{I,M}, I > M
   float* Wt = Lt + (size_t)(NT * (NT - 1) / 2) * TSZ;    // L_JJ^-1
-  uint32_t* stage = reinterpret_cast<uint32_t*>(Lt);     // code staging, once L11 is used
-  __shared__ float red_max[NTHR / 32];
-  __shared__ int red_lit[NTHR / 32];
-  __shared__ float red_min[NTHR / 32];
   __shared__ double red_coh[NTHR / 32];
-  __shared__ float s_rmax[NTHR / TR][TR];
-  __shared__ float s_sq[NTHR / TR][TR];
+  __shared__ float s_rmax[MAXNT][TR];                    // by tile column and row
+  __shared__ float s_sq[MAXNT][TR];
   __shared__ __align__(8) uint64_t barx, lrow[MAXNT], ready[MAXNT];
   __shared__ int s_ok, s_last;
 
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m = n - s - bs;
   const int slab = blockIdx.x;
   const int row0 = s + bs + slab * TR;                   // first global row of the slab
   const int nrows = min(TR, n - row0);
+  const int gi0 = slab * TR;                             // first trailing row of the slab
+  if (tid == 0) {
+    tc::mbar_init(&barx, 1);
+    for (int J = 0; J < NT; ++J) {
+      tc::mbar_init(&lrow[J], 1);
+      tc::mbar_init(&ready[J], 64);
+    }
+    tc::fence_mbar_init();
+    s_last = 0;
+  }
+  __syncthreads();
   tc::grid_dep_wait();   // the POTRF (and the trailing update) before it are complete
+  // the copies, spread over the warps (a copy takes its thread about 80 cycles
+  // to issue): the slab, and each pair its own tile row of L11
+  if (lane == 0) {
+    if (warp == 1) {
+      tc::mbar_expect_tx(&barx, (uint32_t)(TR * bs * sizeof(float)));
+      for (int q = 0; q < RPL; ++q) tc::tma_load_2d(Xs + q * bs * HR, &tmapX, &barx, row0 + HR * q, s);
+    }
+    if ((warp & 1) == 0 && warp / 2 < NT) {
+      const int J = warp / 2;
+      tc::mbar_expect_tx(&lrow[J], (uint32_t)((J + 1) * TSZ * sizeof(float)));
+      tc::bulk_load_1d(Wt + (size_t)J * TSZ, winv + (size_t)J * TSZ, (uint32_t)(TSZ * sizeof(float)), &lrow[J]);
+      for (int M = 0; M < J; ++M)
+        tc::tma_load_2d(Lt + (size_t)tl(J, M) * TSZ, &tmap32, &lrow[J], s + 32 * J, s + 32 * M);
+    }
+  }
   // the previous step's rounding shift for the slab's rows, before this
   // step's sums of squares replace the previous ones in rowsq
   if (prev != nullptr && qa.sh != nullptr && tid < nrows) {
@@ -380,61 +367,76 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
       *shp = __fmaf_rn(unit_roundoff(pp), rowsq[row0 + tid], *shp);
     }
   }
-  if (tid == 0) {
-    s_ok = st->code == 0;
-    tc::mbar_init(&barx, 1);
-    for (int J = 0; J < NT; ++J) {
-      tc::mbar_init(&lrow[J], 1);
-      tc::mbar_init(&ready[J], 64);
+  if (tid == NTHR - 1) s_ok = st->code == 0;
+  // every copy has landed before the CTA may leave (bounded, twice)
+  const bool landed = tc::mbar_wait(&barx, 0) || tc::mbar_wait(&barx, 0);
+  const bool all_landed = !__syncthreads_or(!landed);
+  if (!all_landed && tid == 0) set_status(st, MPCHOL_ERR_TIMEOUT, row0);
+  // a finished pair: its tile's row sums (a chain of FMAs in column order; the
+  // row's sum is the tiles' in order), magnitudes, MX codes and column sums
+  const int mx = (qa.cand >> MXFP8) & 1u       ? MXFP8
+                 : (qa.cand >> MXFP6E2M3) & 1u ? MXFP6E2M3
+                 : (qa.cand >> MXFP6E3M2) & 1u ? MXFP6E3M2
+                 : (qa.cand >> MXFP4) & 1u     ? MXFP4
+                                               : -1;
+  auto post = [&](int J, int t) {
+    if (t < TR) {
+      float v[32], sq = 0.0f, amax = 0.0f;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) v[u] = Xs[xoff<TR>(t, 32 * J + u, bs)];
+#pragma unroll
+      for (int u = 0; u < 32; ++u) {
+        sq = __fmaf_rn(v[u], v[u], sq);
+        amax = fmaxf(amax, fabsf(v[u]));
+      }
+      s_sq[J][t] = sq;
+      s_rmax[J][t] = amax;
+      // an MX-family member of the candidates (at most one: they share the MX
+      // code slot and scales)
+      if (mx >= 0 && t < nrows) {
+        if (mx == MXFP8) put_mx_block<MXFP8>(v, amax, qa, gi0 + t, J);
+        else if (mx == MXFP6E2M3) put_mx_block<MXFP6E2M3>(v, amax, qa, gi0 + t, J);
+        else if (mx == MXFP6E3M2) put_mx_block<MXFP6E3M2>(v, amax, qa, gi0 + t, J);
+        else put_mx_block<MXFP4>(v, amax, qa, gi0 + t, J);
+      }
     }
-    tc::fence_mbar_init();
-  }
-  __syncthreads();
-  const bool issued = s_ok != 0;
-  if (issued && tid == 0) {
-    tc::mbar_expect_tx(&barx, (uint32_t)(TR * bs * sizeof(float)));
-    for (int q = 0; q < RPL; ++q) tc::tma_load_2d(Xs + q * bs * HR, &tmapX, &barx, row0 + HR * q, s);
-    for (int J = 0; J < NT; ++J) {
-      tc::mbar_expect_tx(&lrow[J], (uint32_t)((J + 1) * TSZ * sizeof(float)));
-      for (int M = 0; M < J; ++M)
-        tc::tma_load_2d(Lt + (size_t)tl(J, M) * TSZ, &tmap32, &lrow[J], s + 32 * J, s + 32 * M);
-      tc::bulk_load_1d(Wt + (size_t)J * TSZ, winv + (size_t)J * TSZ, (uint32_t)(TSZ * sizeof(float)),
-                       &lrow[J]);
+    // column sums (coherence rule): a thread sums column c over the slab's
+    // rows, starting at row c % TR so that a warp's threads read different banks
+    // (a fixed order per column), and adds it into copy slab % kColCopies of
+    // colacc (the copies spread the CTAs' atomics over more L2 lines).  The
+    // sums reach colacc as FP64 atomics of FP32 partials, which are exact while
+    // a column's partials span less than 2^20 in magnitude; the order of the
+    // atomics then does not change the result
+    if (colacc != nullptr && t >= 32) {
+      const int c = 32 * J + t - 32;
+      float cs = 0.0f;
+#pragma unroll 8
+      for (int q = 0; q < TR; ++q) {
+        const int r = (q + c) & (TR - 1);
+        cs += (r < nrows) ? Xs[xoff<TR>(r, c, bs)] : 0.0f;
+      }
+      atomicAdd(colacc + (size_t)(slab % kColCopies) * bs + c, (double)cs);
     }
-    if (!tc::mbar_wait(&barx, 0)) {
-      s_ok = 0;
-      set_status(st, MPCHOL_ERR_TIMEOUT, row0);
-      tc::mbar_wait(&barx, 0);
-    }
-  }
-  __syncthreads();
-  if (s_ok) {
-    if (!slab_solve<TR>(Xs, bs, Lt, Wt, lrow, ready, tid)) {
-      s_ok = 0;
-      set_status(st, MPCHOL_ERR_TIMEOUT, row0);
-    }
-  }
-  // every copy into L11's space has landed before it is reused (bounded;
-  // immediate once the solve has seen each tile row)
-  if (issued && tid == 0)
+  };
+  bool solved = all_landed && s_ok;
+  if (solved) solved = slab_solve<TR>(Xs, bs, Lt, Wt, lrow, ready, tid, post);
+  const bool gave_up = all_landed && s_ok && !solved;
+  tc::fence_proxy_async_smem();                          // the slab, to the copies out
+  solved = !__syncthreads_or(!solved);
+  if (gave_up) set_status(st, MPCHOL_ERR_TIMEOUT, row0);
+  if (!solved && tid == 0)                               // no copy in flight at the exit
     for (int J = 0; J < NT; ++J) tc::mbar_wait(&lrow[J], 0);
-  __syncthreads();
-  float bm = 0.0f;   // this CTA's max d/dtilde, min dtilde and literal code
-  float bmin = INFINITY;
-  int bl = 0;
-  if (s_ok) {
-    // ---- write the solved slab back (TMA stores; rows past n are clipped)
-    tc::fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      for (int q = 0; q < RPL; ++q)
-        if (row0 + HR * q < n) tc::tma_store_2d(&tmapX, Xs + q * bs * HR, row0 + HR * q, s);
-      tc::bulk_commit();
-    }
-    // ---- Schur diagonal tracker and switching statistics of the slab -----
-    slab_row_partials<TR>(Xs, bs, s_sq, s_rmax, tid);
-    __syncthreads();
-    if (tid < nrows) {
+  if (solved && tid == NTHR - 1) {                       // the solved slab (rows past n are clipped)
+    for (int q = 0; q < RPL; ++q)
+      if (row0 + HR * q < n) tc::tma_store_2d(&tmapX, Xs + q * bs * HR, row0 + HR * q, s);
+    tc::bulk_commit();
+  }
+  // Schur diagonal tracker and switching statistics of the slab, then the
+  // ticket, by the warps that hold its rows
+  if (warp < SW) {
+    float bm = 0.0f, bmin = INFINITY;   // max d/dtilde, min dtilde and literal code
+    int bl = 0;
+    if (solved && tid < nrows) {
       const int gi = row0 + tid;
       const float sq = row_sq<TR>(s_sq, NT, tid);
       rowsq[gi] = sq;
@@ -448,74 +450,36 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
       // reference list {FP32, FP16, E4M3} with the reference's machine epsilons
       const float ref_eps[3] = {1.1920929e-7f, 0.0009765625f, 0.125f};
       int pick = 0;
-      for (int p = 0; p < 3; ++p)
-        if (ref_eps[p] * dt >= dp.eps_prime * di) { pick = p; break; }
+#pragma unroll
+      for (int p = 2; p >= 0; --p)
+        if (ref_eps[p] * dt >= dp.eps_prime * di) pick = p;
       bl = max(bl, 2 - pick);
       if (next != nullptr && dp.floor_ratio > 0.0f && gi - (s + bs) < next_bs &&
           dt <= dp.floor_ratio * di)
         next->fp64_diag = 1;
     }
-    // ---- column sums of the slab (coherence rule): thread c sums column c
-    // over the slab's rows, starting at row c % TR so that the 32 threads of
-    // a warp read 32 different banks (a fixed order per column), and adds it
-    // into copy slab % kColCopies of colacc (the copies spread the CTAs'
-    // atomics over more L2 lines).  The sums reach colacc as FP64 atomics of
-    // FP32 partials, which are exact while a column's partials span less than
-    // 2^20 in magnitude; the order of the atomics then does not change the
-    // result
-    if (colacc != nullptr && tid < bs) {
-      float cs = 0.0f;
-#pragma unroll 8
-      for (int q = 0; q < TR; ++q) {
-        const int r = (q + tid) & (TR - 1);
-        cs += (r < nrows) ? Xs[xoff<TR>(r, tid, bs)] : 0.0f;
-      }
-      atomicAdd(colacc + (size_t)(slab % kColCopies) * bs + tid, (double)cs);
+    bm = warp_max(bm);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      bl = max(bl, __shfl_xor_sync(0xffffffffu, bl, o));
+      bmin = fminf(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
+    }
+    if (lane == 0) {
+      atomicMax(&step->max_ratio_bits, __float_as_uint(bm));
+      atomicMax(&step->literal_code, bl);
+      if (bmin < INFINITY) atomicMax(&step->not_min_dt_bits, ~__float_as_uint(fmaxf(bmin, 0.0f)));
+    }
+    if (SW > 1) pair_sync(0);
+    if (tid == 0) {
       __threadfence();
+      s_last = atomicAdd(&step->grid_bar, 1) == (int)gridDim.x - 1;
     }
-    // ---- the slab's codes in every candidate format -------------------------
-    if (qa.cand != 0) {
-      const int r = tid % TR;
-      float rmax = 0.0f;
-#pragma unroll
-      for (int q = 0; q < NTHR / TR; ++q) rmax = fmaxf(rmax, s_rmax[q][r]);
-      const int gi0 = slab * TR;                         // first trailing row of the slab
-      const bool f16 = (qa.cand >> FP16) & 1u, f16x2 = (qa.cand >> FP16X2) & 1u;
-      if (f16 || f16x2)
-        quantize_slab<TR>(Xs, bs, nrows, gi0, m, f16x2 ? FP16X2 : FP16, rmax, qa, stage, tid);
-      // E4M3, E5M2 and the MX-family member of the candidates (at most one:
-      // they share the MX code slot and scales)
-      const int f8[6] = {E4M3, E5M2, MXFP8, MXFP6E2M3, MXFP6E3M2, MXFP4};
-      for (int i = 0; i < 6; ++i)
-        if ((qa.cand >> f8[i]) & 1u) quantize_slab<TR>(Xs, bs, nrows, gi0, m, f8[i], rmax, qa, stage, tid);
-    }
-    if (tid == 0) tc::bulk_wait_read();   // the slab's stores are complete before the ticket
   }
-  // the next kernel (the head of the trailing update) may be scheduled once
-  // every CTA is past its solve; it waits for this grid before reading
+  if (solved) quantize_rows_of_slab<TR>(Xs, bs, nrows, gi0, m, s_rmax, qa, tid);
+  if (tid == NTHR - 1) tc::bulk_wait_read();             // the copies out have read the slab
+  // the next kernel (the head of the trailing update) may be scheduled; it
+  // waits for this grid before reading
   tc::grid_dep_trigger();
-  // ---- statistics of the CTA; the last CTA resolves the step --------------
-  bm = warp_max(bm);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    bl = max(bl, __shfl_xor_sync(0xffffffffu, bl, o));
-    bmin = fminf(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
-  }
-  if ((tid & 31) == 0) { red_max[tid >> 5] = bm; red_lit[tid >> 5] = bl; red_min[tid >> 5] = bmin; }
-  __syncthreads();
-  if (tid == 0) {
-    float cm = 0.0f, cmin = INFINITY; int cl = 0;
-    for (int w = 0; w < NTHR / 32; ++w) {
-      cm = fmaxf(cm, red_max[w]);
-      cl = max(cl, red_lit[w]);
-      cmin = fminf(cmin, red_min[w]);
-    }
-    atomicMax(&step->max_ratio_bits, __float_as_uint(cm));
-    atomicMax(&step->literal_code, cl);
-    if (cmin < INFINITY) atomicMax(&step->not_min_dt_bits, ~__float_as_uint(fmaxf(cmin, 0.0f)));
-    __threadfence();
-    s_last = atomicAdd(&step->grid_bar, 1) == (int)gridDim.x - 1;
-  }
   __syncthreads();
   if (!s_last) return;
   __threadfence();                                       // every CTA's statistics
@@ -592,7 +556,7 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
       }
   for (int e = tid; e < NT * TSZ; e += NTHR) Wt[e] = S.winv[e];
   __syncthreads();
-  if (!slab_solve<TR>(Xs, bs, Lt, Wt, nullptr, ready, tid)) {
+  if (!slab_solve<TR>(Xs, bs, Lt, Wt, nullptr, ready, tid, [](int, int) {})) {
     s_ok = 0;
     set_status(S.st, MPCHOL_ERR_TIMEOUT, row0);
   }
@@ -603,7 +567,7 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
     if (r < nrows) S.A[(size_t)(s + c) * ld + row0 + r] = Xs[xoff<TR>(r, c, bs)];
   }
   __shared__ float s_sq[NTHR / TR][TR];
-  slab_row_partials<TR>(Xs, bs, s_sq, nullptr, tid);
+  slab_row_partials<TR>(Xs, bs, s_sq, tid);
   __syncthreads();
   if (tid < nrows) {
     const int gi = row0 + tid;
@@ -660,7 +624,8 @@ cudaError_t launch_trsm_panel(const CUtensorMap& tmapX, const CUtensorMap& tmapX
   // 64-row slabs while the panel has more 32-row slabs than the GPU has SMs
   // (throughput: L11 staged once per 64 rows); below that the smallest slabs
   // that all run at once (latency: a CTA's work follows its rows).  B200, b =
-  // 256, panel solve: T64 us for a 64-row slab, T32 for 32 rows, T16 for 16.
+  // 256, a panel solve inside a factorization: 35 us with 64-row slabs, 22 with 32,
+  // 16 with 16.
   const int nsm = sm_count();
   if (ceil_div(m, 32) > nsm)
     return launch_panel<64>(tmapX, tmap32, A, lda, n, s, bs, winv, d, dtilde, rowsq, step, next,
