@@ -794,26 +794,28 @@ block_inverse_kernel(const float* __restrict__ L, int ldl, int n, float* __restr
   block_inverse_body(L, ldl, n, wsup, blockIdx);
 }
 
-// C(64 x 64) = A(64 x K) B(K x 64), all column-major, FP32 FMA, by 256 threads
-// as four groups of 64: group q takes k = 8 q .. 8 q + 7 of every 32-deep
-// chunk with 8 x 8 outputs per thread, and the groups' sums are added at the
-// end in a fixed order.  A 64 x 64 tile per CTA spreads a super-block's
-// largest doubling over 64 SMs (128 x 128 tiles: 16) and the split of K keeps
-// the 8 x 8 register blocks that shared memory's return path needs (four
-// 16-byte reads per 64 FMAs and k).  The next chunk travels in registers.
-// The six launches of n = 1024 take 107 us (128 x 128 tiles: 266), those of n =
-// 16384 312 us (385).
-// Rows of A past a_rows are zero.  Thread (tx, ty): rows 4 tx.. and 32 + 4
-// tx.., columns ty + 8 j.
-constexpr int GT = 64;
-constexpr int GKC = 32;
+// C(32 x 32) = A(32 x K) B(K x 32), all column-major, FP32 FMA, by 256 threads
+// as four groups of 64: group q takes k = 16 q .. 16 q + 15 of every 64-deep
+// chunk with 4 x 4 outputs per thread, and the groups' sums are added at the
+// end in a fixed order.  The next chunk travels in registers; the lanes' bits
+// interleave into tx and ty so that four neighbouring lanes read two different
+// 16-byte vectors of each operand (2.2 cycles of shared memory a load; 4.0 with
+// four).  A chunk costs its load latency before it costs its FMAs, so the small
+// tile wins at every order: four CTAs per SM in place of two, and 256 tiles for
+// a super-block's largest doubling.  All the levels (B200, n = 1024 / 3000 /
+// 8192 / 16384): 103 / 121 / 176 / 306 us with 64 x 64 tiles and 8 x 8 outputs,
+// 39 / 66 / 137 / 248 with these.
+// Rows of A past a_rows are zero.  K is a multiple of 64.  Thread (tx, ty): rows
+// 4 tx.., columns ty + 8 j.
+constexpr int GT = 32;
+constexpr int GKC = 64;
 constexpr int GLDB = GKC + 4;                        // floats per staged column of B
 constexpr int G_AS = GKC * GT, G_BS = GT * GLDB;
 constexpr int G_SMEM = 2 * (G_AS + G_BS);            // two chunks; the reduction reuses them
 static_assert(G_SMEM >= 2 * GT * GT, "two groups' sums fit");
 
-__device__ __forceinline__ void gemm64_load(const float* A, int lda, int a_rows, const float* B,
-                                            int ldb, int k0, float4 (&ra)[2], float4 (&rb)[2]) {
+__device__ __forceinline__ void gemm32_load(const float* A, int lda, int a_rows, const float* B, int ldb,
+                                            int k0, float4 (&ra)[2], float4 (&rb)[2]) {
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int e = threadIdx.x + NTH * u;
@@ -831,14 +833,22 @@ __device__ __forceinline__ void gemm64_load(const float* A, int lda, int a_rows,
   }
 }
 
-__device__ __forceinline__ void gemm64(const float* A, int lda, int a_rows, const float* B, int ldb,
-                                       int K, float (&acc)[8][8], float* sm) {
-  const int tid = threadIdx.x, grp = tid / 64, tx = tid % 8, ty = (tid % 64) / 8;
+__device__ __forceinline__ void gemm32_lane(int& tx, int& ty) {
+  const int l = threadIdx.x % 32;
+  tx = (l & 1) | ((l >> 1) & 6);
+  ty = ((l >> 1) & 1) | ((l >> 3) & 2) | ((threadIdx.x >> 3) & 4);
+}
+
+__device__ __forceinline__ void gemm32(const float* A, int lda, int a_rows, const float* B, int ldb,
+                                       int K, float (&acc)[4][4], float* sm) {
+  const int tid = threadIdx.x, grp = tid / 64;
+  int tx, ty;
+  gemm32_lane(tx, ty);
   float4 ra[2], rb[2];
-  gemm64_load(A, lda, a_rows, B, ldb, 0, ra, rb);
+  gemm32_load(A, lda, a_rows, B, ldb, 0, ra, rb);
   for (int k0 = 0, buf = 0; k0 < K; k0 += GKC, buf ^= 1) {
-    float* As = sm + buf * (G_AS + G_BS);            // [k][row]
-    float* Bs = As + G_AS;                           // [column][k]
+    float* As = sm + buf * (G_AS + G_BS);          // [k][row]
+    float* Bs = As + G_AS;                          // [column][k]
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int e = tid + NTH * u;
@@ -846,24 +856,23 @@ __device__ __forceinline__ void gemm64(const float* A, int lda, int a_rows, cons
       *reinterpret_cast<float4*>(Bs + (e / (GKC / 4)) * GLDB + 4 * (e % (GKC / 4))) = rb[u];
     }
     __syncthreads();   // this buffer's last reader passed the previous barrier
-    if (k0 + GKC < K) gemm64_load(A, lda, a_rows, B, ldb, k0 + GKC, ra, rb);
+    if (k0 + GKC < K) gemm32_load(A, lda, a_rows, B, ldb, k0 + GKC, ra, rb);
 #pragma unroll 1
-    for (int kq = 0; kq < 8; kq += 4) {
-      const int k = 8 * grp + kq;
-      float4 b[8];
+    for (int kq = 0; kq < GKC / 4; kq += 4) {
+      const int k = GKC / 4 * grp + kq;
+      float4 b[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < 4; ++j)
         b[j] = *reinterpret_cast<const float4*>(Bs + (ty + 8 * j) * GLDB + k);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float4 a0 = *reinterpret_cast<const float4*>(As + (k + e) * GT + 4 * tx);
-        const float4 a1 = *reinterpret_cast<const float4*>(As + (k + e) * GT + 32 + 4 * tx);
-        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const float4 a = *reinterpret_cast<const float4*>(As + (k + e) * GT + 4 * tx);
+        const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 4; ++j) {
           const float bv = e == 0 ? b[j].x : (e == 1 ? b[j].y : (e == 2 ? b[j].z : b[j].w));
 #pragma unroll
-          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(av[i], bv, acc[i][j]);
+          for (int i = 0; i < 4; ++i) acc[i][j] = fmaf(av[i], bv, acc[i][j]);
         }
       }
     }
@@ -875,27 +884,29 @@ __device__ __forceinline__ void gemm64(const float* A, int lda, int a_rows, cons
     if (grp >= half && grp < 2 * half) {
       float* d = sm + (grp - half) * GT * GT + (tid % 64);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) d[(j * 8 + i) * 64] = acc[i][j];
+        for (int i = 0; i < 4; ++i) d[(j * 4 + i) * 64] = acc[i][j];
     }
     __syncthreads();
     if (grp < half) {
       const float* d = sm + grp * GT * GT + (tid % 64);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i][j] += d[(j * 8 + i) * 64];
+        for (int i = 0; i < 4; ++i) acc[i][j] += d[(j * 4 + i) * 64];
     }
   }
 }
 
 // One doubling level of half-size h (a multiple of RB) for pair bid.y of
-// super-block bid.z; bid.x enumerates the (h/GT)^2 output tiles.
+// super-block bid.z; bid.x enumerates the (h/32)^2 output tiles.
 //   PHASE 0:  T(ti,tj) = sum_{kt >= tj} L(h + ti, kt) A^-1(kt, tj)  -> upper-right scratch
 //   PHASE 1:  X(ti,tj) = -sum_{kt <= ti} C^-1(ti, kt) T(kt, tj)     -> lower-left block
-// (64-tile indices relative to the pair's origin a0 = 2 h * pair).  Tiles
-// whose rows start at or past n are skipped: the solves never read them.
+// (indices relative to the pair's origin a0 = 2 h * pair; the sums over k
+// start and end at multiples of 64, where the inverses are zero on the wrong
+// side of the diagonal).  64-row groups that start at or past n are skipped:
+// the solves never read them.
 template <int PHASE>
 __device__ __forceinline__ void
 superinv_gemm_body(const float* __restrict__ L, int ldl, int n, float* __restrict__ wsup, int h, uint3 bid) {
@@ -903,34 +914,34 @@ superinv_gemm_body(const float* __restrict__ L, int ldl, int n, float* __restric
   const int tpr = h / GT;
   const int ti = bid.x / tpr, tj = bid.x % tpr;
   const int S = bid.z, s0 = S * RS, a0 = bid.y * 2 * h;
-  const int grow = s0 + a0 + h + ti * GT;          // first global row of the output tile
-  if (grow >= n) return;
+  const int r0 = ti * GT, c0 = tj * GT;
+  if (s0 + a0 + h + (r0 & ~63) >= n) return;
+  const int grow = s0 + a0 + h + r0;               // first global row of the output tile
   float* W = wsup + (size_t)S * RS * RS;
-  float acc[8][8] = {};
+  float acc[4][4] = {};
   float* out;
   if (PHASE == 0) {
-    gemm64(L + (size_t)(s0 + a0 + tj * GT) * ldl + grow, ldl, min(GT, n - grow),
-           W + (size_t)(a0 + tj * GT) * RS + a0 + tj * GT, RS, h - tj * GT, acc, sm);
-    out = W + (size_t)(a0 + h + tj * GT) * RS + a0 + ti * GT;
+    const int k0 = c0 & ~63;
+    gemm32(L + (size_t)(s0 + a0 + k0) * ldl + grow, ldl, min(GT, n - grow),
+           W + (size_t)(a0 + c0) * RS + a0 + k0, RS, h - k0, acc, sm);
+    out = W + (size_t)(a0 + h + c0) * RS + a0 + r0;
   } else {
-    gemm64(W + (size_t)(a0 + h) * RS + a0 + h + ti * GT, RS, GT,
-           W + (size_t)(a0 + h + tj * GT) * RS + a0, RS, (ti + 1) * GT, acc, sm);
-    out = W + (size_t)(a0 + tj * GT) * RS + a0 + h + ti * GT;
+    gemm32(W + (size_t)(a0 + h) * RS + a0 + h + r0, RS, GT,
+           W + (size_t)(a0 + h + c0) * RS + a0, RS, (r0 & ~63) + 64, acc, sm);
+    out = W + (size_t)(a0 + c0) * RS + a0 + h + r0;
   }
   if (threadIdx.x >= 64) return;                   // group 0 holds the sums
   const float sg = PHASE == 0 ? 1.0f : -1.0f;
-  const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
+  int tx, ty;
+  gemm32_lane(tx, ty);
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh)
-      *reinterpret_cast<float4*>(out + (size_t)(ty + 8 * j) * RS + 32 * hh + 4 * tx) =
-          make_float4(sg * acc[4 * hh][j], sg * acc[4 * hh + 1][j], sg * acc[4 * hh + 2][j],
-                      sg * acc[4 * hh + 3][j]);
+  for (int j = 0; j < 4; ++j)
+    *reinterpret_cast<float4*>(out + (size_t)(ty + 8 * j) * RS + 4 * tx) =
+        make_float4(sg * acc[0][j], sg * acc[1][j], sg * acc[2][j], sg * acc[3][j]);
 }
 
 template <int PHASE>
-__global__ void __launch_bounds__(NTH, 2)
+__global__ void __launch_bounds__(NTH, 4)
 superinv_gemm_kernel(const float* __restrict__ L, int ldl, int n, float* __restrict__ wsup, int h) {
   superinv_gemm_body<PHASE>(L, ldl, n, wsup, h, blockIdx);
 }
@@ -1395,7 +1406,7 @@ block_inverse_batched_kernel(const BatchSys* __restrict__ sys) {
 }
 
 template <int PHASE>
-__global__ void __launch_bounds__(NTH, 2)
+__global__ void __launch_bounds__(NTH, 4)
 superinv_gemm_batched_kernel(const BatchSys* __restrict__ sys, int h, int max_super) {
   const BatchSys& S = sys[blockIdx.z / max_super];
   const int sup = blockIdx.z % max_super;

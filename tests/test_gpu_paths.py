@@ -60,7 +60,7 @@ def test_resources_of_a_freed_factor_serve_the_next_one():
     assert not bad
 
 
-@pytest.mark.parametrize("n", [31, 33, 96, 128, 129, 191, 385, 640, 1023, 1025, 1500])
+@pytest.mark.parametrize("n", [31, 33, 96, 128, 129, 191, 161, 193, 225, 289, 385, 545, 640, 1023, 1025, 1500])
 def test_preconditioner_apply_at_block_and_super_block_edges(n):
     """z = M^-1 r through the block and super-block inverses against the FP64
     solve with the factor itself.  The inverses are exact to FP32 rounding:
