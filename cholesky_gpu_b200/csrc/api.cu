@@ -223,6 +223,10 @@ bool acquire_resources(int device, size_t bytes, Resources* out) {
        cudaStreamCreateWithFlags(&r.capture_stream, cudaStreamNonBlocking) == cudaSuccess;
   for (cudaEvent_t* e : {&r.ev_next, &r.ev_rest, &r.ev_catch})
     ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+  // the slots of the triangular solve start out with no launch's tag, and stay
+  // at the start of the memory whatever factor object it serves
+  ok = ok && cudaMemsetAsync(r.arena, 0, trsv_slot_bytes(), r.aux) == cudaSuccess &&
+       cudaStreamSynchronize(r.aux) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     free_resources(r);
@@ -892,11 +896,12 @@ mpchol_status ensure_solve(mpchol_factor_t* f, cudaStream_t stream) {
 mpchol_status apply_precond(mpchol_factor_t* f, double* w, double* mid, double* out, int nr, const int* skip,
                             cudaStream_t stream) {
   PHASE(MPCHOL_PH_TRSV, 1, stream,
-        launch_trsv_persistent(false, f->A, f->ld, f->n, f->wsup, w, mid, nr, f->trsv_ctr, skip, f->pstatus,
-                               stream));
+        launch_trsv_persistent(false, f->A, f->ld, f->n, f->wsup, w, mid, nr, f->trsv_ctr,
+                               f->res.arena, skip, f->pstatus, stream));
   PHASE(MPCHOL_PH_TRSV, 1, stream,
         launch_trsv_persistent(true, f->A, f->ld, f->n, f->wsup, mid, out, nr,
-                               f->trsv_ctr + trsv_counter_ints(f->n), skip, f->pstatus, stream));
+                               f->trsv_ctr + trsv_counter_ints(f->n), f->res.arena, skip, f->pstatus,
+                               stream));
   return MPCHOL_OK;
 }
 
@@ -1326,7 +1331,7 @@ mpchol_status mpchol_factor_create(const mpchol_opts* opts, int n, mpchol_factor
   const size_t nv = (size_t)n * 8, nbq = (size_t)n * f->b;
   // one device allocation holds every buffer (see Resources)
   auto carve = [&](char* base) -> size_t {
-    size_t off = 0;
+    size_t off = (trsv_slot_bytes() + 255) / 256 * 256;   // first: the triangular solve's slots
     auto take = [&](auto*& p, size_t count) {
       using T = std::remove_reference_t<decltype(*p)>;
       p = base ? reinterpret_cast<T*>(base + off) : nullptr;

@@ -26,13 +26,16 @@ cudaError_t launch_solve_setup(const float* L, int ldl, int n, float* wsup, cuda
 // wsup, one persistent cooperative launch: w is consumed, out (n x nrhs) and
 // the trsv_counter_ints(n) counters are zero on entry.  launch_trsv_prep: w <-
 // in, and for the forward-then-backward pair its targets mid and out and both
-// sets of counters zero.
+// sets of counters zero.  slots: trsv_slot_bytes() of device memory that no two
+// solves use at once, zero when allocated and afterwards written by these
+// launches only.
 size_t trsv_counter_ints(int n);
+size_t trsv_slot_bytes();
 cudaError_t launch_trsv_prep(const double* in, double* w, double* mid, double* out, int n, int nrhs,
                              int* counters, cudaStream_t stream);
 cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n,
                                    const float* wsup, double* w, double* out, int nrhs, int* counters,
-                                   const int* skip, DevStatus* st, cudaStream_t stream);
+                                   void* slots, const int* skip, DevStatus* st, cudaStream_t stream);
 // What the kernels of one solve work on: n x nr vectors (column-major, ld n;
 // nr = 1, 2, 4 or 8), partial sums of pcg_vgrid() blocks, and the scalars
 // that never leave the device.

@@ -173,25 +173,34 @@ __device__ __forceinline__ void tile_pass(const TA* T, int ld, int rows_valid, i
   }
 }
 
-// Reduce the per-warp row partials of tile_pass(NOTRANS) and add sign * sum
-// into out[row0 + r] (rows < nvalid) with FP64 atomics.
+// The per-warp row partials of tile_pass(NOTRANS) in shared memory (ends with a
+// barrier) and the sum of element e = k * RB + r over the warps.
 template <int NR>
-__device__ __forceinline__ void flush_rows(double (&acc)[4][NR], double* red, double* out, int n,
-                                           int row0, int nvalid, double sign) {
+__device__ __forceinline__ void stage_rows(double (&acc)[4][NR], double* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int k = 0; k < NR; ++k) red[(warp * NR + k) * RB + 4 * lane + r] = acc[r][k];
   __syncthreads();
+}
+template <int NR>
+__device__ __forceinline__ double row_sum(const double* red, int e) {
+  double s = 0.0;
+#pragma unroll
+  for (int w = 0; w < NTH / 32; ++w) s += red[w * NR * RB + e];
+  return s;
+}
+
+// Reduce the per-warp row partials and add sign * sum into out[row0 + r]
+// (rows < nvalid) with FP64 atomics.
+template <int NR>
+__device__ __forceinline__ void flush_rows(double (&acc)[4][NR], double* red, double* out, int n,
+                                           int row0, int nvalid, double sign) {
+  stage_rows<NR>(acc, red);
   for (int e = threadIdx.x; e < RB * NR; e += NTH) {
     const int k = e / RB, r = e % RB;
-    if (r < nvalid) {
-      double s = 0.0;
-#pragma unroll
-      for (int w = 0; w < NTH / 32; ++w) s += red[(w * NR + k) * RB + r];
-      atomicAdd(&out[(size_t)k * n + row0 + r], sign * s);
-    }
+    if (r < nvalid) atomicAdd(&out[(size_t)k * n + row0 + r], sign * row_sum<NR>(red, e));
   }
 }
 
@@ -1022,10 +1031,32 @@ panel_body(const float* __restrict__ L, int ldl, int n, int s0, int rs,
 // atomic counter in a topological order (trsv_job: grouped by the
 // super-block they feed), so a unit only ever waits on units already taken
 // by running CTAs; the launch is cooperative, so all CTAs are resident and
-// every wait ends.  Completion is
-// counted per 128-row segment:
-//   seg_in[g]   panel contributions received by segment g (global 128-tile g)
-//   seg_out[g]  TRMV tiles finished that write segment g of the result
+// every wait ends.
+//
+// The chain of a solve is TRMV tile -> panel tile from S into its neighbour
+// S' ("near") -> TRMV tile of S', two links per super-block.  What a link costs
+// beyond its tile is the hand-over.  With 1 or 2 right-hand sides each TRMV and
+// near tile writes its 128 partial sums into a slot of its own, every number
+// beside a tag that names the launch and the super-block, and the tiles that
+// need the segment read the slots of its 1 to 8 contributors until the tags
+// match, adding them in a fixed order: one L2 write and one read, no fence, no
+// counter and no atomic in between.  The other panel tiles ("far") are off the
+// chain: they add into the right-hand side with FP64 atomics and count per
+// 128-row segment:
+//   seg_in[g]   far contributions received by segment g (global 128-tile g)
+//   seg_out[g]  segment g of the result is in `out` (the last TRMV tile that
+//               contributes to it adds the slots and writes it)
+// Slots are used in turn by odd and even super-blocks: a slot is written again
+// only after tiles that wait, through the chain, for every reader of its last
+// use.
+// With 4 or 8 right-hand sides a segment's slots would hold as many bytes as the
+// tile or twice that: there every tile adds with atomics, seg_in counts all
+// panel tiles and seg_out the finished TRMV tiles of the segment (slots for 4:
+// 0 to 5% slower).
+// One right-hand side, forward / backward, against atomics and counters
+// throughout, units in the order of need alone and bound to a CTA a unit early
+// (B200): n = 6144 45 / 49 -> 39 / 45 us, 8192 63 / 69 -> 57 / 65, 16384 172 / 188
+// -> 145 / 158; eight: 16384 291 / 291 -> 282 / 274.
 // Waits are bounded; a wait that runs out records MPCHOL_ERR_TIMEOUT and the
 // unit proceeds (the result is then wrong, but no CTA waits forever).
 constexpr long long kTrsvMaxPolls = 1ll << 24;
@@ -1051,6 +1082,73 @@ __device__ __forceinline__ void signal_count(int* ctr) {
   if (threadIdx.x == 0) atomicAdd(ctr, 1);
 }
 
+// A slot's element: 16 bytes, written and read in one access.
+struct __align__(16) TrsvSlot { double v; unsigned long long tag; };
+constexpr int kSlotSegs = 64;                 // slots per parity and kind: 8 contributors of 8 segments
+constexpr int kSlotNr = 2;                    // most right-hand sides that use them
+constexpr long long kSlotMaxPolls = 1ll << 22;
+
+__device__ __forceinline__ void slot_put(TrsvSlot* p, double v, unsigned long long tag) {
+  asm volatile("{\n.reg .b128 t;\nmov.b128 t, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ void slot_get(const TrsvSlot* p, double& v, unsigned long long& tag) {
+  long long lo;
+  asm volatile("{\n.reg .b128 t;\nld.relaxed.gpu.global.b128 t, [%2];\nmov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(tag)
+               : "l"(p)
+               : "memory");
+  v = __longlong_as_double(lo);
+}
+
+// s[e] = base(e) + the nin (1 to 8) contributions of a segment, in order, once
+// their tags match; base(e): row0 + e of x (null: zero).  One right-hand side:
+// two threads per element, which take the even and the odd contributions (the
+// odd sums pass through tmp).  Ends with a barrier.
+template <int NR>
+__device__ __forceinline__ void gather_slots(const TrsvSlot* slots, int nin, unsigned long long tag,
+                                             const double* x, int n, int row0, int nvalid, double* s,
+                                             double* tmp, DevStatus* st, int unit) {
+  constexpr int STR = NR == 1 ? 2 : 1, PER = 8 / STR;
+  const int half = NR == 1 ? threadIdx.x / RB : 0;
+  long long polls = 0;
+#pragma unroll 1
+  for (int e = NR == 1 ? threadIdx.x % RB : threadIdx.x; e < RB * NR; e += NTH) {
+    const int r = e % RB;
+    double sum = (half == 0 && x != nullptr && r < nvalid) ? __ldcg(x + (size_t)(e / RB) * n + row0 + r) : 0.0;
+    double v[PER];
+    bool all;
+    do {
+      unsigned long long t[PER];
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+        t[q] = tag;
+        v[q] = 0.0;
+        const int p = q * STR + half;
+        if (p < nin) slot_get(slots + (size_t)p * RB * NR + e, v[q], t[q]);
+      }
+      all = true;
+#pragma unroll
+      for (int q = 0; q < PER; ++q) all = all && t[q] == tag;
+      if (!all && ++polls > kSlotMaxPolls) {
+        if (st != nullptr) set_status(st, MPCHOL_ERR_TIMEOUT, unit);
+        break;
+      }
+    } while (!all);
+#pragma unroll
+    for (int q = 0; q < PER; ++q) sum += v[q];
+    if (half == 0) s[e] = sum;
+    else tmp[e] = sum;
+    if (NR == 1) break;
+  }
+  if (NR == 1) {
+    __syncthreads();
+    if (half == 0) s[threadIdx.x] += tmp[threadIdx.x];
+  }
+  __syncthreads();
+}
+
 // One unit of the solve: a tile, the vector segment it reads, where its
 // result goes and the counters it waits on and signals.
 struct TrsvJob {
@@ -1062,104 +1160,151 @@ struct TrsvJob {
   bool panel;           // L panel tile (reads out, writes work) or W_S tile
   const int* wait_ctr;
   int wait_need;
-  int* sig_ctr;
+  int* sig_ctr;         // null: nothing waits on a counter of this unit
+  // slots (0: the input is a vector / the result is added to one)
+  int in_slot, nin;     // first slot and number of the input segment's contributions
+  int in_blk;           // the super-block in their tags
+  int out_slot, out_blk;
+  int fin_slot, nfin;   // the unit that completes a segment: its contributions
 };
 
-// Decode unit u.  Units are grouped by the super-block B they feed, in solve
-// order (forward: B = 0, 1, ..; backward: B = NS-1, NS-2, ..): group B holds
-// the panel tiles that carry an earlier super-block's finished segment of the
-// solution into B's input (sources in solve order, so the ones ready longest
-// come first), then the TRMV tiles of W_B.  Every unit depends only on units
-// of earlier groups or earlier in its own group, so the order is topological
-// (the deadlock-freedom of the persistent loop needs that), and a CTA is
-// never handed far-off panel work while the chain's next TRMV waits in the
-// queue behind it.  Returns false past the last unit.
-template <bool TRANS>
-__device__ __forceinline__ bool trsv_job(int u, const float* L, int ldl, int n, const float* wsup,
-                                         int* seg_in, int* seg_out, TrsvJob& jb) {
+// The order of the units.  Positions count super-blocks in solve order
+// (forward: block p, backward: block NS-1-p); chain(p): the near tiles (p-1 ->
+// p), then the TRMV tiles of p; far (a -> b), b >= a + 2: the other panel tiles.
+//   chain(0);  for p = 0, 1, ..: chain(p+1), far tiles with 3 p + 2 <= 2 a + b < 3 p + 5
+//   (by 2 a + b, then by a)
+// Topological: 2 a + b < 3 p + 5 and b >= a + 2 give a <= p, so the sources of a
+// stage's far tiles are solved by chains before it, and far tiles into p + 2
+// (a <= p, so 2 a + b <= 3 p + 2) stand before chain(p+2).  The chain's tiles
+// stand a stage ahead, so that they are staged when their input arrives, and
+// 2 a + b brings a far tile up between its source and its need, which spreads
+// the far work over the solve (in the order of need alone, grouped by b, half
+// the CTAs waited on unsolved sources while tiles that were ready stood further
+// back, and the chain waited for far tiles from the fourth super-block on).
+// A CTA asks for numbers in increasing order, so the stage is found by moving
+// on from that of its last unit.
+struct TrsvCursor { int stage, first; };     // stage p (-1: chain(0)) and its first unit
+
+template <bool TRANS, bool SLOTS>
+__device__ __forceinline__ bool trsv_job(int u, TrsvCursor& cu, const float* L, int ldl, int n,
+                                         const float* wsup, int* seg_in, int* seg_out, TrsvJob& jb) {
   const int ntiles = ceil_div(n, RB);
   const int NS = ceil_div(n, RS);
   constexpr int NSUB = RS / RB;              // segments of a full super-block
-  for (int t = 0; t < NS; ++t) {
-    const int B = TRANS ? NS - 1 - t : t;
-    const int b0 = B * RS;
-    const int rb = min(RS, n - b0);
-    const int nsubB = ceil_div(rb, RB);
-    const int gB = b0 / RB;                  // first global segment of B
-    // panel tiles feeding B: forward from every T < B (NSUB columns of T x
-    // nsubB rows of B); backward from every T > B (the rows of T x NSUB
-    // columns of B)
-    const int npan = TRANS ? (ntiles - gB - nsubB) * NSUB : B * NSUB * nsubB;
-    if (u < npan) {
-      jb.panel = true;
-      jb.ld = ldl;
-      if (!TRANS) {
-        // w(rows r of B) -= L(r, T col c) y_T(c)
-        const int T = u / (NSUB * nsubB), q = u % (NSUB * nsubB);
-        const int r = q / NSUB, c = q % NSUB;
-        const int r0 = b0 + r * RB, c0 = T * RS + c * RB;
-        jb.T = L + (size_t)c0 * ldl + r0;
-        jb.nrow = min(RB, n - r0); jb.ncol = RB;
-        jb.nt = true;
-        jb.vin_row0 = c0; jb.vin_n = RB;
-        jb.out_row0 = r0; jb.out_n = jb.nrow;
-        jb.wait_ctr = seg_out + T * NSUB + c; jb.wait_need = c + 1;
-        jb.sig_ctr = seg_in + gB + r;
-      } else {
-        // w(col segment c of B) -= L(T row rt, c)^T z_T(rt); sources T from
-        // the last super-block down
-        int q = u, T = NS - 1;
-        for (;; --T) {
-          const int nsubT = ceil_div(min(RS, n - T * RS), RB);
-          if (q < nsubT * NSUB) break;
-          q -= nsubT * NSUB;
-        }
-        const int rt = q / NSUB, c = q % NSUB;
-        const int t0 = T * RS;
-        const int nsubT = ceil_div(min(RS, n - t0), RB);
-        const int r0 = t0 + rt * RB, c0 = b0 + c * RB;
-        jb.T = L + (size_t)c0 * ldl + r0;
-        jb.nrow = min(RB, n - r0); jb.ncol = RB;
-        jb.nt = false;
-        jb.vin_row0 = r0; jb.vin_n = jb.nrow;
-        jb.out_row0 = c0; jb.out_n = RB;
-        jb.wait_ctr = seg_out + T * NSUB + rt; jb.wait_need = nsubT - rt;
-        jb.sig_ctr = seg_in + gB + c;
-      }
-      return true;
+  jb.nin = jb.nfin = 0;
+  jb.out_slot = -1;
+  // first slot of segment q of super-block S: kind 0 its TRMV sums, kind 1 its
+  // near panel contributions
+  auto slot0 = [&](int S, int kind, int q) { return ((S & 1) * 2 + kind) * kSlotSegs + q * NSUB; };
+  auto block = [&](int p) { return TRANS ? NS - 1 - p : p; };
+  auto nsub = [&](int S) { return min(NSUB, ntiles - S * NSUB); };
+  // panel tiles (source position a -> target position b)
+  auto pair_units = [&](int a, int b) { return TRANS ? nsub(block(a)) * NSUB : NSUB * nsub(block(b)); };
+  // far pairs with 2 a + b = k: a = lo .. lo + count - 1; the last super-block,
+  // which may be partial, is in the first of them if in any
+  auto far_lo = [&](int k) { return max(0, (k - NS + 2) / 2); };
+  auto far_count = [&](int k) { return max(0, (k - 2) / 3 - far_lo(k) + 1); };
+  auto far_units = [&](int k) {
+    const int c = far_count(k);
+    return c == 0 ? 0 : pair_units(far_lo(k), k - 2 * far_lo(k)) + (c - 1) * NSUB * NSUB;
+  };
+  auto trmv_units = [&](int p) {
+    const int nb = nsub(block(p));
+    return nb * (nb + 1) / 2;
+  };
+  int a = -1, b = 0;                         // positions; a < 0: a TRMV tile of b
+  bool far = false;
+  for (;; ++cu.stage) {
+    const int p = cu.stage, near = p >= 0 ? pair_units(p, p + 1) : 0, trmv = trmv_units(p + 1);
+    int v = u - cu.first, k = 3 * p + 2;
+    if (v < near + trmv) {
+      if (v < near) a = p;
+      else v -= near;
+      b = p + 1;
+      u = v;
+      break;
     }
-    u -= npan;
-    const int ntr = nsubB * (nsubB + 1) / 2;
-    if (u < ntr) {
-      int i, j;
-      tri_of(u, i, j);
-      const int ri0 = b0 + i * RB, rj0 = b0 + j * RB;
-      jb.T = wsup + (size_t)B * RS * RS + (size_t)(j * RB) * RS + i * RB;
-      jb.ld = RS;
-      jb.nrow = min(RB, b0 + rb - ri0);
-      jb.ncol = min(RB, b0 + rb - rj0);
-      jb.panel = false;
-      if (!TRANS) {
-        // y_B(i) += W(i,j) w_B(j): w_B(j) has all gB panel contributions
-        jb.nt = true;
-        jb.vin_row0 = rj0; jb.vin_n = jb.ncol;
-        jb.out_row0 = ri0; jb.out_n = jb.nrow;
-        jb.wait_ctr = seg_in + gB + j; jb.wait_need = gB;
-        jb.sig_ctr = seg_out + gB + i;
-      } else {
-        // z_B(j) += W(i,j)^T w_B(i): w_B(i) has the contributions of every
-        // segment below B
-        jb.nt = false;
-        jb.vin_row0 = ri0; jb.vin_n = jb.nrow;
-        jb.out_row0 = rj0; jb.out_n = jb.ncol;
-        jb.wait_ctr = seg_in + gB + i; jb.wait_need = ntiles - gB - nsubB;
-        jb.sig_ctr = seg_out + gB + j;
+    v -= near + trmv;
+    int units = 0;
+    if (p >= 0)
+      for (; k < 3 * p + 5; ++k) {
+        units = far_units(k);
+        if (v < units) break;
+        v -= units;
       }
-      return true;
+    if (p >= 0 && k < 3 * p + 5) {
+      far = true;
+      a = far_lo(k);
+      const int first = pair_units(a, k - 2 * a);
+      if (v >= first) { a += 1 + (v - first) / (NSUB * NSUB); v = (v - first) % (NSUB * NSUB); }
+      b = k - 2 * a;
+      u = v;
+      break;
     }
-    u -= ntr;
+    if (p + 2 >= NS) return false;
+    cu.first = u - v;
   }
-  return false;
+  const int B = block(b), b0 = B * RS, nsubB = nsub(B), gB = b0 / RB;
+  const int nsubN = b == 0 ? 0 : nsub(block(b - 1));   // segments of B's neighbour in the chain
+  if (a >= 0) {
+    const int T = block(a), t0 = T * RS, gT = t0 / RB, nsubT = nsub(T);
+    jb.panel = true;
+    jb.ld = ldl;
+    // forward: w(rows r of B) -= L(r, T col c) y_T(c); backward: w(col segment c
+    // of B) -= L(T row r, c)^T z_T(r)
+    const int r = u / NSUB, c = u % NSUB;
+    const int src = TRANS ? r : c, dst = TRANS ? c : r;
+    const int r0 = (TRANS ? t0 : b0) + r * RB, c0 = (TRANS ? b0 : t0) + c * RB;
+    jb.T = L + (size_t)c0 * ldl + r0;
+    jb.nrow = min(RB, n - r0); jb.ncol = RB;
+    jb.nt = !TRANS;
+    jb.vin_row0 = TRANS ? r0 : c0; jb.vin_n = TRANS ? jb.nrow : RB;
+    jb.out_row0 = TRANS ? c0 : r0; jb.out_n = TRANS ? RB : jb.nrow;
+    if (!SLOTS || far) {
+      jb.wait_ctr = seg_out + gT + src;
+      jb.wait_need = SLOTS ? 1 : TRANS ? nsubT - src : src + 1;
+      jb.sig_ctr = seg_in + gB + dst;
+    } else {
+      // polling the slots starts once the source's far contributions are in
+      jb.wait_ctr = seg_in + gT + src;
+      jb.wait_need = TRANS ? max(0, ntiles - gT - 2 * NSUB) : max(0, gT - NSUB);
+      jb.sig_ctr = nullptr;
+      jb.in_slot = slot0(T, 0, src) + (TRANS ? src : 0);
+      jb.nin = TRANS ? nsubT - src : src + 1;
+      jb.in_blk = T;
+      jb.out_slot = slot0(B, 1, dst) + src;
+      jb.out_blk = B;
+    }
+    return true;
+  }
+  int i, j;
+  tri_of(u, i, j);
+  const int ri0 = b0 + i * RB, rj0 = b0 + j * RB;
+  jb.T = wsup + (size_t)B * RS * RS + (size_t)(j * RB) * RS + i * RB;
+  jb.ld = RS;
+  jb.nrow = min(RB, n - ri0);
+  jb.ncol = min(RB, n - rj0);
+  jb.panel = false;
+  jb.nt = !TRANS;
+  // forward: y_B(i) += W(i,j) w_B(j): w_B(j) has all gB panel contributions;
+  // backward: z_B(j) += W(i,j)^T w_B(i): w_B(i) has the contributions of
+  // every segment below B
+  const int in = TRANS ? i : j, o = TRANS ? j : i;
+  jb.vin_row0 = TRANS ? ri0 : rj0; jb.vin_n = TRANS ? jb.nrow : jb.ncol;
+  jb.out_row0 = TRANS ? rj0 : ri0; jb.out_n = TRANS ? jb.ncol : jb.nrow;
+  jb.wait_ctr = seg_in + gB + in;
+  jb.wait_need = TRANS ? ntiles - gB - nsubB : gB;
+  jb.sig_ctr = seg_out + gB + o;
+  if (SLOTS) {
+    jb.wait_need -= nsubN;                   // the near ones come through slots
+    jb.in_slot = slot0(B, 1, in); jb.nin = nsubN; jb.in_blk = B;
+    jb.out_slot = slot0(B, 0, o) + (TRANS ? i : j); jb.out_blk = B;
+    // the last unit of segment o (in the order of the units) completes it
+    const bool last = TRANS ? i == nsubB - 1 : i == j;
+    if (last) { jb.fin_slot = slot0(B, 0, o) + (TRANS ? o : 0); jb.nfin = TRANS ? nsubB - o : i + 1; }
+    else jb.sig_ctr = nullptr;
+  }
+  return true;
 }
 
 template <int NR>
@@ -1176,81 +1321,107 @@ size_t trsv_smem_bytes(int nrhs) {
   }
 }
 
-// Two CTAs per SM, each with one tile stage: a unit's tile copy is issued
-// as soon as the unit is taken and overlaps the wait for its input segment;
-// while one CTA waits on L2 round trips (unit counter, dependency counter,
-// vector segment, fence) the other computes.  The next unit number is taken
-// one unit ahead.  A CTA holds at most two units and finishes the earlier
-// one first; every unit depends only on earlier ones, so the earliest
-// unfinished unit always belongs to a CTA that is working on it, and every
-// wait ends.
+// Two (or three) CTAs per SM, each with one tile stage: a unit's tile copy is
+// issued as soon as the unit is taken and overlaps the wait for its input
+// segment; while one CTA waits on L2 round trips (dependency counter, vector
+// segment, fence) the other computes.  A CTA finishes its unit before it starts
+// the next, whose number it asks for only when the unit's input is there; every
+// unit depends only on earlier ones, so the earliest unfinished unit always
+// belongs to a CTA that is working on it, and every wait ends.
+template <int NR>
+constexpr int trsv_ctas() { return NR == 1 ? 3 : 2; }   // most per SM
+
 template <int NR, bool TRANS>
-__global__ void __launch_bounds__(NTH, 2)
+__global__ void __launch_bounds__(NTH, trsv_ctas<NR>())
 trsv_persistent_kernel(const float* __restrict__ L, int ldl, int n, const float* __restrict__ wsup,
                        double* __restrict__ work, double* __restrict__ out, int* ctr,
-                       const int* skip, DevStatus* st) {
+                       TrsvSlot* slots, const int* skip, DevStatus* st) {
   if (skip != nullptr && *skip) return;
   constexpr bool MMA = NR == 8;
+  constexpr bool SLOTS = NR <= kSlotNr;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   float* Ts = reinterpret_cast<float*>(sm_raw);                           // one stage
   double* s_v = reinterpret_cast<double*>(Ts + (MMA ? BL_TILE : TILE_ELEMS));   // RB x NR
   double* s_col = s_v + RB * NR;                                          // RB x NR
   __shared__ int s_unit[2];
+  __shared__ unsigned long long s_epoch;
   int* next = ctr;
-  int* seg_in = ctr + 1;
+  int* exits = ctr + 1;         // CTAs that are done
+  int* seg_in = ctr + 2;
   int* seg_out = seg_in + ceil_div(n, RB);
-  if (threadIdx.x == 0) s_unit[0] = atomicAdd(next, 1);
+  // The launch's number, which the tags carry: in the slots' header, one more
+  // after each launch (the last CTA to leave raises it).
+  unsigned long long* epoch = reinterpret_cast<unsigned long long*>(slots);
+  if (threadIdx.x == 0) {
+    if (SLOTS) s_epoch = *reinterpret_cast<volatile unsigned long long*>(epoch);
+    s_unit[0] = atomicAdd(next, 1);
+  }
   __syncthreads();
   int ucur = s_unit[0];
+  TrsvSlot* slot = slots + 1;
+  const unsigned long long tag0 = SLOTS ? (s_epoch << 20) + 1 : 0;
+  TrsvCursor cursor{-1, 0};
   TrsvJob cur;
-  bool have = trsv_job<TRANS>(ucur, L, ldl, n, wsup, seg_in, seg_out, cur);
-  for (int it = 1; have; ++it) {
+  for (int it = 1; trsv_job<TRANS, SLOTS>(ucur, cursor, L, ldl, n, wsup, seg_in, seg_out, cur); ++it) {
     if (MMA) stage_tile_bl(Ts, cur.T, cur.ld, cur.nrow, cur.ncol);
     else stage_tile(Ts, cur.T, cur.ld, cur.nrow, cur.ncol);
     cp_async_commit();
-    // the next unit number, taken by a thread of warp 1 so that its round
-    // trip overlaps warp 0's dependency poll; read after this unit's
-    // barriers (s_unit[it & 1] is not read again before its next write)
-    if (threadIdx.x == 32) s_unit[it & 1] = atomicAdd(next, 1);
     wait_count(cur.wait_ctr, cur.wait_need, st, ucur);
-    if (MMA) {
-      load_vec_x8(cur.panel ? out : work, n, cur.vin_row0, cur.vin_n, s_v);
-      cp_async_wait<0>();
-      __syncthreads();
-      double* dst = cur.panel ? work : out;
-      if (cur.nt)
-        tile_mma_x8<false, false, 4, RB / 16, 1>(Ts, s_v, s_v, dst, cur.out_row0, cur.out_n, dst,
-                                                 cur.out_row0, cur.out_n, n, true, false,
-                                                 cur.panel ? -1.0 : 1.0, nullptr);
-      else
-        tile_mma_x8<false, false, 4, RB / 16, 2>(Ts, s_v, s_v, dst, cur.out_row0, cur.out_n, dst,
-                                                 cur.out_row0, cur.out_n, n, false, true,
-                                                 cur.panel ? -1.0 : 1.0, nullptr);
-      signal_count(cur.sig_ctr);   // its barrier also frees the stage and s_v
-      ucur = s_unit[it & 1];
-      have = trsv_job<TRANS>(ucur, L, ldl, n, wsup, seg_in, seg_out, cur);
-      continue;
-    }
-    load_vec<NR>(cur.panel ? out : work, n, cur.vin_row0, cur.vin_n, s_v);
-    cp_async_wait<0>();
-    __syncthreads();
-    double acc[4][NR] = {};
-    tile_pass_staged<NR, false>(Ts, s_v, s_v, acc, s_col, cur.nt, !cur.nt);
-    __syncthreads();
+    // the next number, asked for once this unit's input is there: its round trip
+    // overlaps the tile pass, and no unit is bound to a CTA that still waits
+    // (s_unit[it & 1] is read after this unit's barriers)
+    auto take_next = [&]() {
+      if (threadIdx.x == 32) s_unit[it & 1] = atomicAdd(next, 1);
+    };
     double* dst = cur.panel ? work : out;
     const double sign = cur.panel ? -1.0 : 1.0;
-    if (cur.nt) {
-      flush_rows<NR>(acc, reinterpret_cast<double*>(Ts), dst, n, cur.out_row0, cur.out_n, sign);
+    if constexpr (MMA) {
+      load_vec_x8(cur.panel ? out : work, n, cur.vin_row0, cur.vin_n, s_v);
+      take_next();
+      cp_async_wait<0>();
+      __syncthreads();
+      if (cur.nt)
+        tile_mma_x8<false, false, 4, RB / 16, 1>(Ts, s_v, s_v, dst, cur.out_row0, cur.out_n, dst,
+                                                 cur.out_row0, cur.out_n, n, true, false, sign, nullptr);
+      else
+        tile_mma_x8<false, false, 4, RB / 16, 2>(Ts, s_v, s_v, dst, cur.out_row0, cur.out_n, dst,
+                                                 cur.out_row0, cur.out_n, n, false, true, sign, nullptr);
+      signal_count(cur.sig_ctr);   // its barrier also frees the stage and s_v
     } else {
+      if (cur.nin == 0)
+        load_vec<NR>(cur.panel ? out : work, n, cur.vin_row0, cur.vin_n, s_v);
+      else
+        gather_slots<NR>(slot + (size_t)cur.in_slot * RB * NR, cur.nin, tag0 + cur.in_blk,
+                         cur.panel ? nullptr : work, n, cur.vin_row0, cur.vin_n, s_v, s_col, st, ucur);
+      take_next();
+      cp_async_wait<0>();
+      __syncthreads();
+      double acc[4][NR] = {};
+      tile_pass_staged<NR, false>(Ts, s_v, s_v, acc, s_col, cur.nt, !cur.nt);
+      __syncthreads();
+      double* red = reinterpret_cast<double*>(Ts);
+      if (cur.nt) stage_rows<NR>(acc, red);
       for (int e = threadIdx.x; e < RB * NR; e += NTH) {
-        const int k = e / RB, c = e % RB;
-        if (c < cur.out_n) atomicAdd(&dst[(size_t)k * n + cur.out_row0 + c], sign * s_col[e]);
+        const int r = e % RB;
+        const double v = sign * (cur.nt ? row_sum<NR>(red, e) : s_col[e]);
+        if (cur.out_slot >= 0) slot_put(slot + (size_t)cur.out_slot * RB * NR + e, v, tag0 + cur.out_blk);
+        else if (r < cur.out_n) atomicAdd(&dst[(size_t)(e / RB) * n + cur.out_row0 + r], v);
       }
+      if (cur.nfin > 0) {
+        // the segment's sums into the result (s_v is free; the odd sums pass
+        // through the half of the stage that `red` leaves)
+        gather_slots<NR>(slot + (size_t)cur.fin_slot * RB * NR, cur.nfin, tag0 + cur.out_blk, nullptr, n,
+                         0, 0, s_v, red + TILE_ELEMS / 4, st, ucur);
+        for (int e = threadIdx.x; e < RB * NR; e += NTH)
+          if (e % RB < cur.out_n) __stcg(&out[(size_t)(e / RB) * n + cur.out_row0 + e % RB], s_v[e]);
+      }
+      // the barrier also frees the stage, s_v and s_col
+      if (cur.sig_ctr != nullptr) signal_count(cur.sig_ctr);
+      else __syncthreads();
     }
-    signal_count(cur.sig_ctr);   // its barrier also frees the stage, s_v and s_col
     ucur = s_unit[it & 1];
-    have = trsv_job<TRANS>(ucur, L, ldl, n, wsup, seg_in, seg_out, cur);
   }
+  if (SLOTS && threadIdx.x == 0 && atomicAdd(exits, 1) == (int)gridDim.x - 1) *epoch = s_epoch + 1;
 }
 
 // ---- batched variants: one launch serves every system of a batch --------
@@ -1639,7 +1810,11 @@ cudaError_t launch_trsv_batched(bool backward, const BatchSys* sys, int nsys, in
   return cudaGetLastError();
 }
 
-size_t trsv_counter_ints(int n) { return 1 + 2 * (size_t)ceil_div(n, RB); }
+size_t trsv_slot_bytes() {
+  return sizeof(TrsvSlot) * (1 + (size_t)4 * kSlotSegs * RB * kSlotNr);
+}
+
+size_t trsv_counter_ints(int n) { return 2 + 2 * (size_t)ceil_div(n, RB); }
 
 cudaError_t launch_trsv_prep(const double* in, double* w, double* mid, double* out, int n, int nrhs,
                              int* counters, cudaStream_t stream) {
@@ -1651,25 +1826,31 @@ cudaError_t launch_trsv_prep(const double* in, double* w, double* mid, double* o
 // One cooperative launch over every resident CTA.
 cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n,
                                    const float* wsup, double* work, double* out, int nrhs, int* counters,
-                                   const int* skip, DevStatus* st, cudaStream_t stream) {
+                                   void* slots, const int* skip, DevStatus* st, cudaStream_t stream) {
   cudaError_t e;
-  static int grid_cache[64][2][4] = {};
+  static int grid_cache[64][2][4] = {}, sm_cache[64] = {};
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   const int nri = nrhs == 1 ? 0 : nrhs == 2 ? 1 : nrhs == 4 ? 2 : 3;
-  int& grid = grid_cache[dev & 63][backward ? 1 : 0][nri];
+  int& resident = grid_cache[dev & 63][backward ? 1 : 0][nri];
+  int& sms = sm_cache[dev & 63];
   const size_t smem = trsv_smem_bytes(nrhs);
   auto launch = [&](auto kernel) -> cudaError_t {
-    if (grid == 0) {
+    if (resident == 0) {
       int per_sm = 0, nsm = 0;
       cudaError_t ee = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NTH,
                                                                      smem);
       if (ee == cudaSuccess) ee = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
       if (ee != cudaSuccess) return ee;
-      grid = std::max(1, per_sm) * nsm;
+      resident = std::max(1, per_sm) * nsm;
+      sms = nsm;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    // The third CTA per SM (one right-hand side) pays once far tiles bound the
+    // solve; before that it only slows the chain's tile passes: forward / backward
+    // 57 / 65 us with two and 58 / 67 with three at n = 8192, 78 / 88 and 76 / 82
+    // at 10240, 168 / 185 and 145 / 158 at 16384.
+    cfg.gridDim = dim3(n > 9 * RS ? resident : std::min(resident, 2 * sms));
     cfg.blockDim = dim3(NTH);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -1678,7 +1859,8 @@ cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, L, ldl, n, wsup, work, out, counters, skip, st);
+    return cudaLaunchKernelEx(&cfg, kernel, L, ldl, n, wsup, work, out, counters,
+                              static_cast<TrsvSlot*>(slots), skip, st);
   };
   if (!backward) {
     NR_SWITCH(nrhs, (e = launch(trsv_persistent_kernel<NRC, false>)));

@@ -74,6 +74,26 @@ def test_preconditioner_apply_at_block_and_super_block_edges(n):
     assert ((Z - ref).norm() / ref.norm()).item() < 1e-5
 
 
+@pytest.mark.parametrize("n,nrhs", [(1025, 1), (2049, 2), (2200, 1), (3333, 1), (3200, 2), (3100, 4), (4097, 8),
+                                    (9728, 1), (9601, 2)])
+def test_triangular_solves_over_many_super_blocks(n, nrhs):
+    """The persistent solve for each number of right-hand sides, with partial
+    super-blocks and both grids, twice in a row (its slots are used again)
+    against FP64.  A diagonally dominant A keeps kappa(L) below 2: the FP32
+    inverses leave 1e-6, the bound has another digit."""
+    g = torch.Generator().manual_seed(n)
+    A = (torch.rand(n, n, generator=g) - 0.5).cuda()
+    A = A + A.T
+    A.diagonal().add_(2.0 * n)
+    f = mp.factor(A, block_size=256, precision="fp32")
+    L = f.lower().double()
+    for seed in (1, 2):
+        R = matgen.rhs(n, nrhs, seed).cuda()
+        ref = torch.cholesky_solve(R.reshape(n, -1), L).reshape(R.shape)
+        Z = f.apply_precond(R)
+        assert ((Z - ref).norm() / ref.norm()).item() < 1e-5
+
+
 @pytest.mark.parametrize("n,d,lower", [
     (1, 3, False), (63, 16, True), (65, 17, False), (2047, 15, True), (2305, 33, True),
 ])
