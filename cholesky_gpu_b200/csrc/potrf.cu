@@ -734,15 +734,17 @@ __device__ __forceinline__ void load_tiles(float* tiles, const float* A, int lda
     }
   }
 }
-__device__ __forceinline__ void store_tiles(const float* tiles, float* A, int lda, int bs, int ntiles,
-                                            bool vec, int tid) {
+// Tile t by the calling warp.
+__device__ __forceinline__ void store_tile(const float* tiles, float* A, int lda, int bs, int t, bool vec,
+                                           int lane) {
+  int I, J;
+  tile_of(t, I, J);
+  tiles += t * TSZ;
   if (vec) {
-    const int r4 = 4 * (tid & 7), c = (tid & 255) >> 3;
-#pragma unroll 2
-    for (int t = tid >> 8; t < ntiles; t += 2) {
-      int I, J;
-      tile_of(t, I, J);
-      const float4 v = *reinterpret_cast<const float4*>(tiles + t * TSZ + c * TS + r4);
+    const int r4 = 4 * (lane & 7);
+#pragma unroll 4
+    for (int c = lane >> 3; c < TS; c += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(tiles + c * TS + r4);
       float* g = A + (size_t)(J * TS + c) * lda + I * TS + r4;
       if (I > J || r4 >= c) {
         *reinterpret_cast<float4*>(g) = v;
@@ -753,12 +755,11 @@ __device__ __forceinline__ void store_tiles(const float* tiles, float* A, int ld
       }
     }
   } else {
+    const int r = I * TS + lane;
 #pragma unroll 1
-    for (int e = tid; e < ntiles * TSZ; e += 512) {
-      int I, J;
-      tile_of(e / TSZ, I, J);
-      const int r = I * TS + e % TS, c = J * TS + e % TSZ / TS;
-      if (r < bs && c < bs && r >= c) A[(size_t)c * lda + r] = tiles[e];
+    for (int k = 0; k < TS; ++k) {
+      const int c = J * TS + k;
+      if (r < bs && c < bs && r >= c) A[(size_t)c * lda + r] = tiles[k * TS + lane];
     }
   }
 }
@@ -858,10 +859,13 @@ potrf_f32_block(float* tiles, float* A, int lda, int s, int bs, const float* d, 
       if (log.fail >= 0) atomicMin(&s_fail, I * TS + log.fail);
       if (log.npert) atomicAdd(&s_pert, log.npert);
     }
-    // the inverse for the panel solve, where the SM has issue slots to spare;
-    // the first tiles' and the last one's wait for the end
-    if (I >= 2 && I < NT - 1)
+    // the inverse for the panel solve, where the SM has issue slots to spare: the
+    // first two tiles' beside the last three columns, the last one's beside the
+    // stores
+    if (I < NT - 1) {
+      if (I < 2) ok = tc::mbar_wait(&sub[max(I + 1, NT - 3) * NSUB], 0) && ok;
       invert_tile<float, SUB>(mine, s_inv + I * TS, winv + I * TS * TS, lane);
+    }
   } else {
     // tile (I, K), K >= 2, by columns 0 .. K - 2, in column order over all
     // helpers: a task waits only for tiles that need tasks of earlier columns
@@ -891,9 +895,12 @@ potrf_f32_block(float* tiles, float* A, int lda, int s, int bs, const float* d, 
     if (tid == 0) set_status(st, MPCHOL_ERR_NOT_SPD, s + s_fail);
     return;
   }
-  store_tiles(tiles, Ab, lda, bs, ntiles, vec, tid);
-  if (warp < 2 ? warp < NT : warp == NT - 1)
-    invert_tile<float, SUB>(tiles + tidx(warp, warp) * TSZ, s_inv + warp * TS, winv + warp * TS * TS, lane);
+  if (warp == NT - 1) {
+    invert_tile<float, SUB>(tiles + (ntiles - 1) * TSZ, s_inv + warp * TS, winv + warp * TS * TS, lane);
+  } else {
+    for (int t = warp < NT - 1 ? warp : warp - 1; t < ntiles; t += nwarps - 1)
+      store_tile(tiles, Ab, lda, bs, t, vec, lane);
+  }
   if (tid == 0 && s_pert) atomicAdd(&st->perturbed, s_pert);
 }
 
