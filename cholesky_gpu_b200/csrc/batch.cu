@@ -26,25 +26,33 @@ namespace {
 constexpr int kSlots = 8;
 constexpr int kScal = 64;
 
-// A_i <- the caller's matrix (column-major, ld ldsrc[i]); d = dtilde = diag,
-// sh = 0.
-__global__ void batch_load_kernel(const BatchSys* __restrict__ sys, const float* const* __restrict__ src,
-                                  const int* __restrict__ ldsrc) {
+// A_i <- the lower triangle of the caller's matrix (column-major, ld ldsrc[i];
+// whole 32-row tiles at the diagonal); d = dtilde = diag, sh = 0.  A warp per
+// column, eight loads in flight per lane whatever the order: the pass reads and
+// writes half of what a copy of the square does (128 systems of 64 to 2048: 484
+// -> 120 us).
+__global__ void __launch_bounds__(256)
+batch_load_kernel(const BatchSys* __restrict__ sys, const float* const* __restrict__ src,
+                  const int* __restrict__ ldsrc) {
   const BatchSys& S = sys[blockIdx.y];
   const float* a = src[blockIdx.y];
   const int lda = ldsrc[blockIdx.y];
-  const int n = S.n;
-  // CTA x copies columns x, x + gridDim.x, ..., its threads run down a column
-  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+  const int n = S.n, lane = threadIdx.x & 31, nw = blockDim.x / 32;
+  for (int c = blockIdx.x * nw + threadIdx.x / 32; c < n; c += gridDim.x * nw) {
     const float* ac = a + (size_t)c * lda;
     float* dc = S.A + (size_t)c * S.ld;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
-      const float v = ac[r];
-      dc[r] = v;
-      if (r == c) {
-        S.d[r] = v;
-        S.dtilde[r] = v;
-        S.sh[r] = 0.0f;
+    for (int r0 = c / 32 * 32 + lane; r0 < n; r0 += 256) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r0 + 32 * u < n) v[u] = ac[r0 + 32 * u];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r0 + 32 * u < n) dc[r0 + 32 * u] = v[u];
+      if (r0 == c) {                               // in the column's first 32 rows
+        S.d[c] = v[0];
+        S.dtilde[c] = v[0];
+        S.sh[c] = 0.0f;
       }
     }
   }
@@ -93,6 +101,8 @@ struct mpchol_batch {
   DevStatus* h_st = nullptr;
   int* h_open = nullptr;
   cudaStream_t cap = nullptr;
+  cudaEvent_t ev_loaded = nullptr;     // a factor call has read the caller's matrices
+  cudaEvent_t ev_factored = nullptr;   // ... and is complete
   cudaGraphExec_t fgraph = nullptr;
   cudaGraphExec_t igraph = nullptr;
   double ig_tol2 = -1.0;
@@ -112,16 +122,15 @@ void batch_free(mpchol_batch* B) {
   if (B->fgraph) cudaGraphExecDestroy(B->fgraph);
   if (B->igraph) cudaGraphExecDestroy(B->igraph);
   if (B->cap) cudaStreamDestroy(B->cap);
+  for (cudaEvent_t e : {B->ev_loaded, B->ev_factored})
+    if (e) cudaEventDestroy(e);
   delete B;
 }
 
-// The factor sequence for every system (captured once into B->fgraph).
+// The factor sequence for every system, from the loaded matrices (captured once
+// into B->fgraph).
 mpchol_status enqueue_factor(mpchol_batch* B, cudaStream_t s) {
   const PotrfParams pp{B->opts.diag_pert, B->opts.pert, B->opts.pivot_floor};
-  MPCHOL_CUDA_TRY(cudaMemsetAsync(B->st, 0, sizeof(DevStatus) * B->count, s));
-  batch_load_kernel<<<dim3(64, B->count), 256, 0, s>>>(
-      B->d_sys, reinterpret_cast<const float* const*>(B->d_ptrs), B->d_ld);
-  MPCHOL_CUDA_TRY(cudaGetLastError());
   for (int k = 0; k < B->nsteps; ++k) {
     const int sk = k * B->b;
     const BatchStep* steps = B->d_steps + (size_t)k * B->count;
@@ -302,7 +311,9 @@ mpchol_status mpchol_batch_create(const mpchol_opts* opts, int count, const int*
   if (cudaMemcpy(B->d_sys, B->h_sys.data(), sizeof(BatchSys) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(B->d_steps, B->h_steps.data(), sizeof(BatchStep) * B->h_steps.size(),
                  cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&B->cap, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaStreamCreateWithFlags(&B->cap, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_loaded, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_factored, cudaEventDisableTiming) != cudaSuccess) {
     batch_free(B);
     return MPCHOL_ERR_CUDA;
   }
@@ -328,6 +339,11 @@ mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, con
   MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->d_ptrs, B->h_ptrs, sizeof(void*) * B->count,
                                   cudaMemcpyHostToDevice, s));
   MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->d_ld, B->h_ld, sizeof(int) * B->count, cudaMemcpyHostToDevice, s));
+  MPCHOL_CUDA_TRY(cudaMemsetAsync(B->st, 0, sizeof(DevStatus) * B->count, s));
+  batch_load_kernel<<<dim3(64, B->count), 256, 0, s>>>(
+      B->d_sys, reinterpret_cast<const float* const*>(B->d_ptrs), B->d_ld);
+  MPCHOL_CUDA_TRY(cudaGetLastError());
+  MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_loaded, s));
   if (B->fgraph == nullptr) {
     cudaGraph_t g = nullptr;
     // relaxed: the launchers set kernel attributes (not stream work) as they go
@@ -344,14 +360,17 @@ mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, con
     MPCHOL_CUDA_TRY(ie);
   }
   MPCHOL_CUDA_TRY(cudaGraphLaunch(B->fgraph, s));
-  // the host pointer tables are reused by the next call: finish reading them
-  MPCHOL_CUDA_TRY(cudaStreamSynchronize(s));
+  MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_factored, s));
+  // the caller's matrices and the host pointer tables are free again once they
+  // have been read; the host prepares the solve while the device factors
+  MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_loaded));
   return MPCHOL_OK;
 }
 
 mpchol_status mpchol_batch_lower(const mpchol_batch_t* B, int index, const float** dL, int* ldl,
                                  int* n) {
   if (B == nullptr || dL == nullptr || index < 0 || index >= B->count) return MPCHOL_ERR_BAD_ARG;
+  MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_factored));   // the caller may read it on any stream
   const int i = (int)(std::find(B->order.begin(), B->order.end(), index) - B->order.begin());
   *dL = B->h_sys[i].A;
   if (ldl) *ldl = B->h_sys[i].ld;
@@ -363,6 +382,7 @@ mpchol_status mpchol_batch_info(mpchol_batch_t* B, int* status, int* fail_row, i
                                 mpchol_stream_t stream_) {
   if (B == nullptr || status == nullptr) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  MPCHOL_CUDA_TRY(cudaStreamWaitEvent(s, B->ev_factored, 0));
   MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->h_st, B->st, sizeof(DevStatus) * B->count,
                                   cudaMemcpyDeviceToHost, s));
   MPCHOL_CUDA_TRY(cudaStreamSynchronize(s));
@@ -387,6 +407,7 @@ mpchol_status mpchol_batch_pcg(mpchol_batch_t* B, const float* const* dA, const 
   if (po.check_every < 2) po.check_every = 2;
   if (po.max_it < 0) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  MPCHOL_CUDA_TRY(cudaStreamWaitEvent(s, B->ev_factored, 0));   // the factor call's stream may be another
   const int ns = B->count, nr = B->nr;
   for (int i = 0; i < ns; ++i) {
     const int u = B->order[i];
@@ -469,7 +490,7 @@ mpchol_status mpchol_batch_pcg(mpchol_batch_t* B, const float* const* dA, const 
     MPCHOL_CUDA_TRY(launch_dot_batched(B->d_sys, ns, 0, 0, 3, nr, 0, s));
     MPCHOL_CUDA_TRY(launch_reduce_batched(B->d_sys, ns, 3, 40, nr, 0, s));
     MPCHOL_CUDA_TRY(launch_frob_batched(B->d_sys, ns, s));
-    MPCHOL_CUDA_TRY(launch_reduce_batched(B->d_sys, ns, 3, 48, 1, 0, s));
+    MPCHOL_CUDA_TRY(launch_reduce_batched(B->d_sys, ns, 3, 48, 8, 0, s));   // eight sums of four
     MPCHOL_CUDA_TRY(launch_dot_batched(B->d_sys, ns, 1, 2, 2, nr, 0, s));
     MPCHOL_CUDA_TRY(launch_reduce_batched(B->d_sys, ns, 2, 56, nr, 0, s));
   }
@@ -483,7 +504,9 @@ mpchol_status mpchol_batch_pcg(mpchol_batch_t* B, const float* const* dA, const 
     const double* sc = B->h_scal + (size_t)i * kScal;
     bool conv = true;
     double relmax = 0.0, bemax = 0.0, prmax = 0.0;
-    const double frob = std::sqrt(sc[48]);
+    double fro2 = 0.0;
+    for (int k = 0; k < 8; ++k) fro2 += sc[48 + k];
+    const double frob = std::sqrt(fro2);
     for (int k = 0; k < B->nrhs; ++k) {
       const double rr = sc[32 + k], bb2 = sc[24 + k], xx = sc[40 + k];
       if (!(rr <= tol2 * bb2)) conv = false;

@@ -517,9 +517,11 @@ trsm_panel_kernel(const __grid_constant__ CUtensorMap tmapX, const __grid_consta
 }
 
 // Batched: blockIdx.y = system, blockIdx.x = 32-row slab.  Staging by
-// plain coalesced loads (no per-system tensor maps), the same slab solve;
-// the epilogue keeps the row sums of squares (rounding-shift estimate) and
-// the diagonal tracker.
+// cp.async (no per-system tensor maps), all of it in flight at once: with plain
+// loads, two in flight per thread, staging took as long as the solve (128
+// systems of 64 to 2048, all steps: 1354 -> 788 us).  The same slab solve; the
+// epilogue keeps the row sums of squares (rounding-shift estimate) and the
+// diagonal tracker.
 __global__ void __launch_bounds__(NTHR, 2)
 trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
   constexpr int TR = 32;
@@ -544,17 +546,20 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
     for (int J = 0; J < NT; ++J) tc::mbar_init(&ready[J], 64);
     tc::fence_mbar_init();
   }
-  for (int e = tid; e < bs * TR; e += NTHR) {
-    const int c = e / TR, r = e % TR;
-    Xs[xoff<TR>(r, c, bs)] = (r < nrows) ? A[(size_t)(s + c) * ld + row0 + r] : 0.0f;
+  // everything by 16-byte asynchronous copies, all in flight at once (columns of
+  // the library's storage start on 128-byte boundaries at multiples of 32 rows;
+  // slab rows past n are its padding, whose results are not stored)
+  const int r4 = 4 * (tid & 7);
+  for (int c = tid >> 3; c < bs; c += NTHR / 8)
+    tc::cp_async16(Xs + c * TR + r4, A + (size_t)(s + c) * ld + row0 + r4);
+  for (int q = tid >> 8; q < NT * (NT - 1) / 2; q += NTHR / 256) {   // half a CTA per tile
+    int I = 1;
+    while (tl(I + 1, 0) <= q) ++I;
+    const int M = q - tl(I, 0), c = (tid & 255) >> 3;
+    tc::cp_async16(Lt + q * TSZ + c * 32 + r4, A + (size_t)(s + 32 * M + c) * ld + s + 32 * I + r4);
   }
-  for (int I = 1; I < NT; ++I)
-    for (int M = 0; M < I; ++M)
-      for (int e = tid; e < TSZ; e += NTHR) {
-        const int c = e / 32, r = e % 32;
-        Lt[tl(I, M) * TSZ + e] = A[(size_t)(s + 32 * M + c) * ld + s + 32 * I + r];
-      }
-  for (int e = tid; e < NT * TSZ; e += NTHR) Wt[e] = S.winv[e];
+  for (int e = 4 * tid; e < NT * TSZ; e += 4 * NTHR) tc::cp_async16(Wt + e, S.winv + e);
+  tc::cp_async_wait_all();
   __syncthreads();
   if (!slab_solve<TR>(Xs, bs, Lt, Wt, nullptr, ready, tid, [](int, int) {})) {
     s_ok = 0;
@@ -562,9 +567,15 @@ trsm_batched_kernel(BatchSys* __restrict__ sys, int s, int b) {
   }
   __syncthreads();
   if (!s_ok) return;
-  for (int e = tid; e < bs * TR; e += NTHR) {
-    const int c = e / TR, r = e % TR;
-    if (r < nrows) S.A[(size_t)(s + c) * ld + row0 + r] = Xs[xoff<TR>(r, c, bs)];
+  for (int c = tid >> 3; c < bs; c += NTHR / 8) {
+    const float4 v = *reinterpret_cast<const float4*>(Xs + c * TR + r4);
+    float* g = S.A + (size_t)(s + c) * ld + row0 + r4;
+    if (r4 + 3 < nrows) *reinterpret_cast<float4*>(g) = v;
+    else {
+      if (r4 < nrows) g[0] = v.x;
+      if (r4 + 1 < nrows) g[1] = v.y;
+      if (r4 + 2 < nrows) g[2] = v.z;
+    }
   }
   __shared__ float s_sq[NTHR / TR][TR];
   slab_row_partials<TR>(Xs, bs, s_sq, tid);

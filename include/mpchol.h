@@ -389,8 +389,9 @@ MPCHOL_API mpchol_status mpchol_syrk_update(float* dC, int ldc, int m, int k, in
  * device pointers.  Matrices are FP32 column-major (ld lda[i]) with the lower
  * triangle read; B and X are n_i x nrhs FP64 column-major (ld n_i).
  *   mpchol_batch_factor: one CUDA graph launch factors every system (and
- *     forms the solve data); blocks the host until it has read the pointer
- *     tables.
+ *     forms the solve data); blocks the host until the matrices and the
+ *     pointer tables have been read, not until the factors are complete
+ *     (the calls below wait for them, on whatever stream).
  *   mpchol_batch_pcg: PCG of every system in lockstep (converged ones skip),
  *     FP64 true residual per system; reports[i] per system (may be NULL).
  *     Returns OK if every system converged, PCG_MAXIT otherwise. */
