@@ -28,12 +28,16 @@ def rbf_build(X: torch.Tensor, lengthscale: float, nugget: float, fp64: bool = T
     of X (n x d FP32 CUDA tensor).  Returns (K64, K32); each is an n x n
     tensor whose storage is column-major (symmetric: the lower triangle holds
     K when lower_only)."""
+    return _rbf_build(X, lengthscale, nugget, fp64, fp32, lower_only, torch.zeros)
+
+
+def _rbf_build(X, lengthscale, nugget, fp64, fp32, lower_only, alloc):
     if not X.is_cuda or X.dtype != torch.float32 or X.dim() != 2:
         raise ValueError("X must be an n x d float32 CUDA tensor")
     Xc = X.contiguous()
     n, d = Xc.shape
-    K64 = torch.zeros((n, n), dtype=torch.float64, device=X.device) if fp64 else None
-    K32 = torch.zeros((n, n), dtype=torch.float32, device=X.device) if fp32 else None
+    K64 = alloc((n, n), dtype=torch.float64, device=X.device) if fp64 else None
+    K32 = alloc((n, n), dtype=torch.float32, device=X.device) if fp32 else None
     lib = load()
     check(lib.mpchol_rbf_build(Xc.data_ptr(), n, d, d, float(lengthscale), float(nugget),
                                None if K64 is None else K64.data_ptr(),
@@ -70,7 +74,9 @@ class RBFSolve(torch.autograd.Function):
         max_it = opts.pop("max_it", 500)
         ell = float(lengthscale)
         lam = float(nugget)
-        K64, K32 = rbf_build(X.detach(), ell, lam)
+        # the solves read the lower triangles only: no pass over the matrices to
+        # clear the rest (n = 8192: 108 us)
+        K64, K32 = _rbf_build(X.detach(), ell, lam, True, True, True, torch.empty)
         n = X.shape[0]
         f = Factor(n, **opts)
         f.compute(K32)

@@ -233,3 +233,29 @@ def test_small_solve_stops_at_its_iteration_budget_and_reports_failures():
     with pytest.raises(mp.MpcholError) as e:      # an indefinite operator: p^T A p < 0
         f.pcg(bad, B)
     assert e.value.status == 6
+
+
+@pytest.mark.parametrize("n,opts", [(300, {}), (1300, dict(block_size=128, precision="fp32"))])
+def test_rbf_solve_reads_lower_triangles_only(n, opts):
+    """The kernel matrices of a differentiable solve come from uncleared memory:
+    with NaN in the blocks that the allocator hands out next, the solution and
+    the gradients are those of a solve on zeroed blocks.  Tolerance: two PCG
+    solves to 1e-11 at kappa below 1e4."""
+    from cholesky_gpu_b200 import rbf_solve
+    g = torch.Generator().manual_seed(n)
+    X = torch.randn(n, 3, generator=g).cuda()
+    y = torch.randn(n, generator=g, dtype=torch.float64).cuda()
+
+    def run(fill):
+        torch.cuda.empty_cache()
+        held = [torch.full((n, n), fill, dtype=t, device="cuda") for t in (torch.float64, torch.float32)]
+        torch.cuda.synchronize()
+        del held
+        Xr = X.clone().requires_grad_(True)
+        x = rbf_solve(Xr, 1.0, 0.5, y, rel_tol=1e-11, **opts)
+        (gX,) = torch.autograd.grad((x * y).sum(), Xr)
+        return x.detach(), gX
+
+    (x0, g0), (x1, g1) = run(0.0), run(float("nan"))
+    assert ((x1 - x0).norm() / x0.norm()).item() < 1e-6
+    assert ((g1 - g0).norm() / g0.norm()).item() < 1e-6
