@@ -512,82 +512,65 @@ __device__ __forceinline__ void stage_tile_4b(float* dst, const float* T, int ld
   }
 }
 
-// Shared memory of the staged SYMV: STAGES x (tile + x_J + x_I) + column sums.
-// 8 rhs: one 84 KB stage per CTA and two CTAs per SM (each CTA's load
-// overlaps the other's tile pass; 16 warps hide the DMMA and shared-memory
-// latencies better than one CTA with two stages: 306 vs 331 us at n = 16384)
+// CTAs per SM of the staged SYMV, each with one stage (tile + x_J + x_I, and the
+// column sums): a CTA's load overlaps the others' tile passes, and 16 or 24
+// warps hide the FP64 and shared-memory latencies better than one CTA with its
+// tiles staged two ahead.  One rhs, n = 8192: 36 us -> 30; two, 4100: 15.3 ->
+// 13.8; four, 2999: 21.5 -> 18.3; eight, 16384: 331 -> 306.
 template <int NR>
-constexpr int symv_stages() { return NR >= 8 ? 1 : 3; }
+constexpr int symv_ctas() { return NR == 1 ? 3 : 2; }
 template <int NR>
 constexpr size_t symv_staged_smem() {
   if (NR == 8)   // blocked tiles and padded segments, no column-sum buffer
-    return (size_t)symv_stages<NR>() * (BL_TILE * sizeof(float) + 2 * (size_t)XS * 8 * sizeof(double));
-  return (size_t)symv_stages<NR>() * (TILE_ELEMS * sizeof(float) + 2 * RB * NR * sizeof(double)) +
-         (size_t)RB * NR * sizeof(double);
+    return BL_TILE * sizeof(float) + 2 * (size_t)XS * 8 * sizeof(double);
+  return TILE_ELEMS * sizeof(float) + 3 * (size_t)RB * NR * sizeof(double);
 }
 
 // ---- y += A x, FP32 symmetric A (lower triangle), persistent over the tiles.
-// CTA b takes tiles b, b + grid, ...; each tile is staged symv_stages - 1
-// tiles ahead together with its two vector segments.  The row partials are
+// CTA b takes tiles b, b + grid, ...; each tile is staged together with its two
+// vector segments.  The row partials are
 // reduced in the stage's own tile buffer once the tile has been used.
 // fro != nullptr: CTA b also writes its share of ||A||_F^2 (lower triangle,
 // off-diagonal entries twice) to fro[b] and zeroes fro[gridDim.x ..nfro).
 template <int NR>
-__global__ void __launch_bounds__(NTH, NR >= 8 ? 2 : 1)
+__global__ void __launch_bounds__(NTH, symv_ctas<NR>())
 symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __restrict__ x,
                    double* __restrict__ y, const int* skip, double* fro, int nfro, int al16) {
   if (skip != nullptr && *skip) return;
-  constexpr int STAGES = symv_stages<NR>();
   constexpr bool MMA = NR == 8;
-  constexpr int TE = MMA ? BL_TILE : TILE_ELEMS;      // floats per staged tile
+  constexpr int TE = MMA ? BL_TILE : TILE_ELEMS;      // floats of the staged tile
   constexpr int VEC = MMA ? XS * 8 : RB * NR;         // doubles per staged segment
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  float* tiles = reinterpret_cast<float*>(sm_raw);
-  double* vecs = reinterpret_cast<double*>(tiles + STAGES * TE);   // [stage][xJ, xI]
-  double* s_col = vecs + STAGES * 2 * VEC;
+  float* Ts = reinterpret_cast<float*>(sm_raw);
+  double* xJ = reinterpret_cast<double*>(Ts + TE);
+  double* xI = xJ + VEC;
+  double* s_col = xI + VEC;
   const int T = ceil_div(n, RB);
   const int ntiles = T * (T + 1) / 2;
-  auto issue = [&](int t, int stage) {
-    int I, J;
-    tri_of(t, I, J);
-    const int i0 = I * RB, j0 = J * RB;
-    const int ni = min(RB, n - i0), nj = min(RB, n - j0);
+  auto issue = [&](int i0, int ni, int j0, int nj) {
     const float* T = A + (size_t)j0 * lda + i0;
     if (MMA) {
-      if (al16) stage_tile_bl(tiles + stage * TE, T, lda, ni, nj);
-      else stage_tile_4b<true>(tiles + stage * TE, T, lda, ni, nj);
-      stage_vec_x8(x, n, j0, nj, vecs + (2 * stage) * VEC);
-      stage_vec_x8(x, n, i0, ni, vecs + (2 * stage + 1) * VEC);
+      if (al16) stage_tile_bl(Ts, T, lda, ni, nj);
+      else stage_tile_4b<true>(Ts, T, lda, ni, nj);
+      stage_vec_x8(x, n, j0, nj, xJ);
+      stage_vec_x8(x, n, i0, ni, xI);
     } else {
-      if (al16) stage_tile(tiles + stage * TE, T, lda, ni, nj);
-      else stage_tile_4b<false>(tiles + stage * TE, T, lda, ni, nj);
-      stage_vec<NR>(x, n, j0, nj, vecs + (2 * stage) * VEC);
-      stage_vec<NR>(x, n, i0, ni, vecs + (2 * stage + 1) * VEC);
+      if (al16) stage_tile(Ts, T, lda, ni, nj);
+      else stage_tile_4b<false>(Ts, T, lda, ni, nj);
+      stage_vec<NR>(x, n, j0, nj, xJ);
+      stage_vec<NR>(x, n, i0, ni, xI);
     }
   };
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    const int t = blockIdx.x + s * gridDim.x;
-    if (t < ntiles) issue(t, s);
-    cp_async_commit();
-  }
-  int stage = 0;
   double fsq = 0.0;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    {
-      const int tn = t + (STAGES - 1) * gridDim.x;
-      if (tn < ntiles) issue(tn, (stage + STAGES - 1) % STAGES);
-      cp_async_commit();
-    }
-    cp_async_wait<STAGES - 1>();
-    __syncthreads();
     int I, J;
     tri_of(t, I, J);
     const int i0 = I * RB, j0 = J * RB;
     const int ni = min(RB, n - i0), nj = min(RB, n - j0);
-    float* Ts = tiles + stage * TE;
-    const double* xJ = vecs + (2 * stage) * VEC;
-    const double* xI = xJ + VEC;
+    issue(i0, ni, j0, nj);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
     if (MMA) {
       // row sums to y_I, column sums to y_J, straight from the fragments
       if (fro != nullptr) {
@@ -598,7 +581,6 @@ symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __
         else tile_mma_x8<false, false>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, true, 1.0, nullptr);
       }
       __syncthreads();   // the stage is free again
-      stage = (stage + 1) % STAGES;
       continue;
     }
     double acc[4][NR] = {};
@@ -616,15 +598,13 @@ symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __
     }
     flush_rows<NR>(acc, reinterpret_cast<double*>(Ts), y, n, i0, ni, 1.0);
     __syncthreads();   // the stage and s_col are free again
-    stage = (stage + 1) % STAGES;
   }
-  cp_async_wait<0>();
   if (fro != nullptr) {
     // block sum in a fixed order: warps, then the CTA's warps in turn
     double v = fsq;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    double* wsum = reinterpret_cast<double*>(tiles);   // the stages are free
+    double* wsum = reinterpret_cast<double*>(Ts);   // the stage is free
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1723,7 +1703,7 @@ cudaError_t launch_symv_skip(const TA* A, int lda, int n, const double* x, doubl
   const int T = ceil_div(n, RB);
   const int ntiles = T * (T + 1) / 2;
   if constexpr (sizeof(TA) == 4) {
-    int grid = std::min(ntiles, (nrhs >= 8 ? 2 : 1) * sm_count());
+    int grid = std::min(ntiles, (nrhs == 1 ? symv_ctas<1>() : symv_ctas<2>()) * sm_count());
     if (fro != nullptr) grid = std::min(grid, nfro);   // one Frobenius partial per CTA
     const int al16 = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
     NR_SWITCH(nrhs, (symv_staged_kernel<NRC><<<grid, NTH, symv_staged_smem<NRC>(), stream>>>(A, lda, n, x, y, skip, fro, nfro, al16)));
