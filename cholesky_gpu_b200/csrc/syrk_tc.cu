@@ -167,14 +167,49 @@ __device__ __forceinline__ TileCtx tile_ctx(int t, const TcBatch& bt, float* C, 
   return c;
 }
 
-// The kernel body for one format.  mhi / mlo / mc point at tensor maps in the
-// launch's parameter space (TMA reads them from there).
+// A CTA's barriers and TMEM, set up once before the body of whichever format
+// runs; one kernel can then set them up before it knows the format, while the
+// kernel before it still runs.
+constexpr int MAX_STAGES = 4;
+struct TcShared {
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES];
+  uint64_t accf[2], acce[2];
+  uint64_t cld[EPI_WARPS][2];   // LDST: each warp's C boxes landed
+  uint32_t tmem;
+  volatile int abort;
+};
+__device__ __forceinline__ void tc_setup(TcShared& sh, uint32_t tmem_cols) {
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MAX_STAGES; ++s) { tc::mbar_init(&sh.full[s], 1); tc::mbar_init(&sh.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { tc::mbar_init(&sh.accf[b], 1); tc::mbar_init(&sh.acce[b], EPI_WARPS); }
+    for (int w = 0; w < EPI_WARPS; ++w) { tc::mbar_init(&sh.cld[w][0], 1); tc::mbar_init(&sh.cld[w][1], 1); }
+    tc::fence_mbar_init();
+    sh.abort = 0;
+  }
+  if ((threadIdx.x >> 5) == 1) tc::tmem_alloc(&sh.tmem, tmem_cols);
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+}
+__device__ __forceinline__ void tc_teardown(TcShared& sh, uint32_t tmem_cols) {
+  tc::tc_fence_before();
+  __syncthreads();
+  if ((threadIdx.x >> 5) == 1) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(sh.tmem, tmem_cols);
+  }
+}
+template <int FMT>
+constexpr uint32_t tc_tmem_cols() { return TcCfg<FMT>::MX ? 4 * TM : 2 * TM; }  // accumulators (+ scales)
+
+// The work of one format between set-up and tear-down.  mhi / mlo / mc point at
+// tensor maps in the launch's parameter space (TMA reads them from there).
 template <int FMT, bool BATCH, bool WIDE>
 __device__ __forceinline__ void
 syrk_tc_body(const CUtensorMap* mhi, const CUtensorMap* mlo, const CUtensorMap* mc,
              float* __restrict__ C, int ldc, int m, int k, const int8_t* __restrict__ rowexp,
              const uint8_t* __restrict__ mxexp, int ldmx, DevStatus* st, const TcBatch& bt,
-             int ntiles_b, TileSel sel) {
+             int ntiles_b, TileSel sel, TcShared& sh) {
   using Cfg = TcCfg<FMT>;
   using Plan = TcPlan<FMT, BATCH, WIDE>;
   if (st != nullptr && st->code != 0) return;
@@ -183,7 +218,6 @@ syrk_tc_body(const CUtensorMap* mhi, const CUtensorMap* mlo, const CUtensorMap* 
   constexpr bool MX = Cfg::MX;
   // A sets, B sets, then (MXFP8) the A and B scales of the chunk
   constexpr int STAGE_BYTES = 2 * NSETS * STRIP + (MX ? 2 * SF_BYTES : 0);
-  constexpr uint32_t TMEM_COLS = MX ? 4 * TM : 2 * TM;  // accumulators (+ scales)
   constexpr bool RED = Plan::RED;
   constexpr bool LDST = Plan::LDST;
   constexpr int KSTEP = 32;                             // bytes of K per MMA
@@ -192,34 +226,24 @@ syrk_tc_body(const CUtensorMap* mhi, const CUtensorMap* mlo, const CUtensorMap* 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full_bar[NS];
-  __shared__ __align__(8) uint64_t empty_bar[NS];
-  __shared__ __align__(8) uint64_t accf_bar[2];
-  __shared__ __align__(8) uint64_t acce_bar[2];
-  __shared__ __align__(8) uint64_t cld_bar[EPI_WARPS][2];   // LDST: each warp's C boxes landed
-  __shared__ uint32_t tmem_base_sh;
-  __shared__ volatile int abort_sh;
+  static_assert(NS <= MAX_STAGES, "one barrier pair per stage");
+  auto& full_bar = sh.full;
+  auto& empty_bar = sh.empty;
+  auto& accf_bar = sh.accf;
+  auto& acce_bar = sh.acce;
+  auto& cld_bar = sh.cld;
+  auto& abort_sh = sh.abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = (m + TM - 1) / TM;
   const int ntiles = BATCH ? ntiles_b : sel_tile_count(T, sel);
   const int nchunks = (k * Cfg::ESIZE) / CHUNK;
 
+  const uint32_t tmem = sh.tmem;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NS; ++s) { tc::mbar_init(&full_bar[s], 1); tc::mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { tc::mbar_init(&accf_bar[b], 1); tc::mbar_init(&acce_bar[b], EPI_WARPS); }
-    if (LDST)
-      for (int w = 0; w < EPI_WARPS; ++w) { tc::mbar_init(&cld_bar[w][0], 1); tc::mbar_init(&cld_bar[w][1], 1); }
-    tc::fence_mbar_init();
     tc::prefetch_tmap(mhi);
     if (NSETS == 2) tc::prefetch_tmap(mlo);
-    abort_sh = 0;
   }
-  if (warp == 1) tc::tmem_alloc(&tmem_base_sh, TMEM_COLS);
-  tc::tc_fence_before();
-  __syncthreads();
-  tc::tc_fence_after();
-  const uint32_t tmem = tmem_base_sh;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -497,12 +521,6 @@ syrk_tc_body(const CUtensorMap* mhi, const CUtensorMap* mlo, const CUtensorMap* 
   }
   // reduce-adds and stores performed before exit
   if ((RED || LDST) && warp >= 2 && lane == 0) tc::bulk_wait_read();
-  tc::tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc::tc_fence_after();
-    tc::tmem_dealloc(tmem, TMEM_COLS);
-  }
 }
 
 template <int FMT, bool BATCH, bool WIDE>
@@ -511,8 +529,11 @@ syrk_tc_kernel(const __grid_constant__ TcMaps maps, float* __restrict__ C, int l
                const int8_t* __restrict__ rowexp, const uint8_t* __restrict__ mxexp, int ldmx,
                const int* prec_sel, DevStatus* st, TcBatch bt, int ntiles_b, TileSel sel) {
   if (prec_sel != nullptr && *prec_sel != FMT) return;
+  __shared__ __align__(8) TcShared sh;
+  tc_setup(sh, tc_tmem_cols<FMT>());
   syrk_tc_body<FMT, BATCH, WIDE>(&maps.hi, &maps.lo, &maps.c, C, ldc, m, k, rowexp, mxexp, ldmx, st,
-                                 bt, ntiles_b, sel);
+                                 bt, ntiles_b, sel, sh);
+  tc_teardown(sh, tc_tmem_cols<FMT>());
 }
 
 // K beyond the format's load / store epilogue (see TcCfg)
@@ -535,18 +556,20 @@ syrk_tc_dispatch_kernel(const __grid_constant__ TcMapsAll maps, float* __restric
                         const int8_t* __restrict__ rexp_e5m2, const int8_t* __restrict__ rexp_f16,
                         const uint8_t* __restrict__ mxexp, int ldmx, unsigned fmt_mask,
                         const int* prec_sel, DevStatus* st, TileSel sel) {
+  __shared__ __align__(8) TcShared sh;
+  tc_setup(sh, 4 * TM);     // the most any format needs
   tc::grid_dep_wait();      // the panel solve that resolved the step is complete
   tc::grid_dep_trigger();   // the POTRF after this (head) launch may be scheduled
-  const int f = *prec_sel;
-  if (f < 0 || f > 31 || ((fmt_mask >> f) & 1u) == 0) return;
+  int f = *prec_sel;
+  if (f < 0 || f > 31 || ((fmt_mask >> f) & 1u) == 0) f = FP32;   // not this kernel's
   const TcBatch nb{};
   // one body per format and epilogue (the K test is uniform over the grid)
 #define TC_BODY(F, MHI, MLO, REXP, MX, LDMX)                                                     \
   do {                                                                                        \
     if (tc_wide<F>(k))                                                                        \
-      syrk_tc_body<F, false, true>(MHI, MLO, &maps.c, C, ldc, m, k, REXP, MX, LDMX, st, nb, 0, sel); \
+      syrk_tc_body<F, false, true>(MHI, MLO, &maps.c, C, ldc, m, k, REXP, MX, LDMX, st, nb, 0, sel, sh); \
     else                                                                                      \
-      syrk_tc_body<F, false, false>(MHI, MLO, &maps.c, C, ldc, m, k, REXP, MX, LDMX, st, nb, 0, sel); \
+      syrk_tc_body<F, false, false>(MHI, MLO, &maps.c, C, ldc, m, k, REXP, MX, LDMX, st, nb, 0, sel, sh); \
   } while (0)
   switch (f) {
     case FP16:
@@ -554,7 +577,7 @@ syrk_tc_dispatch_kernel(const __grid_constant__ TcMapsAll maps, float* __restric
       break;
     case FP16X2:   // reduce-add epilogue at every K
       syrk_tc_body<FP16X2, false, false>(&maps.h16, &maps.l16, &maps.c, C, ldc, m, k, rexp_f16,
-                                         nullptr, 0, st, nb, 0, sel);
+                                         nullptr, 0, st, nb, 0, sel, sh);
       break;
     case E4M3:
       TC_BODY(E4M3, &maps.h8[0], &maps.h8[0], rexp_e4m3, nullptr, 0);
@@ -572,6 +595,7 @@ syrk_tc_dispatch_kernel(const __grid_constant__ TcMapsAll maps, float* __restric
       break;
   }
 #undef TC_BODY
+  tc_teardown(sh, 4 * TM);
 }
 
 template <int FMT, bool BATCH, bool WIDE = false>
