@@ -528,11 +528,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 syrk_tc_kernel(const __grid_constant__ TcMaps maps, float* __restrict__ C, int ldc, int m, int k,
                const int8_t* __restrict__ rowexp, const uint8_t* __restrict__ mxexp, int ldmx,
                const int* prec_sel, DevStatus* st, TcBatch bt, int ntiles_b, TileSel sel) {
-  if (prec_sel != nullptr && *prec_sel != FMT) return;
   __shared__ __align__(8) TcShared sh;
   tc_setup(sh, tc_tmem_cols<FMT>());
-  syrk_tc_body<FMT, BATCH, WIDE>(&maps.hi, &maps.lo, &maps.c, C, ldc, m, k, rowexp, mxexp, ldmx, st,
-                                 bt, ntiles_b, sel, sh);
+  tc::grid_dep_wait();      // as in the dispatch kernel below
+  tc::grid_dep_trigger();
+  if (prec_sel == nullptr || *prec_sel == FMT)
+    syrk_tc_body<FMT, BATCH, WIDE>(&maps.hi, &maps.lo, &maps.c, C, ldc, m, k, rowexp, mxexp, ldmx, st,
+                                   bt, ntiles_b, sel, sh);
   tc_teardown(sh, tc_tmem_cols<FMT>());
 }
 
@@ -631,9 +633,10 @@ cudaError_t launch_fmt(const TcMaps& maps, float* C, int ldc, int m, int k, cons
   auto go = [&](auto kernel, size_t smem) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, NTHREADS, smem, stream>>>(maps, C, ldc, m, k, rowexp, mxexp, ldmx, prec_sel, st,
-                                             bt, ntiles_b, sel);
-    return cudaGetLastError();
+    PdlLaunch L(dim3(grid), dim3(NTHREADS), smem, stream);
+    e = cudaLaunchKernelEx(&L.cfg, kernel, maps, C, ldc, m, k, rowexp, mxexp, ldmx, prec_sel, st, bt,
+                           ntiles_b, sel);
+    return e != cudaSuccess ? e : cudaGetLastError();
   };
   if constexpr (!BATCH)
     if (tc_wide<FMT>(k)) return go(syrk_tc_kernel<FMT, false, true>, tc_smem<FMT, false, true>());
