@@ -330,6 +330,7 @@ mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, con
                                   mpchol_stream_t stream_) {
   if (B == nullptr || dA == nullptr || lda == nullptr) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  MPCHOL_CUDA_TRY(cudaStreamWaitEvent(s, B->ev_factored, 0));   // an earlier call, on whatever stream
   for (int i = 0; i < B->count; ++i) {
     const int u = B->order[i];
     if (dA[u] == nullptr || lda[u] < B->n[u]) return MPCHOL_ERR_BAD_ARG;

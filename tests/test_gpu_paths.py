@@ -259,3 +259,29 @@ def test_rbf_solve_reads_lower_triangles_only(n, opts):
     (x0, g0), (x1, g1) = run(0.0), run(float("nan"))
     assert ((x1 - x0).norm() / x0.norm()).item() < 1e-6
     assert ((g1 - g0).norm() / g0.norm()).item() < 1e-6
+
+
+@pytest.mark.parametrize("precision,block", [("fp16x2", 128), ("fp16", 64)])
+def test_batch_calls_on_different_streams(precision, block):
+    """The factor call returns before the factors are complete: a second factor
+    call, the status and the solve on other streams wait for it.  Orders at tile
+    edges, one of two super-blocks; the true residual is FP64."""
+    ns = [64, 1, 33, 130, 1100, 257]
+    As = [matgen.spd_matrix(n, 1e2, n).cuda() if n > 1 else torch.full((1, 1), 3.0, device="cuda") for n in ns]
+    other = [2.0 * A for A in As]
+    Bs = [matgen.rhs(n, 2, n).cuda().reshape(n, 2) for n in ns]
+    bt = mp.Batch(ns, nrhs=2, block_size=block, precision=precision)
+    torch.cuda.synchronize()
+    s1, s2, s3 = (torch.cuda.Stream() for _ in range(3))
+    with torch.cuda.stream(s1):
+        bt.factor(other)
+    with torch.cuda.stream(s2):
+        bt.factor(As)
+    with torch.cuda.stream(s3):
+        assert bt.info()[0] == [0] * len(ns)
+        Xs, reps, _ = bt.pcg(As, Bs, rel_tol=1e-10)
+    torch.cuda.synchronize()
+    for A, B, X, r in zip(As, Bs, Xs, reps):
+        assert r.converged
+        S = torch.tril(A.double()) + torch.tril(A.double(), -1).T
+        assert ((S @ X - B).norm() / B.norm()).item() < 2e-10
