@@ -254,9 +254,11 @@ MPCHOL_API mpchol_status mpchol_factor_prepare_solve(mpchol_factor_t* f, mpchol_
  * The iterations run in a device-side loop (a CUDA graph the object keeps)
  * that stops when the recursive residual meets the tolerance or max_it is
  * reached; `stream` is synchronized after each such loop and the answer is
- * re-checked on the true residual (restarting from it if needed).  When the
- * runtime refuses the graph, or profiling is on, iterations are launched
- * directly and `stream` is synchronized every check_every iterations.
+ * re-checked on the true residual (restarting from it if needed).  On the
+ * first two calls with the same operands, when the runtime refuses the graph,
+ * and when profiling is on, iterations are launched directly and `stream` is
+ * synchronized every check_every iterations.  Systems of n <= 1024 are solved
+ * in one launch and one synchronization.
  * report may be NULL.  A factor whose factorization failed (NOT_SPD,
  * TIMEOUT) is not used: the solve returns the factor's status without
  * iterating.  The solve has a device status word of its own (breakdown,
