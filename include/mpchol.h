@@ -257,8 +257,9 @@ MPCHOL_API mpchol_status mpchol_factor_prepare_solve(mpchol_factor_t* f, mpchol_
  * re-checked on the true residual (restarting from it if needed).  On the
  * first two calls with the same operands, when the runtime refuses the graph,
  * and when profiling is on, iterations are launched directly and `stream` is
- * synchronized every check_every iterations.  Systems of n <= 1024 are solved
- * in one launch and one synchronization.
+ * synchronized every check_every iterations.  Systems of n <= 1024 whose rows
+ * and vectors fit the SMs' shared memory (all but the largest with 8 columns)
+ * are solved in one launch and one synchronization.
  * report may be NULL.  A factor whose factorization failed (NOT_SPD,
  * TIMEOUT) is not used: the solve returns the factor's status without
  * iterating.  The solve has a device status word of its own (breakdown,
