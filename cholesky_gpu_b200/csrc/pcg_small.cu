@@ -68,8 +68,8 @@ __device__ __forceinline__ void load8(const T* strip, int n, int j, double (&s)[
 
 template <int NR, typename TA>
 __global__ void __launch_bounds__(NTH, 1)
-pcg_small_kernel(const TA* __restrict__ A, int lda, const double* __restrict__ B, int nrhs,
-                 double* __restrict__ X, const float* __restrict__ W, PcgVectors g, double tol2, int max_it,
+pcg_small_kernel(const TA* __restrict__ A, int lda, const double* B, int nrhs, double* X,
+                 const float* __restrict__ W, PcgVectors g, double tol2, int max_it,
                  int max_restarts, bool x0, const DevStatus* factor_st, unsigned* bar) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   const int n = g.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x;
@@ -338,10 +338,12 @@ pcg_small_kernel(const TA* __restrict__ A, int lda, const double* __restrict__ B
   }
   if (!ok) return;
   // ---- results -------------------------------------------------------------------
-  if (slice && sk < nrhs) X[so] = xv;
   put_partial(g.part_rz, slice ? rs[so] * zv : 0.0);
   grid_bar();
-  if (!ok || blockIdx.x != 0) return;
+  if (!ok) return;
+  // X may be B itself: every CTA has read B for the last time before this barrier
+  if (slice && sk < nrhs) X[so] = xv;
+  if (blockIdx.x != 0) return;
   double rz[NR];
   sum_partials(g.part_rz, rz);
   if (warp == 0) {

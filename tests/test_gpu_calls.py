@@ -1,0 +1,64 @@
+"""How calls share memory, streams and threads: solves in place, objects freed
+while others work, calls from several threads at once."""
+import ctypes
+
+import pytest
+import torch
+
+import cholesky_gpu_b200 as mp
+from cholesky_gpu_b200 import _lib, matgen
+
+pytestmark = pytest.mark.gpu
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("n", [9, 512, 1000, 1024, 1025])
+@pytest.mark.parametrize("nrhs", [1, 4])
+@pytest.mark.parametrize("f64", [False, True])
+def test_the_solution_may_overwrite_the_right_hand_side(n, nrhs, f64):
+    """mpchol_pcg, mpchol_pcg_f64 and mpchol_adjoint_solve with the solution's
+    buffer as the right-hand side's, on both sides of the one-launch solve's
+    range.  Two solutions with relative residuals of 1e-10 at kappa = 1e2 differ
+    by at most 2 * 1e-10 * 1e2."""
+    lib = _lib.load()
+    A = matgen.spd_matrix(n, 1e2, n).cuda()
+    if f64:
+        A = A.double()
+    B = matgen.rhs(n, nrhs, n + 1).cuda().reshape(n, nrhs).t().contiguous()    # column-major
+    f = mp.factor(A.float(), block_size=128, precision="fp16")
+    solve = lib.mpchol_pcg_f64 if f64 else lib.mpchol_pcg
+    po, rep = _lib.default_pcg_opts(rel_tol=1e-10), _lib.Report()
+    X = torch.empty_like(B)
+
+    def call(b, x):
+        return solve(f.handle, A.data_ptr(), n, b.data_ptr(), x.data_ptr(), nrhs, ctypes.byref(po),
+                     ctypes.byref(rep), _stream())
+    assert call(B, X) == _lib.OK
+    bar = 2e-8 * X.norm().item()
+    for _ in range(50):
+        b = B.clone()
+        assert call(b, b) == _lib.OK and rep.converged
+        assert (b - X).norm().item() <= bar
+    if f64:
+        for _ in range(10):
+            b = B.clone()
+            assert lib.mpchol_adjoint_solve(f.handle, A.data_ptr(), n, X.data_ptr(), b.data_ptr(), b.data_ptr(),
+                                            nrhs, None, n, ctypes.byref(po), ctypes.byref(rep),
+                                            _stream()) == _lib.OK
+            assert (b - X).norm().item() <= bar
+
+
+@pytest.mark.parametrize("n", [512, 1000, 1100])
+def test_the_drop_in_driver_solves_in_place(n):
+    A = matgen.spd_matrix(n, 1e2, n).cuda().double()
+    b = matgen.rhs(n, 1, n).cuda().reshape(n)
+    x = torch.empty_like(b)
+    args = dict(eps_prime=1e-3, rel_tol=1e-10)
+    assert mp.precond_CG(A, x, b, n, 128, **args) == 0
+    for _ in range(20):
+        y = b.clone()
+        assert mp.precond_CG(A, y, y, n, 128, **args) == 0
+        assert (y - x).norm().item() <= 2e-8 * x.norm().item()
