@@ -74,6 +74,7 @@ cudaError_t launch_update_p(const PcgVectors& v, double tol2, const cudaGraphCon
 // word; v's status zero on entry.  Writes X (n x nrhs), the scalars of v, done
 // (converged, iterations).
 bool pcg_small_ok(int n, int nr, int elem, int nsm);
+cudaError_t pcg_small_set_attributes();   // by solve_init_attributes
 template <typename TA>
 cudaError_t launch_pcg_small(const TA* A, int lda, const double* B, int nrhs, double* X, const float* W,
                              const PcgVectors& v, double tol2, int max_it, int max_restarts, bool x0,

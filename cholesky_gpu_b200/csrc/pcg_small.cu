@@ -365,23 +365,23 @@ pcg_small_kernel(const TA* __restrict__ A, int lda, const double* B, int nrhs, d
   }
 }
 
-template <int NR, typename TA>
-size_t small_smem(int n) {
-  return (size_t)ROWS * n * (sizeof(TA) + 2 * sizeof(float)) + (size_t)2 * NR * n * sizeof(double);
+// Dynamic shared memory: the strips of A (elem bytes an element) and W, r and p.
+size_t small_smem(int n, int nr, int elem) {
+  return (size_t)ROWS * n * (elem + 2 * sizeof(float)) + (size_t)2 * nr * n * sizeof(double);
+}
+// What an SM leaves for it beside the static reduction buffers.
+size_t small_smem_max(int nr) {
+  return (size_t)227 * 1024 - (sizeof(double) * (NW * ROWS * nr + 8) + 64);
 }
 
 template <int NR, typename TA>
 cudaError_t launch_small(const TA* A, int lda, const double* B, int nrhs, double* X, const float* W,
                          const PcgVectors& v, double tol2, int max_it, int max_restarts, bool x0,
                          const DevStatus* factor_st, unsigned* bar, cudaStream_t stream) {
-  const size_t smem = small_smem<NR, TA>(v.n);
-  cudaError_t e = cudaFuncSetAttribute(pcg_small_kernel<NR, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ceil_div(v.n, ROWS));
   cfg.blockDim = dim3(NTH);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = small_smem(v.n, NR, sizeof(TA));
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -396,12 +396,29 @@ cudaError_t launch_small(const TA* A, int lda, const double* B, int nrhs, double
 
 // One super-block (its inverse is the whole preconditioner), one CTA per SM
 // for every eight rows, and the strips and replicated vectors in an SM's shared
-// memory.  Static shared memory: the reduction buffers.
+// memory.
 bool pcg_small_ok(int n, int nr, int elem, int nsm) {
   if (n > LDW || ceil_div(n, ROWS) > nsm) return false;
-  const size_t dyn = (size_t)ROWS * n * (elem + 8) + (size_t)16 * nr * n;
-  const size_t stat = sizeof(double) * (NW * ROWS * nr + 8) + 64;
-  return dyn + stat <= (size_t)227 * 1024;
+  return small_smem(n, nr, elem) <= small_smem_max(nr);
+}
+
+// The most any n takes, once per device: the attribute is the kernel's, not the
+// launch's, and a value set for one call would bound a concurrent one.
+cudaError_t pcg_small_set_attributes() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto kernel, int nr) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem_max(nr));
+  };
+  set(pcg_small_kernel<1, float>, 1);
+  set(pcg_small_kernel<2, float>, 2);
+  set(pcg_small_kernel<4, float>, 4);
+  set(pcg_small_kernel<8, float>, 8);
+  set(pcg_small_kernel<1, double>, 1);
+  set(pcg_small_kernel<2, double>, 2);
+  set(pcg_small_kernel<4, double>, 4);
+  set(pcg_small_kernel<8, double>, 8);
+  return e;
 }
 
 template <typename TA>

@@ -1676,7 +1676,7 @@ cudaError_t solve_set_attributes() {
   if ((e = set_dyn(panel_batched_kernel<NRC, true>, red_bytes(NRC))) != cudaSuccess) return e;
   SET_NRB(1) SET_NRB(2) SET_NRB(4) SET_NRB(8)
 #undef SET_NRB
-  return cudaSuccess;
+  return pcg_small_set_attributes();
 }
 
 int sm_count() {

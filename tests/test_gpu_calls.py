@@ -62,3 +62,39 @@ def test_the_drop_in_driver_solves_in_place(n):
         y = b.clone()
         assert mp.precond_CG(A, y, y, n, 128, **args) == 0
         assert (y - x).norm().item() <= 2e-8 * x.norm().item()
+
+
+def _threads(*work):
+    """Runs each function in a thread of its own; returns what they raised."""
+    import threading
+    raised = []
+
+    def guard(fn):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                fn()
+        except Exception as e:      # a thread's exception does not fail the test by itself
+            raised.append(e)
+    ts = [threading.Thread(target=guard, args=(fn,)) for fn in work]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    return raised
+
+
+def test_small_solves_of_different_orders_in_threads():
+    """One-launch solves of one number of right-hand sides need shared memory by
+    their order: none may bound another thread's."""
+    def solver(n, turns):
+        A = matgen.spd_matrix(n, 1e2, n).cuda()
+        B = matgen.rhs(n, 1, n).cuda().reshape(n)
+        f = mp.factor(A, block_size=128, precision="fp16")
+        torch.cuda.synchronize()
+
+        def run():
+            for _ in range(turns):
+                _, rep = f.pcg(A, B, rel_tol=1e-10)
+                assert rep.converged and rep.rel_residual <= 1e-10
+        return run
+    assert _threads(solver(1000, 300), solver(64, 600), solver(500, 400), solver(9, 600)) == []
