@@ -1640,18 +1640,48 @@ size_t solve_wsup_elems(int n) {
   return (size_t)nbs * RS * RS;
 }
 
-cudaError_t solve_init_attributes() {
-  // once per device (kernel attributes are per device)
+// What the launchers ask of a device: its SMs, and the resident CTAs per SM of
+// the triangular solve (by direction; 1, 2, 4, 8 right-hand sides).
+struct DeviceLimits {
+  int sms = 0, trsv[2][4] = {};
+};
+// The kernels' attributes are set and the limits asked for once per device (both
+// are per device), under a lock until all is complete: threads may make their
+// first calls at the same time.
+cudaError_t device_limits(const DeviceLimits** out) {
   static std::mutex mu;
-  static bool done[64] = {};
+  static DeviceLimits limits[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lk(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  e = solve_set_attributes();
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
-  return e;
+  DeviceLimits& d = limits[dev & 63];
+  if (d.sms == 0) {
+    DeviceLimits f;
+    e = solve_set_attributes();
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&f.sms, cudaDevAttrMultiProcessorCount, dev);
+    auto ask = [&](auto kernel, size_t smem, int& n) {
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, NTH, smem);
+      n = std::max(1, n);
+    };
+    auto both = [&](auto fwd, auto bwd, size_t smem, int i) {
+      ask(fwd, smem, f.trsv[0][i]);
+      ask(bwd, smem, f.trsv[1][i]);
+    };
+    both(trsv_persistent_kernel<1, false>, trsv_persistent_kernel<1, true>, trsv_staged_smem<1>(), 0);
+    both(trsv_persistent_kernel<2, false>, trsv_persistent_kernel<2, true>, trsv_staged_smem<2>(), 1);
+    both(trsv_persistent_kernel<4, false>, trsv_persistent_kernel<4, true>, trsv_staged_smem<4>(), 2);
+    both(trsv_persistent_kernel<8, false>, trsv_persistent_kernel<8, true>, trsv_staged_smem<8>(), 3);
+    if (e != cudaSuccess) return e;
+    d = f;
+  }
+  *out = &d;
+  return cudaSuccess;
+}
+
+cudaError_t solve_init_attributes() {
+  const DeviceLimits* lim = nullptr;
+  return device_limits(&lim);
 }
 
 cudaError_t solve_set_attributes() {
@@ -1679,15 +1709,6 @@ cudaError_t solve_set_attributes() {
   return pcg_small_set_attributes();
 }
 
-int sm_count() {
-  static int cache[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-  int& c = cache[dev & 63];
-  if (c == 0 && cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) c = 148;
-  return c;
-}
-
 cudaError_t launch_zero_vec(double* y, long long count, cudaStream_t stream) {
   zero_vec_kernel<<<148, 256, 0, stream>>>(y, count);
   return cudaGetLastError();
@@ -1703,7 +1724,10 @@ cudaError_t launch_symv_skip(const TA* A, int lda, int n, const double* x, doubl
   const int T = ceil_div(n, RB);
   const int ntiles = T * (T + 1) / 2;
   if constexpr (sizeof(TA) == 4) {
-    int grid = std::min(ntiles, (nrhs == 1 ? symv_ctas<1>() : symv_ctas<2>()) * sm_count());
+    const DeviceLimits* lim = nullptr;
+    const cudaError_t le = device_limits(&lim);
+    if (le != cudaSuccess) return le;
+    int grid = std::min(ntiles, (nrhs == 1 ? symv_ctas<1>() : symv_ctas<2>()) * lim->sms);
     if (fro != nullptr) grid = std::min(grid, nfro);   // one Frobenius partial per CTA
     const int al16 = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
     NR_SWITCH(nrhs, (symv_staged_kernel<NRC><<<grid, NTH, symv_staged_smem<NRC>(), stream>>>(A, lda, n, x, y, skip, fro, nfro, al16)));
@@ -1748,7 +1772,9 @@ cudaError_t launch_symv_batched(const BatchSys* sys, int nsys, int ntiles, int x
   cudaError_t e = launch_vec_slot_batched(sys, nsys, -1, yslot, nr, use_skip, stream);
   if (e != cudaSuccess) return e;
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = std::min(ntiles, 2 * sm_count());
+  const DeviceLimits* lim = nullptr;
+  if ((e = device_limits(&lim)) != cudaSuccess) return e;
+  const int grid = std::min(ntiles, 2 * lim->sms);
   NR_SWITCH(nr, (symv_staged_batched_kernel<NRC><<<grid, NTH, symv_batched_smem<NRC>(), stream>>>(sys, nsys, ntiles, xslot, yslot, use_skip)));
   return cudaGetLastError();
 }
@@ -1807,30 +1833,19 @@ cudaError_t launch_trsv_prep(const double* in, double* w, double* mid, double* o
 cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n,
                                    const float* wsup, double* work, double* out, int nrhs, int* counters,
                                    void* slots, const int* skip, DevStatus* st, cudaStream_t stream) {
-  cudaError_t e;
-  static int grid_cache[64][2][4] = {}, sm_cache[64] = {};
-  int dev = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  const DeviceLimits* lim = nullptr;
+  cudaError_t e = device_limits(&lim);
+  if (e != cudaSuccess) return e;
   const int nri = nrhs == 1 ? 0 : nrhs == 2 ? 1 : nrhs == 4 ? 2 : 3;
-  int& resident = grid_cache[dev & 63][backward ? 1 : 0][nri];
-  int& sms = sm_cache[dev & 63];
+  const int per_sm = lim->trsv[backward ? 1 : 0][nri];
   const size_t smem = trsv_smem_bytes(nrhs);
   auto launch = [&](auto kernel) -> cudaError_t {
-    if (resident == 0) {
-      int per_sm = 0, nsm = 0;
-      cudaError_t ee = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NTH,
-                                                                     smem);
-      if (ee == cudaSuccess) ee = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-      if (ee != cudaSuccess) return ee;
-      resident = std::max(1, per_sm) * nsm;
-      sms = nsm;
-    }
     cudaLaunchConfig_t cfg = {};
     // The third CTA per SM (one right-hand side) pays once far tiles bound the
     // solve; before that it only slows the chain's tile passes: forward / backward
     // 57 / 65 us with two and 58 / 67 with three at n = 8192, 78 / 88 and 76 / 82
     // at 10240, 168 / 185 and 145 / 158 at 16384.
-    cfg.gridDim = dim3(n > 9 * RS ? resident : std::min(resident, 2 * sms));
+    cfg.gridDim = dim3((n > 9 * RS ? per_sm : std::min(per_sm, 2)) * lim->sms);
     cfg.blockDim = dim3(NTH);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

@@ -98,3 +98,40 @@ def test_small_solves_of_different_orders_in_threads():
                 assert rep.converged and rep.rel_residual <= 1e-10
         return run
     assert _threads(solver(1000, 300), solver(64, 600), solver(500, 400), solver(9, 600)) == []
+
+
+_FIRST_SOLVES = """
+import threading
+import torch
+import cholesky_gpu_b200 as mp
+from cholesky_gpu_b200 import matgen
+n = 1100
+A = matgen.spd_matrix(n, 1e2, n).cuda()
+fs = [mp.factor(A, block_size=128, precision="fp16") for _ in range(8)]
+Bs = [matgen.rhs(n, k, k).cuda().reshape(n, k) for k in (1, 2, 4, 8) * 2]
+torch.cuda.synchronize()
+gate, done = threading.Barrier(8), []
+def first(f, B):
+    with torch.cuda.stream(torch.cuda.Stream()):
+        gate.wait()
+        X, rep = f.pcg(A, B, rel_tol=1e-10)
+        assert rep.converged
+        done.append(1)
+ts = [threading.Thread(target=first, args=a) for a in zip(fs, Bs)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+assert len(done) == 8, len(done)
+"""
+
+
+def test_the_first_solves_of_a_process_in_threads():
+    """A process whose first eight solves (each number of columns twice, general
+    path) start together: what the launchers look up once per device is complete
+    for every one of them."""
+    import subprocess
+    import sys
+    from .conftest import ROOT
+    for _ in range(3):
+        r = subprocess.run([sys.executable, "-c", _FIRST_SOLVES], cwd=ROOT, capture_output=True, text=True,
+                           timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
