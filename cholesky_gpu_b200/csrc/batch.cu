@@ -329,22 +329,11 @@ mpchol_status mpchol_batch_destroy(mpchol_batch_t* B) {
 mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, const int* lda,
                                   mpchol_stream_t stream_) {
   if (B == nullptr || dA == nullptr || lda == nullptr) return MPCHOL_ERR_BAD_ARG;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  MPCHOL_CUDA_TRY(cudaStreamWaitEvent(s, B->ev_factored, 0));   // an earlier call, on whatever stream
-  for (int i = 0; i < B->count; ++i) {
-    const int u = B->order[i];
+  for (int u = 0; u < B->count; ++u)
     if (dA[u] == nullptr || lda[u] < B->n[u]) return MPCHOL_ERR_BAD_ARG;
-    B->h_ptrs[i] = const_cast<float*>(dA[u]);
-    B->h_ld[i] = lda[u];
-  }
-  MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->d_ptrs, B->h_ptrs, sizeof(void*) * B->count,
-                                  cudaMemcpyHostToDevice, s));
-  MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->d_ld, B->h_ld, sizeof(int) * B->count, cudaMemcpyHostToDevice, s));
-  MPCHOL_CUDA_TRY(cudaMemsetAsync(B->st, 0, sizeof(DevStatus) * B->count, s));
-  batch_load_kernel<<<dim3(64, B->count), 256, 0, s>>>(
-      B->d_sys, reinterpret_cast<const float* const*>(B->d_ptrs), B->d_ld);
-  MPCHOL_CUDA_TRY(cudaGetLastError());
-  MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_loaded, s));
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  // captured before anything reads the caller's matrices: a capture that fails
+  // leaves nothing in flight
   if (B->fgraph == nullptr) {
     cudaGraph_t g = nullptr;
     // relaxed: the launchers set kernel attributes (not stream work) as they go
@@ -360,12 +349,30 @@ mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, con
     cudaGraphDestroy(g);
     MPCHOL_CUDA_TRY(ie);
   }
-  MPCHOL_CUDA_TRY(cudaGraphLaunch(B->fgraph, s));
-  MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_factored, s));
-  // the caller's matrices and the host pointer tables are free again once they
-  // have been read; the host prepares the solve while the device factors
-  MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_loaded));
-  return MPCHOL_OK;
+  auto enqueue = [&]() -> mpchol_status {
+    MPCHOL_CUDA_TRY(cudaStreamWaitEvent(s, B->ev_factored, 0));   // an earlier call, on whatever stream
+    for (int i = 0; i < B->count; ++i) {
+      B->h_ptrs[i] = const_cast<float*>(dA[B->order[i]]);
+      B->h_ld[i] = lda[B->order[i]];
+    }
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->d_ptrs, B->h_ptrs, sizeof(void*) * B->count,
+                                    cudaMemcpyHostToDevice, s));
+    MPCHOL_CUDA_TRY(cudaMemcpyAsync(B->d_ld, B->h_ld, sizeof(int) * B->count, cudaMemcpyHostToDevice, s));
+    MPCHOL_CUDA_TRY(cudaMemsetAsync(B->st, 0, sizeof(DevStatus) * B->count, s));
+    batch_load_kernel<<<dim3(64, B->count), 256, 0, s>>>(
+        B->d_sys, reinterpret_cast<const float* const*>(B->d_ptrs), B->d_ld);
+    MPCHOL_CUDA_TRY(cudaGetLastError());
+    MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_loaded, s));
+    MPCHOL_CUDA_TRY(cudaGraphLaunch(B->fgraph, s));
+    MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_factored, s));
+    // the caller's matrices and the host pointer tables are free again once they
+    // have been read; the host prepares the solve while the device factors
+    MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_loaded));
+    return MPCHOL_OK;
+  };
+  const mpchol_status e = enqueue();
+  if (e != MPCHOL_OK) cudaStreamSynchronize(s);   // ... on an error too
+  return e;
 }
 
 mpchol_status mpchol_batch_lower(const mpchol_batch_t* B, int index, const float** dL, int* ldl,
