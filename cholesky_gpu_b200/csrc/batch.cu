@@ -103,6 +103,7 @@ struct mpchol_batch {
   cudaStream_t cap = nullptr;
   cudaEvent_t ev_loaded = nullptr;     // a factor call has read the caller's matrices
   cudaEvent_t ev_factored = nullptr;   // ... and is complete
+  mutable bool lower_given = false;    // a caller may hold a pointer to a factor
   cudaGraphExec_t fgraph = nullptr;
   cudaGraphExec_t igraph = nullptr;
   double ig_tol2 = -1.0;
@@ -366,8 +367,9 @@ mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, con
     MPCHOL_CUDA_TRY(cudaGraphLaunch(B->fgraph, s));
     MPCHOL_CUDA_TRY(cudaEventRecord(B->ev_factored, s));
     // the caller's matrices and the host pointer tables are free again once they
-    // have been read; the host prepares the solve while the device factors
-    MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_loaded));
+    // have been read; the host prepares the solve while the device factors (unless
+    // the caller can read a factor without asking for it again)
+    MPCHOL_CUDA_TRY(cudaEventSynchronize(B->lower_given ? B->ev_factored : B->ev_loaded));
     return MPCHOL_OK;
   };
   const mpchol_status e = enqueue();
@@ -378,7 +380,8 @@ mpchol_status mpchol_batch_factor(mpchol_batch_t* B, const float* const* dA, con
 mpchol_status mpchol_batch_lower(const mpchol_batch_t* B, int index, const float** dL, int* ldl,
                                  int* n) {
   if (B == nullptr || dL == nullptr || index < 0 || index >= B->count) return MPCHOL_ERR_BAD_ARG;
-  MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_factored));   // the caller may read it on any stream
+  MPCHOL_CUDA_TRY(cudaEventSynchronize(B->ev_factored));   // the caller may read it on any stream,
+  B->lower_given = true;                                   // also after a later factor call
   const int i = (int)(std::find(B->order.begin(), B->order.end(), index) - B->order.begin());
   *dL = B->h_sys[i].A;
   if (ldl) *ldl = B->h_sys[i].ld;

@@ -394,7 +394,9 @@ MPCHOL_API mpchol_status mpchol_syrk_update(float* dC, int ldc, int m, int k, in
  *   mpchol_batch_factor: one CUDA graph launch factors every system (and
  *     forms the solve data); blocks the host until the matrices and the
  *     pointer tables have been read, not until the factors are complete
- *     (the calls below wait for them, on whatever stream).
+ *     (the calls below wait for them, on whatever stream).  Once a pointer
+ *     has been given out by mpchol_batch_lower it blocks until the factors
+ *     are complete: the pointer stays good for every later factor call.
  *   mpchol_batch_pcg: PCG of every system in lockstep (converged ones skip),
  *     FP64 true residual per system; reports[i] per system (may be NULL).
  *     Returns OK if every system converged, PCG_MAXIT otherwise. */

@@ -135,3 +135,27 @@ def test_the_first_solves_of_a_process_in_threads():
         r = subprocess.run([sys.executable, "-c", _FIRST_SOLVES], cwd=ROOT, capture_output=True, text=True,
                            timeout=300)
         assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_a_pointer_to_a_batch_factor_outlives_the_next_factor_call():
+    """A pointer from mpchol_batch_lower is read on a stream of its own right
+    after a second factor call on another one: it holds the second factor."""
+    from cholesky_gpu_b200.api import _wrap_device
+    ns = [2048, 300, 1500]
+    As = [matgen.spd_matrix(n, 1e2, n).cuda() for n in ns]
+    bt = mp.Batch(ns, block_size=128, precision="fp16x2")
+    bt.factor([4.0 * A for A in As])
+    p, ld, n = ctypes.c_void_p(), ctypes.c_int(), ctypes.c_int()
+    assert _lib.load().mpchol_batch_lower(bt.handle, 0, ctypes.byref(p), ctypes.byref(ld),
+                                          ctypes.byref(n)) == _lib.OK
+    view = _wrap_device(p.value, (n.value, ld.value), torch.float32)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s1):
+        bt.factor(As)
+    with torch.cuda.stream(s2):
+        got = view.clone()
+    torch.cuda.synchronize()
+    assert torch.equal(got[:, : n.value].t().tril(), bt.lower(0))
+    L = torch.linalg.cholesky(As[0].double())
+    assert ((bt.lower(0) - L).norm() / L.norm()).item() < 1e-5
