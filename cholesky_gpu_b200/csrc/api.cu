@@ -146,18 +146,13 @@ struct PcgGraph {
 // 0.5 ms, ten times that on a busy host, and the drop-in entry points make
 // and free a factor object on every call.  So the resources of a freed object
 // are kept for the next one of about its size: at most kCacheCount sets of
-// kCacheBytes in all, idle ones only (the device is synchronized when a set
-// is put away, as a cudaFree would), given back by mpchol_release_cached, when
-// an allocation of the library fails, or when newer ones take their room.
+// kCacheBytes in all, given back by mpchol_release_cached, when an allocation
+// of the library fails, or when newer ones take their room.  Only idle sets
+// are kept: the object's last work is waited for by its event, never by the
+// device (which would end the captures of other threads), and a set whose
+// memory work unknown to the library may still use (see note_use) is freed.
 // Create + destroy at n = 3072: 3.6 ms with one allocation per buffer, 0.70
 // with one for all.
-// The scalar block of a factor object (doubles): misc at 0, ||b||^2 at 32, rho
-// at 40, the factor's and the solve's status at 56, done and loop control at 60,
-// the small solve's barrier at 62.
-constexpr int kScalBnorm = 32, kScalRho = 40, kScalStatus = 56, kScalDone = 60, kScalBarrier = 62,
-              kScalDoubles = 64;
-static_assert(sizeof(DevStatus) == 16, "two status words take four doubles");
-
 struct Resources {
   int device = -1;
   char* arena = nullptr;
@@ -170,18 +165,26 @@ struct Resources {
   cudaEvent_t ev_next = nullptr;    // the next block's columns are updated
   cudaEvent_t ev_rest = nullptr;    // the rest of the step's update is done
   cudaEvent_t ev_catch = nullptr;   // a step's catch-ups are done
+  cudaEvent_t ev_used = nullptr;    // the last call's work on the caller's stream is done
 };
 constexpr size_t kCacheBytes = (size_t)512 << 20;
 constexpr size_t kCacheCount = 4;
 std::mutex g_cache_mu;
 std::vector<Resources> g_cache;   // oldest first
 
+// The scalar block of a factor object (doubles): misc at 0, ||b||^2 at 32, rho
+// at 40, the factor's and the solve's status at 56, done and loop control at 60,
+// the small solve's barrier at 62.
+constexpr int kScalBnorm = 32, kScalRho = 40, kScalStatus = 56, kScalDone = 60, kScalBarrier = 62,
+              kScalDoubles = 64;
+static_assert(sizeof(DevStatus) == 16, "two status words take four doubles");
+
 void free_resources(Resources& r) {
   if (r.arena) cudaFree(r.arena);
   if (r.h_scal) cudaFreeHost(r.h_scal);
   if (r.aux) cudaStreamDestroy(r.aux);
   if (r.capture_stream) cudaStreamDestroy(r.capture_stream);
-  for (cudaEvent_t e : {r.ev_next, r.ev_rest, r.ev_catch})
+  for (cudaEvent_t e : {r.ev_next, r.ev_rest, r.ev_catch, r.ev_used})
     if (e) cudaEventDestroy(e);
   r = Resources{};
 }
@@ -221,7 +224,7 @@ bool acquire_resources(int device, size_t bytes, Resources* out) {
   ok = ok && cudaMallocHost(reinterpret_cast<void**>(&r.h_scal), sizeof(double) * kScalDoubles) == cudaSuccess &&
        cudaStreamCreateWithFlags(&r.aux, cudaStreamNonBlocking) == cudaSuccess &&
        cudaStreamCreateWithFlags(&r.capture_stream, cudaStreamNonBlocking) == cudaSuccess;
-  for (cudaEvent_t* e : {&r.ev_next, &r.ev_rest, &r.ev_catch})
+  for (cudaEvent_t* e : {&r.ev_next, &r.ev_rest, &r.ev_catch, &r.ev_used})
     ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
   // the slots of the triangular solve start out with no launch's tag, and stay
   // at the start of the memory whatever factor object it serves
@@ -236,18 +239,31 @@ bool acquire_resources(int device, size_t bytes, Resources* out) {
   return true;
 }
 
-// Puts a set away (or frees it when it is larger than the cache may hold).
-void put_away_resources(Resources& r) {
-  if (r.arena == nullptr || r.bytes > kCacheBytes) {
+// Lets this thread ask for the state of the library's own events while other
+// streams are captured in whatever mode: neither event nor stream is part of
+// a capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Puts a set away, once the work behind its event and on aux is done.  A set
+// larger than the cache may hold is freed, and so is one that is not known to
+// become idle with those two: cudaFree waits for whatever uses the memory.
+void put_away_resources(Resources& r, bool known) {
+  if (r.arena == nullptr) {
     free_resources(r);
     return;
   }
-  int cur = 0;
-  const bool there = cudaGetDevice(&cur) == cudaSuccess;
-  if (there && cur != r.device) cudaSetDevice(r.device);
-  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
-  if (there && cur != r.device) cudaSetDevice(cur);
-  if (!idle) {
+  if (known && r.bytes <= kCacheBytes) {
+    const RelaxedCapture relaxed;
+    if (cudaEventSynchronize(r.ev_used) != cudaSuccess || cudaStreamSynchronize(r.aux) != cudaSuccess) {
+      cudaGetLastError();            // not an error of the caller's next call
+      known = false;
+    }
+  }
+  if (!known || r.bytes > kCacheBytes) {
     free_resources(r);
     return;
   }
@@ -293,6 +309,10 @@ struct mpchol_factor {
   int n = 0, ld = 0, b = 0, nsteps = 0;
   int device = 0;
   Resources res;              // device memory that holds the buffers down to loop_ctl, streams, ...
+  // What may use that memory (see note_use): work up to res.ev_used, which was
+  // last recorded on the stream with this number, or work the library cannot see.
+  mutable bool used = false, unseen = false;
+  mutable unsigned long long used_stream = 0;
   float* A = nullptr;         // n columns x ld rows, factor in the lower triangle
   float* d = nullptr;         // original diagonal
   float* dtilde = nullptr;    // Schur-complement diagonal tracker
@@ -396,15 +416,55 @@ void free_factor(mpchol_factor_t* f) {
     if (p) cudaFree(p);
   if (f->graph.exec) cudaGraphExecDestroy(f->graph.exec);
   if (f->fgraph.exec) cudaGraphExecDestroy(f->fgraph.exec);
-  if (f->cp) cudaStreamDestroy(f->cp);
+  if (f->cp) {
+    cudaStreamSynchronize(f->cp);   // copies into the memory put away below
+    cudaStreamDestroy(f->cp);
+  }
   for (cudaEvent_t e : f->ev_grp)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : {f->ev_start, f->ev_diag})
     if (e) cudaEventDestroy(e);
   if (f->h_diag) cudaFreeHost(f->h_diag);
-  put_away_resources(f->res);
+  put_away_resources(f->res, !f->unseen);
   delete f;
 }
+
+// Records that a call has enqueued work on the object's memory on s.  Work the
+// library cannot wait for when the object is freed makes the memory `unseen`:
+// a call under a capture (the caller's graph may run at any time), an earlier
+// call's work still running on another stream, and, in the calls that give out
+// pointers into the memory, the caller's own.
+void note_use(const mpchol_factor_t* f, cudaStream_t s) {
+  if (f->unseen) return;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  bool ok = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+            cudaStreamGetId(s, &id) == cudaSuccess;
+  if (ok && f->used && id != f->used_stream) {
+    const RelaxedCapture relaxed;
+    ok = cudaEventQuery(f->res.ev_used) == cudaSuccess;
+  }
+  ok = ok && cudaEventRecord(f->res.ev_used, s) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    f->unseen = true;
+    return;
+  }
+  f->used = true;
+  f->used_stream = id;
+}
+// ... at the end of a call, however it ends, unless that has waited for s itself.
+struct UseScope {
+  const mpchol_factor_t* f;
+  cudaStream_t s;
+  bool waited = false;
+  UseScope(const mpchol_factor_t* f_, cudaStream_t s_) : f(f_), s(s_) {}
+  ~UseScope() {
+    if (!waited) note_use(f, s);
+  }
+  UseScope(const UseScope&) = delete;
+  UseScope& operator=(const UseScope&) = delete;
+};
 
 DecisionParams make_dp(const mpchol_opts& o) {
   DecisionParams dp;
@@ -923,6 +983,7 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
   if (popts) po = *popts;
   if (po.check_every < 1) po.check_every = 1;
   if (po.max_it < 0) return MPCHOL_ERR_BAD_ARG;
+  UseScope use(f, stream);
   const int n = f->n;
   const int nr = pcg_padded_nrhs(nrhs);
   const size_t nv = (size_t)n * 8;
@@ -1013,6 +1074,7 @@ mpchol_status run_pcg(mpchol_factor_t* f, const TA* dA, int lda, const double* d
                                reinterpret_cast<unsigned*>(f->scal + kScalBarrier), stream));
     mpchol_status rs = read_back();
     if (rs != MPCHOL_OK) return rs;
+    use.waited = true;
   } else if ((ss = true_residual(true)) != MPCHOL_OK) {
     return ss;
   }
@@ -1407,6 +1469,7 @@ mpchol_status mpchol_factor_compute(mpchol_factor_t* f, const float* dA, int lda
                                     mpchol_stream_t stream) {
   if (f == nullptr || dA == nullptr || lda < f->n) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const UseScope use(f, s);
   PHASE(MPCHOL_PH_SETUP, 1, s, launch_copy_lower(dA, lda, f->A, f->ld, f->n, f->b, 0, f->n, s));
   return launch_factor(f, s);
 }
@@ -1436,6 +1499,7 @@ mpchol_status mpchol_factor_codes(const mpchol_factor_t* f, int fmt, const void*
     *dScales = is_mx(fmt) ? static_cast<const void*>(mx)
                             : static_cast<const void*>(rexp + (size_t)rexp_slot(fmt) * f->n);
   }
+  f->unseen = true;
   *ldq = f->b;
   *rows = f->n - s - f->b;
   *col0 = s;
@@ -1449,6 +1513,7 @@ mpchol_status mpchol_solve_host(mpchol_factor_t* f, const float* hA, int lda, co
       nrhs < 1 || nrhs > 8)
     return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  UseScope use(f, s);
   const int n = f->n, b = f->b;
   if (f->op == nullptr) {
     MPCHOL_CUDA_TRY(dmalloc(&f->op, (size_t)f->ld * n));
@@ -1518,6 +1583,7 @@ mpchol_status mpchol_solve_host(mpchol_factor_t* f, const float* hA, int lda, co
   if (st != MPCHOL_OK && st != MPCHOL_PCG_MAXIT) return st;
   MPCHOL_CUDA_TRY(cudaMemcpyAsync(hX, f->hx, sizeof(double) * n * nrhs, cudaMemcpyDeviceToHost, s));
   MPCHOL_CUDA_TRY(cudaStreamSynchronize(s));
+  use.waited = true;
   return st;
 }
 
@@ -1584,12 +1650,14 @@ mpchol_status mpchol_factor_info_get(const mpchol_factor_t* fc, mpchol_factor_in
   mpchol_factor_t* f = const_cast<mpchol_factor_t*>(fc);
   if (f == nullptr || info == nullptr) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  UseScope use(f, s);
   std::vector<StepState> steps(f->nsteps + 1);
   DevStatus st;
   MPCHOL_CUDA_TRY(cudaMemcpyAsync(steps.data(), f->steps, sizeof(StepState) * (f->nsteps + 1),
                                   cudaMemcpyDeviceToHost, s));
   MPCHOL_CUDA_TRY(cudaMemcpyAsync(&st, f->status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   MPCHOL_CUDA_TRY(cudaStreamSynchronize(s));
+  use.waited = true;
   memset(info, 0, sizeof(*info));
   info->status = st.code;
   info->fail_row = st.code == MPCHOL_ERR_NOT_SPD ? st.row : -1;
@@ -1608,6 +1676,7 @@ mpchol_status mpchol_factor_info_get(const mpchol_factor_t* fc, mpchol_factor_in
 
 mpchol_status mpchol_factor_lower(const mpchol_factor_t* f, const float** dL, int* ldl, int* n) {
   if (f == nullptr) return MPCHOL_ERR_BAD_ARG;
+  f->unseen = true;
   if (dL) *dL = f->A;
   if (ldl) *ldl = f->ld;
   if (n) *n = f->n;
@@ -1645,6 +1714,7 @@ mpchol_status mpchol_factor_save(const mpchol_factor_t* fc, void* blob, size_t c
   if (blob == nullptr) return MPCHOL_OK;
   if (cap < total) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  UseScope use(f, s);
   // a failed factorization is not saved
   DevStatus fst;
   if (read_status(f->status, s, &fst) != 0) return MPCHOL_ERR_CUDA;
@@ -1652,6 +1722,7 @@ mpchol_status mpchol_factor_save(const mpchol_factor_t* fc, void* blob, size_t c
   unsigned char* out = static_cast<unsigned char*>(blob);
   MPCHOL_CUDA_TRY(blob_copy(f, out + sizeof(FactorBlobHeader), true, s));
   MPCHOL_CUDA_TRY(cudaStreamSynchronize(s));
+  use.waited = true;
   FactorBlobHeader h{};
   memcpy(h.magic, kBlobMagic, 8);
   h.version = 1;
@@ -1675,9 +1746,11 @@ mpchol_status mpchol_factor_load(mpchol_factor_t* f, const void* blob, size_t si
   if (st != MPCHOL_OK) return st;
   if (n != f->n || b != f->b) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  UseScope use(f, s);
   unsigned char* in = const_cast<unsigned char*>(static_cast<const unsigned char*>(blob));
   MPCHOL_CUDA_TRY(blob_copy(f, in + sizeof(FactorBlobHeader), false, s));
   MPCHOL_CUDA_TRY(cudaStreamSynchronize(s));
+  use.waited = true;
   f->solve_ready = false;
   // the saved status word is the blob's last field
   DevStatus fst;
@@ -1689,6 +1762,7 @@ mpchol_status mpchol_factor_load(mpchol_factor_t* f, const void* blob, size_t si
 
 mpchol_status mpchol_factor_diags(const mpchol_factor_t* f, const float** dD, const float** dDt) {
   if (f == nullptr) return MPCHOL_ERR_BAD_ARG;
+  f->unseen = true;
   if (dD) *dD = f->d;
   if (dDt) *dDt = f->dtilde;
   return MPCHOL_OK;
@@ -1696,6 +1770,7 @@ mpchol_status mpchol_factor_diags(const mpchol_factor_t* f, const float** dD, co
 
 mpchol_status mpchol_factor_prepare_solve(mpchol_factor_t* f, mpchol_stream_t stream) {
   if (f == nullptr) return MPCHOL_ERR_BAD_ARG;
+  const UseScope use(f, reinterpret_cast<cudaStream_t>(stream));
   return ensure_solve(f, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -1733,6 +1808,7 @@ mpchol_status mpchol_apply_precond(mpchol_factor_t* f, const double* dR, double*
                                    mpchol_stream_t stream) {
   if (f == nullptr || dR == nullptr || dZ == nullptr || nrhs < 1 || nrhs > 8) return MPCHOL_ERR_BAD_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  UseScope use(f, s);
   mpchol_status ss = ensure_solve(f, s);
   if (ss != MPCHOL_OK) return ss;
   const int nr = pcg_padded_nrhs(nrhs);
@@ -1750,6 +1826,7 @@ mpchol_status mpchol_apply_precond(mpchol_factor_t* f, const double* dR, double*
                                     sizeof(double) * f->n, nrhs, cudaMemcpyDeviceToDevice, s));
   DevStatus st;
   if (read_status(f->pstatus, s, &st) != 0) return MPCHOL_ERR_CUDA;
+  use.waited = true;
   return (mpchol_status)st.code;
 }
 
@@ -1780,27 +1857,30 @@ int mpchol_precond_cg(double* dA, double* dX, double* dB, int n, int r, double n
   mpchol_factor_t* f = nullptr;
   mpchol_status st = mpchol_factor_create(&o, n, &f);
   if (st != MPCHOL_OK) return -(100 + st);
-  // FP64 -> FP32 directly into the factor's storage (src/mixed_cholesky.cu:122)
-  if (launch_copy_lower(dA, n, f->A, f->ld, n, f->b, 0, n, s) != cudaSuccess) {
-    free_factor(f);
-    return -(100 + MPCHOL_ERR_CUDA);
-  }
-  st = run_factor(f, s);
-  mpchol_factor_info info;
-  if (st == MPCHOL_OK) st = mpchol_factor_info_get(f, &info, nullptr, nullptr, stream);
-  if (st != MPCHOL_OK) { free_factor(f); return -(100 + st); }
-  if (info.status == MPCHOL_ERR_NOT_SPD) { free_factor(f); return info.fail_row + 1; }
-  if (info.status != MPCHOL_OK) { free_factor(f); return -(100 + info.status); }
-  mpchol_pcg_opts po;
-  mpchol_pcg_opts_default(&po);
-  po.rel_tol = rel_tol;
-  po.max_it = max_it;
-  po.x0_precond = 1;
-  st = run_pcg<double>(f, dA, n, dB, dX, 1, &po, nullptr, s);
+  // the factor, the solve; everything is on s
+  auto run = [&]() -> int {
+    // FP64 -> FP32 directly into the factor's storage (src/mixed_cholesky.cu:122)
+    if (launch_copy_lower(dA, n, f->A, f->ld, n, f->b, 0, n, s) != cudaSuccess) return -(100 + MPCHOL_ERR_CUDA);
+    st = run_factor(f, s);
+    mpchol_factor_info info;
+    if (st == MPCHOL_OK) st = mpchol_factor_info_get(f, &info, nullptr, nullptr, stream);
+    if (st != MPCHOL_OK) return -(100 + st);
+    if (info.status == MPCHOL_ERR_NOT_SPD) return info.fail_row + 1;
+    if (info.status != MPCHOL_OK) return -(100 + info.status);
+    mpchol_pcg_opts po;
+    mpchol_pcg_opts_default(&po);
+    po.rel_tol = rel_tol;
+    po.max_it = max_it;
+    po.x0_precond = 1;
+    st = run_pcg<double>(f, dA, n, dB, dX, 1, &po, nullptr, s);
+    if (st == MPCHOL_OK) return 0;
+    if (st == MPCHOL_PCG_MAXIT) return -1;
+    return -(100 + st);
+  };
+  const int code = run();
+  note_use(f, s);
   free_factor(f);
-  if (st == MPCHOL_OK) return 0;
-  if (st == MPCHOL_PCG_MAXIT) return -1;
-  return -(100 + st);
+  return code;
 }
 
 int mpchol_switching_chol(float* dA, int n, int b, float* d_diagVals, float* updated_diag,
@@ -1831,6 +1911,7 @@ int mpchol_switching_chol(float* dA, int n, int b, float* d_diagVals, float* upd
     if (cudaStreamSynchronize(s) != cudaSuccess) st = MPCHOL_ERR_CUDA;
     if (st == MPCHOL_OK) st = (mpchol_status)info.status;
   }
+  note_use(f, s);
   free_factor(f);
   return st;
 }

@@ -7,8 +7,10 @@
  *     reference, src/micro_chol.hpp:18-20, src/sChol.cuh:278-279).
  *   - All pointers named d* are device pointers; h* are host pointers.
  *   - Every call is ordered on the caller's stream; the library never
- *     synchronizes the device except where a call is documented to return a
- *     host-visible result (reports, info), and then only that stream.
+ *     synchronizes the device.  A call that is documented to return a
+ *     host-visible result (reports, info) synchronizes that stream.  Destroying
+ *     an object waits for the object's own work (a cudaFree inside it, where
+ *     memory goes back to the driver, waits for more).
  *   - Errors are status codes.  The library never calls exit(), never destroys
  *     caller-owned handles or streams, and its kernels never trap.
  *   - Objects are re-entrant across different factor objects; one stream per
@@ -195,7 +197,10 @@ MPCHOL_API mpchol_status mpchol_factor_destroy(mpchol_factor_t* f);
 /* The device memory, streams and events of destroyed factor objects are kept
  * for the next object of about the same size (at most 4 sets, 512 MiB in all,
  * per process); this gives them back to the driver.  An allocation of the
- * library that fails does the same before it reports MPCHOL_ERR_ALLOC. */
+ * library that fails does the same before it reports MPCHOL_ERR_ALLOC.  Not
+ * kept, but freed by cudaFree: the memory of an object that gave out pointers
+ * into it (mpchol_factor_lower, _diags, _codes), was used under a stream
+ * capture, or was used on a stream while its work on another one still ran. */
 MPCHOL_API void mpchol_release_cached(void);
 /* Synchronizes `stream`; fills info; hStepPrec (nullable, length nsteps)
  * receives each step's trailing-update precision, hStepFp64 (nullable) the

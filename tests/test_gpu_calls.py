@@ -159,3 +159,115 @@ def test_a_pointer_to_a_batch_factor_outlives_the_next_factor_call():
     assert torch.equal(got[:, : n.value].t().tril(), bt.lower(0))
     L = torch.linalg.cholesky(As[0].double())
     assert ((bt.lower(0) - L).norm() / L.norm()).item() < 1e-5
+
+
+def _solved(f, A, B):
+    f.compute(A)
+    X, rep = f.pcg(A, B, rel_tol=1e-10)
+    assert rep.converged
+    return X
+
+
+def test_dropping_a_factor_leaves_a_capture_in_another_thread_alone():
+    """A factor object destroyed by one thread while another captures a graph in
+    the thread-local mode: the capture ends well and its graph runs."""
+    import threading
+    n = 700
+    A, B = matgen.spd_matrix(n, 1e2, n).cuda(), matgen.rhs(n, 1, n).cuda().reshape(n)
+    held = [mp.Factor(n, block_size=128, precision="fp16") for _ in range(2)]
+    for f in held:
+        _solved(f, A, B)
+    del f
+    x, y = torch.ones(1000, device="cuda"), torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        y.copy_(x)
+        t = threading.Thread(target=held.clear)
+        t.start()
+        t.join()
+        y.add_(x)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, 2 * x)
+    X = _solved(mp.Factor(n, block_size=128, precision="fp16"), A, B)     # no error is left behind
+    assert ((A.double() @ X - B).norm() / B.norm()).item() < 2e-10
+
+
+def test_factors_come_and_go_while_others_capture():
+    """One thread makes and drops factor objects while two others make batches
+    and factor objects that capture their graphs: every call succeeds."""
+    ns = [300, 64, 700]
+    As = [matgen.spd_matrix(n, 1e2, n).cuda() for n in ns]
+    Bs = [matgen.rhs(n, 1, n).cuda().reshape(n) for n in ns]
+    big, rhs = matgen.spd_matrix(1300, 1e2, 5).cuda(), matgen.rhs(1300, 1, 5).cuda().reshape(1300)
+    torch.cuda.synchronize()
+
+    def drops():
+        for i in range(200):
+            _solved(mp.Factor(ns[i % 3], block_size=128, precision="fp16"), As[i % 3], Bs[i % 3])
+
+    def batches():
+        for _ in range(15):
+            bt = mp.Batch(ns, nrhs=1, block_size=128, precision="fp16")
+            bt.factor(As)
+            Xs, reps, st = bt.pcg(As, Bs, rel_tol=1e-10)
+            assert st == _lib.OK and all(r.converged for r in reps)
+
+    def graphs():
+        for _ in range(15):
+            f = mp.Factor(1300, block_size=128, precision="fp16")
+            for _ in range(4):                       # the factor's graph, then the loop's
+                _solved(f, big, rhs)
+    assert _threads(drops, batches, graphs) == []
+
+
+def test_memory_is_not_reused_before_its_last_reader():
+    """The memory of a freed object serves the next one only after what still
+    used it: the caller's copy through a pointer, and a factorization still
+    waiting on another stream."""
+    from cholesky_gpu_b200.api import _wrap_device
+    n = 640
+    opts = dict(block_size=128, precision="fp32")
+    A1, A2 = matgen.spd_matrix(n, 1e2, 1).cuda(), 9.0 * matgen.spd_matrix(n, 1e2, 2).cuda()
+    L1, L2 = mp.factor(A1, **opts).lower(), mp.factor(A2, **opts).lower()
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+    f = mp.factor(A1, **opts)
+    p = ctypes.c_void_p()
+    assert _lib.load().mpchol_factor_lower(f.handle, ctypes.byref(p), None, None) == _lib.OK
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(40_000_000)
+        got = _wrap_device(p.value, (n, n), torch.float32).clone()
+        del f
+    with torch.cuda.stream(other):
+        h = mp.factor(A2, **opts)
+    torch.cuda.synchronize()
+    assert torch.equal(got.t().tril(), L1) and torch.equal(h.lower(), L2)
+    del h
+    for _ in range(3):
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(40_000_000)
+            f = mp.factor(A1, **opts)                # enqueued behind the wait
+            del f
+        with torch.cuda.stream(other):
+            h = mp.factor(A2, **opts)
+        torch.cuda.synchronize()
+        assert torch.equal(h.lower(), L2)
+
+
+def test_freed_memory_serves_the_next_solves_in_threads():
+    """Objects that give out no pointer, made and freed in turn in three threads:
+    each solve is that of a lone object."""
+    ns = (200, 900, 513, 1100)
+    mats = {n: (matgen.spd_matrix(n, 1e2, n).cuda(), matgen.rhs(n, 1, n).cuda().reshape(n)) for n in ns}
+    torch.cuda.synchronize()
+
+    def worker(order):
+        def run():
+            for n in order * 6:
+                A, B = mats[n]
+                X = _solved(mp.Factor(n, block_size=128, precision="fp16x2"), A, B)
+                assert ((A.double() @ X - B).norm() / B.norm()).item() < 2e-10
+        return run
+    assert _threads(worker(ns), worker(ns[::-1]), worker((900, 200))) == []
