@@ -86,18 +86,26 @@ def _threads(*work):
 def test_small_solves_of_different_orders_in_threads():
     """One-launch solves of one number of right-hand sides need shared memory by
     their order: none may bound another thread's."""
-    def solver(n, turns):
-        A = matgen.spd_matrix(n, 1e2, n).cuda()
-        B = matgen.rhs(n, 1, n).cuda().reshape(n)
-        f = mp.factor(A, block_size=128, precision="fp16")
+    lib = _lib.load()
+
+    def solver(n):
+        A, B = matgen.spd_matrix(n, 1e2, n).cuda(), matgen.rhs(n, 1, n).cuda().reshape(n)
+        X, f, side = torch.empty_like(B), mp.factor(A, block_size=128, precision="fp16"), torch.cuda.Stream()
+        po, rep = _lib.default_pcg_opts(rel_tol=1e-10), _lib.Report()
+        short = _lib.default_pcg_opts(rel_tol=1e-10, max_it=0, x0_precond=0)
         torch.cuda.synchronize()
 
+        def call(o):
+            return lib.mpchol_pcg(f.handle, A.data_ptr(), n, B.data_ptr(), X.data_ptr(), 1, ctypes.byref(o),
+                                  ctypes.byref(rep), side.cuda_stream)
+
         def run():
-            for _ in range(turns):
-                _, rep = f.pcg(A, B, rel_tol=1e-10)
-                assert rep.converged and rep.rel_residual <= 1e-10
+            for _ in range(5000):                    # the launches are what meets
+                st = call(short)
+                assert st == _lib.PCG_MAXIT, (n, st)
+            assert call(po) == _lib.OK and rep.rel_residual <= 1e-10
         return run
-    assert _threads(solver(1000, 300), solver(64, 600), solver(500, 400), solver(9, 600)) == []
+    assert _threads(solver(1000), solver(64), solver(500), solver(9)) == []
 
 
 _FIRST_SOLVES = """
