@@ -971,8 +971,9 @@ cudaError_t launch_potrf_batched(BatchSys* sys, int nact, int s, int b, const Po
                                  cudaStream_t stream) {
   if (nact <= 0) return cudaSuccess;
   const size_t smem = potrf_smem_bytes(b);
-  cudaError_t e = cudaFuncSetAttribute(potrf_batched_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the kernel's limit, not the launch's: the most any block needs
+  cudaError_t e = cudaFuncSetAttribute(potrf_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)potrf_smem_bytes(256));
   if (e != cudaSuccess) return e;
   potrf_batched_kernel<<<nact, 512, smem, stream>>>(sys, s, b, p);
   return cudaGetLastError();

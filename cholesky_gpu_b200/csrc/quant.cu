@@ -98,6 +98,8 @@ __global__ void quantize_hash_kernel(unsigned long long first, unsigned long lon
 }
 
 size_t qtile_smem(int k) { return (size_t)k * (QROWS + 1) * sizeof(float); }
+// The kernels' limit, not a launch's (concurrent calls share it): K <= 256.
+size_t qtile_smem_max() { return qtile_smem(256); }
 
 }  // namespace
 
@@ -106,7 +108,7 @@ cudaError_t launch_quantize_rows(const float* P, int ldp, int m, int k, int fmt,
   if (m <= 0) return cudaSuccess;
   const size_t smem = qtile_smem(k);
   cudaError_t e = cudaFuncSetAttribute(quantize_rows_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qtile_smem_max());
   if (e != cudaSuccess) return e;
   quantize_rows_kernel<<<ceil_div(m, QROWS), QTHR, smem, stream>>>(P, ldp, m, k, fmt, q, ldq, rowexp,
                                                                    mxexp, ldmx);
@@ -139,7 +141,7 @@ cudaError_t launch_quantize_batched(BatchSys* sys, const BatchStep* steps, int n
   if (nact <= 0 || max_m <= 0) return cudaSuccess;
   const size_t smem = qtile_smem(b);
   cudaError_t e = cudaFuncSetAttribute(quantize_batched_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qtile_smem_max());
   if (e != cudaSuccess) return e;
   quantize_batched_kernel<<<dim3(ceil_div(max_m, QROWS), nact), QTHR, smem, stream>>>(
       sys, steps, s, b, fmt, q, qrows, rowexp, mxexp, diag_pert);

@@ -653,8 +653,9 @@ cudaError_t launch_trsm_batched(BatchSys* sys, int nact, int s, int b, int max_m
   if (nact <= 0 || max_m <= 0) return cudaSuccess;
   if (b % 32 != 0 || b > 32 * MAXNT) return cudaErrorInvalidValue;
   const size_t smem = trsm_smem_floats(32, b) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(trsm_batched_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the kernel's limit, not the launch's: the most any block needs
+  cudaError_t e = cudaFuncSetAttribute(trsm_batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(trsm_smem_floats(32, 32 * MAXNT) * sizeof(float)));
   if (e != cudaSuccess) return e;
   trsm_batched_kernel<<<dim3(ceil_div(max_m, 32), nact), NTHR, smem, stream>>>(sys, s, b);
   return cudaGetLastError();

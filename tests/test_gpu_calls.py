@@ -279,3 +279,21 @@ def test_freed_memory_serves_the_next_solves_in_threads():
                 assert ((A.double() @ X - B).norm() / B.norm()).item() < 2e-10
         return run
     assert _threads(worker(ns), worker(ns[::-1]), worker((900, 200))) == []
+
+
+def test_batches_of_different_blocks_in_threads():
+    """Batches whose block sizes ask for different amounts of shared memory are
+    made, factored and solved at the same time."""
+    ns = [200, 64, 400]
+    As = [matgen.spd_matrix(n, 1e2, n).cuda() for n in ns]
+    Bs = [matgen.rhs(n, 1, n).cuda().reshape(n) for n in ns]
+    torch.cuda.synchronize()
+
+    def batches(block):
+        def run():
+            for _ in range(25):
+                bt = mp.Batch(ns, nrhs=1, block_size=block, precision="fp16")
+                bt.factor(As)                        # the launches are captured here
+                assert bt.pcg(As, Bs, rel_tol=1e-10)[2] == _lib.OK
+        return run
+    assert _threads(batches(192), batches(64), batches(256), batches(128)) == []
