@@ -384,8 +384,9 @@ def switching_chol(d_A: torch.Tensor, n: int, b: int, d_diagVals: torch.Tensor,
                    updated_diag: torch.Tensor, eps_prime: float, perturb_diag: bool = False,
                    microscal_size: int = 32, scales: torch.Tensor | None = None) -> int:
     """The reference's switching_chol (src/switching_chol.cuh:19-22): in-place
-    FP32 factor of the n x n column-major matrix d_A with block b.  Returns a
-    status code (0 = ok) where the reference returns nothing."""
+    FP32 factor of the n x n column-major matrix d_A with block b (nothing above
+    the diagonal is written).  Returns a status code (0 = ok) where the
+    reference returns nothing."""
     _require_cuda(d_A, torch.float32, "d_A")
     if d_A.stride(0) != 1 and not d_A.is_contiguous():
         raise ValueError("d_A must be column-major or contiguous symmetric")

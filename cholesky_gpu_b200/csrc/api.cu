@@ -1901,9 +1901,9 @@ int mpchol_switching_chol(float* dA, int n, int b, float* d_diagVals, float* upd
   mpchol_factor_info info;
   st = mpchol_factor_info_get(f, &info, nullptr, nullptr, stream);
   if (st == MPCHOL_OK) {
-    if (cudaMemcpy2DAsync(dA, sizeof(float) * n, f->A, sizeof(float) * f->ld, sizeof(float) * n, n,
-                          cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-      st = MPCHOL_ERR_CUDA;
+    // the lower triangle only: above it the factor's storage holds leftovers, dA the
+    // caller's values
+    if (launch_copy_lower(f->A, f->ld, dA, n, n, 1, 0, n, s) != cudaSuccess) st = MPCHOL_ERR_CUDA;
     if (d_diagVals && cudaMemcpyAsync(d_diagVals, f->d, sizeof(float) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       st = MPCHOL_ERR_CUDA;
     if (updated_diag && cudaMemcpyAsync(updated_diag, f->dtilde, sizeof(float) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess)

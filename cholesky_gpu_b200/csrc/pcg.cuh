@@ -84,8 +84,8 @@ cudaError_t launch_pcg_small(const TA* A, int lda, const double* B, int nrhs, do
 cudaError_t launch_extract_diag(const float* A, int lda, int n, float* d, float* dtilde,
                                 cudaStream_t stream);
 // Columns [c0, c1) of the lower block columns (rows from the column's block
-// diagonal down, block b) of src (FP32, or FP64 rounded to FP32) into dst, in
-// one launch.
+// diagonal down, block b; b = 1: the lower triangle) of src (FP32, or FP64
+// rounded to FP32) into dst, in one launch.
 template <typename TS>
 cudaError_t launch_copy_lower(const TS* src, int lds, float* dst, int ldd, int n, int b, int c0,
                               int c1, cudaStream_t stream);

@@ -33,14 +33,15 @@ __global__ void extract_diag_kernel(const float* __restrict__ A, int lda, int n,
 // an FP64 source, a pass over the full square with an index division per
 // element: B200, n = 16384: 664 us in 64 copies against 183 us; n = 8192: 300
 // against 41 us; FP64 source at n = 3072: 28 against 7 us.  VEC: 16-byte accesses, for a
-// source whose columns all start on 16-byte boundaries.
+// source and a destination whose columns all start on 16-byte boundaries and b a
+// multiple of 4.  b = 1: exactly the lower triangle.
 template <typename TS, bool VEC>
 __global__ void __launch_bounds__(256)
 copy_lower_kernel(const TS* __restrict__ src, int lds, float* __restrict__ dst, int ldd, int n,
                   int b, int c0, int c1) {
   constexpr int V = VEC ? 4 : 1;
   for (int c = c0 + (int)blockIdx.x; c < c1; c += gridDim.x) {
-    const int r0 = c / b * b;                      // a multiple of 32
+    const int r0 = c / b * b;                      // VEC: a multiple of 4
     const TS* s = src + (size_t)c * lds;
     float* t = dst + (size_t)c * ldd;
     const int step = V * (int)blockDim.x;
@@ -195,9 +196,8 @@ cudaError_t launch_copy_lower(const TS* src, int lds, float* dst, int ldd, int n
   c1 = std::min(c1, n);
   if (c1 <= c0) return cudaSuccess;
   const int grid = std::min(c1 - c0, 148 * 8);
-  // rows start at multiples of b (of 32); dst is the library's own storage
   if constexpr (sizeof(TS) == 4) {
-    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 &&
+    if (b % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 &&
         lds % 4 == 0 && ldd % 4 == 0) {
       copy_lower_kernel<TS, true><<<grid, 256, 0, stream>>>(src, lds, dst, ldd, n, b, c0, c1);
       return cudaGetLastError();

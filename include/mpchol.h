@@ -351,7 +351,8 @@ MPCHOL_API int mpchol_precond_cg(double* dA, double* dX, double* dB, int n, int 
                       float eps_prime, float flr, int perturb_diag, int microscal_size,
                       double rel_tol, int max_it, mpchol_stream_t stream);
 /* switching_chol semantics: in-place factor of the FP32 matrix dA (ld = n)
- * with block b; d_diagVals (n) receives the original diagonal and
+ * with block b (the lower triangle becomes L, what lies above it is left as it
+ * is); d_diagVals (n) receives the original diagonal and
  * updated_diag (n) the Schur-complement diagonal tracker (the reference's
  * caller fills both, src/mixed_cholesky.cu:128-131; here the library fills
  * them).  scales (nullable) receives the last MX step's E8M0 codes.

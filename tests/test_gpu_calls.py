@@ -297,3 +297,24 @@ def test_batches_of_different_blocks_in_threads():
                 assert bt.pcg(As, Bs, rel_tol=1e-10)[2] == _lib.OK
         return run
     assert _threads(batches(192), batches(64), batches(256), batches(128)) == []
+
+
+@pytest.mark.parametrize("n,block", [(1, 128), (31, 128), (33, 256), (127, 128), (257, 128), (514, 256)])
+def test_the_drop_in_factorization_leaves_the_upper_triangle_alone(n, block):
+    """switching_chol writes L into the lower triangle of its column-major matrix
+    and nothing else, whatever the memory that the library works in held before
+    (a larger system's solve and factor)."""
+    big = matgen.spd_matrix(600, 1e2, 1).cuda()
+    _solved(mp.Factor(600, block_size=128, precision="fp16"), big, matgen.rhs(600, 1, 1).cuda().reshape(600))
+    A = matgen.spd_matrix(n, 1e2, n).cuda() if n > 1 else torch.full((1, 1), 4.0, device="cuda")
+    store = A.clone()                                # row j of the storage is column j
+    above = torch.ones((n, n), dtype=torch.bool, device="cuda").tril(-1)   # of the storage: i < j
+    store[above] = torch.arange(int(above.sum()), device="cuda", dtype=torch.float32) + 1000.0
+    before = store.clone()
+    d, dt = torch.empty(n, device="cuda"), torch.empty(n, device="cuda")
+    assert mp.switching_chol(store, n, block, d, dt, 1e-3) == 0
+    assert torch.equal(store[above], before[above])
+    L = torch.linalg.cholesky(A.double())
+    got = store.t().tril().double()
+    assert ((got - L).norm() / L.norm()).item() < 1e-3
+    assert torch.equal(d, torch.diagonal(A))
