@@ -68,7 +68,7 @@ __device__ __forceinline__ void sum_partials(const double* partials, double (&ou
 // Each of these vector passes also prepares what the next kernels start from
 // (zeroed accumulation targets, the triangular solves' input and counters), so
 // that an iteration is seven launches; a boundary costs 1.5 us or more of an
-// iteration that takes 20 at n = 1024.
+// iteration that takes 40 at n = 1500.
 
 // The inputs of one application z = M^-1 r: work = r, tmp and z zero, the two
 // triangular solves' counters zero.

@@ -447,7 +447,8 @@ __device__ void potrf_block(T* tiles, float* A, int lda, int s, int bs, const fl
 // instruction fetch, not arithmetic, bounded fully unrolled forms, whose code
 // was refetched in every phase.  One SM's FP32 rate is the floor: 116 K warp
 // fmas, about 41 K cycles at the 0.7 of peak that three-operand fmas reach.
-// 256 x 256: 47 us a launch alone and 53 - 68 us beside a trailing update; one
+// 256 x 256: 46 us a launch alone and 46 - 68 us (median 55, n = 8192) beside a
+// trailing update, from its early start on; one
 // pivot per shared-memory round trip with block barriers between tile solves
 // and updates took 72 us, and 77 - 105 us beside the update.
 constexpr int NPW = 8;          // panel warps: warp w holds tile row w
@@ -557,7 +558,10 @@ __device__ __forceinline__ void chain_tile(float (&a)[TS], float* t, float* inv,
 #pragma unroll
     for (int k = 0; k < SUB; ++k) {
       const float piv = d[k][k] + sh[k];
-      float r;   // rsqrtf's value for every normal argument, at less than half its latency
+      // rsqrtf's result (the bits agree for every positive normal argument, checked
+      // over all of them; 2^-22.9 of the exact value at worst) at less than half its
+      // latency.  A denormal pivot takes the full rule.
+      float r;
       asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
       plain = plain && piv > th[k] && piv <= 3.402823466e38f;
       my_inv = lane == k ? r : my_inv;

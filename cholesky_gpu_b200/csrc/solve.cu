@@ -10,14 +10,17 @@
 // once per factor, the inverses W_S of the 1024-row diagonal super-blocks
 // L_SS are formed by recursive doubling (FP64 128-block inverses, FP32 GEMM
 // tiles above that).  A
-// forward solve is then n/1024 steps of two fully parallel kernels:
+// forward solve is then n/1024 steps of two fully parallel passes over tiles:
 //     y_S  = W_S w_S                      (TRMV over the super-block's lower tiles)
 //     w_T -= L_TS y_S   for T > S         (GEMV over the panel below)
-// and the backward solve mirrors it with transposes.  The applied operator is
+// and the backward solve mirrors it with transposes; a single system's tiles
+// run in one persistent launch, a batch's in a launch per pass.  The applied operator is
 // (Lt Lt^T)^-1 with Lt = blockdiag(W_S^-1) + strictly-block-lower(L), which is
 // symmetric positive definite whenever the W_S are nonsingular, so PCG stays
 // well defined; it equals (L L^T)^-1 up to the FP32 rounding of the W_S.
-// Partial sums are combined with FP64 atomics.
+// Partial sums of the products, of far panel tiles and of a batch's passes are
+// combined with FP64 atomics; those on the persistent solve's chain go through
+// tagged slots where there are one or two right-hand sides.
 #include <algorithm>
 #include <mutex>
 
@@ -49,11 +52,6 @@ __device__ __forceinline__ void load4<float>(const float* p, int nvalid, float o
 // Tile loaded into registers: lane covers rows 4*lane..4*lane+3, warp covers
 // CH consecutive columns starting at col0.  Elements outside (rows_valid,
 // cols_valid) are zero.  Every load of the batch is issued before any use.
-template <typename TA, int CH>
-struct TileRegs {
-  double v[CH][4];
-};
-
 // Tile values stay in the matrix's own type in registers (FP32 tiles take
 // half the registers of a widened copy); they are widened at each use.
 template <int CH>
@@ -224,14 +222,11 @@ __device__ __forceinline__ void tri_of(int t, int& i, int& j) {
   j = t - a * (a + 1) / 2;
 }
 
-template <typename TA> struct ChunkOf { static constexpr int value = 16; };
-template <> struct ChunkOf<double> { static constexpr int value = 8; };
-
 // ---- tiles staged in shared memory -------------------------------------------
 // The streaming kernels (SYMV, the persistent triangular solve) copy each
-// 128 x 128 FP32 tile into shared memory with cp.async, one or two tiles
-// ahead of its use: the copies hold no registers, so an SM keeps 128-192 KB
-// of HBM reads in flight while it computes on the current tile.
+// 128 x 128 FP32 tile into shared memory with cp.async, one stage per CTA and
+// two or three CTAs per SM: the copies hold no registers, and one CTA's copy is
+// in flight (64 KB) while the others compute on theirs.
 constexpr int TILE_ELEMS = RB * RB;   // 64 KB of FP32
 constexpr int SCH = 8;                // columns per widened chunk
 
@@ -636,8 +631,7 @@ symv_body(const TA* __restrict__ A, int lda, int n, const double* __restrict__ x
   __syncthreads();
   double acc[4][NR] = {};
   const bool diag = (I == J);
-  tile_pass<TA, NR, ChunkOf<TA>::value>(A + (size_t)j0 * lda + i0, lda, ni, nj, s_xJ, s_xI, acc,
-                                        s_col, diag ? 1 : 0, diag ? 2 : 0, true, true);
+  tile_pass<TA, NR, 8>(A + (size_t)j0 * lda + i0, lda, ni, nj, s_xJ, s_xI, acc, s_col, diag ? 1 : 0, diag ? 2 : 0, true, true);
   __syncthreads();
   // column sums go to y_J
   for (int e = threadIdx.x; e < RB * NR; e += NTH) {
@@ -658,7 +652,7 @@ symv_kernel(const TA* __restrict__ A, int lda, int n, const double* __restrict__
 // For a lower-triangular [A 0; B C], inv = [A^-1 0; X C^-1] with
 // X = -C^-1 (B A^-1).  The inverses W_S of the RS-row diagonal super-blocks
 // are built bottom-up: the 128-row diagonal blocks in FP64 (32-row tiles on
-// the FP64 tensor cores), then the 128 -> 1024 doublings as 64 x 64 FP32 GEMM
+// the FP64 tensor cores), then the 128 -> 1024 doublings as 32 x 32 FP32 GEMM
 // tiles over all super-blocks at once.
 // Storage: W_S is RS x RS column-major at wsup + S*RS*RS.  Its lower 128-tiles
 // hold the inverse (diagonal tiles with a zero upper part); the strictly
@@ -1036,7 +1030,10 @@ panel_body(const float* __restrict__ L, int ldl, int n, int s0, int rs,
 // One right-hand side, forward / backward, against atomics and counters
 // throughout, units in the order of need alone and bound to a CTA a unit early
 // (B200): n = 6144 45 / 49 -> 39 / 45 us, 8192 63 / 69 -> 57 / 65, 16384 172 / 188
-// -> 145 / 158; eight: 16384 291 / 291 -> 282 / 274.
+// -> 145 / 158; eight: 16384 291 / 291 -> 282 / 274.  With two super-blocks, where
+// every unit runs at once, the decoding of the order shows: n = 2048, two
+// right-hand sides, 13.7 / 16.7 -> 15.6 / 18.9 (the launches saved around a pair
+// of solves make up for it: 86 -> 84 us for mpchol_apply_precond).
 // Waits are bounded; a wait that runs out records MPCHOL_ERR_TIMEOUT and the
 // unit proceeds (the result is then wrong, but no CTA waits forever).
 constexpr long long kTrsvMaxPolls = 1ll << 24;
@@ -1462,78 +1459,62 @@ template <int NR>
 __global__ void __launch_bounds__(NTH, 2)
 symv_staged_batched_kernel(const BatchSys* __restrict__ sys, int nsys, int ntiles, int xslot,
                            int yslot, int use_skip) {
-  constexpr int STAGES = 1;
   constexpr bool MMA = NR == 8;
   constexpr int TE = MMA ? BL_TILE : TILE_ELEMS;
   constexpr int VEC = MMA ? XS * 8 : RB * NR;
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  __shared__ SymvUnit s_unit[STAGES];
-  float* tiles = reinterpret_cast<float*>(sm_raw);
-  double* vecs = reinterpret_cast<double*>(tiles + STAGES * TE);
-  double* s_col = vecs + STAGES * 2 * VEC;
-  auto issue = [&](int t, int stage) {
-    const SymvUnit u = symv_unit<NR>(sys, nsys, t, xslot, yslot, use_skip);
-    if (threadIdx.x == 0) s_unit[stage] = u;
-    if (u.A == nullptr) return;
+  float* Ts = reinterpret_cast<float*>(sm_raw);
+  double* xJ = reinterpret_cast<double*>(Ts + TE);
+  double* xI = xJ + VEC;
+  double* s_col = xI + VEC;
+  __shared__ SymvUnit s_unit;   // read again after the copies: no registers held through the tile pass
+  auto issue = [&](const SymvUnit& u) {
     const int i0 = u.I * RB, j0 = u.J * RB;
     const int ni = min(RB, u.n - i0), nj = min(RB, u.n - j0);
     const float* T = u.A + (size_t)j0 * u.lda + i0;
-    float* dst = tiles + stage * TE;
     if (MMA) {
-      if (u.al16) stage_tile_bl(dst, T, u.lda, ni, nj);
-      else stage_tile_4b<true>(dst, T, u.lda, ni, nj);
-      stage_vec_x8(u.x, u.n, j0, nj, vecs + (2 * stage) * VEC);
-      stage_vec_x8(u.x, u.n, i0, ni, vecs + (2 * stage + 1) * VEC);
+      if (u.al16) stage_tile_bl(Ts, T, u.lda, ni, nj);
+      else stage_tile_4b<true>(Ts, T, u.lda, ni, nj);
+      stage_vec_x8(u.x, u.n, j0, nj, xJ);
+      stage_vec_x8(u.x, u.n, i0, ni, xI);
     } else {
-      if (u.al16) stage_tile(dst, T, u.lda, ni, nj);
-      else stage_tile_4b<false>(dst, T, u.lda, ni, nj);
-      stage_vec<NR>(u.x, u.n, j0, nj, vecs + (2 * stage) * VEC);
-      stage_vec<NR>(u.x, u.n, i0, ni, vecs + (2 * stage + 1) * VEC);
+      if (u.al16) stage_tile(Ts, T, u.lda, ni, nj);
+      else stage_tile_4b<false>(Ts, T, u.lda, ni, nj);
+      stage_vec<NR>(u.x, u.n, j0, nj, xJ);
+      stage_vec<NR>(u.x, u.n, i0, ni, xI);
     }
   };
-#pragma unroll
-  for (int st = 0; st < STAGES - 1; ++st) {
-    const int t = blockIdx.x + st * gridDim.x;
-    if (t < ntiles) issue(t, st);
-    cp_async_commit();
-  }
-  int stage = 0;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     {
-      const int tn = t + (STAGES - 1) * gridDim.x;
-      if (tn < ntiles) issue(tn, (stage + STAGES - 1) % STAGES);
-      cp_async_commit();
+      const SymvUnit u = symv_unit<NR>(sys, nsys, t, xslot, yslot, use_skip);
+      if (u.A == nullptr) continue;                // uniform over the CTA
+      if (threadIdx.x == 0) s_unit = u;
+      issue(u);
     }
-    cp_async_wait<STAGES - 1>();
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
-    const SymvUnit u = s_unit[stage];
-    if (u.A != nullptr) {
-      const int i0 = u.I * RB, j0 = u.J * RB;
-      const int ni = min(RB, u.n - i0), nj = min(RB, u.n - j0);
-      float* Ts = tiles + stage * TE;
-      const double* xJ = vecs + (2 * stage) * VEC;
-      const double* xI = xJ + VEC;
-      if (MMA) {
-        if (u.I == u.J)
-          tile_mma_x8<true, false>(Ts, xJ, xI, u.y, i0, ni, u.y, j0, nj, u.n, true, true, 1.0, nullptr);
-        else
-          tile_mma_x8<false, false>(Ts, xJ, xI, u.y, i0, ni, u.y, j0, nj, u.n, true, true, 1.0, nullptr);
-      } else {
-        double acc[4][NR] = {};
-        if (u.I == u.J) tile_pass_staged<NR, true>(Ts, xJ, xI, acc, s_col, true, true);
-        else tile_pass_staged<NR, false>(Ts, xJ, xI, acc, s_col, true, true);
-        __syncthreads();
-        for (int e = threadIdx.x; e < VEC; e += NTH) {
-          const int k = e / RB, c = e % RB;
-          if (c < nj) atomicAdd(&u.y[(size_t)k * u.n + j0 + c], s_col[e]);
-        }
-        flush_rows<NR>(acc, reinterpret_cast<double*>(Ts), u.y, u.n, i0, ni, 1.0);
+    const SymvUnit u = s_unit;
+    const int i0 = u.I * RB, j0 = u.J * RB;
+    const int ni = min(RB, u.n - i0), nj = min(RB, u.n - j0);
+    if (MMA) {
+      if (u.I == u.J)
+        tile_mma_x8<true, false>(Ts, xJ, xI, u.y, i0, ni, u.y, j0, nj, u.n, true, true, 1.0, nullptr);
+      else
+        tile_mma_x8<false, false>(Ts, xJ, xI, u.y, i0, ni, u.y, j0, nj, u.n, true, true, 1.0, nullptr);
+    } else {
+      double acc[4][NR] = {};
+      if (u.I == u.J) tile_pass_staged<NR, true>(Ts, xJ, xI, acc, s_col, true, true);
+      else tile_pass_staged<NR, false>(Ts, xJ, xI, acc, s_col, true, true);
+      __syncthreads();
+      for (int e = threadIdx.x; e < VEC; e += NTH) {
+        const int k = e / RB, c = e % RB;
+        if (c < nj) atomicAdd(&u.y[(size_t)k * u.n + j0 + c], s_col[e]);
       }
+      flush_rows<NR>(acc, reinterpret_cast<double*>(Ts), u.y, u.n, i0, ni, 1.0);
     }
-    __syncthreads();   // the stage, its unit record and s_col are free again
-    stage = (stage + 1) % STAGES;
+    __syncthreads();   // the stage, the unit's record and s_col are free again
   }
-  cp_async_wait<0>();
 }
 
 // dst slot = 0 (src < 0) or a copy of the src slot
@@ -1841,10 +1822,13 @@ cudaError_t launch_trsv_persistent(bool backward, const float* L, int ldl, int n
   const size_t smem = trsv_smem_bytes(nrhs);
   auto launch = [&](auto kernel) -> cudaError_t {
     cudaLaunchConfig_t cfg = {};
-    // The third CTA per SM (one right-hand side) pays once far tiles bound the
-    // solve; before that it only slows the chain's tile passes: forward / backward
-    // 57 / 65 us with two and 58 / 67 with three at n = 8192, 78 / 88 and 76 / 82
-    // at 10240, 168 / 185 and 145 / 158 at 16384.
+    // The third CTA per SM (one right-hand side, or eight) pays once far tiles
+    // bound the solve; before that it only slows the chain's tile passes.  Two and
+    // three per SM, forward / backward in us.  One right-hand side: 24.0 / 27.5 and
+    // 27.7 / 32.1 at n = 4096, 55 / 60 and 56 / 63 at 8192, 65 / 70 and 63 / 70 at
+    // 9200, 78 / 88 and 76 / 82 at 10240, 168 / 185 and 145 / 158 at 16384.  Eight:
+    // 22.8 / 23.4 and 24.7 / 26.8 at 2048, 46 / 46 and 51 / 51 at 4096, 100 / 98 and
+    // 112 / 112 at 8192.  (With two or four only two fit.)
     cfg.gridDim = dim3((n > 9 * RS ? per_sm : std::min(per_sm, 2)) * lim->sms);
     cfg.blockDim = dim3(NTH);
     cfg.dynamicSmemBytes = smem;

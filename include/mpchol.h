@@ -455,7 +455,7 @@ MPCHOL_API mpchol_status mpchol_rbf_grad(const float* dX, int n, int d, int ldx,
  * synchronize the device (stalling every other stream), and a process whose
  * device memory is held by a caching allocator may have none to give.
  *   n <= MPCHOL_POTRF_STATIC_MAX (larger n: MPCHOL_ERR_BAD_ARG, nothing runs);
- *   dA 16-byte aligned and lda a multiple of 4 (TMA); lda >= n.
+ *   dA 16-byte aligned and lda a multiple of 4 (MPCHOL_ERR_BAD_ARG); lda >= n.
  *   pivot_floor > 0: pivots <= pivot_floor * A(i,i) are raised to that value
  *   (max(|pivot|, floor) repair); pivot_floor = 0: no repair.
  *   dInfo (device int): 0 on success, i + 1 if pivot i was not positive
