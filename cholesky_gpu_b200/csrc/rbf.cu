@@ -224,6 +224,10 @@ rbf_grad_kernel(const float* __restrict__ X, int n, int d, int ldx, double inv2l
     double r2[R][C] = {};
 #pragma unroll 4
     for (int k = 0; k < d; ++k) dist_step<R, C>(xi + k * LI, xj + k * LJX, rows, cols, r2);
+    // s by tiles, then over the tiles: one chain of R C terms a tile loses more than
+    // 32-row CTAs with half the terms did (relative error at n = 8192, d = 64,
+    // geometric mean of 24 draws: 7.3e-16 with those, 1.3e-15 in one chain, 4.2e-16)
+    double s_tile = 0.0;
 #pragma unroll
     for (int v = 0; v < C; ++v) {
       const int jl = cols[v / 2] + v % 2;
@@ -233,7 +237,7 @@ rbf_grad_kernel(const float* __restrict__ X, int n, int d, int ldx, double inv2l
       for (int u = 0; u < R; ++u) {
         const bool in = i0 + rows[u / 2] + u % 2 < n && j0 + jl < n;
         kv[u] = in ? exp(-r2[u][v] * inv2l2) : 0.0;
-        s_acc += in ? ai[u] * bv * kv[u] * r2[u][v] : 0.0;
+        s_tile += in ? ai[u] * bv * kv[u] * r2[u][v] : 0.0;
         pa[u] = fma(kv[u], av, pa[u]);
         pb[u] = fma(kv[u], bv, pb[u]);
       }
@@ -241,6 +245,7 @@ rbf_grad_kernel(const float* __restrict__ X, int n, int d, int ldx, double inv2l
       for (int u = 0; u < R / 2; ++u)
         *reinterpret_cast<double2*>(kt + jl * LI + rows[u]) = make_double2(kv[2 * u], kv[2 * u + 1]);
     }
+    s_acc += s_tile;
     __syncthreads();
     if (j0 + JT < n) fetch(j0 + JT);
 #pragma unroll 2
