@@ -23,6 +23,7 @@
 // tagged slots where there are one or two right-hand sides.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -419,7 +420,9 @@ __device__ __forceinline__ void load_vec_x8(const double* x, int n, int row0, in
 // fixes the product at compile time (1: row sums, 2: column sums, 0: by
 // do_nt / do_t).  Both products: KC = 8, UNR = 2 (the 128 registers of two
 // CTAs per SM allow no more); one product: KC = 4 fully unrolled.
-template <bool DIAG, bool FRO, int KC = 8, int UNR = 2, int ONLY = 0>
+// NACC accumulators share the k-steps of an output in turn: each is a chain of
+// 32 / NACC DMMAs.
+template <bool DIAG, bool FRO, int KC = 8, int UNR = 2, int ONLY = 0, int NACC = 2>
 __device__ __forceinline__ void tile_mma_x8(const float* Ts, const double* x_c, const double* x_r,
                                             double* y_rows, int row0, int nrows, double* y_cols,
                                             int col0, int ncols, int n, bool do_nt_rt, bool do_t_rt,
@@ -429,11 +432,11 @@ __device__ __forceinline__ void tile_mma_x8(const float* Ts, const double* x_c, 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int B0 = 16 * warp;
-  // accumulators: [m-block][k-step parity] -- eight independent DMMA chains
-  // per warp when both products run
-  double dn[2][2][2] = {};
-  double dt[2][2][2] = {};
-  static_assert(KC % 2 == 0, "k-step parity picks the accumulator: chunks hold an even count");
+  // accumulators: [m-block][k-step % NACC] -- eight independent DMMA chains
+  // per warp when both products run with two
+  double dn[2][NACC][2] = {};
+  double dt[2][NACC][2] = {};
+  static_assert(KC % NACC == 0, "a chunk's k-steps go round the accumulators whole times");
 #pragma unroll(UNR)
   for (int kb = 0; kb < RB; kb += 4 * KC) {
     // every fragment of the chunk is loaded (and widened) before its DMMAs
@@ -471,17 +474,26 @@ __device__ __forceinline__ void tile_mma_x8(const float* Ts, const double* x_c, 
             const int r = B0 + 8 * mb + g, c = kb + 4 * j + t;
             *fsq = fma((DIAG && r == c) ? a : 2.0 * a, a, *fsq);
           }
-          dmma_m8n8k4(dn[mb][j & 1], a, bn[j]);
+          dmma_m8n8k4(dn[mb][j % NACC], a, bn[j]);
         }
       }
       if (do_t) {
 #pragma unroll
-        for (int mb = 0; mb < 2; ++mb) dmma_m8n8k4(dt[mb][j & 1], (double)at[mb][j], bt[j]);
+        for (int mb = 0; mb < 2; ++mb) dmma_m8n8k4(dt[mb][j % NACC], (double)at[mb][j], bt[j]);
       }
     }
   }
 #pragma unroll
   for (int mb = 0; mb < 2; ++mb) {
+#pragma unroll
+    for (int h = NACC / 2; h > 1; h >>= 1)             // the accumulators in pairs
+#pragma unroll
+      for (int q = 0; q < h; ++q)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          dn[mb][q][i] += dn[mb][q + h][i];
+          dt[mb][q][i] += dt[mb][q + h][i];
+        }
     const int idx = B0 + 8 * mb + g;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -527,7 +539,13 @@ constexpr size_t symv_staged_smem() {
 // reduced in the stage's own tile buffer once the tile has been used.
 // fro != nullptr: CTA b also writes its share of ||A||_F^2 (lower triangle,
 // off-diagonal entries twice) to fro[b] and zeroes fro[gridDim.x ..nfro).
-template <int NR>
+// al16: the columns of A start on 16-byte boundaries.  Eight right-hand sides
+// (AL, fixed at compile time there): columns that do not start so used to be
+// summed in short chains by FMAs, so their DMMA passes, one product at a time,
+// spread the sums over eight accumulators (relative error of a product at n =
+// 2999: 2.4e-16 with FMAs, 44 us; 3.3e-16 with two accumulators, 17.4; 2.5e-16
+// with eight, 16.8).
+template <int NR, bool AL = true>
 __global__ void __launch_bounds__(NTH, symv_ctas<NR>())
 symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __restrict__ x,
                    double* __restrict__ y, const int* skip, double* fro, int nfro, int al16) {
@@ -545,7 +563,7 @@ symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __
   auto issue = [&](int i0, int ni, int j0, int nj) {
     const float* T = A + (size_t)j0 * lda + i0;
     if (MMA) {
-      if (al16) stage_tile_bl(Ts, T, lda, ni, nj);
+      if (AL) stage_tile_bl(Ts, T, lda, ni, nj);
       else stage_tile_4b<true>(Ts, T, lda, ni, nj);
       stage_vec_x8(x, n, j0, nj, xJ);
       stage_vec_x8(x, n, i0, ni, xI);
@@ -568,12 +586,21 @@ symv_staged_kernel(const float* __restrict__ A, int lda, int n, const double* __
     __syncthreads();
     if (MMA) {
       // row sums to y_I, column sums to y_J, straight from the fragments
+      auto pass = [&](auto diag, auto f) {
+        constexpr bool D = decltype(diag)::value, F = decltype(f)::value;
+        if constexpr (AL) {
+          tile_mma_x8<D, F>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, true, 1.0, &fsq);
+        } else {
+          tile_mma_x8<D, F, 8, 2, 1, 8>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, false, 1.0, &fsq);
+          tile_mma_x8<D, false, 8, 2, 2, 8>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, false, true, 1.0, nullptr);
+        }
+      };
       if (fro != nullptr) {
-        if (I == J) tile_mma_x8<true, true>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, true, 1.0, &fsq);
-        else tile_mma_x8<false, true>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, true, 1.0, &fsq);
+        if (I == J) pass(std::true_type{}, std::true_type{});
+        else pass(std::false_type{}, std::true_type{});
       } else {
-        if (I == J) tile_mma_x8<true, false>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, true, 1.0, nullptr);
-        else tile_mma_x8<false, false>(Ts, xJ, xI, y, i0, ni, y, j0, nj, n, true, true, 1.0, nullptr);
+        if (I == J) pass(std::true_type{}, std::false_type{});
+        else pass(std::false_type{}, std::false_type{});
       }
       __syncthreads();   // the stage is free again
       continue;
@@ -1678,6 +1705,7 @@ cudaError_t solve_set_attributes() {
   if ((e = set_dyn(symv_staged_kernel<NRC>, symv_staged_smem<NRC>())) != cudaSuccess) return e;
   SET_NRP(1) SET_NRP(2) SET_NRP(4) SET_NRP(8)
 #undef SET_NRP
+  if ((e = set_dyn(symv_staged_kernel<8, false>, symv_staged_smem<8>())) != cudaSuccess) return e;
   if ((e = set_dyn(block_inverse_batched_kernel, kBlockInvSmem)) != cudaSuccess) return e;
 #define SET_NRB(NRC)                                                                              \
   if ((e = set_dyn(symv_staged_batched_kernel<NRC>, symv_batched_smem<NRC>())) != cudaSuccess) return e; \
@@ -1711,7 +1739,10 @@ cudaError_t launch_symv_skip(const TA* A, int lda, int n, const double* x, doubl
     int grid = std::min(ntiles, (nrhs == 1 ? symv_ctas<1>() : symv_ctas<2>()) * lim->sms);
     if (fro != nullptr) grid = std::min(grid, nfro);   // one Frobenius partial per CTA
     const int al16 = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0;
-    NR_SWITCH(nrhs, (symv_staged_kernel<NRC><<<grid, NTH, symv_staged_smem<NRC>(), stream>>>(A, lda, n, x, y, skip, fro, nfro, al16)));
+    if (nrhs == 8 && !al16)
+      symv_staged_kernel<8, false><<<grid, NTH, symv_staged_smem<8>(), stream>>>(A, lda, n, x, y, skip, fro, nfro, 0);
+    else
+      NR_SWITCH(nrhs, (symv_staged_kernel<NRC><<<grid, NTH, symv_staged_smem<NRC>(), stream>>>(A, lda, n, x, y, skip, fro, nfro, al16)));
   } else {
     NR_SWITCH(nrhs, (symv_kernel<TA, NRC><<<ntiles, NTH, red_bytes(NRC), stream>>>(A, lda, n, x, y, skip)));
   }

@@ -285,3 +285,23 @@ def test_batch_calls_on_different_streams(precision, block):
         assert r.converged
         S = torch.tril(A.double()) + torch.tril(A.double(), -1).T
         assert ((S @ X - B).norm() / B.norm()).item() < 2e-10
+
+
+@pytest.mark.parametrize("n,pad", [(127, 0), (125, 2), (128, 1)])
+def test_eight_column_products_of_unaligned_columns_sum_in_short_chains(n, pad):
+    """A matrix of ones times vectors of one 1 among numbers t = 2^-56.  A partial
+    sum that holds the 1 loses each t (or four of them) added after it, so the
+    result shows how many terms share a chain: at most 16 here, and two
+    roundings to 2^-53 where the parts meet."""
+    from cholesky_gpu_b200 import _lib
+    ld = n + pad
+    A = torch.ones((n, ld), device="cuda")
+    t = 2.0 ** -56
+    X = torch.full((8, n), t, device="cuda", dtype=torch.float64)
+    for k in range(8):
+        X[k, (k * n) // 8] = 1.0
+    Y = torch.empty_like(X)
+    _lib.check(_lib.load().mpchol_symv(A.data_ptr(), ld, n, X.data_ptr(), Y.data_ptr(), 8,
+                                       torch.cuda.current_stream().cuda_stream))
+    lost = (n - 1) * t - (Y - 1.0)          # Y - 1 is exact; below 2^-46
+    assert lost.abs().max().item() <= 16 * t + 2 * 2.0 ** -53
