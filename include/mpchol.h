@@ -139,7 +139,8 @@ typedef struct {
   int converged;           /* 1 if every rhs met rel_tol on the true residual */
   double rel_residual;     /* max over rhs of ||b - A x|| / ||b||, FP64, recomputed from x */
   double backward_error;   /* max over rhs of ||b - A x|| / (||A||_F ||x|| + ||b||) */
-  double precond_residual; /* max over rhs of sqrt(r^T z)/||b|| (the reference's stopping quantity) */
+  double precond_residual; /* max over rhs of sqrt(r^T z)/||b|| (the reference's stopping quantity), z of the
+                              last iteration; 0 if none ran */
 } mpchol_report;
 
 typedef struct mpchol_factor mpchol_factor_t;
